@@ -37,26 +37,26 @@ DRAFT = 4
 def listed():
     return [
         # the smallest call: a four-layer model of width 256, where launches and latencies are all there is
-        dict(name="tiny hybrid, generate", model="hybrid", size="tiny", op="generate", tokens=16, new=8, batch=1, ctx=0, form="int4"),
+        dict(name="tiny hybrid: generate", model="hybrid", size="tiny", op="generate", tokens=16, new=8, batch=1, ctx=0, form="int4"),
         # one user who is answered: 27B, INT4 weights, a short context (the headline benchmark)
-        dict(name="27b, decode", model="hybrid", size="27b", op="decode", tokens=0, new=8, batch=1, ctx=133, form="int4"),
+        dict(name="27b: decode", model="hybrid", size="27b", op="decode", tokens=0, new=8, batch=1, ctx=133, form="int4"),
         # the prompt of the headline benchmark
-        dict(name="27b, prompt of 512", model="hybrid", size="27b", op="prompt", tokens=512, new=0, batch=1, ctx=0, form="int4"),
+        dict(name="27b: prompt of 512", model="hybrid", size="27b", op="prompt", tokens=512, new=0, batch=1, ctx=0, form="int4"),
         # a busy server: 16 sequences of about 4000 tokens, four drafted tokens each, half of them right
-        dict(name="27b, verify 16 drafts", model="hybrid", size="27b", op="verify", tokens=0, new=1, batch=16, ctx=4051, form="int4"),
+        dict(name="27b: verify 16 drafts", model="hybrid", size="27b", op="verify", tokens=0, new=1, batch=16, ctx=4051, form="int4"),
         # the published checkpoint's form: attention and recurrence weights in fp16; a few users, long contexts
-        dict(name="hybrid 5k fp16, decode 5", model="hybrid", size="5k", op="decode", tokens=0, new=8, batch=5, ctx=7001, form="fp16"),
+        dict(name="hybrid 5k fp16: decode 5", model="hybrid", size="5k", op="decode", tokens=0, new=8, batch=5, ctx=7001, form="fp16"),
         # a batch too large for the few-row kernels
-        dict(name="hybrid 2k, decode 24", model="hybrid", size="2k", op="decode", tokens=0, new=4, batch=24, ctx=700, form="int4"),
+        dict(name="hybrid 2k: decode 24", model="hybrid", size="2k", op="decode", tokens=0, new=4, batch=24, ctx=700, form="int4"),
         # a chat turn
-        dict(name="hybrid 4k, prompt of 77", model="hybrid", size="4k", op="prompt", tokens=77, new=0, batch=1, ctx=0, form="int4"),
+        dict(name="hybrid 4k: prompt of 77", model="hybrid", size="4k", op="prompt", tokens=77, new=0, batch=1, ctx=0, form="int4"),
         # a document
-        dict(name="hybrid 4k, prompt of 3001", model="hybrid", size="4k", op="prompt", tokens=3001, new=0, batch=1, ctx=0, form="int4"),
+        dict(name="hybrid 4k: prompt of 3001", model="hybrid", size="4k", op="prompt", tokens=3001, new=0, batch=1, ctx=0, form="int4"),
         # the dense-weight decoders: a user who is answered, a prompt, everything in 32 bits, a small batch
-        dict(name="degedra 4k, decode", model="degedra", size="4k", op="decode", tokens=0, new=8, batch=1, ctx=1500, form="bf16"),
-        dict(name="degedra 5k, prompt of 1000", model="degedra", size="5k", op="prompt", tokens=1000, new=0, batch=1, ctx=0, form="bf16"),
-        dict(name="degedra 2k fp32, prompt of 200", model="degedra", size="2k", op="prompt", tokens=200, new=0, batch=1, ctx=0, form="fp32"),
-        dict(name="vekerax 4k, generate", model="vekerax", size="4k", op="generate", tokens=300, new=16, batch=1, ctx=0, form="bf16"),
+        dict(name="degedra 4k: decode", model="degedra", size="4k", op="decode", tokens=0, new=8, batch=1, ctx=1500, form="bf16"),
+        dict(name="degedra 5k: prompt of 1000", model="degedra", size="5k", op="prompt", tokens=1000, new=0, batch=1, ctx=0, form="bf16"),
+        dict(name="degedra 2k fp32: prompt of 200", model="degedra", size="2k", op="prompt", tokens=200, new=0, batch=1, ctx=0, form="fp32"),
+        dict(name="vekerax 4k: generate", model="vekerax", size="4k", op="generate", tokens=300, new=16, batch=1, ctx=0, form="bf16"),
     ]
 
 
