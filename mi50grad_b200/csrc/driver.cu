@@ -779,6 +779,10 @@ static int mixer_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, in
         p.w = (const float*)L.w; p.x = (const float*)x; p.out = out; p.ldw = L.ldw; p.ldx = ldx; p.K = L.K; p.N = L.N; p.T = T;
         p.ldo = ldo; p.mode = mode; p.softcap = softcap;
         if (mode == DG_STORE) p.act_cols = act; else p.act = act;
+        if (max_ks > 1) {
+            p.max_splits = max_ks; p.plane_stride = (long long)d->m.max_prefill * ldo;
+            *planes = b2_gemm_f32_splits(L.N, L.K, T, max_ks);
+        }
         return b2_gemm_f32(&p, s);
     }
     GemmTcParams p;

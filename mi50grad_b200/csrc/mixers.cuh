@@ -140,6 +140,8 @@ struct GemmF32Params {
     const float* w; const float* x; void* out;
     int ldw, ldx, K, N, T, ldo, mode, act;
     float softcap; int act_cols;
+    long long plane_stride;  // DG_STORE_F32: floats between the planes of a product split over K (0: no split)
+    int max_splits, pad;
 };
 
 // ---- one mixer: windowed attention and / or a linear recurrence (csrc/attention_window.cu, csrc/ssd.cu).
@@ -200,6 +202,7 @@ struct MixRun {
 
 B2_API int b2_gemv_dense(const DenseGemvParams* p, cudaStream_t s);
 B2_API int b2_gemm_f32(const GemmF32Params* p, cudaStream_t s);
+B2_API int b2_gemm_f32_splits(int N, int K, int T, int max_splits);      // planes a launch leaves
 B2_API int b2_embed_rows(const void* embed, const int* row_tokens, const void* rows, const void* seqs, float* h, void* xb,
                          int ldx, int n_rows, int H, int vocab, int dt, cudaStream_t s);
 B2_API int b2_post_norm(float* h, const float* m, const float* w, const float* final_w, void* xb, int ldx, int n_rows, int H,

@@ -108,6 +108,23 @@ def test_gate_up_pair(dt, F, K, rows):
     _close(out[:, :F], ref, tol)
 
 
+@pytest.mark.parametrize("N,K,T_,pad", [(1, 1, 1, 0), (130, 15, 17, 3), (128, 16, 33, 4), (257, 50, 41, 4), (2048, 1000, 200, 0), (96, 6144, 49, 8),
+                                        (4500, 66, 57, 2), (12288, 36, 65, 4), (16, 2049, 300, 1)])
+def test_gemm_f32_tiles_and_splits(N, K, T_, pad):
+    """Every tile height, ragged edges, rows that allow 16-byte copies and rows that do not, splits over K.  Two fp32
+    chains of at most K terms: the error stays below sqrt(K) roundings of terms of size K ** -0.5."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    w, x = _rnd(N, K + pad, std=K ** -0.5).cuda()[:, :K], _rnd(T_, K + pad, seed=1).cuda()[:, :K]
+    ref = x.double() @ w.double().T
+    out = torch.full((T_, N + 1), 7.0, device="cuda")
+    K_.gemm_f32(w, x, out[:, :N], L.DG_STORE_F32)
+    _close(out[:, :N], ref, 1e-5)
+    assert bool((out[:, N] == 7.0).all())
+    planes = K_.gemm_f32(w, x, torch.full((4, T_, N), float("nan"), device="cuda"), L.DG_STORE_F32)
+    _close(planes.sum(0), ref, 1e-5)
+
+
 @pytest.mark.parametrize("N,K,T_", [(37, 90, 9), (300, 200, 64), (640, 1032, 130), (129, 4096, 511)])
 def test_many_row_gemms(N, K, T_):
     from mi50grad_b200.ops import kernels as K_
