@@ -23,9 +23,7 @@
 //    state of every linear-attention layer in one launch.
 //  * kv_compact: moves the accepted nodes' K/V from slot len+node to slot len+depth in every
 //    full-attention layer (a no-op for chains).
-#include <cooperative_groups.h>
 #include "kernels.cuh"
-namespace cg = cooperative_groups;
 
 #define DN_THREADS 256
 #define DN_COLS 32
@@ -33,240 +31,273 @@ namespace cg = cooperative_groups;
 
 __device__ __forceinline__ int top_bit(unsigned m) { return m ? 31 - __clz(m) : -1; }
 
+#define VF_THREADS 256
+#define VF_CHUNK 4               // nodes whose products with the state are reduced together
+
+// One CTA per value head and sequence.  Bound: the states (64 KB a head; 50 MB for 16 sequences of 48 heads), and behind
+// them the latencies between the steps, so nothing is done node by node that does not have to be: the convolution, the
+// norms, the dot products of all pairs (node, ancestor) and S0^T k, S0^T q of all nodes are formed side by side, and
+// only the recursion of the update vectors over a path is serial, per column, without a barrier.  The state stays in
+// registers (4 columns x DK / groups rows a thread, read once, 16 bytes at a time) and is requested before anything else.
+// Measured for 16 sequences of 5 nodes and 48 heads of 128 x 128: 55 us a layer; a cluster of four CTAs per head
+// that walked the nodes with five barriers each took 127.
 template <int DK, int DV>
-__global__ void __launch_bounds__(DN_THREADS) deltanet_verify_kernel(const DeltaParams p, const SpecStage st,
-                                                                      int layer) {
-    constexpr int CB = DV / DN_COLS;
-    constexpr int RPT = DK / 8;
-    constexpr int NCH = 2 * DK + DN_COLS;
-    cg::cluster_group cluster = cg::this_cluster();
+struct VerifySmem {
+    static constexpr int NCH = 2 * DK + DV, LPR = DV / 4, RG = VF_THREADS / LPR;
+    float cq[NM][DK], ck[NM][DK], cv[NM][DV];             // convolved inputs (unscaled)
+    float mm[NM][DV], sq[NM][DV];                         // S0^T k, S0^T q; later the update vectors and the outputs
+    float dk[NM][NM], dq[NM][NM];                         // k_t . k_a, q_t . k_a (t == a: k.k, q.k), then their coefficients
+    float qq[NM], invq[NM], invk[NM], gl[NM], G[NM], beta[NM], ab[NM][2];
+    float ss[NM][DV / 32];
+    float abp[VF_THREADS / 32][VF_CHUNK][2];
+    unsigned anc[NM];
+    __half xraw[NM][NCH];
+    float4 red[2][VF_CHUNK][RG][LPR];
+};
+
+template <int DK, int DV>
+__global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const DeltaParams p, const SpecStage st, int layer) {
+    typedef VerifySmem<DK, DV> Smem;
+    constexpr int NCH = Smem::NCH, LPR = Smem::LPR, RG = Smem::RG, RPT = DK / RG, WARPS = VF_THREADS / 32;
+    constexpr int CB = DV / DN_COLS, HCH = 2 * DK + DN_COLS;          // the history is kept per 32 columns of a head
+    extern __shared__ float4 vf_smem[];
+    Smem& sm = *(Smem*)vf_smem;
     pdl_launch_dependents();
-    const int cb = blockIdx.x, j = blockIdx.y, si = blockIdx.z;
-    const int tid = threadIdx.x, lane = tid & 31, kr = tid >> 5, vcol = lane;
+    const int j = blockIdx.x, si = blockIdx.y;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rep = p.nv / p.nk, kh = j / rep;
     const int r0 = p.seq_rows[si], r1 = p.seq_rows[si + 1];
-    if (r0 >= r1) return;                        // uniform over the whole cluster
+    if (r0 >= r1) return;
     const int N = min(r1 - r0, NM);
     const int seq = p.rows[r0].seq;
+    const int rg = tid / LPR, c4 = tid % LPR;                          // rows rg * RPT .., columns 4 c4 ..
 
-    __shared__ float hist[NCH][3];
-    __shared__ float cw[NCH][4];
-    __shared__ __half xraw[NM][NCH];
-    __shared__ float khat[NM][DK];
-    __shared__ float uu[NM][DN_COLS], yy[NM][DN_COLS];
-    __shared__ float Gs[NM], dkk[NM], dkq[NM];
-    __shared__ float cq[DK], ck[DK], cv[DN_COLS];
-    __shared__ float red_m[8][DN_COLS], red_q[8][DN_COLS];
-    __shared__ float red32[8];
-    __shared__ float cl_ss[NM];
+    float4 S[RPT];
+    const float4* sp = (const float4*)(p.state + (((size_t)seq * p.nv + j) * DK + rg * RPT) * DV) + c4;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) S[i] = sp[i * (DV / 4)];
 
     auto chan = [&](int c) -> int {
         if (c < DK) return kh * DK + c;
         if (c < 2 * DK) return p.nk * DK + kh * DK + (c - DK);
-        return 2 * p.nk * DK + j * DV + cb * DN_COLS + (c - 2 * DK);
+        return 2 * p.nk * DK + j * DV + (c - 2 * DK);
     };
     auto proj_col = [&](int c) -> int {
         if (c < DK) return p.off_q + kh * DK + c;
         if (c < 2 * DK) return p.off_k + kh * DK + (c - DK);
-        return p.off_v + j * DV + cb * DN_COLS + (c - 2 * DK);
+        return p.off_v + j * DV + (c - 2 * DK);
     };
-    const __half* my_hist = p.conv_state + ((((size_t)seq * p.nv + j) * CB + cb) * NCH) * 3;
-    for (int c = tid; c < NCH; c += DN_THREADS) {
-#pragma unroll
-        for (int t = 0; t < 3; ++t) hist[c][t] = __half2float(my_hist[c * 3 + t]);
-        const __half* w = p.conv_w + (size_t)chan(c) * 4;
-#pragma unroll
-        for (int t = 0; t < 4; ++t) cw[c][t] = __half2float(w[t]);
+    for (int i = tid; i < N * NCH; i += VF_THREADS) {
+        const int t = i / NCH, c = i - t * NCH;
+        sm.xraw[t][c] = p.proj[(size_t)(r0 + t) * p.ld + proj_col(c)];
     }
-    float S[RPT];
-    const float* sp = p.state + (((size_t)seq * p.nv + j) * DK) * DV + cb * DN_COLS + vcol;
-#pragma unroll
-    for (int i = 0; i < RPT; ++i) S[i] = sp[(size_t)(kr + 8 * i) * DV];
-    const float neg_expA = -__expf(p.A_log[j]);
-    const float dtb = __half2float(p.dt_bias[j]);
-    const float nw = __half2float(p.norm_w[cb * DN_COLS + vcol]);
+    // ancestors of a node inside this sequence's block (bit a <-> node a)
+    if (tid < N) sm.anc[tid] = (unsigned)(p.rows[r0 + tid].mask & 0xFFFFull) & ((1u << tid) - 1u);
+    // ---- a / b inputs of the gates
     const bool inkernel_ab = p.off_a < 0;
-    __syncthreads();
-
-    for (int t = 0; t < N; ++t) {
-        const int r = r0 + t;
-        const __half* pr = p.proj + (size_t)r * p.ld;
-        // ancestors of node t inside this sequence's block (bit a <-> node a), nearest first
-        const unsigned anc = (unsigned)(p.rows[r].mask & 0xFFFFull) & ((1u << t) - 1u);
-        const int d = __popc(anc);
-        const int p1 = top_bit(anc);
-        const unsigned a2 = p1 >= 0 ? anc & ~(1u << p1) : 0u;
-        const int p2 = top_bit(a2);
-        const int p3 = top_bit(p2 >= 0 ? a2 & ~(1u << p2) : 0u);
-        // ---- phase A: a/b partial sums, conv + SiLU along the node's path
-        float sa = 0.f, sb = 0.f;
-        if (inkernel_ab) {
-            const __half* wa = p.wa + (size_t)j * p.H;
-            const __half* wb = p.wb + (size_t)j * p.H;
-            if (p.ln.h) {
-                const float* hr = p.ln.h + (size_t)r * p.ln.H;
-                for (int i = tid * 2; i < p.H; i += DN_THREADS * 2) {
-                    float2 hv = *(const float2*)(hr + i);
-                    float2 ww = __half22float2(*(const __half2*)(p.ln.w + i));
-                    float2 av = __half22float2(*(const __half2*)(wa + i));
-                    float2 bv = __half22float2(*(const __half2*)(wb + i));
-                    float x0 = hv.x * ww.x, x1 = hv.y * ww.y;
-                    sa += x0 * av.x + x1 * av.y;
-                    sb += x0 * bv.x + x1 * bv.y;
-                }
-            } else {
-                const __half* x = p.xn + (size_t)r * p.ldx;
-                for (int i = tid * 2; i < p.H; i += DN_THREADS * 2) {
-                    float2 xv = __half22float2(*(const __half2*)(x + i));
-                    float2 av = __half22float2(*(const __half2*)(wa + i));
-                    float2 bv = __half22float2(*(const __half2*)(wb + i));
-                    sa += xv.x * av.x + xv.y * av.y;
-                    sb += xv.x * bv.x + xv.y * bv.y;
+    if (inkernel_ab) {
+        const __half* wa = p.wa + (size_t)j * p.H;
+        const __half* wb = p.wb + (size_t)j * p.H;
+        for (int t0 = 0; t0 < N; t0 += VF_CHUNK) {
+            float sa[VF_CHUNK], sb[VF_CHUNK];
+#pragma unroll
+            for (int u = 0; u < VF_CHUNK; ++u) sa[u] = sb[u] = 0.f;
+            for (int i = tid * 2; i < p.H; i += VF_THREADS * 2) {
+                const float2 av = __half22float2(*(const __half2*)(wa + i)), bv = __half22float2(*(const __half2*)(wb + i));
+                float2 ww = make_float2(1.f, 1.f);
+                if (p.ln.h) ww = __half22float2(*(const __half2*)(p.ln.w + i));
+#pragma unroll
+                for (int u = 0; u < VF_CHUNK; ++u) {
+                    const int r = r0 + min(t0 + u, N - 1);
+                    float2 x = p.ln.h ? *(const float2*)(p.ln.h + (size_t)r * p.ln.H + i) : __half22float2(*(const __half2*)(p.xn + (size_t)r * p.ldx + i));
+                    x.x *= ww.x; x.y *= ww.y;
+                    sa[u] += x.x * av.x + x.y * av.y;
+                    sb[u] += x.x * bv.x + x.y * bv.y;
                 }
             }
-            sa = warp_sum(sa);
-            sb = warp_sum(sb);
-            if (lane == 0) { red_m[kr][0] = sa; red_m[kr][1] = sb; }
-        }
-        for (int c = tid; c < NCH; c += DN_THREADS) {
-            const __half xh = pr[proj_col(c)];
-            xraw[t][c] = xh;
-            const float x = __half2float(xh);
-            // taps at distance 1..3 along the path; beyond the root they come from the history
-            const float x1 = d >= 1 ? __half2float(xraw[p1][c]) : hist[c][2];
-            const float x2 = d >= 2 ? __half2float(xraw[p2][c]) : hist[c][1 + d];
-            const float x3 = d >= 3 ? __half2float(xraw[p3][c]) : hist[c][d];
-            float o = x3 * cw[c][0] + x2 * cw[c][1] + x1 * cw[c][2] + x * cw[c][3];
-            o = silu_f(o);
-            if (c < DK) cq[c] = o; else if (c < 2 * DK) ck[c - DK] = o; else cv[c - 2 * DK] = o;
-        }
-        __syncthreads();
-        // ---- phase B: norms, q.k, and the dot products with every ancestor's key
-        for (int idx = kr; idx < 3 + 2 * d; idx += 8) {
-            float s = 0.f;
-            if (idx < 3) {
-                for (int i = lane; i < DK; i += 32) {
-                    float a = (idx == 1) ? ck[i] : cq[i], b = (idx == 0) ? cq[i] : ck[i];
-                    s += a * b;                  // 0: q.q  1: k.k  2: q.k
-                }
-                s = warp_sum(s);
-                if (lane == 0) red32[idx] = s;
-            } else {
-                int ord = (idx - 3) >> 1;
-                unsigned m = anc;
-                for (int q = 0; q < ord; ++q) m &= m - 1;          // drop the `ord` lowest ancestors
-                const int a = __ffs(m) - 1;
-                const float* other = ((idx - 3) & 1) ? cq : ck;
-                for (int i = lane; i < DK; i += 32) s += khat[a][i] * other[i];
-                s = warp_sum(s);
-                if (lane == 0) { if ((idx - 3) & 1) dkq[a] = s; else dkk[a] = s; }
+#pragma unroll
+            for (int u = 0; u < VF_CHUNK; ++u) {
+                sa[u] = warp_sum(sa[u]);
+                sb[u] = warp_sum(sb[u]);
+                if (lane == 0) { sm.abp[warp][u][0] = sa[u]; sm.abp[warp][u][1] = sb[u]; }
             }
-        }
-        if (kr == 7) {
-            float a_in, b_in;
-            if (inkernel_ab) {
-                float inv = p.ln.h ? lazy_inv_rms(p.ln, r, lane) : 1.f;
+            __syncthreads();
+            if (warp < VF_CHUNK && t0 + warp < N) {
+                const int t = t0 + warp;
+                const float inv = p.ln.h ? lazy_inv_rms(p.ln, r0 + t, lane) : 1.f;
                 float ta = 0.f, tb = 0.f;
 #pragma unroll
-                for (int w = 0; w < 8; ++w) { ta += red_m[w][0]; tb += red_m[w][1]; }
-                a_in = __half2float(__float2half(ta * inv));
-                b_in = __half2float(__float2half(tb * inv));
-            } else {
-                a_in = __half2float(pr[p.off_a + j]);
-                b_in = __half2float(pr[p.off_b + j]);
+                for (int w = 0; w < WARPS; ++w) { ta += sm.abp[w][warp][0]; tb += sm.abp[w][warp][1]; }
+                if (lane == 0) { sm.ab[t][0] = __half2float(__float2half(ta * inv)); sm.ab[t][1] = __half2float(__float2half(tb * inv)); }
             }
-            if (lane == 0) { red32[3] = a_in; red32[4] = b_in; }
+            __syncthreads();
+        }
+    } else if (tid < N) {
+        const __half* pr = p.proj + (size_t)(r0 + tid) * p.ld;
+        sm.ab[tid][0] = __half2float(pr[p.off_a + j]);
+        sm.ab[tid][1] = __half2float(pr[p.off_b + j]);
+    }
+    __syncthreads();
+    // ---- convolution + SiLU along every node's path: a thread keeps its channel's taps and history
+    for (int c = tid; c < NCH; c += VF_THREADS) {
+        const int blk = c < 2 * DK ? 0 : (c - 2 * DK) / DN_COLS, hc = c < 2 * DK ? c : 2 * DK + (c - 2 * DK) % DN_COLS;
+        const __half* hp = p.conv_state + ((((size_t)seq * p.nv + j) * CB + blk) * HCH + hc) * 3;
+        const __half* w = p.conv_w + (size_t)chan(c) * 4;
+        float hist[3], cw[4];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) hist[q] = __half2float(hp[q]);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cw[q] = __half2float(w[q]);
+        for (int t = 0; t < N; ++t) {
+            // taps at distance 1..3 along the path; beyond the root they come from the history
+            const unsigned a1 = sm.anc[t];
+            const int d = __popc(a1), p1 = top_bit(a1);
+            const unsigned a2 = p1 >= 0 ? a1 & ~(1u << p1) : 0u;
+            const int p2 = top_bit(a2), p3 = top_bit(p2 >= 0 ? a2 & ~(1u << p2) : 0u);
+            const float x1 = d >= 1 ? __half2float(sm.xraw[p1][c]) : hist[2];
+            const float x2 = d >= 2 ? __half2float(sm.xraw[p2][c]) : (d == 1 ? hist[2] : hist[1]);
+            const float x3 = d >= 3 ? __half2float(sm.xraw[p3][c]) : (d == 2 ? hist[2] : (d == 1 ? hist[1] : hist[0]));
+            const float o = silu_f(x3 * cw[0] + x2 * cw[1] + x1 * cw[2] + __half2float(sm.xraw[t][c]) * cw[3]);
+            if (c < DK) sm.cq[t][c] = o; else if (c < 2 * DK) sm.ck[t][c - DK] = o; else sm.cv[t][c - 2 * DK] = o;
+        }
+    }
+    __syncthreads();
+    // ---- dot products of every node with itself and with its ancestors, a warp each
+    {
+        int n = 0;
+        for (int t = 0; t < N; ++t)
+            for (unsigned m = sm.anc[t] | (1u << t); m; m &= m - 1, ++n) {
+                if (n % WARPS != warp) continue;
+                const int a = __ffs(m) - 1;
+                float kk = 0.f, qk = 0.f, qq = 0.f;
+                for (int i = lane; i < DK; i += 32) {
+                    const float ka = sm.ck[a][i], q = sm.cq[t][i];
+                    kk = fmaf(sm.ck[t][i], ka, kk);
+                    qk = fmaf(q, ka, qk);
+                    qq = fmaf(q, q, qq);
+                }
+                kk = warp_sum(kk);
+                qk = warp_sum(qk);
+                if (a == t) qq = warp_sum(qq);
+                if (lane == 0) { sm.dk[t][a] = kk; sm.dq[t][a] = qk; if (a == t) sm.qq[t] = qq; }
+            }
+    }
+    __syncthreads();
+    if (tid < N) {
+        sm.invq[tid] = rsqrtf(sm.qq[tid] + 1e-6f) * rsqrtf((float)DK);
+        sm.invk[tid] = rsqrtf(sm.dk[tid][tid] + 1e-6f);
+        const float x = sm.ab[tid][0] + __half2float(p.dt_bias[j]);
+        sm.gl[tid] = fmaxf(-__expf(p.A_log[j]) * (x > 20.f ? x : log1pf(__expf(x))), -20.f);
+        sm.beta[tid] = sigmoid_f(sm.ab[tid][1]);
+    }
+    __syncthreads();
+    if (tid < N) {
+        float g = 0.f;                                    // summed log-decay along the path
+        for (unsigned m = sm.anc[tid] | (1u << tid); m; m &= m - 1) g += sm.gl[__ffs(m) - 1];
+        sm.G[tid] = g;
+    }
+    // ---- S0^T k and S0^T q of all nodes
+    for (int t0 = 0; t0 < N; t0 += VF_CHUNK) {
+#pragma unroll 1
+        for (int u = 0; u < VF_CHUNK && t0 + u < N; ++u) {
+            const float* kp = sm.ck[t0 + u] + rg * RPT;
+            const float* qp = sm.cq[t0 + u] + rg * RPT;
+            float4 m = make_float4(0.f, 0.f, 0.f, 0.f), q = m;
+#pragma unroll
+            for (int i = 0; i < RPT; i += 4) {
+                const float4 k4 = *(const float4*)(kp + i), q4 = *(const float4*)(qp + i);
+                const float kv[4] = {k4.x, k4.y, k4.z, k4.w}, qv[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    m.x = fmaf(S[i + e].x, kv[e], m.x); m.y = fmaf(S[i + e].y, kv[e], m.y); m.z = fmaf(S[i + e].z, kv[e], m.z); m.w = fmaf(S[i + e].w, kv[e], m.w);
+                    q.x = fmaf(S[i + e].x, qv[e], q.x); q.y = fmaf(S[i + e].y, qv[e], q.y); q.z = fmaf(S[i + e].z, qv[e], q.z); q.w = fmaf(S[i + e].w, qv[e], q.w);
+                }
+            }
+            sm.red[0][u][rg][c4] = m;
+            sm.red[1][u][rg][c4] = q;
         }
         __syncthreads();
-        const float invq = rsqrtf(red32[0] + 1e-6f) * rsqrtf((float)DK);
-        const float invk = rsqrtf(red32[1] + 1e-6f);
-        const float kq = red32[2] * invq * invk;
-        const float a_in = red32[3], b_in = red32[4];
-        float gl = neg_expA * (a_in + dtb > 20.f ? a_in + dtb : log1pf(__expf(a_in + dtb)));
-        gl = fmaxf(gl, -20.f);
-        const float decay = __expf(gl);
-        const float beta = sigmoid_f(b_in);
-        const float Gp = p1 >= 0 ? Gs[p1] : 0.f;
-        const float Gt = Gp + gl;
-        // ---- phase C: S0^T k and S0^T q for this CTA's columns
-        float mp = 0.f, qp = 0.f;
+        const int cnt = min(VF_CHUNK, N - t0);
+        for (int i = tid; i < 2 * cnt * DV; i += VF_THREADS) {
+            const int which = i / (cnt * DV), u = (i / DV) % cnt, c = i % DV;
+            const float* rp = (const float*)&sm.red[which][u][0][0] + c;
+            float s = 0.f;
 #pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-            mp = fmaf(S[i], ck[kr + 8 * i], mp);
-            qp = fmaf(S[i], cq[kr + 8 * i], qp);
+            for (int g = 0; g < RG; ++g) s += rp[g * DV];
+            if (which) sm.sq[t0 + u][c] = s * sm.invq[t0 + u]; else sm.mm[t0 + u][c] = s * sm.invk[t0 + u];
         }
-        red_m[kr][vcol] = mp * invk;
-        red_q[kr][vcol] = qp * invq;
-        for (int i = tid; i < DK; i += DN_THREADS) khat[t][i] = ck[i] * invk;
-        __syncthreads();
-        float mm = 0.f, sq = 0.f;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) { mm += red_m[w][vcol]; sq += red_q[w][vcol]; }
-        float Sk = __expf(Gp) * mm;              // S_parent^T k_t
-        float ys = __expf(Gt) * sq;              // decayed S0 part of S_t^T q_t
-        for (unsigned m = anc; m; m &= m - 1) {
-            const int a = __ffs(m) - 1;
-            const float ua = uu[a][vcol], Ga = Gs[a];
-            Sk = fmaf(__expf(Gp - Ga) * ua, dkk[a] * invk, Sk);
-            ys = fmaf(__expf(Gt - Ga) * ua, dkq[a] * invq, ys);
-        }
-        const float delta = (cv[vcol] - decay * Sk) * beta;
-        const float y = ys + delta * kq;
-        const float ss = warp_sum(y * y);
-        __syncthreads();                          // all reads of Gs/uu/red_* of this node are done
-        if (kr == 0) { uu[t][vcol] = delta; yy[t][vcol] = y; }
-        if (tid == 0) { cl_ss[t] = ss; Gs[t] = Gt; }
         __syncthreads();
     }
-    cluster.sync();
-    // ---- gated RMSNorm over the head's dv outputs, one warp per node
-    for (int t = kr; t < N; t += 8) {
-        float tot = 0.f;
-#pragma unroll
-        for (int c = 0; c < CB; ++c) tot += *cluster.map_shared_rank(&cl_ss[t], c);
-        const __half* pr = p.proj + (size_t)(r0 + t) * p.ld;
-        const float z = __half2float(pr[p.off_z + j * DV + cb * DN_COLS + vcol]);
-        const float o = yy[t][vcol] * rsqrtf(tot / (float)DV + p.eps) * nw * silu_f(z);
-        p.out[(size_t)(r0 + t) * p.ldo + j * DV + cb * DN_COLS + vcol] = __float2half(o);
+    // ---- coefficients of an ancestor's update vector in S_parent^T k_t and in S_t^T q_t
+    for (int i = tid; i < N * NM; i += VF_THREADS) {
+        const int t = i / NM, a = i % NM;
+        const unsigned m = sm.anc[t];
+        if (a == t) sm.dq[t][t] *= sm.invq[t] * sm.invk[t];
+        else if (m >> a & 1) {
+            const float Gp = sm.G[top_bit(m)], Ga = sm.G[a];
+            sm.dk[t][a] *= sm.invk[a] * sm.invk[t] * __expf(Gp - Ga);
+            sm.dq[t][a] *= sm.invk[a] * sm.invq[t] * __expf(sm.G[t] - Ga);
+        }
     }
-    // ---- staging for the commit
+    __syncthreads();
+    // ---- the recursion, one thread per column
+    if (tid < DV) {
+        for (int t = 0; t < N; ++t) {
+            const unsigned m0 = sm.anc[t];
+            const float Gp = m0 ? sm.G[top_bit(m0)] : 0.f;
+            float Sk = __expf(Gp) * sm.mm[t][tid], ys = __expf(sm.G[t]) * sm.sq[t][tid];
+            for (unsigned m = m0; m; m &= m - 1) {
+                const int a = __ffs(m) - 1;
+                const float u = sm.mm[a][tid];
+                Sk = fmaf(sm.dk[t][a], u, Sk);
+                ys = fmaf(sm.dq[t][a], u, ys);
+            }
+            const float delta = (sm.cv[t][tid] - __expf(sm.gl[t]) * Sk) * sm.beta[t];
+            const float y = fmaf(delta, sm.dq[t][t], ys);
+            sm.mm[t][tid] = delta;
+            sm.sq[t][tid] = y;
+            const float s = warp_sum(y * y);
+            if (lane == 0) sm.ss[t][warp] = s;
+        }
+    }
+    __syncthreads();
+    // ---- gated RMSNorm over the head's dv outputs; staging for the commit
     unsigned char* blk = st.base + (size_t)layer * st.layer_stride + (size_t)si * st.seq_stride;
     float* su = (float*)(blk + st.off_u);
-    for (int t = kr; t < N; t += 8) su[((size_t)t * p.nv + j) * DV + cb * DN_COLS + vcol] = uu[t][vcol];
+    for (int i = tid; i < N * DV; i += VF_THREADS) {
+        const int t = i / DV, c = i - t * DV;
+        float tot = 0.f;
+#pragma unroll
+        for (int q = 0; q < DV / 32; ++q) tot += sm.ss[t][q];
+        const float z = __half2float(p.proj[(size_t)(r0 + t) * p.ld + p.off_z + j * DV + c]);
+        const float o = sm.sq[t][c] * rsqrtf(tot / (float)DV + p.eps) * __half2float(p.norm_w[c]) * silu_f(z);
+        p.out[(size_t)(r0 + t) * p.ldo + j * DV + c] = __float2half(o);
+        su[((size_t)t * p.nv + j) * DV + c] = sm.mm[t][c];
+    }
     const int conv_dim = 2 * p.nk * DK + p.nv * DV;
     __half* sx = (__half*)(blk + st.off_x);
-    const bool key_owner = (cb == 0) && (j % rep == 0);
-    for (int i = tid; i < N * NCH; i += DN_THREADS) {
+    const bool key_owner = j % rep == 0;
+    for (int i = tid; i < N * NCH; i += VF_THREADS) {
         const int t = i / NCH, c = i - t * NCH;
-        if (c >= 2 * DK || key_owner) sx[(size_t)t * conv_dim + chan(c)] = xraw[t][c];
+        if (c >= 2 * DK || key_owner) sx[(size_t)t * conv_dim + chan(c)] = sm.xraw[t][c];
     }
-    if (cb == 0 && tid < N) ((float*)(blk + st.off_g))[tid * p.nv + j] = Gs[tid];
+    if (tid < N) ((float*)(blk + st.off_g))[tid * p.nv + j] = sm.G[tid];
     if (key_owner) {
         float* sk = (float*)(blk + st.off_k);
-        for (int i = tid; i < N * DK; i += DN_THREADS) {
+        for (int i = tid; i < N * DK; i += VF_THREADS) {
             const int t = i / DK, e = i - t * DK;
-            sk[((size_t)t * p.nk + kh) * DK + e] = khat[t][e];
+            sk[((size_t)t * p.nk + kh) * DK + e] = sm.ck[t][e] * sm.invk[t];
         }
     }
-    cluster.sync();                              // no CTA leaves while a peer may still read its shared memory
 }
 
 template <int DK, int DV>
 static int launch_verify(const DeltaParams* p, const SpecStage* st, int layer, cudaStream_t s) {
-    constexpr int CB = DV / DN_COLS;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(CB, p->nv, p->n_seqs);
-    cfg.blockDim = dim3(DN_THREADS);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = CB;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, deltanet_verify_kernel<DK, DV>, *p, *st, layer);
+    constexpr size_t smem = sizeof(VerifySmem<DK, DV>);
+    static SmemOptIn optin;
+    if (cudaError_t e = optin.ensure(deltanet_verify_kernel<DK, DV>, smem)) return e;
+    deltanet_verify_kernel<DK, DV><<<dim3(p->nv, p->n_seqs), VF_THREADS, smem, s>>>(*p, *st, layer);
+    return cudaGetLastError();
 }
 
 B2_API int b2_deltanet_verify(const DeltaParams* p, const SpecStage* st, int layer, int dk, int dv, cudaStream_t s) {

@@ -140,3 +140,81 @@ def test_tp_engine_tree_hooks_match_oracle():
     eng.set_eagle_mode(True, k_draft=3)
     d = eng.generate_eagle_drafts(hs[0], 3)
     assert len(d) == 3 and d[0] == int(torch.argmax(orc.compute_logits(ref[0])))
+
+
+def _tree(n, kind):
+    if kind == "chain":
+        return [i - 1 for i in range(n)]
+    g = torch.Generator().manual_seed(n)
+    return [-1] + [int(torch.randint(-1 if kind == "forest" else 0, i, (1,), generator=g)) for i in range(1, n)]
+
+
+@pytest.mark.parametrize("dk,nk,nv,sizes,kind,ab", [(128, 2, 6, [5, 1, 16], "chain", "proj"), (128, 1, 2, [16, 4, 7], "tree", "lazy"),
+                                                    (64, 2, 4, [3, 16, 9], "forest", "proj"), (64, 1, 1, [8], "tree", "xn")])
+def test_verify_outputs_equal_steps_along_every_path(dk, nk, nv, sizes, kind, ab):
+    """The output of every node of a draft tree is that of feeding its path to the step kernel, token by token; both
+    are fp32 sums rounded to fp16 once, so they differ by an ulp or so."""
+    import ctypes as C
+    from mi50grad_b200.ops import kernels as K
+    from mi50grad_b200.ops import lib as L
+    g = torch.Generator().manual_seed(3)
+    rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+    dv, H, R, ns = dk, 512, sum(sizes), len(sizes)
+    kd = nk * dk
+    conv_dim = 2 * kd + nv * dv
+    ld = conv_dim + nv * dv + 2 * nv
+    proj = rnd(R, ld).half().cuda()
+    conv_w, A_log = (rnd(conv_dim, 4) * 0.3).half().cuda(), (torch.rand(nv, generator=g) * 1.5 - 1.0).cuda()
+    dt_bias, norm_w = (rnd(nv) * 0.5).half().cuda(), (torch.rand(dv, generator=g) + 0.5).half().cuda()
+    state, hist0 = (rnd(ns, nv, dk, dv) * 0.1).cuda(), rnd(ns, conv_dim, 3).half()
+    conv = torch.zeros(ns, nv, dv // 32, 2 * dk + 32, 3, dtype=torch.float16)
+    for j in range(nv):
+        kh = j // (nv // nk)
+        for cb in range(dv // 32):
+            ch = [kh * dk + i for i in range(dk)] + [kd + kh * dk + i for i in range(dk)] + [2 * kd + j * dv + cb * 32 + i for i in range(32)]
+            conv[:, j, cb] = hist0[:, ch]
+    conv = conv.cuda()
+    wa, wb, xn = (rnd(nv, H) * 0.05).half().cuda(), (rnd(nv, H) * 0.05).half().cuda(), rnd(R, H).half().cuda()
+    hres, wnorm = (rnd(R, H) * 3).cuda(), (torch.rand(H, generator=g) + 0.5).half().cuda()
+    offs = (0, kd, 2 * kd, conv_dim) + ((conv_dim + nv * dv, conv_dim + nv * dv + nv) if ab == "proj" else (-1, -1))
+    lazy = lambda rows: K.lazy_norm(hres[rows], torch.cat([hres[rows].pow(2).sum(-1, keepdim=True), torch.zeros(len(rows), 3, device="cuda")], 1), wnorm)  # noqa: E731
+    starts = [sum(sizes[:i]) for i in range(ns + 1)]
+    parents = [_tree(n, kind) for n in sizes]
+    paths, entries = [], []
+    for s, par in enumerate(parents):
+        up = []
+        for t, q in enumerate(par):
+            up.append((up[q] if q >= 0 else []) + [t])
+            entries.append((s, 0, 0, 0, sum(1 << a for a in up[t])))
+        paths += [(s, [starts[s] + a for a in u]) for u in up]
+    rows, seq_rows = K.make_rows(entries, "cuda"), torch.tensor(starts, dtype=torch.int32, device="cuda")
+    out = torch.zeros(R, nv * dv, dtype=torch.float16, device="cuda")
+    p, st = L.DeltaParams(), L.SpecStage()
+    p.proj, p.ld = proj.data_ptr(), ld
+    p.off_q, p.off_k, p.off_v, p.off_z, p.off_a, p.off_b = offs
+    p.xn, p.ldx, p.H, p.wa, p.wb = xn.data_ptr(), H, H, wa.data_ptr(), wb.data_ptr()
+    every = list(range(R))
+    keep = lazy(every) if ab == "lazy" else None
+    if keep is not None:
+        p.ln = keep
+    p.conv_w, p.conv_state, p.state = conv_w.data_ptr(), conv.data_ptr(), state.data_ptr()
+    p.A_log, p.dt_bias, p.norm_w = A_log.data_ptr(), dt_bias.data_ptr(), norm_w.data_ptr()
+    p.seq_rows, p.rows, p.out, p.ldo = seq_rows.data_ptr(), rows.data_ptr(), out.data_ptr(), out.stride(0)
+    p.nk, p.nv, p.n_seqs, p.eps = nk, nv, ns, 1e-6
+    off = [C.c_int() for _ in range(4)]
+    L.lib().b2_spec_stage_layout.restype = C.c_longlong
+    blk = int(L.lib().b2_spec_stage_layout(nk, nv, dk, dv, *[C.byref(o) for o in off]))
+    stage = torch.zeros(ns * blk, dtype=torch.uint8, device="cuda")
+    st.base, st.seq_stride, st.layer_stride = stage.data_ptr(), blk, ns * blk
+    st.off_k, st.off_u, st.off_g, st.off_x = (o.value for o in off)
+    s0, c0 = state.clone(), conv.clone()
+    L.check(L.lib().b2_deltanet_verify(C.byref(p), C.byref(st), 0, dk, dv, L.stream()), "verify")
+    assert torch.equal(state, s0) and torch.equal(conv, c0)
+    for r, (s, path) in enumerate(paths):
+        one = torch.tensor([0, len(path)], dtype=torch.int32, device="cuda")
+        ref = K.deltanet_step(proj[path].contiguous(), offs, conv_w, conv.clone(), state.clone(), A_log, dt_bias, norm_w,
+                              K.make_rows([(s, 0, 0, 0, 1)] * len(path), "cuda"), one, nk, nv, dk, dv,
+                              xn=xn[path].contiguous() if ab == "xn" else None, wa=wa if ab != "proj" else None,
+                              wb=wb if ab != "proj" else None, ln=lazy(path) if ab == "lazy" else None)[-1]
+        err = float((out[r].float() - ref.float()).abs().max() / ref.float().abs().max())
+        assert err < 2e-3, (r, err)
