@@ -255,6 +255,29 @@ def test_attn_rows_tensor_core(K, hd, nq, nkv, splits):
         assert _rel(out[r].cpu().view(nq, hd), o[0]) < 4e-3, f"row {r}"
 
 
+@pytest.mark.parametrize("hd,nq,nkv,sizes,splits", [(256, 24, 4, [5, 5, 5], 2), (256, 6, 1, [1, 5, 2, 3], 1), (256, 4, 2, [1] * 9, 3),
+                                                    (256, 8, 1, [2, 1], 1), (64, 4, 2, [8, 7], 4), (64, 2, 2, [16, 1, 1], 1),
+                                                    (64, 3, 1, [5, 0, 1], 2), (256, 5, 1, [6, 6], 7)])
+def test_attn_rows_few_rows_per_sequence(K, hd, nq, nkv, sizes, splits):
+    """Drafts and batched decode, whose heads share the MMA tiles: one and two tiles, ragged sequences (one of them
+    longer than a tile), empty ones, contexts that end inside a block, slices without a visible slot."""
+    from mi50grad_b200.models import oracle as O
+    gen = torch.Generator().manual_seed(16)
+    d = _dev()
+    max_seq, ctxs = 700, [0, 63, 64, 650, 300, 1, 129, 15, 16]
+    kc, vc = torch.randn(len(sizes), max_seq, nkv, hd, generator=gen).half(), torch.randn(len(sizes), max_seq, nkv, hd, generator=gen).half()
+    entries = [(s, ctxs[s], ctxs[s] + i, ctxs[s], (1 << i) | (0 if i % 3 == 2 else (1 << i) - 1)) for s, n in enumerate(sizes) for i in range(n)]
+    seq_rows = torch.tensor([sum(sizes[:i]) for i in range(len(sizes) + 1)], dtype=torch.int32)
+    q = torch.randn(len(entries), 2 * nq * hd, generator=gen).half()
+    out = K.attn_rows(q.to(d), K.make_rows(entries, d), seq_rows.to(d), kc.to(d), vc.to(d), nq, nkv, hd, gate_off=nq * hd, splits=splits)
+    for r, (s_, _, _, ctx, mask) in enumerate(entries):
+        vis = list(range(ctx)) + [ctx + j for j in range(64) if (mask >> j) & 1]
+        o = O.attention(q[r:r + 1, :nq * hd].float().view(1, nq, hd), kc[s_, vis].float(), vc[s_, vis].float(),
+                        torch.ones(1, len(vis), dtype=torch.bool))
+        o = o * torch.sigmoid(q[r, nq * hd:].float().view(1, nq, hd))
+        assert _rel(out[r].cpu().view(nq, hd), o[0]) < 4e-3, f"row {r}"
+
+
 @pytest.mark.parametrize("hd,nq,nkv,T,past", [(64, 4, 2, 40, 5), (64, 2, 1, 200, 0), (256, 6, 1, 130, 7),
                                               (256, 12, 2, 512, 0), (128, 4, 4, 300, 64)])
 def test_attn_prefill_tcgen05(K, hd, nq, nkv, T, past):
