@@ -1249,58 +1249,99 @@ B2_API int b2_deltanet_chunk(const DeltaParams* p, const void* ab, int ld_ab, vo
 }
 B2_API long long b2_deltanet_tw_floats(int nv, int n_rows) { return (long long)nv * ((n_rows + DC_C - 1) / DC_C) * 2 * DC_C * DC_C; }
 
-// a/b projections for many rows: ab[r][o] = x[r] . w[o], o < 2 nv (tiny dense weights).  A CTA stages
-// AB_ROWS activation rows in shared memory and computes 8 outputs (one per warp) for all of them:
-// grid = (row groups, output groups).
-#define AB_ROWS 8
-__global__ void __launch_bounds__(256) ab_proj_kernel(const __half* __restrict__ x, int ldx, const __half* __restrict__ wa,
-                                                      const __half* __restrict__ wb, int nv, int H,
-                                                      __half* __restrict__ ab, int ld_ab, int rows) {
-    extern __shared__ __align__(16) __half xs[];           // [AB_ROWS][H]
+__device__ __forceinline__ void ab_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// a / b gate projections of many rows: ab[t][o] = x[t] . w[o] (o < nv: wa, else wb), a handful of outputs over the whole
+// width, so neither a GEMM tile nor a dot product per warp fills the GPU: as one dense tcgen05 launch a CTA walked all of K
+// alone, with a warp per output on the FMA pipes 24 rows of 2048 took 9.5 us.  A CTA takes 16 rows x 32 outputs and its 8
+// warps divide K in steps of 32; they meet in shared memory.  The order of k inside a product is free, so lane t of a row
+// quad takes 8 adjacent k of its rows (16 bytes) and these are its fragments of two mma.sync.  Measured: 8.4 us for 512 rows of
+// 5120 and 96 outputs (27 before), 4.8 us for 24 rows of 2048.
+#define AB_TOK 16
+#define AB_OUT 32
+#define AB_WARPS 8
+#define AB_RING 4
+#define AB_ITEMS (2 + AB_OUT / 8)   // 16-byte pieces of a lane and step: two token rows, four output rows
+__global__ void __launch_bounds__(AB_WARPS * 32) ab_proj_kernel(const __half* __restrict__ x, int ldx, const __half* __restrict__ wa,
+                                                                const __half* __restrict__ wb, int nv, int H,
+                                                                __half* __restrict__ ab, int ld_ab, int rows) {
+    extern __shared__ uint4 ab_smem[];               // [AB_WARPS][AB_RING][AB_ITEMS][32 lanes]
     pdl_launch_dependents();
-    const int r0 = blockIdx.x * AB_ROWS, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nr = min(AB_ROWS, rows - r0);
-    for (int i = tid * 8; i < AB_ROWS * H; i += 256 * 8) {
-        const int r = i / H, c = i - r * H;
-        *(uint4*)(xs + i) = r < nr ? *(const uint4*)(x + (size_t)(r0 + r) * ldx + c) : make_uint4(0u, 0u, 0u, 0u);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    uint4* ring = ab_smem + warp * (AB_RING * AB_ITEMS * 32) + lane;
+    const int r0 = blockIdx.x * AB_TOK, o0 = blockIdx.y * AB_OUT;
+    const __half* xr[2];
+    const __half* wr[AB_OUT / 8];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) xr[i] = x + (size_t)min(r0 + g + 8 * i, rows - 1) * ldx + 8 * t;
+#pragma unroll
+    for (int n = 0; n < AB_OUT / 8; ++n) {
+        const int o = min(o0 + 8 * n + g, 2 * nv - 1);
+        wr[n] = (o < nv ? wa + (size_t)o * H : wb + (size_t)(o - nv) * H) + 8 * t;
+    }
+    float acc[AB_OUT / 8][4];
+#pragma unroll
+    for (int n = 0; n < AB_OUT / 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+    // a lane copies what it reads back itself (cp.async), AB_RING - 1 steps ahead: no barrier
+    auto issue = [&](int i, int slot) {
+        const int k0 = (i * AB_WARPS + warp) * 32;
+        uint4* d = ring + slot * AB_ITEMS * 32;
+        if (k0 + 8 * t < H) {                        // (H is a multiple of 8)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) cp_async16(d + q * 32, xr[q] + k0);
+#pragma unroll
+            for (int n = 0; n < AB_OUT / 8; ++n) cp_async16(d + (2 + n) * 32, wr[n] + k0);
+        } else {
+#pragma unroll
+            for (int q = 0; q < AB_ITEMS; ++q) d[q * 32] = make_uint4(0u, 0u, 0u, 0u);
+        }
+    };
+    const int steps = (H + AB_WARPS * 32 - 1) / (AB_WARPS * 32);
+#pragma unroll
+    for (int i = 0; i < AB_RING - 1; ++i) {
+        if (i < steps) issue(i, i);
+        cp_async_commit();
+    }
+    for (int i = 0; i < steps; ++i) {
+        if (i + AB_RING - 1 < steps) issue(i + AB_RING - 1, (i + AB_RING - 1) % AB_RING);
+        cp_async_commit();
+        cp_async_wait<AB_RING - 1>();
+        const uint4* v = ring + (i % AB_RING) * AB_ITEMS * 32;
+        const uint4 lo = v[0], hi = v[32];
+        const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
+#pragma unroll
+        for (int n = 0; n < AB_OUT / 8; ++n) {
+            const uint4 w = v[(2 + n) * 32];
+            ab_mma(acc[n], a0, w.x, w.y);
+            ab_mma(acc[n], a1, w.z, w.w);
+        }
+    }
+    __syncthreads();                                 // the partial sums take the ring's place
+    float (*red)[AB_TOK][AB_OUT + 2] = (float (*)[AB_TOK][AB_OUT + 2])ab_smem;
+#pragma unroll
+    for (int n = 0; n < AB_OUT / 8; ++n) {
+        *(float2*)&red[warp][g][8 * n + 2 * t] = make_float2(acc[n][0], acc[n][1]);
+        *(float2*)&red[warp][g + 8][8 * n + 2 * t] = make_float2(acc[n][2], acc[n][3]);
     }
     __syncthreads();
-    for (int o = blockIdx.y * 8 + warp; o < min(2 * nv, (int)blockIdx.y * 8 + 8); o += 8) {
-        const __half* w = (o < nv) ? wa + (size_t)o * H : wb + (size_t)(o - nv) * H;
-        float acc[AB_ROWS];
+    for (int i = tid; i < AB_TOK * AB_OUT; i += AB_WARPS * 32) {
+        const int r = i / AB_OUT, o = i % AB_OUT;
+        float s = 0.f;
 #pragma unroll
-        for (int r = 0; r < AB_ROWS; ++r) acc[r] = 0.f;
-        for (int i = lane * 8; i < H; i += 256) {
-            const uint4 wv = *(const uint4*)(w + i);
-            const __half2* w2 = (const __half2*)&wv;
-            float2 wf[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) wf[q] = __half22float2(w2[q]);
-#pragma unroll
-            for (int r = 0; r < AB_ROWS; ++r) {
-                const uint4 xv = *(const uint4*)(xs + r * H + i);
-                const __half2* x2 = (const __half2*)&xv;
-#pragma unroll
-                for (int q = 0; q < 4; ++q) { const float2 b = __half22float2(x2[q]); acc[r] += wf[q].x * b.x + wf[q].y * b.y; }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < AB_ROWS; ++r) {
-            const float v = warp_sum(acc[r]);
-            if (lane == 0 && r < nr) ab[(size_t)(r0 + r) * ld_ab + o] = __float2half(v);
-        }
+        for (int w = 0; w < AB_WARPS; ++w) s += red[w][r][o];
+        if (r0 + r < rows && o0 + o < 2 * nv) ab[(size_t)(r0 + r) * ld_ab + o0 + o] = __float2half(s);
     }
 }
 B2_API int b2_ab_proj(const void* x, int ldx, const void* wa, const void* wb, int nv, int H, void* ab, int ld_ab,
                       int rows, cudaStream_t s) {
     if (H % 8 || (ldx % 8)) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)AB_ROWS * H * 2;
+    constexpr size_t smem = (size_t)AB_WARPS * AB_RING * AB_ITEMS * 32 * 16;
     static SmemOptIn optin;
-    {
-        cudaError_t e = optin.ensure(ab_proj_kernel, smem);
-        if (e != cudaSuccess) return e;
-    }
-    ab_proj_kernel<<<dim3((rows + AB_ROWS - 1) / AB_ROWS, (2 * nv + 7) / 8), 256, smem, s>>>((const __half*)x, ldx, (const __half*)wa,
-                                                                     (const __half*)wb, nv, H, (__half*)ab, ld_ab, rows);
+    if (cudaError_t e = optin.ensure(ab_proj_kernel, smem)) return e;
+    ab_proj_kernel<<<dim3((rows + AB_TOK - 1) / AB_TOK, (2 * nv + AB_OUT - 1) / AB_OUT), AB_WARPS * 32, smem, s>>>(
+        (const __half*)x, ldx, (const __half*)wa, (const __half*)wb, nv, H, (__half*)ab, ld_ab, rows);
     return cudaGetLastError();
 }

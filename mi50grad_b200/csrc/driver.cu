@@ -62,7 +62,6 @@ struct LayerDesc {
     int q8_group, q8_F, pad_q8;   // group size of the W4A8 scales; local FFN width
     const void* q8_w[3];          // int8 [N][K] or signed nibbles int32 [N][K/8]
     const void* q8_s[3];          // fp32 [N] (W8A8) or fp16 [K/group][N] (W4A8)
-    const void* wab;              // DeltaNet: [wa; wb] as one fp16 [2*nv][H] matrix (many-row steps run it as a GEMM)
 };
 
 struct ModelDesc {
@@ -683,17 +682,7 @@ static int rows_impl(Driver* d, int T, int n_seqs, int flags, cudaStream_t s) {
             // else one small dense kernel for all rows into spare columns of the projection buffer
             const void* ab = (const __half*)m.p_proj + (L.off_a >= 0 ? L.off_a : 0);
             if (L.off_a < 0 && m.ab_off >= 0) {
-                if (L.wab && T >= 64 && m.H % 64 == 0) {
-                    // the two small gate projections of all rows as one dense tensor-core GEMM (weights by TMA)
-                    GemmTcParams g;
-                    memset(&g, 0, sizeof(g));
-                    g.K = m.H; g.T = T; g.t_tile = 64;
-                    g.n_valid = 2 * m.la_nv; g.ldo = m.ld_proj; g.epi = TC_EPI_STORE_F16;
-                    g.out = (__half*)m.p_proj + m.ab_off; g.status = m.tc_status;
-                    CK(b2_gemm_f16_tc(&g, L.wab, m.H, m.p_xn, m.H, s));
-                } else {
-                    CK(b2_ab_proj(m.p_xn, m.H, L.wa, L.wb, m.la_nv, m.H, (__half*)m.p_proj + m.ab_off, m.ld_proj, T, s));
-                }
+                CK(b2_ab_proj(m.p_xn, m.H, L.wa, L.wb, m.la_nv, m.H, (__half*)m.p_proj + m.ab_off, m.ld_proj, T, s));
                 d->launches++;
                 ab = (const __half*)m.p_proj + m.ab_off;
                 q.off_a = m.ab_off; q.off_b = m.ab_off + m.la_nv;

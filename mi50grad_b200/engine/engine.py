@@ -512,10 +512,6 @@ class InferenceEngine:
             else:
                 d.wa = None if dl.wa is None else dl.wa.data_ptr()
                 d.wb = None if dl.wb is None else dl.wb.data_ptr()
-                if dl.wa is not None and dl.wb is not None:
-                    if getattr(dl, "wab", None) is None:
-                        dl.wab = torch.cat([dl.wa, dl.wb], dim=0).contiguous()
-                    d.wab = dl.wab.data_ptr()
                 d.conv_w, d.A_log = dl.conv_w.data_ptr(), dl.A_log.data_ptr()
                 d.dt_bias, d.la_norm = dl.dt_bias.data_ptr(), dl.la_norm.data_ptr()
                 d.conv_state = self.states.dn.layer_conv(i).data_ptr()

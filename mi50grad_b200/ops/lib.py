@@ -144,7 +144,7 @@ class LayerDesc(C.Structure):
                 ("A_log", vp), ("dt_bias", vp), ("la_norm", vp),
                 ("off_q", i32), ("off_k", i32), ("off_v", i32), ("off_z", i32), ("off_a", i32), ("off_b", i32),
                 ("ffn_kind", i32), ("q8_group", i32), ("q8_F", i32), ("pad_q8", i32),
-                ("q8_w", vp * 3), ("q8_s", vp * 3), ("wab", vp)]
+                ("q8_w", vp * 3), ("q8_s", vp * 3)]
 
 
 class SampleParams(C.Structure):

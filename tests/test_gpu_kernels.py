@@ -228,6 +228,15 @@ def test_decode_attn(K, hd, nq, nkv, splits):
         assert _rel(out[r].cpu().view(nq, hd), o[0]) < 3e-3, f"row {r}"
 
 
+@pytest.mark.parametrize("rows,nv,H", [(1, 1, 8), (16, 16, 256), (17, 17, 264), (80, 48, 5120), (33, 3, 2056)])
+def test_ab_proj_edges(K, rows, nv, H):
+    """Row and output tiles of 16 and 32, widths that end inside a step: fp32 sums rounded to fp16 once."""
+    gen = torch.Generator().manual_seed(22)
+    x, wa, wb = (torch.randn(n, H, generator=gen).half() for n in (rows, nv, nv))
+    ab = K.ab_proj(x.to(_dev()), wa.to(_dev()), wb.to(_dev())).cpu()[:, :2 * nv]
+    assert _rel(ab, torch.cat([x.double() @ wa.double().t(), x.double() @ wb.double().t()], 1)) < 1e-3
+
+
 @pytest.mark.parametrize("hd,nq,nkv,splits", [(256, 6, 1, 1), (256, 24, 4, 3), (64, 4, 2, 1), (64, 6, 2, 4)])
 def test_attn_rows_tensor_core(K, hd, nq, nkv, splits):
     """Many-row attention: a 40-row causal prompt chunk behind 5 cached tokens (three tiles, the last
