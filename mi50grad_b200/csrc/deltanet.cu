@@ -539,8 +539,7 @@ __device__ __forceinline__ float silu_fast(float x) { return __fdividef(x, 1.f +
 
 template <int DK, int DV>
 __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_chunk_kernel(const DeltaParams p, const __half* __restrict__ ab, int ld_ab,
-                                                                      const __half* __restrict__ qk_pre, int ld_qk,
-                                                                      const float* __restrict__ tw_pre, int n_chunks) {
+                                                                      const __half* __restrict__ qk_pre, int ld_qk) {
     constexpr int CB = DV / DN_COLS;
     constexpr int MT = DK / 16;               // 16-row tiles of the state slice, one or two per warp
     constexpr int SPW = (MT + 7) / 8;         // state m-tiles per warp
@@ -563,8 +562,9 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_chunk_kernel(const Del
     float* Us = Ks + DC_C * LDK;              // [C][LDU]  v -> b -> u (in place)
     float* QSs = Us + DC_C * DC_LDU;          // [C][32]   exp(G) Q S0
     float* Ys = QSs + DC_C * DN_COLS;         // [C][32]
-    float* As0 = Ys + DC_C * DN_COLS;         // [2][2][C][LDA]: (A or T, W) of this chunk and, with the pre-pass, of the next
-    float* S0t = As0 + 4 * DC_C * DC_LDA;     // [32][LDK]  transposed copy of the state slice (a B operand)
+    float* As = Ys + DC_C * DN_COLS;          // [C][LDA]
+    float* Ws = As + DC_C * DC_LDA;           // [C][LDA]
+    float* S0t = Ws + DC_C * DC_LDA;          // [32][LDK]  transposed copy of the state slice (a B operand)
     float* hist = S0t + DN_COLS * LDK;        // [NCH][3]
     float* cw = hist + NCH * 3;               // [NCH][4]
     float* Gs = cw + NCH * 4;                 // [C] running log-decay
@@ -641,18 +641,6 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_chunk_kernel(const Del
         }
         cp_async_commit();
     };
-    // T = (I + A)^-1 and W of a chunk from the pre-pass: 32 x 32 floats each, into the chunk's pair of buffers
-    auto stage_tw = [&](int ci) {
-        if (!tw_pre) return;
-        float* dstb = As0 + (ci & 1) * 2 * DC_C * DC_LDA;
-        const float* src = tw_pre + ((size_t)j * n_chunks + ci) * 2 * DC_C * DC_C;
-        for (int idx = tid; idx < 2 * DC_C * (DC_C / 4); idx += DN_THREADS) {
-            const int mat = idx / (DC_C * (DC_C / 4)), rem = idx % (DC_C * (DC_C / 4));
-            const int row = rem / (DC_C / 4), pc = rem % (DC_C / 4);
-            cp_async16(dstb + mat * DC_C * DC_LDA + row * DC_LDA + pc * 4, src + mat * DC_C * DC_C + row * DC_C + pc * 4);
-        }
-    };
-    stage_tw(0);
     stage_raw(r0);
     // the gate inputs of a chunk are fetched one chunk ahead (a global round trip off the critical path)
     float a_pre = 0.f, b_pre = 0.f;
@@ -712,9 +700,7 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_chunk_kernel(const Del
             cl_ss[slot * DC_C + tid] = 0.f;
         }
         __syncthreads();
-        if (rb + DC_C < r1) { stage_tw(chunk_idx + 1); stage_raw(rb + DC_C); }          // fly while this chunk is processed
-        float* As = As0 + (tw_pre ? (chunk_idx & 1) * 2 * DC_C * DC_LDA : 0);
-        float* Ws = As + DC_C * DC_LDA;
+        if (rb + DC_C < r1) stage_raw(rb + DC_C);          // fly while this chunk is processed
         fetch_gates(rb + DC_C);
         // output gates of this chunk, needed only at its end
         float zf[DC_C / 8];
@@ -790,7 +776,7 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_chunk_kernel(const Del
         const int a_row = (lane & 7) + ((lane >> 3) & 1) * 8, a_col = (lane >> 4) * 4;       // A operand addressing
         const int b_row = (lane & 7) + (lane >> 4) * 8, b_col = ((lane >> 3) & 1) * 4;       // B operand, two 8-column tiles
         {
-            for (int tile = kr; tile < (tw_pre ? 0 : MB * (MB + 1)); tile += 8) {
+            for (int tile = kr; tile < MB * (MB + 1); tile += 8) {
                 int mi = 0, ni = tile;                 // row block mi holds tiles ni = 0 .. 2 mi + 1
                 while (ni >= 2 * mi + 2) { ni -= 2 * mi + 2; ++mi; }
                 float kk[4] = {0.f, 0.f, 0.f, 0.f}, qk[4] = {0.f, 0.f, 0.f, 0.f};
@@ -855,36 +841,6 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_chunk_kernel(const Del
         // ---- P5: (I + A) U = B by forward substitution, 8 rows per block: every warp first removes
         // the contribution of all earlier blocks from its row, then warp 0 solves the 8x8 triangle
         // with one column per lane in registers
-        if (tw_pre) {
-            // U = T B with T = (I + A)^-1 from the pre-pass: one 16x8 tile per warp, split-TF32 operands
-            // (hi + lo parts) so that the product keeps fp32 accuracy like the substitution it replaces
-            const int mi5 = kr % MB, nb5 = (kr / MB) * NTW;
-            float u[NTW][4];
-#pragma unroll
-            for (int n = 0; n < NTW; ++n) u[n][0] = u[n][1] = u[n][2] = u[n][3] = 0.f;
-            const float* ta = As + (16 * mi5 + a_row) * DC_LDA + a_col;
-            for (int k0 = 0; k0 < 16 * (mi5 + 1); k0 += 8) {
-                float fa[4], hi[4], lo[4];
-                ldsm4(fa, ta + k0);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) { hi[e] = tf32r(fa[e]); lo[e] = tf32r(fa[e] - hi[e]); }
-#pragma unroll
-                for (int n = 0; n < NTW; ++n) {
-                    const float b0 = Us[(k0 + t) * DC_LDU + 8 * (nb5 + n) + g], b1 = Us[(k0 + t + 4) * DC_LDU + 8 * (nb5 + n) + g];
-                    const float b0h = tf32r(b0), b1h = tf32r(b1);
-                    mma_tf32(u[n], lo[0], lo[1], lo[2], lo[3], b0h, b1h);
-                    mma_tf32(u[n], hi[0], hi[1], hi[2], hi[3], tf32r(b0 - b0h), tf32r(b1 - b1h));
-                    mma_tf32(u[n], hi[0], hi[1], hi[2], hi[3], b0h, b1h);
-                }
-            }
-            __syncthreads();                               // every warp has read B before anyone overwrites it
-#pragma unroll
-            for (int n = 0; n < NTW; ++n)
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    Us[(16 * mi5 + g + (e >> 1) * 8) * DC_LDU + 8 * (nb5 + n) + 2 * t + (e & 1)] = u[n][e];
-            __syncthreads();
-        } else
         for (int blk = 0; blk < DC_C / 8; ++blk) {
             const int i = 8 * blk + kr;
             float acc = Us[i * DC_LDU + vcol];
@@ -1074,23 +1030,53 @@ __global__ void __launch_bounds__(2 * DK) deltanet_qk_prep_kernel(const DeltaPar
 }
 
 // ---------------------------------------------------------------------------
-// Second pre-pass of the chunked scan: everything of a chunk that does not depend on the state, for every
-// (value head, chunk) in parallel: the gates, A = beta decay (K K^T) below the diagonal, W = decay (Q K^T) on
-// and below it, and T = (I + A)^-1 (forward substitution on the 32 x 32 unit triangle, one column per lane).
-// The scan then replaces its per-chunk products and its sequential triangular solve by loads and U = T B.
-// Output fp32 [nv][n_chunks][T | W][32][32].  grid = (chunks, value heads), 256 threads.
+// The scan of one prompt, in three parts.  With T = (I + A)^-1 the update vectors of a chunk are
+//     U = T (beta (V - exp(G) K S0)) = U0 - Wt S0,     U0 = T diag(beta) V,   Wt = T diag(beta exp(G)) K,
+// and U0, Wt and W do not depend on the state.  So a first kernel forms them for every (value head, chunk) side by side
+// (deltanet_tw_prep_kernel), and what is left to the serial walk over the chunks is two dependent products a chunk:
+// [Wt; Q] S0, then W U and K^T U (deltanet_scan_kernel).  The raw outputs go back into U0's place; a third kernel
+// norms, gates and rounds them (deltanet_scan_out_kernel), which also keeps the sum over a head's columns, and with it
+// the cluster, out of the walk.
+//
+// Per (value head, chunk) the work buffer holds Wt [32][DK] | U0, later Y [32][DV] | W [32][32] | exp(G) [32] |
+// exp(G_C - G) [32] | exp(G_C).
 // ---------------------------------------------------------------------------
-template <int DK>
+#define DC_GATES (2 * DC_C + 4)
+template <int DK, int DV> struct ScanBlock {
+    static constexpr int U0 = DC_C * DK, W = U0 + DC_C * DV, GATES = W + DC_C * DC_C, FLOATS = GATES + DC_GATES;
+};
+
+// hi + lo = x with hi a TF32 value; the tensor core ignores the low 13 bits of lo, which leaves 2^-21 of x
+__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
+    hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
+    lo = x - hi;
+}
+__device__ __forceinline__ void ldsm4_h(uint32_t (&r)[4], const __half* row_ptr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(row_ptr)));
+}
+__device__ __forceinline__ void ldsm4_ht(uint32_t (&r)[4], const __half* row_ptr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(row_ptr)));
+}
+__device__ __forceinline__ float2 h2f(uint32_t x) { return __half22float2(*(const __half2*)&x); }
+
+// Everything of a chunk that does not depend on the state: the gates, A = beta decay (K K^T) below the diagonal,
+// W = decay (Q K^T) on and below it, T = (I + A)^-1 (forward substitution on the 32 x 32 unit triangle, one column per
+// lane), the convolved values V, and with them U0 and Wt.  T enters its products as hi + lo TF32 parts (and V too; K is
+// fp16), so they keep fp32 accuracy.  grid = (chunks, value heads), 256 threads.
+template <int DK, int DV>
 __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const DeltaParams p, const __half* __restrict__ ab, int ld_ab,
                                                                       const __half* __restrict__ qk_pre, int ld_qk,
                                                                       float* __restrict__ tw, int n_chunks) {
     static_assert(DC_C == 32, "one lane per column of the triangle");
-    constexpr int LDK = DC_LDK(DK);
+    constexpr int LDK = DC_LDK(DK), LDV = DV + 8;
     constexpr int MB = DC_C / 16;
     extern __shared__ __align__(16) float psm[];
     float* Qs = psm;                          // [C][LDK]
     float* Ks = Qs + DC_C * LDK;
-    float* As = Ks + DC_C * LDK;              // [C][LDA]
+    float* Vs = Ks + DC_C * LDK;              // [C][LDV]
+    float* As = Vs + DC_C * LDV;              // [C][LDA]
     float* Ws = As + DC_C * DC_LDA;
     float* Ts = Ws + DC_C * DC_LDA;
     float* Gs = Ts + DC_C * DC_LDA;           // [C]
@@ -1101,7 +1087,7 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const Delt
     const int r0 = p.seq_rows[0], r1 = p.seq_rows[1];
     const int rb = r0 + ci * DC_C;
     if (rb >= r1) return;
-    const int Ce = min(DC_C, r1 - rb);
+    const int Ce = min(DC_C, r1 - rb), seq = p.rows[r0].seq;
     for (int idx = tid; idx < DC_C * (DK / 8) * 2; idx += DN_THREADS) {
         const int which = idx / (DC_C * (DK / 8)), rem = idx % (DC_C * (DK / 8));
         const int row = rem / (DK / 8), c = (rem % (DK / 8)) * 8;
@@ -1111,6 +1097,23 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const Delt
         float* dst = (which ? Ks : Qs) + row * LDK + c;
 #pragma unroll
         for (int q = 0; q < 4; ++q) { const float2 f = __half22float2(h2[q]); dst[2 * q] = f.x; dst[2 * q + 1] = f.y; }
+    }
+    // values: causal convolution + SiLU of a channel over a run of rows; rows before the sequence come from the history
+    for (int idx = tid; idx < DV * (DC_C / 8); idx += DN_THREADS) {
+        const int c = idx % DV, i0 = idx / DV * 8;
+        const __half* hist = p.conv_state + ((((size_t)seq * p.nv + j) * (DV / DN_COLS) + c / DN_COLS) * (2 * DK + DN_COLS) + 2 * DK + c % DN_COLS) * 3;
+        const __half* w = p.conv_w + (size_t)(2 * p.nk * DK + j * DV + c) * 4;
+        const float w0 = __half2float(w[0]), w1 = __half2float(w[1]), w2 = __half2float(w[2]), w3 = __half2float(w[3]);
+        const __half* col = p.proj + p.off_v + j * DV + c;
+        float x[11];
+#pragma unroll
+        for (int i = 0; i < 11; ++i) {
+            const int ri = rb + i0 - 3 + i;
+            x[i] = ri >= r1 ? 0.f : (ri >= r0 ? __half2float(col[(size_t)ri * p.ld]) : __half2float(hist[ri - r0 + 3]));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            Vs[(i0 + i) * LDV + c] = i0 + i < Ce ? silu_fast(x[i] * w0 + x[i + 1] * w1 + x[i + 2] * w2 + x[i + 3] * w3) : 0.f;
     }
     if (tid < DC_C) {
         float gl = 0.f, beta = 0.f;
@@ -1137,7 +1140,7 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const Delt
     {
         const int a_row = (lane & 7) + ((lane >> 3) & 1) * 8, a_col = (lane >> 4) * 4;
         for (int tile = kr; tile < MB * (MB + 1); tile += 8) {
-            int mi = 0, ni = tile;
+            int mi = 0, ni = tile;                 // row block mi holds tiles ni = 0 .. 2 mi + 1
             while (ni >= 2 * mi + 2) { ni -= 2 * mi + 2; ++mi; }
             float kk[4] = {0.f, 0.f, 0.f, 0.f}, qk[4] = {0.f, 0.f, 0.f, 0.f};
             const float* ka = Ks + (16 * mi + a_row) * LDK + a_col;
@@ -1179,11 +1182,258 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const Delt
         }
     }
     __syncthreads();
-    float* dst = tw + ((size_t)j * n_chunks + ci) * 2 * DC_C * DC_C;
-    for (int idx = tid; idx < 2 * DC_C * DC_C; idx += DN_THREADS) {
-        const int mat = idx / (DC_C * DC_C), rem = idx % (DC_C * DC_C);
-        dst[idx] = (mat ? Ws : Ts)[(rem / DC_C) * DC_LDA + rem % DC_C];
+    typedef ScanBlock<DK, DV> B;
+    float* dst = tw + ((size_t)j * n_chunks + ci) * B::FLOATS;
+    for (int idx = tid; idx < DC_C * DC_C; idx += DN_THREADS) dst[B::W + idx] = Ws[(idx / DC_C) * DC_LDA + idx % DC_C];
+    if (tid < DC_C) {
+        dst[B::GATES + tid] = __expf(Gs[tid]);
+        dst[B::GATES + DC_C + tid] = __expf(Gs[DC_C - 1] - Gs[tid]);
+        if (tid == 0) dst[B::GATES + 2 * DC_C] = __expf(Gs[DC_C - 1]);
     }
+    // ---- Wt = (T diag(beta exp(G))) K and U0 = (T diag(beta)) V: 16 x 8 tiles, T is zero above the diagonal
+    // (a warp keeps to one row tile, so T's fragments are split once per product)
+    const int mi = kr % MB;
+#pragma unroll
+    for (int kind = 0; kind < 2; ++kind) {
+        const bool is_k = kind == 0;
+        const float* src = is_k ? Ks + g : Vs + g;
+        const int lds = is_k ? LDK : LDV, ldo = is_k ? DK : DV;
+        float* o = dst + (is_k ? 0 : B::U0) + 2 * t;
+        float hi[DC_C / 8][4], lo[DC_C / 8][4];
+#pragma unroll
+        for (int k8 = 0; k8 < DC_C / 8; ++k8)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int k = 8 * k8 + t + 4 * (e >> 1);
+                split_tf32(Ts[(16 * mi + g + 8 * (e & 1)) * DC_LDA + k] * bs[k] * (is_k ? __expf(Gs[k]) : 1.f), hi[k8][e], lo[k8][e]);
+            }
+        for (int n0 = kr / MB * 8; n0 < ldo; n0 += DN_THREADS / 32 / MB * 8) {
+            float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int k8 = 0; k8 < DC_C / 8; ++k8) {
+                if (8 * k8 >= 16 * (mi + 1)) break;
+                float h0, l0, h1, l1;
+                split_tf32(src[n0 + (8 * k8 + t) * lds], h0, l0);
+                split_tf32(src[n0 + (8 * k8 + t + 4) * lds], h1, l1);
+                mma_tf32(acc, lo[k8][0], lo[k8][1], lo[k8][2], lo[k8][3], h0, h1);
+                if (!is_k) mma_tf32(acc, hi[k8][0], hi[k8][1], hi[k8][2], hi[k8][3], l0, l1);      // (K is exact)
+                mma_tf32(acc, hi[k8][0], hi[k8][1], hi[k8][2], hi[k8][3], h0, h1);
+            }
+            *(float2*)(o + (16 * mi + g) * ldo + n0) = make_float2(acc[0], acc[1]);
+            *(float2*)(o + (16 * mi + g + 8) * ldo + n0) = make_float2(acc[2], acc[3]);
+        }
+    }
+}
+
+// The walk over the chunks.  A CTA owns 32 columns of a value head's state: as accumulator fragments in registers (warp w:
+// rows 16 w ..) and, TF32-rounded and transposed, as the B operand in shared memory.  Two barriers a chunk:
+//   A  warp (m, n) forms its 16 x 8 tiles of Wt S0 (Wt as hi + lo) and Q S0, and writes U, twice (plain, and times
+//      exp(G_C - G) for the state), as a transposed B operand;
+//   B  the same warp finishes its tile of Y = exp(G) Q S0 + W U, and every warp updates its rows of the state.
+// The operands of the next chunk travel meanwhile (cp.async, two stages).  The order of k inside a product is free: a
+// 16-k block is taken as (2t, 2t + 1) and (8 + 2t, 9 + 2t), which is what ldmatrix gives of fp16 rows and one 8-byte
+// load of fp32 rows.  Bound: the latency of this chain.  Measured (48 value heads of 128, 512 rows):
+// 60 us, and 37 + 8 us for the parts before and behind it; one kernel with nine barriers a chunk took 144 + 16 us.
+#define SC_LDH(D) ((D) + 8)      // halfs: 16-byte rows of 8 adjacent lanes meet no bank twice
+#define SC_LDF(D) ((D) + 8)      // floats: the 8-byte reads of a half warp neither
+template <int DK>
+struct ScanStage {
+    __half q[DC_C][SC_LDH(DK)], k[DC_C][SC_LDH(DK)];
+    float wt[DC_C][SC_LDF(DK)], w[DC_C][SC_LDF(DC_C)], gates[DC_GATES];
+};
+template <int DK>
+struct ScanSmem {
+    ScanStage<DK> st[2];
+    float s0[DN_COLS][SC_LDF(DK)], u[DN_COLS][SC_LDF(DC_C)], ut[DN_COLS][SC_LDF(DC_C)];
+};
+
+template <int DK, int DV>
+__global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const DeltaParams p, const __half* __restrict__ qk_pre, int ld_qk,
+                                                                     float* __restrict__ tw, int n_chunks) {
+    typedef ScanBlock<DK, DV> B;
+    constexpr int MT = DK / 16;                   // warps that own 16 rows of the state
+    static_assert(DC_C == 32 && DN_COLS == 32 && MT <= 8, "eight warps: two row tiles by four column tiles");
+    extern __shared__ __align__(16) float dsm[];
+    ScanSmem<DK>& sm = *(ScanSmem<DK>*)dsm;
+    const int cb = blockIdx.x, j = blockIdx.y, kh = j / (p.nv / p.nk);
+    const int tid = threadIdx.x, lane = tid & 31, kr = tid >> 5, g = lane >> 2, t = lane & 3;
+    const int r0 = p.seq_rows[0], r1 = p.seq_rows[1];
+    if (r0 >= r1) return;
+    const int seq = p.rows[r0].seq, chunks = min((r1 - r0 + DC_C - 1) / DC_C, n_chunks);
+    float* blocks = tw + (size_t)j * n_chunks * B::FLOATS;
+
+    auto stage = [&](int ci) {
+        ScanStage<DK>& s = sm.st[ci & 1];
+        const float* src = blocks + (size_t)ci * B::FLOATS;
+        for (int i = tid; i < DC_C * (DK / 8) * 2; i += DN_THREADS) {
+            const int which = i / (DC_C * (DK / 8)), row = i / (DK / 8) % DC_C, c = i % (DK / 8) * 8, ri = ci * DC_C + row;
+            __half* d = which ? &s.k[row][c] : &s.q[row][c];
+            if (r0 + ri < r1) cp_async16(d, qk_pre + (size_t)ri * ld_qk + (which ? p.nk * DK : 0) + kh * DK + c);
+            else *(uint4*)d = make_uint4(0u, 0u, 0u, 0u);
+        }
+        for (int i = tid; i < DC_C * (DK / 4); i += DN_THREADS) cp_async16(&s.wt[i / (DK / 4)][i % (DK / 4) * 4], src + 4 * i);
+        for (int i = tid; i < DC_C * (DC_C / 4); i += DN_THREADS) cp_async16(&s.w[i / (DC_C / 4)][i % (DC_C / 4) * 4], src + B::W + 4 * i);
+        if (tid < DC_GATES / 4) cp_async16(&s.gates[4 * tid], src + B::GATES + 4 * tid);
+        cp_async_commit();
+    };
+    // this lane's elements of its 16 x 8 tile of U0 (and later Y)
+    const int mi = kr & 1, ni = kr >> 1;
+    const size_t u0_off = (size_t)B::U0 + (size_t)(16 * mi + g) * DV + cb * DN_COLS + 8 * ni + 2 * t;
+    float2 u0[2], u0n[2] = {};
+    auto load_u0 = [&](int ci) {
+        const float* src = blocks + (size_t)ci * B::FLOATS + u0_off;
+        u0n[0] = *(const float2*)src;
+        u0n[1] = *(const float2*)(src + 8 * DV);
+    };
+    stage(0);
+    load_u0(0);
+    float S[4][4];
+    float* sp = p.state + (((size_t)seq * p.nv + j) * DK) * DV + cb * DN_COLS;
+    auto put_s0 = [&]() {
+        if (kr < MT) {
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) sm.s0[8 * n + 2 * t + (e & 1)][16 * kr + g + 8 * (e >> 1)] = tf32r(S[n][e]);
+        }
+    };
+    if (kr < MT) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            const float2 lo = *(const float2*)(sp + (size_t)(16 * kr + g) * DV + 8 * n + 2 * t);
+            const float2 hi = *(const float2*)(sp + (size_t)(16 * kr + g + 8) * DV + 8 * n + 2 * t);
+            S[n][0] = lo.x; S[n][1] = lo.y; S[n][2] = hi.x; S[n][3] = hi.y;
+        }
+    }
+    put_s0();
+    const int a_row = lane & 15, a_col = (lane >> 4) * 8;                              // fp16 A operand (ldmatrix)
+    const int kt_row = (lane & 7) + (lane & 8), kt_col = (lane >> 4) * 8;              // its transpose: chunk rows x state rows
+    for (int ci = 0; ci < chunks; ++ci) {
+        cp_async_wait<0>();
+        __syncthreads();                          // the chunk's operands and S0 are in place; everyone left the chunk before
+        if (ci + 1 < chunks) stage(ci + 1);
+        u0[0] = u0n[0]; u0[1] = u0n[1];
+        if (ci + 1 < chunks) load_u0(ci + 1);
+        const ScanStage<DK>& s = sm.st[ci & 1];
+        // ---- A
+        float wh[4] = {0.f, 0.f, 0.f, 0.f}, wl[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+        {
+            const float* wr = &s.wt[16 * mi + g][2 * t];
+            const float* br = &sm.s0[8 * ni + g][2 * t];
+            const __half* qr = &s.q[16 * mi + a_row][a_col];
+#pragma unroll
+            for (int k0 = 0; k0 < DK; k0 += 16) {
+                uint32_t q[4];
+                ldsm4_h(q, qr + k0);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float2 b = *(const float2*)(br + k0 + 8 * h);
+                    const float2 x = *(const float2*)(wr + k0 + 8 * h), z = *(const float2*)(wr + 8 * SC_LDF(DK) + k0 + 8 * h);
+                    const float2 qa = h2f(q[2 * h]), qb = h2f(q[2 * h + 1]);
+                    float hi[4], lo[4];
+                    split_tf32(x.x, hi[0], lo[0]); split_tf32(z.x, hi[1], lo[1]);
+                    split_tf32(x.y, hi[2], lo[2]); split_tf32(z.y, hi[3], lo[3]);
+                    mma_tf32(wh, hi[0], hi[1], hi[2], hi[3], b.x, b.y);
+                    mma_tf32(wl, lo[0], lo[1], lo[2], lo[3], b.x, b.y);
+                    mma_tf32(y, qa.x, qb.x, qa.y, qb.y, b.x, b.y);
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int i = 16 * mi + g + 8 * (e >> 1), c = 8 * ni + 2 * t + (e & 1);
+            const float u = ((e & 2) ? ((e & 1) ? u0[1].y : u0[1].x) : ((e & 1) ? u0[0].y : u0[0].x)) - (wh[e] + wl[e]);
+            sm.u[c][i] = tf32r(u);
+            sm.ut[c][i] = tf32r(u * s.gates[DC_C + i]);
+            y[e] *= s.gates[i];
+        }
+        __syncthreads();
+        // ---- B: Y
+        {
+            const float* wr = &s.w[16 * mi + g][2 * t];
+            const float* br = &sm.u[8 * ni + g][2 * t];
+#pragma unroll
+            for (int k0 = 0; k0 < DC_C; k0 += 8) {
+                if (k0 >= 16 * (mi + 1)) break;   // (W is zero above the diagonal)
+                const float2 x = *(const float2*)(wr + k0), z = *(const float2*)(wr + 8 * SC_LDF(DC_C) + k0);
+                const float2 b = *(const float2*)(br + k0);
+                mma_tf32(y, x.x, z.x, x.y, z.y, b.x, b.y);
+            }
+            float* dst = blocks + (size_t)ci * B::FLOATS + u0_off;
+            *(float2*)dst = make_float2(y[0], y[1]);
+            *(float2*)(dst + 8 * DV) = make_float2(y[2], y[3]);
+        }
+        // ---- B: S' = exp(G_C) S0 + K^T (exp(G_C - G) U)
+        if (kr < MT) {
+            const float egC = s.gates[2 * DC_C];
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) S[n][e] *= egC;
+#pragma unroll
+            for (int k0 = 0; k0 < DC_C; k0 += 16) {
+                uint32_t kt[4];                   // chunk rows k0 + 2t, state row g | k0 + 8 + 2t, g | k0 + 2t, g + 8 | k0 + 8 + 2t, g + 8
+                ldsm4_ht(kt, &s.k[k0 + kt_row][16 * kr + kt_col]);
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const float2 lo = h2f(kt[h]), hi = h2f(kt[2 + h]);
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        const float2 b = *(const float2*)&sm.ut[8 * n + g][k0 + 8 * h + 2 * t];
+                        mma_tf32(S[n], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
+                    }
+                }
+            }
+        }
+        put_s0();                                 // (every warp read S0 before the second barrier)
+    }
+    if (!p.commit) return;
+    if (kr < MT) {
+#pragma unroll
+        for (int n = 0; n < 4; ++n) {
+            *(float2*)(sp + (size_t)(16 * kr + g) * DV + 8 * n + 2 * t) = make_float2(S[n][0], S[n][1]);
+            *(float2*)(sp + (size_t)(16 * kr + g + 8) * DV + 8 * n + 2 * t) = make_float2(S[n][2], S[n][3]);
+        }
+    }
+}
+
+// Gated RMSNorm of the raw outputs, one warp per (row, value head); the CTAs behind the rows store the last three raw
+// convolution inputs of every channel (older history shifts in when the prompt was shorter than that).
+template <int DK, int DV>
+__global__ void __launch_bounds__(DN_THREADS) deltanet_scan_out_kernel(const DeltaParams p, const float* __restrict__ tw, int n_chunks, int row_ctas) {
+    typedef ScanBlock<DK, DV> B;
+    constexpr int PL = DV / 32;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int r0 = p.seq_rows[0], r1 = p.seq_rows[1];
+    if (r0 >= r1) return;
+    if ((int)blockIdx.x >= row_ctas) {
+        if (!p.commit) return;
+        constexpr int NCH = 2 * DK + DN_COLS, CB = DV / DN_COLS;
+        const int hb = blockIdx.x - row_ctas, j = hb / CB, cb = hb % CB, kh = j / (p.nv / p.nk);
+        __half* hist = p.conv_state + ((((size_t)p.rows[r0].seq * p.nv + j) * CB + cb) * NCH) * 3;
+        for (int c = tid; c < NCH; c += DN_THREADS) {
+            const int col = c < DK ? p.off_q + kh * DK + c : (c < 2 * DK ? p.off_k + kh * DK + c - DK : p.off_v + j * DV + cb * DN_COLS + c - 2 * DK);
+            __half x[3];
+#pragma unroll
+            for (int q = 0; q < 3; ++q) { const int ri = r1 - 3 + q; x[q] = ri >= r0 ? p.proj[(size_t)ri * p.ld + col] : hist[c * 3 + (ri - r0 + 3)]; }
+#pragma unroll
+            for (int q = 0; q < 3; ++q) hist[c * 3 + q] = x[q];
+        }
+        return;
+    }
+    const int item = blockIdx.x * (DN_THREADS / 32) + (tid >> 5), i = item / p.nv, j = item % p.nv;
+    if (i >= r1 - r0) return;
+    const float* y = tw + ((size_t)j * n_chunks + i / DC_C) * B::FLOATS + B::U0 + (i % DC_C) * DV + lane * PL;
+    const __half* zp = p.proj + (size_t)(r0 + i) * p.ld + p.off_z + j * DV + lane * PL;
+    float v[PL], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < PL; e += 2) { const float2 f = *(const float2*)(y + e); v[e] = f.x; v[e + 1] = f.y; }
+#pragma unroll
+    for (int e = 0; e < PL; ++e) ss += v[e] * v[e];
+    const float inv = rsqrtf(warp_sum(ss) / (float)DV + p.eps);
+    __half* o = p.out + (size_t)(r0 + i) * p.ldo + j * DV + lane * PL;
+#pragma unroll
+    for (int e = 0; e < PL; ++e) o[e] = __float2half(v[e] * inv * __half2float(p.norm_w[lane * PL + e]) * silu_fast(__half2float(zp[e])));
 }
 
 template <int DK, int DV>
@@ -1195,20 +1445,23 @@ static int launch_delta_chunk(const DeltaParams* p, const void* ab, int ld_ab, _
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    const int n_chunks = (n_rows + DC_C - 1) / DC_C;
     if (qk_pre && tw) {
-        const size_t psm = (size_t)(2 * DC_C * DC_LDK(DK) + 3 * DC_C * DC_LDA + 3 * DC_C) * sizeof(float);
-        static SmemOptIn opt_tw;
-        if (int e = opt_tw.ensure(deltanet_tw_prep_kernel<DK>, psm)) return e;
-        deltanet_tw_prep_kernel<DK><<<dim3(n_chunks, p->nv), DN_THREADS, psm, s>>>(*p, (const __half*)ab, ld_ab, qk_pre, ld_qk, tw, n_chunks);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    } else {
-        tw = nullptr;
+        const int n_chunks = (n_rows + DC_C - 1) / DC_C;
+        constexpr size_t psm = (size_t)(2 * DC_C * DC_LDK(DK) + DC_C * (DV + 8) + 3 * DC_C * DC_LDA + 3 * DC_C) * sizeof(float);
+        static SmemOptIn opt_tw, opt_scan;
+        if (cudaError_t e = opt_tw.ensure(deltanet_tw_prep_kernel<DK, DV>, psm)) return e;
+        deltanet_tw_prep_kernel<DK, DV><<<dim3(n_chunks, p->nv), DN_THREADS, psm, s>>>(*p, (const __half*)ab, ld_ab, qk_pre, ld_qk, tw, n_chunks);
+        if (cudaError_t e = cudaGetLastError()) return e;
+        if (cudaError_t e = opt_scan.ensure(deltanet_scan_kernel<DK, DV>, sizeof(ScanSmem<DK>))) return e;
+        deltanet_scan_kernel<DK, DV><<<dim3(DV / DN_COLS, p->nv), DN_THREADS, sizeof(ScanSmem<DK>), s>>>(*p, qk_pre, ld_qk, tw, n_chunks);
+        if (cudaError_t e = cudaGetLastError()) return e;
+        const int row_ctas = (int)(((long long)n_rows * p->nv + DN_THREADS / 32 - 1) / (DN_THREADS / 32));
+        deltanet_scan_out_kernel<DK, DV><<<row_ctas + p->nv * (DV / DN_COLS), DN_THREADS, 0, s>>>(*p, tw, n_chunks, row_ctas);
+        return cudaGetLastError();
     }
     constexpr int CB = DV / DN_COLS;
     constexpr int NCH = 2 * DK + DN_COLS;
-    size_t smem = (size_t)(2 * DC_C * DC_LDK(DK) + DC_C * DC_LDU + 2 * DC_C * DN_COLS + 4 * DC_C * DC_LDA + DN_COLS * DC_LDK(DK) + NCH * 7 +
+    size_t smem = (size_t)(2 * DC_C * DC_LDK(DK) + DC_C * DC_LDU + 2 * DC_C * DN_COLS + 2 * DC_C * DC_LDA + DN_COLS * DC_LDK(DK) + NCH * 7 +
                            3 * DC_C + 2 * DC_C) * sizeof(float) + (size_t)(DC_C + 3) * NCH * sizeof(__half);
     static SmemOptIn optin;
     {
@@ -1227,15 +1480,14 @@ static int launch_delta_chunk(const DeltaParams* p, const void* ab, int ld_ab, _
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, deltanet_chunk_kernel<DK, DV>, *p, (const __half*)ab, ld_ab, (const __half*)qk_pre, ld_qk,
-                              (const float*)tw, n_chunks);
+    return cudaLaunchKernelEx(&cfg, deltanet_chunk_kernel<DK, DV>, *p, (const __half*)ab, ld_ab, (const __half*)qk_pre, ld_qk);
 }
 
 // ab: [rows][ld_ab] fp16 with a at column head and b at column nv + head.
 // qk_scratch (optional): fp16 [n_rows][ld_qk >= 2 * nk * dk] work buffer; with it, and ONE launched sequence of
 // n_rows rows, the q / k convolution and norms run once in a parallel pre-pass instead of inside the scan.
-// tw_scratch (optional, needs qk_scratch): fp32 [nv][ceil(n_rows / 32)][2][32][32]; with it the state-independent
-// products of every chunk and the inverse of its triangle are computed in a second parallel pre-pass.
+// tw_scratch (optional, needs qk_scratch): b2_deltanet_tw_floats(nv, n_rows) floats; with it the scan runs in three parts,
+// of which only the middle one walks over the chunks.
 B2_API int b2_deltanet_chunk(const DeltaParams* p, const void* ab, int ld_ab, void* qk_scratch, int ld_qk, int n_rows,
                              void* tw_scratch, int dk, int dv, cudaStream_t s) {
     if (p->nv % p->nk || !ab) return cudaErrorInvalidValue;
@@ -1247,7 +1499,7 @@ B2_API int b2_deltanet_chunk(const DeltaParams* p, const void* ab, int ld_ab, vo
     if (dk == 64 && dv == 64) return launch_delta_chunk<64, 64>(p, ab, ld_ab, qk, ld_qk, n_rows, tw, s);
     return cudaErrorInvalidValue;
 }
-B2_API long long b2_deltanet_tw_floats(int nv, int n_rows) { return (long long)nv * ((n_rows + DC_C - 1) / DC_C) * 2 * DC_C * DC_C; }
+B2_API long long b2_deltanet_tw_floats(int nv, int n_rows) { return (long long)nv * ((n_rows + DC_C - 1) / DC_C) * ScanBlock<128, 128>::FLOATS; }
 
 __device__ __forceinline__ void ab_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"

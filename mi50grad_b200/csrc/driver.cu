@@ -90,6 +90,7 @@ struct ModelDesc {
     float* p_h; void* p_xn; void* p_proj; void* p_attn; void* p_act; float* p_partial;
     void* p_rows; void* p_rows_tmpl; int* p_row_tokens; int* tc_status;
     void* p_ab;                            // [max_prefill][2*la_nv] fp16 a/b projections of the DeltaNet layers
+    void* p_scan;                          // DeltaNet scan: b2_deltanet_tw_floats(la_nv, max_prefill) floats
     float* coll_gather[B2_MAX_TP]; float* coll_mc_gather; int* coll_counters;
     // many-row steps (batched decode, speculative verification): logits and arg-max scratch for p_logit_rows rows
     float* p_logits; float* p_argmax_scratch; int* p_argmax_counters; int* p_out_tokens;
@@ -690,17 +691,14 @@ static int rows_impl(Driver* d, int T, int n_seqs, int flags, cudaStream_t s) {
             if (flags & STEP_SPEC) {
                 CK(b2_deltanet_verify(&q, &m.spec, L.type_index, m.la_dk, m.la_dv, s));
             } else if (n_seqs == 1 && T >= 16) {
-                // the FFN activation buffer is idle here: it holds the outputs of the two pre-passes (q | k of all rows,
-                // then T | W of every chunk and value head) when it is large enough
+                // the FFN activation buffer is idle here: it holds q | k of all rows when it is large enough
                 const int ld_qk = 2 * m.la_nk * m.la_dk;
                 const size_t cap = (size_t)m.max_prefill * m.F_pad * sizeof(__half);
-                const size_t qk_bytes = (((size_t)T * ld_qk * sizeof(__half)) + 255) & ~(size_t)255;
-                const size_t tw_bytes = (size_t)b2_deltanet_tw_floats(m.la_nv, T) * sizeof(float);
-                void* qk = (d->scan_prepass && qk_bytes <= cap) ? m.p_act : nullptr;
-                void* tw = (qk && d->scan_prepass > 1 && qk_bytes + tw_bytes <= cap) ? (void*)((char*)m.p_act + qk_bytes) : nullptr;
+                void* qk = (d->scan_prepass && (size_t)T * ld_qk * sizeof(__half) <= cap) ? m.p_act : nullptr;
+                void* tw = (qk && d->scan_prepass > 1) ? m.p_scan : nullptr;
                 CK(b2_deltanet_chunk(&q, ab, m.ld_proj, qk, ld_qk, T, tw, m.la_dk, m.la_dv, s));
                 if (qk) d->launches++;
-                if (tw) d->launches++;
+                if (tw) d->launches += 2;
             } else {
                 CK(b2_deltanet_step(&q, m.la_dk, m.la_dv, s));
             }

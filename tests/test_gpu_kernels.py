@@ -237,6 +237,31 @@ def test_ab_proj_edges(K, rows, nv, H):
     assert _rel(ab, torch.cat([x.double() @ wa.double().t(), x.double() @ wb.double().t()], 1)) < 1e-3
 
 
+@pytest.mark.parametrize("dk,nk,nv,rows", [(128, 1, 2, 1), (128, 2, 2, 31), (64, 1, 3, 33), (128, 1, 1, 64), (64, 2, 2, 2), (128, 1, 2, 1000)])
+def test_deltanet_scan_in_parts_equals_one_kernel(K, dk, nk, nv, rows):
+    """The three-part scan against the one-kernel form (which is tested against the oracle) where chunks and the convolution's
+    history begin and end.  Both round the state and U to TF32 once a chunk: an ulp of fp16 in the outputs."""
+    gen = torch.Generator().manual_seed(23)
+    rnd = lambda *s: torch.randn(*s, generator=gen)  # noqa: E731
+    kd, vd = nk * dk, nv * dk
+    conv_dim = 2 * kd + vd
+    proj, ab = rnd(rows, conv_dim + vd).half().cuda(), rnd(rows, 2 * nv).half().cuda()
+    w = [(rnd(conv_dim, 4) * 0.3).half().cuda(), (torch.rand(nv, generator=gen) * 1.5 - 1.0).cuda(), (rnd(nv) * 0.5).half().cuda(), (torch.rand(dk, generator=gen) + 0.5).half().cuda()]
+    S0, hist = (rnd(1, nv, dk, dk) * 0.1).cuda(), rnd(1, nv, dk // 32, 2 * dk + 32, 3).half().cuda()
+    hist[:, :, :, :2 * dk] = hist[:, :, :1, :2 * dk]
+    for j in range(nv):
+        hist[:, j, :, :2 * dk] = hist[:, j // (nv // nk) * (nv // nk), :, :2 * dk]
+    rows_meta, seq_rows = K.make_rows([(0, 0, 0, 0, 1)] * rows, _dev()), torch.tensor([0, rows], dtype=torch.int32, device=_dev())
+    got = []
+    for prepass in (0, 2):
+        S, h = S0.clone(), hist.clone()
+        out = K.deltanet_chunk(proj, (0, kd, 2 * kd, conv_dim, -1, -1), ab, w[0], h, S, w[1], w[2], w[3], rows_meta, seq_rows, nk, nv, dk, dk, prepass=prepass)
+        got.append((out, S, h))
+    assert _rel(got[1][0].cpu(), got[0][0].cpu().float()) < 4e-3
+    assert _rel(got[1][1].cpu(), got[0][1].cpu()) < 2e-3
+    assert torch.equal(got[1][2], got[0][2])
+
+
 @pytest.mark.parametrize("hd,nq,nkv,splits", [(256, 6, 1, 1), (256, 24, 4, 3), (64, 4, 2, 1), (64, 6, 2, 4)])
 def test_attn_rows_tensor_core(K, hd, nq, nkv, splits):
     """Many-row attention: a 40-row causal prompt chunk behind 5 cached tokens (three tiles, the last
