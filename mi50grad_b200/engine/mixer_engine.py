@@ -33,6 +33,9 @@ from ..ops import lib as L
 from .engine import InferenceEngine
 from .state import MixerStates
 
+PROMPT_ROWS = 2048      # rows of a prompt per pass (the planes of split projections and the scan's states grow with it)
+MAX_STEP_ROWS = 512     # rows of a step that can have logits
+
 DTYPES = {"bfloat16": (torch.bfloat16, L.DT_BF16, L.LIN_BF16), "float32": (torch.float32, L.DT_F32, L.LIN_F32)}
 
 
@@ -236,7 +239,7 @@ class MixerEngine(InferenceEngine):
         if any(l is None for l in self.layers) or self.embed is None or self.lm_head is None or self.final_norm is None:
             raise RuntimeError("weights are not fully loaded")
         cfg, R, T = self.config, self.max_rows, self.dtype
-        H, P = cfg.hidden_size, min(512, self.max_seq_len)
+        H, P = cfg.hidden_size, min(PROMPT_ROWS, self.max_seq_len)
         self.max_prefill = P
         runs, n_runs = [self.layers[i] for i in self.runs], len(self.runs)
         alloc = self._work_allocator()
@@ -284,7 +287,7 @@ class MixerEngine(InferenceEngine):
         b["out_tokens"], b["p_out_tokens"], b["tc_status"] = i32(R), i32(P), i32(4)
         # rows of a many-row step that can have logits: what the caller asked for, or 64 MB of them
         want = self.ecfg.max_step_rows or max(8 * self.max_batch, (64 << 20) // (4 * b["ld_logits"]))
-        self.step_rows = min(P, max(8, want))
+        self.step_rows = min(P, MAX_STEP_ROWS, max(8, want))
         b["p_logits"] = f32(self.step_rows, b["ld_logits"])
         b["p_argmax_scratch"], b["p_argmax_counters"] = f32(self.step_rows * self.argmax_blocks * 2), i32(self.step_rows + 8)
 

@@ -292,3 +292,23 @@ def test_whole_model_int8_activation_formats(fmt):
         out = eng2.step_tokens(p40[i:i + 8], logits=i + 8 >= 40)
     assert cosine(eng.residual_stream(1)[0].float().cpu(), eng2.residual_stream(8)[7].float().cpu()) > 0.995
     assert eng.launches_per_step() > 0 and 0 <= first < cfg.vocab_size
+
+
+def test_long_prompt_in_one_pass_equals_passes_of_512():
+    """1100 rows in one pass over the layers: the state, the cache and the next tokens are those of three passes."""
+    from mi50grad_b200.config import tiny_config
+    from mi50grad_b200.engine.engine import InferenceEngine
+    from mi50grad_b200.models.weights import random_model
+    cfg = tiny_config()
+    eng = InferenceEngine(cfg, max_seq_len=1200)
+    eng.load_model(random_model(cfg, 4))
+    ids, got = _prompt(cfg, 1100, seed=5), []
+    eng._ensure_driver()
+    assert eng.max_prefill >= 1100 and eng.step_rows <= 512
+    for rows in (eng.max_prefill, 512):
+        eng.max_prefill = rows
+        toks = eng.generate_tokens(ids, 4)
+        got.append((toks, eng.states.dn.S.clone(), eng.states.kv.k[:, 0, :1100].float()))
+    assert got[0][0] == got[1][0]
+    for a, b in zip(got[0][1:], got[1][1:]):
+        assert (a - b).abs().max() <= 2e-2 * b.abs().max()
