@@ -8,51 +8,52 @@
 // instead of host-patched arguments.  Visibility of cache slot s for a row:
 //     s < ctx   or   (s - ctx < 64 and mask bit (s - ctx) set).
 //
-// grid = (kv_heads, rows, splits); a CTA handles every query head of its KV
-// head (GQA), so K/V are read once per group.  Each warp takes batches of cache
-// slots whose rows are all requested before any is used, lanes split the head
-// dimension (HD/32 elements each), scores are reduced with shuffles, and
-// (max, sum, acc) are merged across warps in shared memory and across splits
-// through a scratch buffer by the last CTA to arrive.
+// grid = (kv_heads, rows, splits); a CTA handles every query head of its KV head (GQA), so K/V are read
+// once per group.  Each warp takes 16 cache slots at a time and multiplies them on the tensor cores with the
+// heads as the narrow side: S^T = K Q^T is [16 slots x 8 heads] and O^T += V^T P^T [16 dims x 8 heads] a
+// mma.sync m16n8k16, so up to eight heads cost one column tile and no shuffles but those of the running
+// maximum.  The soft-max weights enter the second product as the sum of two fp16 terms (22 bits); everything
+// else in it is fp16 already, sums are fp32.  (max, sum, O) are merged across warps in shared memory and
+// across splits through a scratch buffer by the last CTA to arrive.
+//
+// Bound: the cache, and with short contexts the latency of one pass.  With dot products on the FMA pipes a
+// slot cost about 180 warp instructions for six heads (here 10), which was the bound.  Measured per layer,
+// 5 sequences of 7000 slots, 4 KV heads of 256, 5 query heads each (143 MB), inside the step: 60 us against 121.
 #include "kernels.cuh"
 
-#define ATT_WARPS 8
+#define ATT_WARPS 4
 #define ATT_THREADS (ATT_WARPS * 32)
 #define ATT_MAX_G 8
-#define ATT_BATCH 8              // cache slots a warp has in flight
-#define ATT_GROUP 4              // slots per soft-max update
-#define ATT_MIN_SPLIT_LEN (ATT_WARPS * ATT_BATCH)      // one pass of one CTA
+#define ATT_SLOTS 16             // cache slots a warp takes at a time
+#define ATT_MIN_SPLIT_LEN (ATT_WARPS * ATT_SLOTS)      // one pass of one CTA
+#define ATT_LDH(HD) ((HD) + 8)   // halfs per staged row: the 16-byte rows of a matrix meet no bank twice
 
-// HD / 32 fp16 values of one cache row held by one lane
-template <int EPL>
-struct KVecT {
-    uint32_t w[EPL / 2];
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int i = 0; i < EPL / 2; ++i) w[i] = 0u;
-    }
-    __device__ __forceinline__ void load(const __half* p) {
-        if constexpr (EPL == 8) { uint4 v = *(const uint4*)p; w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w; }
-        else if constexpr (EPL == 4) { uint2 v = *(const uint2*)p; w[0] = v.x; w[1] = v.y; }
-        else { w[0] = *(const uint32_t*)p; }
-    }
-    __device__ __forceinline__ float get(int e) const {
-        const __half2 h = *(const __half2*)&w[e >> 1];
-        return (e & 1) ? __high2float(h) : __low2float(h);
-    }
-};
+__device__ __forceinline__ void at_ldsm4(uint32_t (&r)[4], const __half* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void at_ldsm4_t(uint32_t (&r)[4], const __half* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ void at_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t at_transpose(uint32_t x) {      // 8 x 8 matrix of 16-bit values over the warp
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(x));
+    return r;
+}
 
-
-// GT: compile-time bound of the query heads per KV head (registers are sized by it).
-template <int HD, int GT>
+template <int HD>
 __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnParams p) {
-    constexpr int EPL = HD / 32;                 // elements per lane
-    using KVec = KVecT<EPL>;
-    constexpr int LB = EPL * 2;                  // bytes of a cache row held by one lane
+    constexpr int LD = ATT_LDH(HD), KS = HD / 16, PPR = HD / 8;
     const int kvh = blockIdx.x, r = blockIdx.y, sp = blockIdx.z;
     pdl_launch_dependents();
     pdl_wait();                                  // Q, and the K/V row of this step, come from the kernels before
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const int G = p.nq / p.nkv;
     const RowMeta rm = p.rows[r];
     const int extra = rm.mask ? 64 - __clzll((long long)rm.mask) : 0;
@@ -64,122 +65,123 @@ __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnPara
     const int s0 = sp * per, s1 = min(total, s0 + per);
 
     __shared__ float sm_m[ATT_WARPS][ATT_MAX_G], sm_l[ATT_WARPS][ATT_MAX_G];
-    // dynamic shared memory: during the walk over the cache a ring of K/V rows per warp
-    // [2 stages][ATT_WARPS][ATT_BATCH][K | V][32 lanes][LB bytes]; afterwards the merge buffer [ATT_WARPS][G][HD]
+    // dynamic shared memory: [ATT_WARPS][K | V][16 slots][LD]; afterwards the merge buffer [ATT_WARPS][G][HD + 8]
     extern __shared__ __align__(16) unsigned char att_smem[];
     float* sm_acc = (float*)att_smem;
-    unsigned char* ring = att_smem + ((size_t)warp * ATT_BATCH * 2 * 32 + lane) * LB;     // this lane's first entry
-    constexpr size_t STAGE_B = (size_t)ATT_WARPS * ATT_BATCH * 2 * 32 * LB;
+    __half* Kw = (__half*)att_smem + (size_t)warp * 2 * ATT_SLOTS * LD;
+    __half* Vw = Kw + ATT_SLOTS * LD;
     __shared__ int s_last;
     __shared__ float sm_f[32][ATT_MAX_G], sm_ls[32][ATT_MAX_G], sm_linv[ATT_MAX_G];
 
-    float q[GT][EPL], acc[GT][EPL], m[GT], l[GT];
-#pragma unroll
-    for (int h = 0; h < GT; ++h) {
-        m[h] = -INFINITY; l[h] = 0.f;
-        KVec qv;
-        qv.zero();
-        if (h < G) qv.load(p.q + (size_t)r * p.ldq + (kvh * G + h) * HD + lane * EPL);
-#pragma unroll
-        for (int e = 0; e < EPL; ++e) { acc[h][e] = 0.f; q[h][e] = qv.get(e) * p.scale; }
-    }
-    const size_t base = ((size_t)rm.seq * p.max_seq) * p.nkv * HD + (size_t)kvh * HD + lane * EPL;
+    // A warp stages its own slots (slot = sb + row), so no barrier is involved; the K rows of its next pass are
+    // requested as soon as the scores are formed, the V rows as soon as the output is.
+    const size_t base = ((size_t)rm.seq * p.max_seq) * p.nkv * HD + (size_t)kvh * HD;
     const size_t stride = (size_t)p.nkv * HD;
-    // A warp takes ATT_BATCH cache slots at a time (slot = sb + i * ATT_WARPS + warp).  Their K and V rows
-    // travel by cp.async into the warp's ring (each lane copies, and later reads back, only its own bytes, so
-    // no barrier is involved), and the rows of the next batch are already on their way while this one is
-    // processed: a pass costs no exposed trip to memory.  The scores of ATT_GROUP slots go through the
-    // soft-max update together.
-    auto issue = [&](int sb, int stage) {
-#pragma unroll
-        for (int i = 0; i < ATT_BATCH; ++i) {
-            const int s = sb + i * ATT_WARPS + warp;
-            if (s < s1) {
-                unsigned char* dst = ring + stage * STAGE_B + (size_t)i * 2 * 32 * LB;
-                const __half* kp = p.kcache + base + (size_t)s * stride;
-                const __half* vp = p.vcache + base + (size_t)s * stride;
-                if constexpr (LB == 16) { cp_async16(dst, kp); cp_async16(dst + 32 * LB, vp); }
-                else if constexpr (LB == 8) { cp_async8(dst, kp); cp_async8(dst + 32 * LB, vp); }
-                else { cp_async4(dst, kp); cp_async4(dst + 32 * LB, vp); }
-            }
+    auto stage = [&](__half* dst, const __half* cache, int sb) {
+#pragma unroll 4
+        for (int i = lane; i < ATT_SLOTS * PPR; i += 32) {
+            const int row = i / PPR, c = i % PPR * 8;
+            if (sb + row < s1) cp_async16(dst + row * LD + c, cache + base + (size_t)(sb + row) * stride + c);
+            else *(uint4*)(dst + row * LD + c) = make_uint4(0u, 0u, 0u, 0u);
         }
-        cp_async_commit();
     };
-    constexpr int PASS = ATT_WARPS * ATT_BATCH;
-    if (s0 < s1) issue(s0, 0);
-    int stage = 0;
-    for (int sb = s0; sb < s1; sb += PASS, stage ^= 1) {
-        if (sb + PASS < s1) { issue(sb + PASS, stage ^ 1); cp_async_wait<1>(); }
-        else cp_async_wait<0>();
-#pragma unroll 1
-        for (int g0 = 0; g0 < ATT_BATCH; g0 += ATT_GROUP) {
-            if (sb + g0 * ATT_WARPS + warp >= s1) break;       // uniform per warp: slots grow with i
-            const unsigned char* src = ring + stage * STAGE_B + (size_t)g0 * 2 * 32 * LB;
-            float d[ATT_GROUP][GT];
-            bool vis[ATT_GROUP];
+    int sb = s0 + warp * ATT_SLOTS;
+    stage(Kw, p.kcache, sb);
+    cp_async_commit();
+    stage(Vw, p.vcache, sb);
+    cp_async_commit();
+    // Q as B operand: head g of the group, dims 16 k + 2 t (+ 8)
+    uint32_t qf[KS][2];
+    {
+        const __half* q = p.q + (size_t)r * p.ldq + (size_t)(kvh * G + min(g, G - 1)) * HD + 2 * t;
 #pragma unroll
-            for (int i = 0; i < ATT_GROUP; ++i) {
-                const int s = sb + (g0 + i) * ATT_WARPS + warp;
-                vis[i] = s < s1 && (s < rm.ctx || ((rm.mask >> (s - rm.ctx)) & 1ull));
-                KVec kk;
-                kk.zero();
-                if (s < s1) kk.load((const __half*)(src + (size_t)i * 2 * 32 * LB));
-                float kf[EPL];
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) kf[e] = kk.get(e);
-#pragma unroll
-                for (int h = 0; h < GT; ++h) {
-                    float x = 0.f;
-#pragma unroll
-                    for (int e = 0; e < EPL; ++e) x = fmaf(q[h][e], kf[e], x);
-                    d[i][h] = x;
-                }
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-                for (int i = 0; i < ATT_GROUP; ++i)
-#pragma unroll
-                    for (int h = 0; h < GT; ++h) d[i][h] += __shfl_xor_sync(0xffffffffu, d[i][h], o);
-            float vf[ATT_GROUP][EPL];
-#pragma unroll
-            for (int i = 0; i < ATT_GROUP; ++i) {
-                KVec vv;
-                vv.zero();
-                if (sb + (g0 + i) * ATT_WARPS + warp < s1) vv.load((const __half*)(src + ((size_t)i * 2 + 1) * 32 * LB));
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) vf[i][e] = vv.get(e);
-            }
-#pragma unroll
-            for (int h = 0; h < GT; ++h) {
-                float mn = m[h];
-#pragma unroll
-                for (int i = 0; i < ATT_GROUP; ++i) if (vis[i]) mn = fmaxf(mn, d[i][h]);
-                if (mn == -INFINITY) continue;                 // nothing visible so far
-                const float corr = __expf(m[h] - mn);          // exp(-inf) = 0 on the first visible slot
-                float pw[ATT_GROUP], ps = 0.f;
-#pragma unroll
-                for (int i = 0; i < ATT_GROUP; ++i) { pw[i] = vis[i] ? __expf(d[i][h] - mn) : 0.f; ps += pw[i]; }
-                l[h] = l[h] * corr + ps;
-#pragma unroll
-                for (int e = 0; e < EPL; ++e) {
-                    float a = acc[h][e] * corr;
-#pragma unroll
-                    for (int i = 0; i < ATT_GROUP; ++i) a = fmaf(pw[i], vf[i][e], a);
-                    acc[h][e] = a;
-                }
-                m[h] = mn;
-            }
+        for (int k = 0; k < KS; ++k) {
+            qf[k][0] = g < G ? *(const uint32_t*)(q + 16 * k) : 0u;
+            qf[k][1] = g < G ? *(const uint32_t*)(q + 16 * k + 8) : 0u;
         }
     }
+    const __half* ka = Kw + (lane & 15) * LD + (lane >> 4) * 8;                                  // slots x dims
+    const __half* va = Vw + ((lane & 7) + (lane >> 4) * 8) * LD + ((lane >> 3) & 1) * 8;         // its transpose: dims x slots
+    const float sc = p.scale * 1.44269504f;                      // scores are kept in the log2 domain
+    float o[KS][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};      // o: dims 16 k + g (+ 8), heads 2 t and 2 t + 1
+#pragma unroll
+    for (int k = 0; k < KS; ++k) o[k][0] = o[k][1] = o[k][2] = o[k][3] = 0.f;
+    for (; sb < s1; sb += ATT_MIN_SPLIT_LEN) {
+        const bool more = sb + ATT_MIN_SPLIT_LEN < s1;
+        cp_async_wait<1>();
+        __syncwarp();
+        float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};    // two chains: even and odd k steps
+#pragma unroll
+        for (int k = 0; k < KS; k += 2) {
+            uint32_t a[4], b[4];
+            at_ldsm4(a, ka + 16 * k);
+            at_ldsm4(b, ka + 16 * k + 16);
+            at_mma(s, a, qf[k][0], qf[k][1]);
+            at_mma(s2, b, qf[k + 1][0], qf[k + 1][1]);
+        }
+        __syncwarp();
+        if (more) stage(Kw, p.kcache, sb + ATT_MIN_SPLIT_LEN);
+        cp_async_commit();
+        // slots g, g + 8 (index e >> 1) and heads 2 t, 2 t + 1 (e & 1)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int slot = sb + g + 8 * (e >> 1), d = slot - rm.ctx;
+            const bool vis = slot < s1 && (d < 0 || ((rm.mask >> d) & 1ull));
+            s[e] = vis ? (s[e] + s2[e]) * sc : -INFINITY;
+        }
+        float pw[4];
+        float cor[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float mx = fmaxf(s[h], s[2 + h]);
+#pragma unroll
+            for (int x = 4; x < 32; x <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, x));
+            const float mn = fmaxf(m[h], mx), ref = mn == -INFINITY ? 0.f : mn;
+            cor[h] = exp2f(m[h] - ref);                          // exp2(-inf) = 0 on the first visible slot
+            m[h] = mn;
+            pw[h] = exp2f(s[h] - ref);
+            pw[2 + h] = exp2f(s[2 + h] - ref);
+            l[h] = l[h] * cor[h] + pw[h] + pw[2 + h];
+        }
+        if (__any_sync(0xffffffffu, cor[0] != 1.f || cor[1] != 1.f)) {
+#pragma unroll
+            for (int k = 0; k < KS; ++k) { o[k][0] *= cor[0]; o[k][1] *= cor[1]; o[k][2] *= cor[0]; o[k][3] *= cor[1]; }
+        }
+        uint32_t ph[2], pl[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const __half2 hi = __floats2half2_rn(pw[2 * i], pw[2 * i + 1]);
+            const float2 f = __half22float2(hi);
+            const __half2 lo = __floats2half2_rn(pw[2 * i] - f.x, pw[2 * i + 1] - f.y);
+            ph[i] = at_transpose(*(const uint32_t*)&hi);
+            pl[i] = at_transpose(*(const uint32_t*)&lo);
+        }
+        cp_async_wait<1>();
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < KS; ++k) {
+            uint32_t v[4];
+            at_ldsm4_t(v, va + 16 * k);
+            at_mma(o[k], v, pl[0], pl[1]);
+            at_mma(o[k], v, ph[0], ph[1]);
+        }
+        __syncwarp();
+        if (more) stage(Vw, p.vcache, sb + ATT_MIN_SPLIT_LEN);
+        cp_async_commit();
+    }
+    cp_async_wait<0>();
     __syncthreads();                             // every warp is done with its ring: the merge buffer reuses it
     // ---- merge the warps of this CTA
+    constexpr int LDO = HD + 8;
 #pragma unroll
-    for (int h = 0; h < GT; ++h) {
-        if (h < G) {
-            if (lane == 0) { sm_m[warp][h] = m[h]; sm_l[warp][h] = l[h]; }
+    for (int h = 0; h < 2; ++h) {
 #pragma unroll
-            for (int e = 0; e < EPL; ++e) sm_acc[((size_t)warp * G + h) * HD + lane * EPL + e] = acc[h][e];
+        for (int x = 4; x < 32; x <<= 1) l[h] += __shfl_xor_sync(0xffffffffu, l[h], x);
+        if (2 * t + h < G) {
+            if (g == 0) { sm_m[warp][2 * t + h] = m[h]; sm_l[warp][2 * t + h] = l[h]; }
+            float* d = sm_acc + ((size_t)warp * G + 2 * t + h) * LDO + g;
+#pragma unroll
+            for (int k = 0; k < KS; ++k) { d[16 * k] = o[k][h]; d[16 * k + 8] = o[k][2 + h]; }
         }
     }
     __syncthreads();
@@ -194,9 +196,9 @@ __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnPara
         float ll = 0.f, a = 0.f;
 #pragma unroll
         for (int w = 0; w < ATT_WARPS; ++w) {
-            float f = (sm_m[w][h] == -INFINITY) ? 0.f : __expf(sm_m[w][h] - mm);
+            float f = (sm_m[w][h] == -INFINITY) ? 0.f : exp2f(sm_m[w][h] - mm);
             ll += sm_l[w][h] * f;
-            a += sm_acc[((size_t)w * G + h) * HD + d] * f;
+            a += sm_acc[((size_t)w * G + h) * LDO + d] * f;
         }
         if (nsplit == 1) {
             float o = ll > 0.f ? a / ll : 0.f;
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnPara
         for (int s = 0; s < nsplit; ++s) mm = fmaxf(mm, sm_f[s][tid]);
         float ll = 0.f;
         for (int s = 0; s < nsplit; ++s) {
-            float f = (sm_f[s][tid] == -INFINITY) ? 0.f : __expf(sm_f[s][tid] - mm);
+            float f = (sm_f[s][tid] == -INFINITY) ? 0.f : exp2f(sm_f[s][tid] - mm);
             ll += sm_ls[s][tid] * f;
             sm_f[s][tid] = f;
         }
@@ -272,32 +274,22 @@ __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnPara
     }
 }
 
-template <int HD, int GT>
+template <int HD>
 static int launch_decode_attn(const AttnParams* p, cudaStream_t s) {
     dim3 grid(p->nkv, p->n_rows, p->splits);
-    const size_t ring = (size_t)2 * ATT_WARPS * ATT_BATCH * 2 * HD * sizeof(__half);
-    const size_t merge = (size_t)ATT_WARPS * (p->nq / p->nkv) * HD * sizeof(float);
+    const size_t ring = (size_t)ATT_WARPS * 2 * ATT_SLOTS * ATT_LDH(HD) * sizeof(__half);
+    const size_t merge = (size_t)ATT_WARPS * (p->nq / p->nkv) * (HD + 8) * sizeof(float);
     const size_t smem = ring > merge ? ring : merge;
     static SmemOptIn opt;
-    if (int e = opt.ensure((const void*)decode_attn_kernel<HD, GT>, smem)) return e;
-    return launch_pdl(decode_attn_kernel<HD, GT>, grid, dim3(ATT_THREADS), smem, s, *p);
-}
-template <int HD>
-static int launch_decode_attn_g(const AttnParams* p, int G, cudaStream_t s) {
-    if (G <= 1) return launch_decode_attn<HD, 1>(p, s);
-    if (G <= 2) return launch_decode_attn<HD, 2>(p, s);
-    if (G <= 3) return launch_decode_attn<HD, 3>(p, s);
-    if (G <= 4) return launch_decode_attn<HD, 4>(p, s);
-    if (G <= 6) return launch_decode_attn<HD, 6>(p, s);
-    return launch_decode_attn<HD, 8>(p, s);
+    if (int e = opt.ensure((const void*)decode_attn_kernel<HD>, smem)) return e;
+    return launch_pdl(decode_attn_kernel<HD>, grid, dim3(ATT_THREADS), smem, s, *p);
 }
 
 B2_API int b2_decode_attn(const AttnParams* p, int hd, cudaStream_t s) {
     if (p->nq % p->nkv || p->nq / p->nkv > ATT_MAX_G || p->splits < 1 || p->splits > 32) return cudaErrorInvalidValue;
-    const int G = p->nq / p->nkv;
-    if (hd == 256) return launch_decode_attn_g<256>(p, G, s);
-    if (hd == 128) return launch_decode_attn_g<128>(p, G, s);
-    if (hd == 64) return launch_decode_attn_g<64>(p, G, s);
+    if (hd == 256) return launch_decode_attn<256>(p, s);
+    if (hd == 128) return launch_decode_attn<128>(p, s);
+    if (hd == 64) return launch_decode_attn<64>(p, s);
     return cudaErrorInvalidValue;
 }
 B2_API int b2_sizeof_attn_params() { return (int)sizeof(AttnParams); }

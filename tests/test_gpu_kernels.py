@@ -262,6 +262,25 @@ def test_deltanet_scan_in_parts_equals_one_kernel(K, dk, nk, nv, rows):
     assert torch.equal(got[1][2], got[0][2])
 
 
+@pytest.mark.parametrize("hd,nq,nkv,splits", [(256, 8, 1, 1), (256, 5, 5, 4), (128, 14, 2, 32), (64, 8, 8, 2)])
+def test_decode_attn_slot_edges(K, hd, nq, nkv, splits):
+    """Contexts around the 16 slots of a warp's pass and the 64 of a CTA's, one to eight heads a group, masks with holes,
+    a score far above the others (its weight is one, the rest vanish in the second fp16 term as well)."""
+    from mi50grad_b200.models import oracle as O
+    gen = torch.Generator().manual_seed(18)
+    d = _dev()
+    ctxs = [0, 1, 15, 16, 17, 48, 63, 64, 65, 127, 129, 500]
+    kc, vc = torch.randn(2, 600, nkv, hd, generator=gen).half(), torch.randn(2, 600, nkv, hd, generator=gen).half()
+    kc[1, 40] *= 6
+    entries = [(i & 1, c, c, c, (1, 0b1011, 1 << 20 | 1)[i % 3]) for i, c in enumerate(ctxs)]
+    q = torch.randn(len(entries), nq * hd, generator=gen).half()
+    out = K.decode_attn(q.to(d), K.make_rows(entries, d), kc.to(d), vc.to(d), nq, nkv, hd, splits=splits)
+    for r, (s, _, _, ctx, mask) in enumerate(entries):
+        vis = list(range(ctx)) + [ctx + j for j in range(64) if (mask >> j) & 1]
+        o = O.attention(q[r:r + 1].float().view(1, nq, hd), kc[s, vis].float(), vc[s, vis].float(), torch.ones(1, len(vis), dtype=torch.bool))
+        assert _rel(out[r].cpu().view(nq, hd), o[0]) < 3e-3, f"row {r}"
+
+
 @pytest.mark.parametrize("hd,nq,nkv,splits", [(256, 6, 1, 1), (256, 24, 4, 3), (64, 4, 2, 1), (64, 6, 2, 4)])
 def test_attn_rows_tensor_core(K, hd, nq, nkv, splits):
     """Many-row attention: a 40-row causal prompt chunk behind 5 cached tokens (three tiles, the last
