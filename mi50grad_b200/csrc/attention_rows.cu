@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(AR_MAX_WARPS * 32, 1) attn_rows_kernel(const A
     constexpr int LD = HD + AR_PAD;
     constexpr int NT_O = HD / 8;                 // 8-column tiles of the output
     pdl_launch_dependents();
+    pdl_wait();
     int row0, nrows;
     if (!ar_find_tile(seq_rows, n_seqs, blockIdx.x, row0, nrows)) return;
     const int kvh = blockIdx.y, sp = blockIdx.z;
@@ -247,6 +248,7 @@ __global__ void __launch_bounds__(MT * 128, 1) attn_rows_packed_kernel(const Att
                                                                       int n_seqs, int splits, int tile_rows) {
     constexpr int LD = HD + AR_PAD, NT_O = HD / 8, THREADS = MT * 128, PPR = HD / 8;
     pdl_launch_dependents();
+    pdl_wait();
     int row0, nrows;
     if (!ar_find_tile(seq_rows, n_seqs, blockIdx.x, row0, nrows, tile_rows)) return;
     const int kvh = blockIdx.y, sp = blockIdx.z, G = p.nq / p.nkv, units = nrows * G;
@@ -432,6 +434,7 @@ __global__ void __launch_bounds__(MT * 128, 1) attn_rows_packed_kernel(const Att
 template <int HD>
 __global__ void __launch_bounds__(128) attn_rows_merge_kernel(const AttnParams p, int splits) {
     pdl_launch_dependents();
+    pdl_wait();
     const int item = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= p.n_rows * p.nq) return;
     const int row = item / p.nq, head = item % p.nq;
@@ -468,8 +471,7 @@ static int launch_packed(const AttnParams* p, const int* seq_rows, int n_seqs, i
     static SmemOptIn optin;
     if (cudaError_t e = optin.ensure(attn_rows_packed_kernel<HD, MT>, smem)) return e;
     const int tiles = (p->n_rows + tile_rows - 1) / tile_rows + n_seqs;       // upper bound; surplus CTAs exit at once
-    attn_rows_packed_kernel<HD, MT><<<dim3(tiles, p->nkv, splits), MT * 128, smem, s>>>(*p, seq_rows, n_seqs, splits, tile_rows);
-    return cudaGetLastError();
+    return launch_pdl(attn_rows_packed_kernel<HD, MT>, dim3(tiles, p->nkv, splits), dim3(MT * 128), smem, s, *p, seq_rows, n_seqs, splits, tile_rows);
 }
 
 template <int HD>
@@ -490,12 +492,10 @@ static int launch_rows(const AttnParams* p, const int* seq_rows, int n_seqs, int
     else {
         const int tiles = (p->n_rows + AR_ROWS - 1) / AR_ROWS + n_seqs;       // upper bound; surplus CTAs exit at once
         dim3 grid(tiles, p->nkv, splits);
-        attn_rows_kernel<HD><<<grid, G * 32, smem, s>>>(*p, seq_rows, n_seqs, splits);
-        e = cudaGetLastError();
+        e = launch_pdl(attn_rows_kernel<HD>, grid, dim3(G * 32), smem, s, *p, seq_rows, n_seqs, splits);
     }
     if (e != cudaSuccess || splits == 1) return e;
-    attn_rows_merge_kernel<HD><<<(p->n_rows * p->nq + 3) / 4, 128, 0, s>>>(*p, splits);
-    return cudaGetLastError();
+    return launch_pdl(attn_rows_merge_kernel<HD>, dim3((p->n_rows * p->nq + 3) / 4), dim3(128), 0, s, *p, splits);
 }
 
 // p->splits: cache slices per tile (1 = none; needs scratch of n_rows * nq * splits * (hd + 2) floats).

@@ -77,6 +77,8 @@ attn_prefill_tc_kernel(const AttnParams p, const __grid_constant__ CUtensorMap q
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_launch_dependents();                      // (not before this CTA has its tensor memory: csrc/gemm_tc.cu)
+    pdl_wait();
     const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + AT_KV;
 
     // this thread's row: lane quarter (warp & 3) of tensor memory, row = 32 * (warp & 3) + lane
@@ -270,8 +272,7 @@ static int launch_attn_prefill_tc(const AttnParams* p, const CUtensorMap& qmap, 
     static SmemOptIn opt;
     if (int e = opt.ensure(attn_prefill_tc_kernel<HD>, smem)) return e;
     dim3 grid((n_rows_seq + AT_ROWS - 1) / AT_ROWS, p->nq);
-    attn_prefill_tc_kernel<HD><<<grid, AT_THREADS, smem, s>>>(*p, qmap, kmap, row_base, n_rows_seq, status);
-    return cudaGetLastError();
+    return launch_pdl(attn_prefill_tc_kernel<HD>, grid, dim3(AT_THREADS), smem, s, *p, qmap, kmap, row_base, n_rows_seq, status);
 }
 
 // Rows [row_base, row_base + n_rows_seq) of the launch belong to one sequence, are in position order and carry

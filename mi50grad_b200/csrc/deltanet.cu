@@ -988,6 +988,8 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_chunk_kernel(const Del
 template <int DK>
 __global__ void __launch_bounds__(2 * DK) deltanet_qk_prep_kernel(const DeltaParams p, __half* __restrict__ qk_pre, int ld_qk,
                                                                   int cb_copies, int nch) {
+    pdl_launch_dependents();
+    pdl_wait();
     const int kh = blockIdx.y, c = threadIdx.x, lane = c & 31, warp = c >> 5;
     const int r0 = p.seq_rows[0], r1 = p.seq_rows[1];
     const int rb = r0 + blockIdx.x * QP_ROWS;
@@ -1073,6 +1075,8 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const Delt
     constexpr int LDK = DC_LDK(DK), LDV = DV + 8;
     constexpr int MB = DC_C / 16;
     extern __shared__ __align__(16) float psm[];
+    pdl_launch_dependents();
+    pdl_wait();
     float* Qs = psm;                          // [C][LDK]
     float* Ks = Qs + DC_C * LDK;
     float* Vs = Ks + DC_C * LDK;              // [C][LDV]
@@ -1255,6 +1259,7 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
     static_assert(DC_C == 32 && DN_COLS == 32 && MT <= 8, "eight warps: two row tiles by four column tiles");
     extern __shared__ __align__(16) float dsm[];
     ScanSmem<DK>& sm = *(ScanSmem<DK>*)dsm;
+    pdl_launch_dependents();
     const int cb = blockIdx.x, j = blockIdx.y, kh = j / (p.nv / p.nk);
     const int tid = threadIdx.x, lane = tid & 31, kr = tid >> 5, g = lane >> 2, t = lane & 3;
     const int r0 = p.seq_rows[0], r1 = p.seq_rows[1];
@@ -1285,8 +1290,6 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
         u0n[0] = *(const float2*)src;
         u0n[1] = *(const float2*)(src + 8 * DV);
     };
-    stage(0);
-    load_u0(0);
     float S[4][4];
     float* sp = p.state + (((size_t)seq * p.nv + j) * DK) * DV + cb * DN_COLS;
     auto put_s0 = [&]() {
@@ -1305,6 +1308,9 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
             S[n][0] = lo.x; S[n][1] = lo.y; S[n][2] = hi.x; S[n][3] = hi.y;
         }
     }
+    pdl_wait();                                   // (the state is older than the kernels before)
+    stage(0);
+    load_u0(0);
     put_s0();
     const int a_row = lane & 15, a_col = (lane >> 4) * 8;                              // fp16 A operand (ldmatrix)
     const int kt_row = (lane & 7) + (lane & 8), kt_col = (lane >> 4) * 8;              // its transpose: chunk rows x state rows
@@ -1403,6 +1409,8 @@ template <int DK, int DV>
 __global__ void __launch_bounds__(DN_THREADS) deltanet_scan_out_kernel(const DeltaParams p, const float* __restrict__ tw, int n_chunks, int row_ctas) {
     typedef ScanBlock<DK, DV> B;
     constexpr int PL = DV / 32;
+    pdl_launch_dependents();
+    pdl_wait();
     const int tid = threadIdx.x, lane = tid & 31;
     const int r0 = p.seq_rows[0], r1 = p.seq_rows[1];
     if (r0 >= r1) return;
@@ -1441,23 +1449,18 @@ static int launch_delta_chunk(const DeltaParams* p, const void* ab, int ld_ab, _
                               float* tw, cudaStream_t s) {
     if (qk_pre) {
         dim3 grid((n_rows + QP_ROWS - 1) / QP_ROWS, p->nk);
-        deltanet_qk_prep_kernel<DK><<<grid, 2 * DK, 0, s>>>(*p, qk_pre, ld_qk, DV / DN_COLS, 2 * DK + DN_COLS);
-        cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+        if (cudaError_t e = launch_pdl(deltanet_qk_prep_kernel<DK>, grid, dim3(2 * DK), 0, s, *p, qk_pre, ld_qk, DV / DN_COLS, 2 * DK + DN_COLS)) return e;
     }
     if (qk_pre && tw) {
         const int n_chunks = (n_rows + DC_C - 1) / DC_C;
         constexpr size_t psm = (size_t)(2 * DC_C * DC_LDK(DK) + DC_C * (DV + 8) + 3 * DC_C * DC_LDA + 3 * DC_C) * sizeof(float);
         static SmemOptIn opt_tw, opt_scan;
         if (cudaError_t e = opt_tw.ensure(deltanet_tw_prep_kernel<DK, DV>, psm)) return e;
-        deltanet_tw_prep_kernel<DK, DV><<<dim3(n_chunks, p->nv), DN_THREADS, psm, s>>>(*p, (const __half*)ab, ld_ab, qk_pre, ld_qk, tw, n_chunks);
-        if (cudaError_t e = cudaGetLastError()) return e;
+        if (cudaError_t e = launch_pdl(deltanet_tw_prep_kernel<DK, DV>, dim3(n_chunks, p->nv), dim3(DN_THREADS), psm, s, *p, (const __half*)ab, ld_ab, qk_pre, ld_qk, tw, n_chunks)) return e;
         if (cudaError_t e = opt_scan.ensure(deltanet_scan_kernel<DK, DV>, sizeof(ScanSmem<DK>))) return e;
-        deltanet_scan_kernel<DK, DV><<<dim3(DV / DN_COLS, p->nv), DN_THREADS, sizeof(ScanSmem<DK>), s>>>(*p, qk_pre, ld_qk, tw, n_chunks);
-        if (cudaError_t e = cudaGetLastError()) return e;
+        if (cudaError_t e = launch_pdl(deltanet_scan_kernel<DK, DV>, dim3(DV / DN_COLS, p->nv), dim3(DN_THREADS), sizeof(ScanSmem<DK>), s, *p, qk_pre, ld_qk, tw, n_chunks)) return e;
         const int row_ctas = (int)(((long long)n_rows * p->nv + DN_THREADS / 32 - 1) / (DN_THREADS / 32));
-        deltanet_scan_out_kernel<DK, DV><<<row_ctas + p->nv * (DV / DN_COLS), DN_THREADS, 0, s>>>(*p, tw, n_chunks, row_ctas);
-        return cudaGetLastError();
+        return launch_pdl(deltanet_scan_out_kernel<DK, DV>, dim3(row_ctas + p->nv * (DV / DN_COLS)), dim3(DN_THREADS), 0, s, *p, tw, n_chunks, row_ctas);
     }
     constexpr int CB = DV / DN_COLS;
     constexpr int NCH = 2 * DK + DN_COLS;
@@ -1524,6 +1527,7 @@ __global__ void __launch_bounds__(AB_WARPS * 32) ab_proj_kernel(const __half* __
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     uint4* ring = ab_smem + warp * (AB_RING * AB_ITEMS * 32) + lane;
+    pdl_wait();
     const int r0 = blockIdx.x * AB_TOK, o0 = blockIdx.y * AB_OUT;
     const __half* xr[2];
     const __half* wr[AB_OUT / 8];
@@ -1593,7 +1597,6 @@ B2_API int b2_ab_proj(const void* x, int ldx, const void* wa, const void* wb, in
     constexpr size_t smem = (size_t)AB_WARPS * AB_RING * AB_ITEMS * 32 * 16;
     static SmemOptIn optin;
     if (cudaError_t e = optin.ensure(ab_proj_kernel, smem)) return e;
-    ab_proj_kernel<<<dim3((rows + AB_TOK - 1) / AB_TOK, (2 * nv + AB_OUT - 1) / AB_OUT), AB_WARPS * 32, smem, s>>>(
-        (const __half*)x, ldx, (const __half*)wa, (const __half*)wb, nv, H, (__half*)ab, ld_ab, rows);
-    return cudaGetLastError();
+    return launch_pdl(ab_proj_kernel, dim3((rows + AB_TOK - 1) / AB_TOK, (2 * nv + AB_OUT - 1) / AB_OUT), dim3(AB_WARPS * 32), smem, s,
+                      (const __half*)x, ldx, (const __half*)wa, (const __half*)wb, nv, H, (__half*)ab, ld_ab, rows);
 }

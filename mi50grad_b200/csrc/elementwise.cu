@@ -19,7 +19,7 @@
 // no earlier step used from it (csrc/gemv.cu, tagged split-K hand-off).
 __global__ void prepare_rows_kernel(const RowMeta* __restrict__ tmpl, const SeqState* __restrict__ seqs,
                                     RowMeta* __restrict__ rows, int n, unsigned int* step_word) {
-    pdl_launch_dependents();
+    // (no early start for what follows: kernels of a step read `rows` before they wait for the kernel before them)
     if (step_word && blockIdx.x == 0 && threadIdx.x == 0) *step_word += 1024u;
     int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n) return;
@@ -126,6 +126,8 @@ __global__ void add_rmsnorm_kernel(float* __restrict__ h, const float* __restric
                                    const __half* __restrict__ delta16, const __half* __restrict__ w,
                                    __half* __restrict__ xn, float* __restrict__ xn32, int H, float eps) {
     __shared__ float red[32];
+    pdl_launch_dependents();
+    pdl_wait();
     int r = blockIdx.x;
     float* hr = h + (size_t)r * H;
     float ss = 0.f;
@@ -150,6 +152,7 @@ __global__ void __launch_bounds__(256) add_rmsnorm_vec_kernel(float* __restrict_
                                                               float* __restrict__ xn32, int H, float eps) {
     __shared__ float red[32];
     pdl_launch_dependents();
+    pdl_wait();
     const int r = blockIdx.x, n4 = H >> 2;
     float4* hr = (float4*)(h + (size_t)r * H);
     float4 v[8];
@@ -190,13 +193,9 @@ __global__ void __launch_bounds__(256) add_rmsnorm_vec_kernel(float* __restrict_
 B2_API int b2_add_rmsnorm(float* h, const float* delta32, const void* delta16, const void* w, void* xn,
                           float* xn32, int n_rows, int H, float eps, cudaStream_t s) {
     if (H % 4 == 0 && H <= 8192) {
-        add_rmsnorm_vec_kernel<<<n_rows, 256, 0, s>>>(h, delta32, (const __half*)delta16, (const __half*)w,
-                                                      (__half*)xn, xn32, H, eps);
-        return cudaGetLastError();
+        return launch_pdl(add_rmsnorm_vec_kernel, dim3(n_rows), dim3(256), 0, s, h, delta32, (const __half*)delta16, (const __half*)w, (__half*)xn, xn32, H, eps);
     }
-    add_rmsnorm_kernel<<<n_rows, 256, 0, s>>>(h, delta32, (const __half*)delta16, (const __half*)w,
-                                              (__half*)xn, xn32, H, eps);
-    return cudaGetLastError();
+    return launch_pdl(add_rmsnorm_kernel, dim3(n_rows), dim3(256), 0, s, h, delta32, (const __half*)delta16, (const __half*)w, (__half*)xn, xn32, H, eps);
 }
 
 // ---------------------------------------------------------------------------

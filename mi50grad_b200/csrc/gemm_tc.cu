@@ -40,8 +40,7 @@
 #define TC_BK 64                 // k per stage (128 bytes of fp16: one swizzle row)
 #define TC_BM 128                // outputs per CTA (MMA M)
 #define TC_A_BYTES (TC_BM * TC_BK * 2)
-#define TC_RING_OF(pair) ((pair) ? 2 : 3)     // own k-blocks of packed weights + scales in flight per producer thread (cp.async);
-                                              // CTA pairs trade one for two more pipeline stages (their token stages are half as large)
+#define TC_RING 4                // own k-blocks of packed weights in flight per producer thread (cp.async)
 
 // ---------------------------------------------------------------------------
 // Kernel
@@ -55,6 +54,11 @@ __device__ __forceinline__ uint32_t tc_nib_hi(uint32_t w) {
     uint32_t r;
     asm("lop3.b32 %0, %1, 0x00f000f0, 0x64006400, 0xea;" : "=r"(r) : "r"(w));
     return r;
+}
+
+// four 8 x 8 matrices of 16-bit values: lane l gives the address of row l & 7 of matrix l >> 3
+__device__ __forceinline__ void tc_stmatrix4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" :: "r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }
 
 // 16-bit output element in the operand type of the launch
@@ -90,7 +94,6 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
     // M = 256 over the two SMs: each CTA dequantises its own 128 weight rows and loads only ITS half of every
     // 256-token operand tile, so the shared-memory traffic of the token operand per SM halves
     constexpr bool pair = PAIR;
-    constexpr int TC_RING = TC_RING_OF(PAIR);
     uint32_t crank = 0u;
     if constexpr (PAIR) crank = cluster_ctarank();
     const int MH = p.m_halves == 2 ? 2 : 1;
@@ -105,7 +108,7 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
     uint64_t* peer_full = bars + 2 * S + 1;   // [S] pair mode, leader CTA: the peer's operands of the stage are in place
     uint32_t* tmem_slot = (uint32_t*)(bars + 3 * S + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
-    uint4* wring = (uint4*)(((uintptr_t)(tmem_slot + 2) + 15) & ~(uintptr_t)15);   // [TC_RING][2][512 producer threads]: 16 B of nibbles, 2 x 8 B scale/zero
+    uint4* wring = (uint4*)(((uintptr_t)(tmem_slot + 2) + 15) & ~(uintptr_t)15);   // [TC_RING][512 producer threads]: 16 B of nibbles
 
     int tmem_cols = 32;
     while (tmem_cols < Tm) tmem_cols <<= 1;
@@ -134,6 +137,12 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // Programmatic launch: the next kernel may start once every CTA of this one has its tensor memory (a CTA of the next
+    // that took it first would wait for this kernel while this one waited for it).  This one starts likewise while the kernel
+    // before it ends: barriers, tensor memory and the first stages' weights, which nothing in a step writes, are ready when
+    // the activations are; only the TMA warp and the epilogue wait for them.  (Decode
+    // of 24 sequences at width 2048, 98 launches a token: 1.12 -> 1.00 ms.)
+    pdl_launch_dependents();
     // split-K: this CTA's k-blocks are [kb_lo, kb_lo + KB) of the p.KB blocks of the matrix
     const int per_kb = (p.KB + (int)gridDim.z - 1) / (int)gridDim.z;
     const int kb_lo = (int)blockIdx.z * per_kb;
@@ -145,7 +154,7 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
     if (warp < TC_PRODUCERS) {
         // ================= weight producers =================
         // warp w owns the 16-row tile w of the CTA's 128 outputs: one 16-byte load per k-block and lane
-        const int g = lane >> 2, t = lane & 3;
+        const int g = lane >> 2;
         // MH = 1: two groups of 8 warps take alternate k-blocks; MH = 2: one group of 16 takes every k-block
         const int grp = MH == 2 ? 0 : warp >> 3, w8 = MH == 2 ? warp : warp & 7;
         const int kstep = MH == 2 ? 1 : 2;
@@ -154,43 +163,51 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
         const bool dense = p.dense != 0;          // fp16 weights arrive by TMA: nothing to dequantise
         const __half2 sixteenth = __float2half2_rn(0.0625f);
         const __half2 k1024 = __float2half2_rn(1024.f), k64 = __float2half2_rn(64.f);
-        // swizzled byte offsets of this lane's stores: row & 7 == g for both of its rows
-        const uint32_t row_lo_off = (uint32_t)(w8 * 16 + g) * 128 + t * 4;
-        uint32_t sw[8];
-#pragma unroll
-        for (int c8 = 0; c8 < 8; ++c8) sw[c8] = (uint32_t)((c8 ^ g) << 4);
-        // packed weights and their scale/zero pairs stream through a cp.async ring: TC_RING-1 of
-        // the group's k-blocks are always in flight, each thread later reads back only what it copied
+        // A lane's fragments are those of 8 x 8 matrices (row g, columns 2 t and 2 t + 1), so four of them, the 32 k of a
+        // row block, leave in one stmatrix, for which lane l gives the swizzled address of row l & 7 of matrix l >> 3.
+        const uint32_t st_off = (uint32_t)(w8 * 16 + (lane & 7)) * 128 + (uint32_t)(((lane >> 3) ^ (lane & 7)) << 4);
+        // packed weights stream through a cp.async ring: TC_RING-1 of the group's k-blocks are always in flight, each
+        // thread later reads back only what it copied.  Their scales and zeros are requested one k-block ahead into
+        // registers (and four ahead into L2): in the ring they would take as much room as the nibbles, and pipeline stages
+        // need it more.  Measured, K = 5120, one wave of 256-output tiles, us a k-block: .91 -> .78 at 80 tokens, 1.18 -> 1.06
+        // at 256; 128-output tiles .84 -> .68 at 256 (four stages instead of two).
         uint4* my_ring = wring + tid;
         const uint4* gq = dense ? nullptr : p.qfrag + ((size_t)wt * p.KB * 4 + ti) * 32 + lane + (size_t)(kb_lo + grp) * 128;
         const uint2* gs = dense ? nullptr : p.szfrag + ((size_t)wt * p.G * 4 + ti) * 8 + g;
         const uint32_t gq_step = 128u * kstep;
         const int c_step = 2 * kstep;
-        int c_issue = p.off32 + 2 * (kb_lo + grp);          // 32-k chunk counter of the next k-block to issue
+        int c_sz = p.off32 + 2 * (kb_lo + grp);             // 32-k chunk counter of the next k-block whose scales are loaded
         int slot_issue = 0;
         auto issue = [&]() {
-            uint4* dst = my_ring + slot_issue * 1024;
-            cp_async16(dst, gq);
-            cp_async8((uint2*)(dst + 512), gs + (size_t)(c_issue >> p.gshift) * 32);
-            cp_async8((uint2*)(dst + 512) + 1, gs + (size_t)((c_issue + 1) >> p.gshift) * 32);
-            gq += gq_step; c_issue += c_step;
+            cp_async16(my_ring + slot_issue * (TC_PRODUCERS * 32), gq);
+            gq += gq_step;
             slot_issue = slot_issue == TC_RING - 1 ? 0 : slot_issue + 1;
+        };
+        uint2 sz_next[2] = {};
+        auto load_sz = [&]() {
+            sz_next[0] = __ldg(gs + (size_t)(c_sz >> p.gshift) * 32);
+            sz_next[1] = __ldg(gs + (size_t)((c_sz + 1) >> p.gshift) * 32);
+            asm volatile("prefetch.global.L2 [%0];" :: "l"(gs + (size_t)min((c_sz + 4 * c_step) >> p.gshift, p.G - 1) * 32));
+            c_sz += c_step;
         };
 #pragma unroll
         for (int i = 0; i < TC_RING - 1; ++i) {
             if (grp + kstep * i < KB && !dense) issue();
             cp_async_commit();
         }
+        if (grp < KB && !dense) load_sz();
         bool ok = true;
         int st = grp, slot = 0;
         uint32_t ph = 0;
-        unsigned char* a_stage = sA + (size_t)grp * a_bytes + row_lo_off;
+        const uint32_t a_first = smem_u32(sA) + st_off;
+        uint32_t a_stage = a_first + (uint32_t)(grp * a_bytes);
         for (int kb = grp; kb < KB && !dense; kb += kstep) {
             if (kb + kstep * (TC_RING - 1) < KB) issue();
             cp_async_commit();
             cp_async_wait<TC_RING - 1>();
-            const uint4 wv = my_ring[slot * 1024];
-            const uint4 szq = my_ring[slot * 1024 + 512];
+            const uint4 wv = my_ring[slot * (TC_PRODUCERS * 32)];
+            const uint2 szc[2] = {sz_next[0], sz_next[1]};
+            if (kb + kstep < KB) load_sz();
             slot = slot == TC_RING - 1 ? 0 : slot + 1;
             {   // one lane polls: many pollers on one barrier slow the arrivals down
                 int o = 1;
@@ -198,11 +215,9 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
                 ok = __shfl_sync(0xffffffffu, o, 0) != 0;
             }
             if (!ok) break;
-            unsigned char* a_lo = a_stage;
-            unsigned char* a_hi = a_stage + 8 * 128;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
-                const uint2 sz = j ? make_uint2(szq.z, szq.w) : make_uint2(szq.x, szq.y);
+                const uint2 sz = szc[j];
                 const __half2 s2 = *(const __half2*)&sz.x, z2 = *(const __half2*)&sz.y;
                 const __half2 s_lo = __half2half2(__low2half(s2)), s_hi = __half2half2(__high2half(s2));
                 const __half2 z_lo = __half2half2(__low2half(z2)), z_hi = __half2half2(__high2half(z2));
@@ -211,27 +226,25 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
                 const uint32_t w0 = j ? wv.z : wv.x, w1 = j ? wv.w : wv.y;
                 auto deq_lo = [&](uint32_t x, __half2 c, __half2 sc) {
                     uint32_t r = tc_nib_lo(x);
-                    return __hmul2(__hsub2(*(__half2*)&r, c), sc);
+                    const __half2 v = __hmul2(__hsub2(*(__half2*)&r, c), sc);
+                    return *(const uint32_t*)&v;
                 };
                 auto deq_hi = [&](uint32_t x, __half2 c, __half2 sc) {
                     uint32_t r = tc_nib_hi(x);
-                    return __hmul2(__hfma2(*(__half2*)&r, sixteenth, c), sc);
+                    const __half2 v = __hmul2(__hfma2(*(__half2*)&r, sixteenth, c), sc);
+                    return *(const uint32_t*)&v;
                 };
-                // k = 32 j + 8 m + 2 t: the 16-byte column group is 4 j + m
-                *(__half2*)(a_lo + sw[4 * j + 0]) = deq_lo(w0, cl_lo, s_lo);
-                *(__half2*)(a_hi + sw[4 * j + 0]) = deq_lo(w0 >> 8, cl_hi, s_hi);
-                *(__half2*)(a_lo + sw[4 * j + 2]) = deq_hi(w0, ch_lo, s_lo);
-                *(__half2*)(a_hi + sw[4 * j + 2]) = deq_hi(w0 >> 8, ch_hi, s_hi);
-                *(__half2*)(a_lo + sw[4 * j + 1]) = deq_lo(w1, cl_lo, s_lo);
-                *(__half2*)(a_hi + sw[4 * j + 1]) = deq_lo(w1 >> 8, cl_hi, s_hi);
-                *(__half2*)(a_lo + sw[4 * j + 3]) = deq_hi(w1, ch_lo, s_lo);
-                *(__half2*)(a_hi + sw[4 * j + 3]) = deq_hi(w1 >> 8, ch_hi, s_hi);
+                // k = 32 j + 8 m + 2 t: matrix m, the 16-byte column group 4 j + m
+                const uint32_t a = a_stage ^ (uint32_t)(j << 6);
+                tc_stmatrix4(a, deq_lo(w0, cl_lo, s_lo), deq_lo(w1, cl_lo, s_lo), deq_hi(w0, ch_lo, s_lo), deq_hi(w1, ch_lo, s_lo));
+                tc_stmatrix4(a + 8 * 128, deq_lo(w0 >> 8, cl_hi, s_hi), deq_lo(w1 >> 8, cl_hi, s_hi), deq_hi(w0 >> 8, ch_hi, s_hi),
+                             deq_hi(w1 >> 8, ch_hi, s_hi));
             }
             fence_proxy_async_smem();           // generic-proxy stores -> visible to the tensor core
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[st]);
-            st += kstep; a_stage += kstep * a_bytes;  // two groups: S is even, a group keeps to the stages of its parity
-            if (st >= S) { st -= S; ph ^= 1; a_stage = sA + (size_t)st * a_bytes + row_lo_off; }
+            st += kstep; a_stage += (uint32_t)(kstep * a_bytes);  // two groups: S is even, a group keeps to the stages of its parity
+            if (st >= S) { st -= S; ph ^= 1; a_stage = a_first + (uint32_t)(st * a_bytes); }
         }
         cp_async_wait<0>();
         // ================= epilogue =================
@@ -242,6 +255,7 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
             __syncwarp();
         }
         asm volatile("bar.sync 1, %0;" :: "n"(TC_PRODUCERS * 32) : "memory");
+        pdl_wait();
         ok = ok && !*abort_flag;
         tc_fence_after();
         if (ok) {
@@ -328,6 +342,7 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
             // pair mode: of every 256-token operand tile this CTA loads rows [128 crank, 128 crank + 128)
             const uint32_t tx = (pair ? (uint32_t)(Tm / 2) * 128u : (uint32_t)(boxes * box) * 128u) + (dense ? (uint32_t)a_bytes : 0u);
             const int row_w = blockIdx.x * (TC_BM * MH);
+            pdl_wait();
             int st = 0;
             uint32_t ph = 0;
             unsigned char* a = sA;
@@ -432,7 +447,7 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
 B2_API size_t b2_gemm_tc_smem(int t_tile, int stages, int m_halves, int ring) {
     size_t b = (size_t)((t_tile + 63) / 64) * 64 * 128;
     return 1024 + (size_t)stages * ((size_t)(m_halves == 2 ? 2 : 1) * TC_A_BYTES + b) + (3 * stages + 1) * 8 + 16 + 16 +
-           (size_t)ring * 2 * (TC_PRODUCERS * 32) * 16;
+           (size_t)ring * (TC_PRODUCERS * 32) * 16;
 }
 
 // x: [T][ldx] fp16 activations (ldx multiple of 8, base 16-byte aligned).
@@ -480,8 +495,8 @@ static int launch_tc(const GemmTcParams* p, const void* w, int ldw, int n_rows_w
     size_t per_stage = (size_t)q.m_halves * TC_A_BYTES + (size_t)((q.t_tile + 63) / 64) * 64 * 128 / (q.cta_pair ? 2 : 1);
     // as many stages as shared memory holds next to the weight ring, an even number (the two producer
     // groups alternate stages); deep pipelines matter most for few tokens, where a stage is consumed quickly
-    const int ring = q.dense ? 0 : TC_RING_OF(q.cta_pair != 0);      // (dense weights need no ring of packed weights)
-    const size_t fixed = 1024 + 256 + (size_t)ring * 2 * (TC_PRODUCERS * 32) * 16;
+    const int ring = q.dense ? 0 : TC_RING;      // (dense weights need no ring of packed weights)
+    const size_t fixed = 1024 + 256 + (size_t)ring * (TC_PRODUCERS * 32) * 16;
     int stages = (int)((227 * 1024 - fixed) / per_stage);
     stages = stages > 8 ? 8 : stages;
     q.stages = stages < 2 ? 2 : (q.m_halves == 2 || q.dense ? stages : (stages & ~1));
@@ -507,8 +522,7 @@ static int launch_tc(const GemmTcParams* p, const void* w, int ldw, int n_rows_w
         if (cudaError_t e = optin_pair.ensure(gemm_int4_tc_kernel<true>, smem)) return e;
         return cudaLaunchKernelEx(&cfg, gemm_int4_tc_kernel<true>, q, map, wmap);
     }
-    gemm_int4_tc_kernel<false><<<grid, TC_THREADS, smem, stream>>>(q, map, wmap);
-    return cudaGetLastError();
+    return launch_pdl(gemm_int4_tc_kernel<false>, grid, dim3(TC_THREADS), smem, stream, q, map, wmap);
 }
 B2_API int b2_gemm_int4_tc(const GemmTcParams* p, const void* x, int ldx, cudaStream_t stream) {
     return launch_tc(p, nullptr, 0, 0, x, ldx, stream);

@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
     const float4* sp = (const float4*)(p.state + (((size_t)seq * p.nv + j) * DK + rg * RPT) * DV) + c4;
 #pragma unroll
     for (int i = 0; i < RPT; ++i) S[i] = sp[i * (DV / 4)];
+    pdl_wait();                                  // (states and row descriptors are older than the in-projection)
 
     auto chan = [&](int c) -> int {
         if (c < DK) return kh * DK + c;
@@ -296,8 +297,7 @@ static int launch_verify(const DeltaParams* p, const SpecStage* st, int layer, c
     constexpr size_t smem = sizeof(VerifySmem<DK, DV>);
     static SmemOptIn optin;
     if (cudaError_t e = optin.ensure(deltanet_verify_kernel<DK, DV>, smem)) return e;
-    deltanet_verify_kernel<DK, DV><<<dim3(p->nv, p->n_seqs), VF_THREADS, smem, s>>>(*p, *st, layer);
-    return cudaGetLastError();
+    return launch_pdl(deltanet_verify_kernel<DK, DV>, dim3(p->nv, p->n_seqs), dim3(VF_THREADS), smem, s, *p, *st, layer);
 }
 
 B2_API int b2_deltanet_verify(const DeltaParams* p, const SpecStage* st, int layer, int dk, int dv, cudaStream_t s) {
