@@ -245,10 +245,98 @@ __global__ void qknorm_rope_cachew_kernel(__half* __restrict__ qkv, int ld, cons
     if (is_q) src[i] = __float2half(out);
     else kcache[cache_off + (size_t)(hidx - nq) * hd + i] = __float2half(out);
 }
+// The same for heads of 32 EPL elements (64, 128, 256) on 2 EPL-byte boundaries: a warp per (row, head), EPL adjacent
+// elements a lane in one access, the norm without a barrier.  A rotation partner is in the lane (interleaved) or
+// half / EPL lanes away.  The form above, one element a thread and a CTA per head, took 103 us for 3001 rows of 16
+// query and 2 x 4 cache heads of 256, ten times what their bytes take; the prompt of 8 layers at width 4096 is 1.6% shorter.
+template <int EPL> struct RopeVec { uint32_t w[EPL / 2]; };
+template <> struct __align__(4) RopeVec<2> { uint32_t w[1]; };
+template <> struct __align__(8) RopeVec<4> { uint32_t w[2]; };
+template <> struct __align__(16) RopeVec<8> { uint32_t w[4]; };
+template <int EPL>
+__global__ void __launch_bounds__(256) qknorm_rope_cachew_warp_kernel(__half* __restrict__ qkv, int ld, const RowMeta* __restrict__ rows,
+                                                                      const __half* __restrict__ q_norm, const __half* __restrict__ k_norm,
+                                                                      const float* __restrict__ cos_tab, const float* __restrict__ sin_tab,
+                                                                      __half* __restrict__ kcache, __half* __restrict__ vcache, int n_rows,
+                                                                      int nq, int nkv, int rot, int max_seq, int interleaved, float eps) {
+    constexpr int HD = 32 * EPL;
+    typedef RopeVec<EPL> Vec;
+    const int lane = threadIdx.x & 31, item = blockIdx.x * 8 + (threadIdx.x >> 5), heads = nq + 2 * nkv;
+    const int r = item / heads, hidx = item % heads;
+    pdl_launch_dependents();
+    if (r >= n_rows) return;
+    const bool is_q = hidx < nq, is_v = hidx >= nq + nkv;
+    Vec nw = {};
+    if (!is_v) nw = *(const Vec*)((is_q ? q_norm : k_norm) + lane * EPL);
+    pdl_wait();                             // the in-projection's output
+    const RowMeta rm = rows[r];
+    __half* src = qkv + (size_t)r * ld + (is_q ? hidx : nq + hidx) * HD + lane * EPL;      // (the gate lies behind Q)
+    Vec x = *(const Vec*)src;
+    const size_t cache = (((size_t)rm.seq * max_seq + rm.slot) * nkv) * HD + lane * EPL;
+    if (is_v) {
+        *(Vec*)(vcache + cache + (size_t)(hidx - nq - nkv) * HD) = x;
+        return;
+    }
+    float v[EPL], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < EPL; e += 2) {
+        const float2 f = __half22float2(*(const __half2*)&x.w[e / 2]);
+        v[e] = f.x; v[e + 1] = f.y;
+    }
+#pragma unroll
+    for (int e = 0; e < EPL; ++e) ss += v[e] * v[e];
+    const float inv = rsqrtf(warp_sum(ss) / (float)HD + eps);
+#pragma unroll
+    for (int e = 0; e < EPL; e += 2) {
+        const float2 f = __half22float2(*(const __half2*)&nw.w[e / 2]);
+        v[e] = v[e] * inv * f.x; v[e + 1] = v[e + 1] * inv * f.y;
+    }
+    const int half = rot >> 1, i0 = lane * EPL;
+    const float* cr = cos_tab + (size_t)rm.pos * half;
+    const float* sr = sin_tab + (size_t)rm.pos * half;
+    if (interleaved) {
+#pragma unroll
+        for (int e = 0; e < EPL; e += 2)
+            if (i0 + e < rot) {
+                const float c = cr[(i0 + e) >> 1], s = sr[(i0 + e) >> 1], a = v[e], b = v[e + 1];
+                v[e] = a * c - b * s;
+                v[e + 1] = a * s + b * c;
+            }
+    } else {
+        const bool first = i0 < half;
+        const int partner = first ? lane + half / EPL : lane - half / EPL;
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) {
+            const float other = __shfl_sync(0xffffffffu, v[e], partner & 31);
+            if (i0 < rot) {
+                const int pair = first ? i0 + e : i0 + e - half;
+                const float c = cr[pair], s = sr[pair];
+                v[e] = first ? v[e] * c - other * s : other * s + v[e] * c;
+            }
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < EPL; e += 2) {
+        const __half2 h = __floats2half2_rn(v[e], v[e + 1]);
+        x.w[e / 2] = *(const uint32_t*)&h;
+    }
+    *(Vec*)(is_q ? src : kcache + cache + (size_t)(hidx - nq) * HD) = x;
+}
 B2_API int b2_qknorm_rope_cachew(void* qkv, int ld, const void* rows, const void* q_norm, const void* k_norm,
                                  const float* cos_tab, const float* sin_tab, void* kcache, void* vcache,
                                  int n_rows, int nq, int nkv, int hd, int rot, int max_seq, int interleaved,
                                  float eps, cudaStream_t s) {
+    const int epl = hd / 32;
+    const bool warp_form = (hd == 64 || hd == 128 || hd == 256) && ld % epl == 0 && (rot & 1) == 0 && (interleaved || (rot >> 1) % epl == 0) &&
+        !(((uintptr_t)qkv | (uintptr_t)q_norm | (uintptr_t)k_norm | (uintptr_t)kcache | (uintptr_t)vcache) & (2 * epl - 1));
+    if (warp_form) {
+        const dim3 grid((unsigned)(((long long)n_rows * (nq + 2 * nkv) + 7) / 8));
+        auto go = [&](auto kernel) {
+            return launch_pdl(kernel, grid, dim3(256), 0, s, (__half*)qkv, ld, (const RowMeta*)rows, (const __half*)q_norm, (const __half*)k_norm,
+                              cos_tab, sin_tab, (__half*)kcache, (__half*)vcache, n_rows, nq, nkv, rot, max_seq, interleaved, eps);
+        };
+        return hd == 64 ? go(qknorm_rope_cachew_warp_kernel<2>) : (hd == 128 ? go(qknorm_rope_cachew_warp_kernel<4>) : go(qknorm_rope_cachew_warp_kernel<8>));
+    }
     dim3 grid(nq + 2 * nkv, n_rows);
     return launch_pdl(qknorm_rope_cachew_kernel, grid, dim3(hd), hd * sizeof(float), s,
                       (__half*)qkv, ld, (const RowMeta*)rows, (const __half*)q_norm, (const __half*)k_norm, cos_tab, sin_tab,

@@ -175,6 +175,43 @@ def test_add_rmsnorm_and_embed(K):
     assert _rel(xx.cpu(), e * torch.rsqrt(e.pow(2).mean(-1, keepdim=True) + 1e-6) * w.float()) < 2e-3
 
 
+@pytest.mark.parametrize("hd,rot,style,pad", [(256, 256, "half", 0), (64, 4, "half", 0), (128, 2, "interleaved", 0), (64, 0, "interleaved", 0),
+                                              (256, 64, "half", 1), (96, 24, "half", 0), (128, 24, "half", 0), (128, 128, "half", 0)])
+def test_qknorm_rope_cachew_routes(K, hd, rot, style, pad):
+    """What the warp form takes (rotations of all, some and none of the dims) and what it leaves to the other: row strides off
+    the vector, head sizes between, rotation halves that end inside a lane."""
+    from mi50grad_b200.models import oracle as O
+    gen = torch.Generator().manual_seed(19)
+    d = _dev()
+    nq, nkv, rows, max_seq = 3, 1, 5, 16
+    qkv = torch.randn(rows, 2 * nq * hd + 2 * nkv * hd + pad, generator=gen).half()
+    qn, kn = (torch.rand(hd, generator=gen) + 0.5).half(), (torch.rand(hd, generator=gen) + 0.5).half()
+    pos = torch.tensor([3, 0, 15, 7, 1])
+    ang = torch.arange(max_seq)[:, None] * 0.3 ** torch.arange(max(1, rot // 2))
+    cos, sin = torch.cos(ang).float(), torch.sin(ang).float()
+    meta = K.make_rows([(0, int(p), i, 0, 1) for i, p in enumerate(pos)], d)
+    kc = torch.zeros(1, max_seq, nkv, hd, dtype=torch.float16, device=d)
+    vc, buf = torch.zeros_like(kc), qkv.to(d).clone()
+    K.qknorm_rope_cachew(buf, meta, qn.to(d), kn.to(d), cos.to(d), sin.to(d), kc, vc, nq, nkv, hd, rot, interleaved=(style == "interleaved"))
+    n = lambda x, w: O.rmsnorm(x, w, 1e-6)  # noqa: E731
+
+    def turn(x):
+        y, h = x.clone(), rot // 2
+        c, s = cos[pos][:, None, :h], sin[pos][:, None, :h]
+        a, b = (x[..., 0:rot:2], x[..., 1:rot:2]) if style == "interleaved" else (x[..., :h], x[..., h:rot])
+        u, w = a * c - b * s, a * s + b * c
+        if style == "interleaved":
+            y[..., 0:rot:2], y[..., 1:rot:2] = u, w
+        else:
+            y[..., :h], y[..., h:rot] = u, w
+        return y
+    q, k = qkv[:, :nq * hd].float().view(rows, nq, hd), qkv[:, 2 * nq * hd:(2 * nq + nkv) * hd].float().view(rows, nkv, hd)
+    v = qkv[:, (2 * nq + nkv) * hd:(2 * nq + 2 * nkv) * hd].view(rows, nkv, hd)
+    assert _rel(buf[:, :nq * hd].cpu().view(rows, nq, hd), turn(n(q, qn))) < 2e-3
+    assert _rel(kc[0, :rows].cpu(), turn(n(k, kn))) < 2e-3 and torch.equal(vc[0, :rows].cpu(), v)
+    assert torch.equal(buf[:, nq * hd:].cpu(), qkv[:, nq * hd:])
+
+
 @pytest.mark.parametrize("hd,rot,style", [(256, 64, "interleaved"), (64, 16, "interleaved"), (128, 32, "half")])
 def test_qknorm_rope_cachew(K, hd, rot, style):
     from mi50grad_b200.config import QwenConfig
