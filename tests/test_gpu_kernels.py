@@ -318,6 +318,29 @@ def test_decode_attn_slot_edges(K, hd, nq, nkv, splits):
         assert _rel(out[r].cpu().view(nq, hd), o[0]) < 3e-3, f"row {r}"
 
 
+@pytest.mark.parametrize("hd,T,past", [(256, 130, 100), (64, 65, 0), (128, 129, 320), (256, 64, 1)])
+def test_attn_prefill_growing_scores_and_poisoned_slots(K, hd, T, past):
+    """Scores that grow along the cache (the reference maximum moves many times, and stays behind by up to 2^8 between), a
+    sequence that ends inside a tile whose other slots hold NaN, rows that end inside a row tile."""
+    from mi50grad_b200.models import oracle as O
+    gen = torch.Generator().manual_seed(37)
+    d = _dev()
+    n = past + T
+    kc, vc = torch.full((2, n + 70, 1, hd), float("nan")).half(), torch.full((2, n + 70, 1, hd), float("nan")).half()
+    q = torch.randn(T, 2 * hd, generator=gen).half()
+    q[:, :hd] = (q[:, :hd].float() + 0.5).half()
+    kc[0, :n] = (torch.randn(n, 1, hd, generator=gen) + torch.linspace(0, 8, n)[:, None, None] * (64 / hd)).half()
+    vc[0, :n] = torch.randn(n, 1, hd, generator=gen).half()
+    entries = [(0, past + i, past + i, past + i + 1, 0) for i in range(T)]
+    out = K.attn_prefill_tc(q.to(d), K.make_rows(entries, d), kc.to(d), vc.to(d), 2, 1, hd)
+    torch.cuda.synchronize()
+    K.gemm_tc_check_status()
+    for r in list(range(0, T, 5)) + [T - 1]:
+        o = O.attention(q[r:r + 1].float().view(1, 2, hd), kc[0, :past + r + 1].float(), vc[0, :past + r + 1].float(),
+                        torch.ones(1, past + r + 1, dtype=torch.bool))
+        assert _rel(out[r].cpu().view(2, hd), o[0]) < 4e-3, r
+
+
 @pytest.mark.parametrize("hd,nq,nkv,splits", [(256, 6, 1, 1), (256, 24, 4, 3), (64, 4, 2, 1), (64, 6, 2, 4)])
 def test_attn_rows_tensor_core(K, hd, nq, nkv, splits):
     """Many-row attention: a 40-row causal prompt chunk behind 5 cached tokens (three tiles, the last
