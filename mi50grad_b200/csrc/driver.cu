@@ -177,7 +177,6 @@ struct Driver {
                                           // 2 = also the state-independent products and the triangle inverse of every chunk
     bool attn_tc = true;                  // prompt attention on tcgen05 (csrc/attention_tc.cu)
     bool gemm_m256 = true;                // 256-output GEMM tiles where the grid stays large enough
-    int gemm_m256_min_ctas = 100;
     bool gemm_splitk = true;              // split-K in the many-row GEMMs that add into the residual stream
     const void* pf_span = nullptr; long long pf_span_bytes = 0;   // see run_linear
     bool pf_state = false;                // the in-projection of a DeltaNet layer prefetches that layer's state into L2
@@ -529,51 +528,37 @@ static int run_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, int 
     memset(&p, 0, sizeof(p));
     p.qfrag = (const uint4*)L.w; p.szfrag = (const uint2*)L.sz;
     p.K = L.K; p.KB = L.KB; p.NTL = L.NTL; p.G = L.G; p.off32 = L.off32; p.gshift = L.gshift;
-    // tokens per CTA: as many as tensor memory holds, unless that leaves most SMs without a CTA
-    // (N = 5120 gives only 40 output tiles): then split the tokens so that the grid fills, but does
-    // not exceed, one wave of 148 CTAs (one CTA per SM: a second partial wave would double the time)
-    const int ctas_n = L.NTL * 16 / 128;
-    int tt = T >= 512 ? 512 : ((T + 15) & ~15);
-    int ks = 1;
-    if (ctas_n < 148) {
-        int parts = 148 / ctas_n;                          // token tiles that still fit one wave
-        int need = (T + parts - 1) / parts;
-        need = (need + 15) & ~15;
-        if (need < 64) need = 64;
-        if (need < tt) tt = need;
-        if (epi == TC_EPI_RESID_F32 && d->gemm_splitk) {
-            // ... or split K instead (the partial products meet in the residual stream through atomic adds):
-            // a k-block of a CTA costs about max(0.46, 0.0021 x tokens) us, so few wide token tiles over a
-            // third of K beat many narrow ones over all of it.  Pick the cheapest (token tile, splits) pair.
-            double best = 1e30;
-            const int tmax = T >= 512 ? 512 : ((T + 15) & ~15);
-            for (int tiles = 1; tiles <= 8; ++tiles) {
-                int t1 = ((T + tiles - 1) / tiles + 15) & ~15;
-                if (t1 > tmax) continue;
-                if (t1 < 16) t1 = 16;
-                const int nt = (T + t1 - 1) / t1;
-                int s1 = 148 / (ctas_n * nt);
-                if (s1 < 1) continue;
-                if (s1 > L.KB / 8) s1 = L.KB / 8 > 0 ? L.KB / 8 : 1;
-                const double blk = 0.0021 * t1 > 0.46 ? 0.0021 * t1 : 0.46;
-                const double cost = ((L.KB + s1 - 1) / s1) * blk + (s1 > 1 ? 4.0 : 0.0);
-                if (cost < best) { best = cost; tt = t1; ks = s1; }
+    // Token tile, outputs per CTA (128, or 256 as two accumulators that share an activation tile) and K splits (only
+    // where the product is added to the residual stream; the parts meet through atomic adds) with the least time by a
+    // model of one CTA per SM: whole waves of CTAs, each a walk over its k-blocks plus a start and an epilogue, and the
+    // traffic of the atomic adds.  us of a 64-k block, measured with one wave: 128 outputs: .39 at 16 tokens, .47 at 128,
+    // .51 at 192, .58 at 256 (to there four pipeline stages fit, beyond it two), .86 at 320, 1.1 at 512; 256 outputs: .64 at
+    // 16, .71 at 128, .84 at 192, .96 at 256.
+    // (256-output tiles of a residual product with few rows would need so many splits that the adds cost more than they
+    // give: at 80 rows the 27B verification step is 2% slower with them.)  Measured against one wave of the widest
+    // tile that fits: prompt of 512 at 27B 37.4 -> 36.1 ms, of 3001 at width 4096 17.5 -> 16.1 ms, of 77 1.78 -> 1.74 ms.
+    auto block_us = [](int t, bool wide) -> double {
+        if (wide) return t <= 128 ? 0.625 + 0.00065 * t : 0.47 + 0.0019 * t;
+        return t <= 192 ? 0.375 + 0.0007 * t : (t <= 256 ? 0.30 + 0.0011 * t : 0.46 + 0.00125 * t);
+    };
+    const bool wide_ok = d->gemm_m256 && (L.NTL * 16) % 256 == 0 && (epi == TC_EPI_STORE_F16 || epi == TC_EPI_SILU_PAIR || epi == TC_EPI_STORE_F32 ||
+                         (epi == TC_EPI_RESID_F32 && T >= 256));
+    const int max_ks = epi == TC_EPI_RESID_F32 && d->gemm_splitk ? 8 : 1;
+    int tt = 16, ks = 1;
+    bool wide = false;
+    double best = 1e30;
+    for (int w = 0; w <= (wide_ok ? 1 : 0); ++w) {
+        const int ctas_n = L.NTL * 16 / (w ? 256 : 128), t_max = w ? 256 : 512, nt0 = (T + t_max - 1) / t_max;
+        for (int nt = nt0; nt <= 2 * nt0 + 8; ++nt) {
+            const int t = ((T + nt - 1) / nt + 15) & ~15;
+            for (int k = 1; k <= max_ks && (k == 1 || L.KB / k >= 8); ++k) {
+                const int waves = (ctas_n * ((T + t - 1) / t) * k + 147) / 148;
+                const double cost = waves * ((L.KB + k - 1) / k * block_us(t, w) + 6.0 + 0.01 * t) + (k > 1 ? 2e-6 * k * T * n_valid : 0.0);
+                if (cost < best - 1e-9) { best = cost; tt = t; ks = k; wide = w; }
             }
         }
     }
-    p.T = T; p.t_tile = tt; p.k_splits = ks;
-    // 256-output tiles (two accumulators sharing each activation tile, weights dequantised once for both) where
-    // they still give the GPU enough CTAs.
-    // Measured (27B, one GPU): with few token rows a weight tile dequantised once for 256 outputs pays (80-row
-    // verify step 26.7 -> 26.1 ms); at 512 rows both forms are bound by the shared-memory traffic of the MMA
-    // operands and the 256-output form is slightly slower in the prompt (41.9 -> 42.5 ms), so it is used below
-    // 256 rows only.
-    if (d->gemm_m256 && T < 256 && (L.NTL * 16) % 256 == 0 &&
-        (epi == TC_EPI_STORE_F16 || epi == TC_EPI_SILU_PAIR || epi == TC_EPI_STORE_F32)) {
-        const int tt2 = T >= 256 ? 256 : ((T + 15) & ~15);
-        const int ctas = (L.NTL * 16 / 256) * ((T + tt2 - 1) / tt2);
-        if (ctas >= d->gemm_m256_min_ctas) { p.m_halves = 2; p.t_tile = tt2; p.k_splits = 1; }
-    }
+    p.T = T; p.t_tile = tt; p.k_splits = ks; p.m_halves = wide ? 2 : 1;
     p.n_valid = n_valid; p.ldo = ldo; p.epi = epi; p.out = out; p.status = d->m.tc_status;
     if (epi == TC_EPI_PUSH_F32) {
         const CommCtx& c = d->m.comm;
@@ -1087,7 +1072,6 @@ B2_API void* b2_driver_create(const ModelDesc* m, const LayerDesc* layers) {
     // 208.7 with 8, against 213.9 without: the gaps between GEMVs are not waiting on HBM.
     const char* g256 = getenv("B200GRAD_GEMM_M256");
     d->gemm_m256 = !(g256 && atoi(g256) == 0);
-    if (g256 && atoi(g256) > 1) d->gemm_m256_min_ctas = atoi(g256);
     const char* gsk = getenv("B200GRAD_GEMM_SPLITK");
     d->gemm_splitk = !(gsk && atoi(gsk) == 0);
     const char* spp = getenv("B200GRAD_SCAN_PREPASS");
