@@ -759,21 +759,27 @@ static int mixer_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, in
     }
     GemmTcParams p;
     memset(&p, 0, sizeof(p));
-    // Token tile and K splits from a fit to measured times (us): a 64-k block of a [128 x t] tile costs about
-    // 0.22 + t / 1000 (the tensor instructions' issue), a tile about 6 + t / 33 outside its k loop, a further
-    // plane 0.7 in its consumer.
-    const int ctas_n = (L.N + 127) / 128, KB = (L.K + 63) / 64, Tr = (T + 15) & ~15;
-    int best_t = 64, best_ks = 1;
+    // Token tile, outputs per CTA and K splits from a fit to measured times (us): a 64-k block of a [128 x t] tile costs
+    // about 0.22 + t / 1000, of a [256 x t] tile (both halves share the activation tile, so a product of the same size
+    // moves two thirds of the bytes out of L2, which is what bounds the narrow form) 0.20 + 2.6 t / 1000; a tile about
+    // 6 + t / 33, or 8, outside its k loop, a further plane 0.7 in its consumer.  1000 rows: 5120 -> 18512 204 -> 157 us
+    // (1206 TFLOP/s), 17408 -> 5120 245 -> 144 us.
+    const int KB = (L.K + 63) / 64, Tr = (T + 15) & ~15;
+    int best_t = 64, best_ks = 1, best_w = 1;
     double best = 1e30;
-    for (int t = 64; t <= 256; t += 16) {
-        if (t >= Tr + 16) break;
-        for (int ks = 1; ks <= max_ks; ++ks) {
-            const int k1 = b2_gemm_tc_splits(L.K, ks), waves = (ctas_n * ((T + t - 1) / t) * k1 + 147) / 148;
-            const double cost = waves * ((KB + k1 - 1) / k1 * (0.22 + 0.001 * t) + 6.0 + 0.03 * t) + 0.7 * (k1 - 1);
-            if (cost < best - 1e-9) { best = cost; best_t = t; best_ks = ks; }
+    for (int w = 1; w <= 2; ++w) {
+        const int ctas_n = (L.N + 128 * w - 1) / (128 * w);
+        for (int t = 64; t <= 256; t += 16) {
+            if (t >= Tr + 16) break;
+            for (int ks = 1; ks <= max_ks; ++ks) {
+                const int k1 = b2_gemm_tc_splits(L.K, ks), waves = (ctas_n * ((T + t - 1) / t) * k1 + 147) / 148;
+                const double tile = w == 1 ? (KB + k1 - 1) / k1 * (0.22 + 0.001 * t) + 6.0 + 0.03 * t : (KB + k1 - 1) / k1 * (0.20 + 0.0026 * t) + 8.0;
+                const double cost = waves * tile + 0.7 * (k1 - 1);
+                if (cost < best - 1e-9) { best = cost; best_t = t; best_ks = k1; best_w = w; }
+            }
         }
     }
-    p.K = L.K; p.T = T; p.t_tile = best_t > Tr ? Tr : best_t; p.k_splits = best_ks;
+    p.K = L.K; p.T = T; p.t_tile = best_t > Tr ? Tr : best_t; p.k_splits = best_ks; p.m_halves = best_w;
     p.ldo = ldo; p.out = out; p.status = d->m.tc_status; p.bf16 = 1; p.softcap = softcap;
     if (planes) { *planes = b2_gemm_tc_splits(L.K, best_ks); p.plane_stride = (long long)d->m.max_prefill * ldo; }
     p.n_valid = mode == DG_GATE_PAIR ? L.N / 2 : L.N;

@@ -483,11 +483,11 @@ static int launch_tc(const GemmTcParams* p, const void* w, int ldw, int n_rows_w
     GemmTcParams q = *p;
     q.box_rows = box_rows;
     q.dense = w ? 1 : 0;
-    // 256-output tiles: only with at most 256 tokens per CTA (two accumulators of 256 columns) and a matrix that
-    // is a whole number of such tiles
-    if (q.m_halves == 2 && (q.t_tile > 256 || (q.NTL * 16) % (2 * TC_BM) != 0)) q.m_halves = 1;
+    // 256-output tiles: only with at most 256 tokens per CTA (two accumulators of 256 columns) and, with INT4 weights, a
+    // matrix that is a whole number of such tiles (dense rows behind the last are zero-filled and not stored)
+    if (q.m_halves == 2 && (q.t_tile > 256 || (!q.dense && (q.NTL * 16) % (2 * TC_BM) != 0))) q.m_halves = 1;
     if (q.m_halves != 2) q.m_halves = 1;
-    dim3 grid(q.NTL * 16 / (TC_BM * q.m_halves), (q.T + q.t_tile - 1) / q.t_tile, 1);
+    dim3 grid((q.NTL * 16 + TC_BM * q.m_halves - 1) / (TC_BM * q.m_halves), (q.T + q.t_tile - 1) / q.t_tile, 1);
     // CTA pairs: 256-token operand tiles, an even number of 128-output CTAs (with dense weights a surplus tile
     // is made up: its rows are zero-filled and not stored)
     if (q.cta_pair && q.dense && q.m_halves == 1) grid.x += grid.x & 1;

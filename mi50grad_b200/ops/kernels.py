@@ -602,9 +602,9 @@ def post_norm_(h: torch.Tensor, m: Optional[torch.Tensor], w: Optional[torch.Ten
 
 def gemm_bf16_tc(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, epi: int = L.TC_EPI_STORE_F32,
                  t_tile: Optional[int] = None, softcap: float = 0.0, cta_pair: bool = False, k_splits: int = 1,
-                 act: int = L.ACT_SILU, act_cols: int = 0):
+                 act: int = L.ACT_SILU, act_cols: int = 0, m_halves: int = 1):
     """out[t][n] (epi) = x[t] . w[n] for bf16 operands on the tcgen05 tensor cores; any K (row strides
-    multiples of 8).  k_splits > 1: out is [planes][T][N] fp32, the product is the sum of its planes."""
+    multiples of 8).  m_halves = 2: 256 outputs a CTA (t_tile <= 256).  k_splits > 1: out is [planes][T][N] fp32, the product is the sum of its planes."""
     T, dev = x.shape[0], x.device
     st = _tc_status.get(dev)
     if st is None:
@@ -613,7 +613,7 @@ def gemm_bf16_tc(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, epi: int =
     p.K, p.T, p.t_tile, p.epi = x.shape[1], T, t_tile or min(256, -(-T // 16) * 16), epi
     p.n_valid = w.shape[0] // 2 if epi == L.TC_EPI_SILU_PAIR else w.shape[0]
     p.ldo, p.out, p.status, p.bf16, p.softcap = out.stride(-2), out.data_ptr(), st.data_ptr(), 1, softcap
-    p.act, p.act_cols = act, act_cols
+    p.act, p.act_cols, p.m_halves = act, act_cols, m_halves
     p.cta_pair, p.k_splits, p.plane_stride = int(cta_pair), k_splits, out.stride(0) if out.dim() == 3 else 0
     L.check(L.lib().b2_gemm_f16_tc(C.byref(p), C.c_void_p(w.data_ptr()), w.stride(0), C.c_void_p(x.data_ptr()),
                                    x.stride(0), L.stream()), "gemm_bf16_tc")

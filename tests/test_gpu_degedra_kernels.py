@@ -172,6 +172,26 @@ def test_gemm_cta_pairs_and_k_splits(N, K, T_, t):
     K_.gemm_tc_check_status()
 
 
+@pytest.mark.parametrize("N,K,T_,t,ks", [(37, 90, 9, 16, 1), (300, 200, 64, 64, 2), (640, 1032, 130, 128, 1), (129, 4096, 511, 256, 3), (1000, 520, 300, 176, 4)])
+def test_dense_gemm_of_256_outputs(N, K, T_, t, ks):
+    """Matrices that end inside a 256-output tile or one of its halves, token tails, planes, and the gate / up pair."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    w, x = _lin(_rnd(N, K, std=K ** -0.5), torch.bfloat16, 8).w, _lin(_rnd(T_, K, seed=1), torch.bfloat16, 8).w
+    ref = x[:, :K].double() @ w[:, :K].double().T
+    out = torch.full((ks, T_, N + 3), 7.0, device="cuda")
+    K_.gemm_bf16_tc(w[:, :K], x[:, :K], out[:, :, :N] if ks > 1 else out[0, :, :N], t_tile=t, k_splits=ks, m_halves=2)
+    planes = 1 if ks == 1 else -(-(-(-K // 64)) // -(-(-(-K // 64)) // ks))
+    _close(out[:planes, :, :N].sum(0), ref, 1e-5)
+    assert bool((out[:, :, N:] == 7.0).all())
+    n = N // 16 * 16
+    pair = torch.full((T_, n // 2 + 8), 7.0, dtype=torch.bfloat16, device="cuda")
+    K_.gemm_bf16_tc(w[:n, :K], x[:, :K], pair[:, :n // 2], L.TC_EPI_SILU_PAIR, t_tile=t, m_halves=2)
+    both = ref[:, :n].reshape(T_, n // 16, 2, 8)
+    _close(pair[:, :n // 2], (torch.nn.functional.silu(both[:, :, 0]) * both[:, :, 1]).reshape(T_, n // 2), 2e-2)
+    assert bool((pair[:, n // 2:] == 7.0).all())
+
+
 @pytest.mark.parametrize("dt", ["bf16", "f32"])
 @pytest.mark.parametrize("H", [90, 168, 4096])
 def test_post_norm(dt, H):
