@@ -9,7 +9,7 @@
 // b2_gemm_f32_splits.
 // Operands reach the registers at 32 floats a clock and an 8 x 8 thread tile asks for a quarter of a float per FMA, so
 // shared memory and the FMA pipes are about equally busy.  Measured in a prompt of 200 rows (12 layers of width 2048):
-// 22 TFLOP/s, the whole prompt 18.1 ms; 64 x 64 tiles staged by scalar loads gave 5.6 TFLOP/s and 55.9 ms.
+// 30 TFLOP/s, the whole prompt 14.5 ms; 64 x 64 tiles staged by scalar loads gave 5.6 TFLOP/s and 55.9 ms.
 #include "mixers.cuh"
 
 #define GF_BN 128
@@ -126,18 +126,20 @@ static int launch_f32(const GemmF32Params* p, int splits, cudaStream_t s) {
     return launch_pdl(gemm_f32_kernel<RT, VEC>, grid, dim3(GF_THREADS), smem, s, *p);
 }
 
-// Tokens of a CTA (8 rt) and splits over K with the least work on the busiest SM: CTAs per SM, times the k-blocks of
-// one, times what a k-block costs (rt + 1: eight columns of FMAs a token row, and the reads of the weights), plus the
-// start and end of a CTA (about 20 k-blocks) and of a further plane in its consumer.
+// Tokens of a CTA (8 rt) and splits over K with the least time on the busiest SM.  Measured, us a 16-k block with n CTAs
+// on an SM: about 0.5 + s n, s = .38, .54, .62, .73, .85, 1.02 for rt = 2, 4, 5, 6, 7, 8 (one CTA alone does not cover its own
+// latencies, so splits pay beyond one CTA an SM: 200 rows, 4096 -> 2048 in two splits 192 us, in four 129 us); a start
+// and an end cost 10, a further plane 1 in its consumer.
 static void plan_f32(int N, int K, int T, int max_splits, int* rt, int* splits) {
+    static const double slope[9] = {0, 0, 0.38, 0, 0.54, 0.62, 0.73, 0.85, 1.02};
     const int nt = (N + GF_BN - 1) / GF_BN, blocks = (K + GF_K - 1) / GF_K;
     double best = 1e30;
     for (int r = 8; r >= 2; --r) {
         if (r == 3) continue;
         for (int want = 1; want <= max_splits; ++want) {
             const int per = (blocks + want - 1) / want, ks = (blocks + per - 1) / per;      // no split is empty
-            const int ctas = nt * ((T + 8 * r - 1) / (8 * r)) * ks, waves = (ctas + 147) / 148;
-            const double cost = waves * (per + 20.0) * (r + 1) + 60.0 * (ks - 1);
+            const int n = (nt * ((T + 8 * r - 1) / (8 * r)) * ks + 147) / 148;
+            const double cost = per * (0.5 + slope[r] * n) + 10.0 + (ks - 1);
             if (cost < best - 1e-9) { best = cost; *rt = r; *splits = ks; }
         }
     }
