@@ -624,8 +624,15 @@ __global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_int4_kernel(const GemvIn
 // ---------------------------------------------------------------------------
 // fp16-weight kernel (lm_head, fp16-attention checkpoints).  Replaces the
 // reference's gemv_fp16_v2 (reference: src/kernels/gemv_fp16_v2.hip:22-88).
-// CTA tile: 128 outputs x kslice; each warp owns 16 outputs, 4 at a time.
+// CTA tile: 128 outputs x kslice; each warp owns 16 outputs.  One row: 4 outputs at a time on the FMA pipes.  More rows: all
+// 16 as the A operand of mma.sync with the rows as its 8 columns; the order of k inside a product is free, so lane t of a
+// row quad takes 8 adjacent k (16 bytes) of weights and activations and these are its fragments of two products.  The
+// weights of F16_DEPTH blocks of 64 k are in flight, the first of them while the activations are staged.  On the FMA pipes
+// 5 rows cost 8 conversions and 16 FMAs a row and 16 bytes of weights, twice the time of the weights.  Decode of 5 sequences
+// with fp16 attention weights at width 5120: 1.34 -> 1.08 ms a token.
 // ---------------------------------------------------------------------------
+#define F16_DEPTH 4
+#define F16_PAD(MR) ((MR) > 1 ? 32 : 0)      // halfs: the 16-byte reads of two adjacent rows meet no bank twice
 template <int MR>
 __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Params p) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -634,11 +641,26 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Par
     const int k0 = blockIdx.y * p.kslice;
     const int klen = min(p.kslice, p.K - k0);
     pdl_launch_dependents();
-    __half* xs = (__half*)smem;                                      // [MR][kslice]
-    float* ybuf = (float*)(smem + (size_t)MR * p.kslice * 2);        // [8][128]
+    const int ldx_s = p.kslice + F16_PAD(MR);
+    __half* xs = (__half*)smem;                                      // [MR][ldx_s]
+    float* ybuf = (float*)(smem + (size_t)MR * ldx_s * 2);           // [8][128]
     float* red32 = ybuf + B2_MAX_ROWS * GEMV_TILE_N;
     int* s_flag = (int*)(red32 + 32);
     const uint32_t epoch_next = (p.epi.mode == EPI_FINISH && p.comm.tp > 1) ? (*p.comm.epoch + 1u) : 0u;
+    const int n_base = blockIdx.x * GEMV_TILE_N + warp * 16, g = lane >> 2, t = lane & 3;
+    uint4 wbuf[MR > 1 ? F16_DEPTH : 1][4];
+    const __half* w_lo = p.w + (size_t)min(n_base + g, p.N - 1) * p.ldw + k0 + t * 8;
+    const __half* w_hi = p.w + (size_t)min(n_base + g + 8, p.N - 1) * p.ldw + k0 + t * 8;
+    auto load_w = [&](uint4 (&b)[4], int k) {                        // rows g and g + 8, k .. k + 63 of the slice
+        const bool a = k + t * 8 < klen, c = k + 32 + t * 8 < klen;
+        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+        b[0] = a ? ldg_nc_v4(w_lo + k) : z; b[1] = a ? ldg_nc_v4(w_hi + k) : z;
+        b[2] = c ? ldg_nc_v4(w_lo + k + 32) : z; b[3] = c ? ldg_nc_v4(w_hi + k + 32) : z;
+    };
+    if constexpr (MR > 1) {
+#pragma unroll
+        for (int d = 0; d < F16_DEPTH; ++d) load_w(wbuf[d], 64 * d);
+    }
 
     // stage the activations (normalised on the way when the input is the lazy fp32 stream): the loads of up
     // to GEMV_STAGE_UN pieces per thread, and under them the partial sums of the norm, are requested before
@@ -686,14 +708,38 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Par
                     o[q] = __floats2half2_rn(hv[u][q].x * inv * ww.x, hv[u][q].y * inv * ww.y);
                 }
             }
-            *(uint4*)(xs + i) = v;
+            *(uint4*)(xs + m * ldx_s + i % p.kslice) = v;
         }
     }
     if (!inv_ready) __syncthreads();
     for (int i = tid; i < B2_MAX_ROWS * GEMV_TILE_N; i += GEMV_THREADS) ybuf[i] = 0.f;
     __syncthreads();
 
-    const int n_base = blockIdx.x * GEMV_TILE_N + warp * 16;
+    if constexpr (MR > 1) {
+        float acc[2][4] = {};
+        const __half* xr = xs + (g < MR ? g : 0) * ldx_s + t * 8;
+        for (int kb = 0; kb < klen; kb += 64 * F16_DEPTH) {
+#pragma unroll
+            for (int d = 0; d < F16_DEPTH; ++d) {
+                const int k = kb + 64 * d;
+                if (k < klen) {                                      // (kslice is a multiple of 256: no read behind a row)
+                    uint4 x0 = *(const uint4*)(xr + k), x1 = *(const uint4*)(xr + k + 32);
+                    if (g >= MR) { x0 = make_uint4(0u, 0u, 0u, 0u); x1 = x0; }
+                    mma16816(acc[0], wbuf[d][0].x, wbuf[d][1].x, wbuf[d][0].y, wbuf[d][1].y, x0.x, x0.y);
+                    mma16816(acc[1], wbuf[d][0].z, wbuf[d][1].z, wbuf[d][0].w, wbuf[d][1].w, x0.z, x0.w);
+                    mma16816(acc[0], wbuf[d][2].x, wbuf[d][3].x, wbuf[d][2].y, wbuf[d][3].y, x1.x, x1.y);
+                    mma16816(acc[1], wbuf[d][2].z, wbuf[d][3].z, wbuf[d][2].w, wbuf[d][3].w, x1.z, x1.w);
+                    load_w(wbuf[d], k + 64 * F16_DEPTH);
+                }
+            }
+        }
+        // outputs g and g + 8, rows 2 t and 2 t + 1
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int m = 2 * t + (e & 1);
+            if (m < M) ybuf[m * GEMV_TILE_N + warp * 16 + g + 8 * (e >> 1)] = acc[0][e] + acc[1][e];
+        }
+    } else
 #pragma unroll 1
     for (int rb = 0; rb < 16; rb += 4) {
         float acc[4][MR];
@@ -713,7 +759,7 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Par
             for (int r = 0; r < 4; ++r) wv[r] = ldg_nc_v4(wr[r] + kk);
 #pragma unroll
             for (int m = 0; m < MR; ++m) {
-                uint4 xv = *(const uint4*)(xs + m * p.kslice + kk);
+                uint4 xv = *(const uint4*)(xs + m * ldx_s + kk);
                 const __half2* x2 = (const __half2*)&xv;
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
@@ -823,7 +869,7 @@ B2_API int b2_gemv_int4(const GemvInt4Params* p, cudaStream_t stream) {
 
 template <int MR>
 static int launch_f16(const GemvF16Params* p, cudaStream_t stream) {
-    size_t smem = (size_t)MR * p->kslice * 2 + (B2_MAX_ROWS * GEMV_TILE_N + 32 + 4) * 4;
+    size_t smem = (size_t)MR * (p->kslice + F16_PAD(MR)) * 2 + (B2_MAX_ROWS * GEMV_TILE_N + 32 + 4) * 4;
     static SmemOptIn optin;
     {
         cudaError_t e = optin.ensure(gemv_f16_kernel<MR>, smem);

@@ -133,6 +133,25 @@ def test_gemv_finish_local_residual_and_lazy_norm(K, rows, ks):
     assert _rel(h2.cpu(), h0 + 2 * y) < 1e-4
 
 
+@pytest.mark.parametrize("N,Kd,rows,lazy", [(16, 8, 5, False), (130, 264, 2, True), (1000, 5128, 8, False), (257, 9216, 4, False),
+                                            (129, 8200, 7, True), (64, 320, 6, True)])
+def test_gemv_f16_several_rows(K, N, Kd, rows, lazy):
+    """Widths that end inside a 64-k block, ragged outputs, slices over K, and a lazily normalised input."""
+    from mi50grad_b200.engine.engine import DeviceLinear
+    from mi50grad_b200.ops import lib as L
+    gen = torch.Generator().manual_seed(29)
+    d = _dev()
+    w, x = (torch.randn(N, Kd, generator=gen) * 0.05).half(), torch.randn(rows, Kd, generator=gen).half()
+    out, ln = torch.zeros(rows, N, dtype=torch.float32, device=d), None
+    if lazy:
+        h, wn = torch.randn(rows, Kd, generator=gen) * 3, (torch.rand(Kd, generator=gen) + 0.5).half()
+        x = (h * torch.rsqrt(h.pow(2).mean(-1, keepdim=True) + 1e-6) * wn.float()).half()
+        ln = K.lazy_norm(h.to(d), torch.cat([h.pow(2).sum(-1, keepdim=True), torch.zeros(rows, 3)], 1).to(d), wn.to(d))
+    K.gemv(DeviceLinear(dense=w.to(d)), None if lazy else x.to(d), out=out, mode=L.EPI_STORE_F32, ln=ln, rows=rows if lazy else None)
+    # (the lazy input may round to the neighbouring fp16 value)
+    assert _rel(out.cpu(), x.double() @ w.double().t()) < (1e-3 if lazy else 1e-4)
+
+
 @pytest.mark.parametrize("N,Kd,rows", [(1000, 512, 1), (4096, 5120, 3), (300, 6144, 8)])
 def test_gemv_f16(K, N, Kd, rows):
     from mi50grad_b200.engine.engine import DeviceLinear
