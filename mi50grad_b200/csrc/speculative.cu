@@ -39,7 +39,7 @@ __device__ __forceinline__ int top_bit(unsigned m) { return m ? 31 - __clz(m) : 
 // norms, the dot products of all pairs (node, ancestor) and S0^T k, S0^T q of all nodes are formed side by side, and
 // only the recursion of the update vectors over a path is serial, per column, without a barrier.  The state stays in
 // registers (4 columns x DK / groups rows a thread, read once, 16 bytes at a time) and is requested before anything else.
-// Measured for 16 sequences of 5 nodes and 48 heads of 128 x 128: 55 us a layer; a cluster of four CTAs per head
+// Measured for 16 sequences of 5 nodes and 48 heads of 128 x 128: 46 us a layer; a cluster of four CTAs per head
 // that walked the nodes with five barriers each took 127.
 template <int DK, int DV>
 struct VerifySmem {
@@ -51,7 +51,7 @@ struct VerifySmem {
     float ss[NM][DV / 32];
     float abp[VF_THREADS / 32][VF_CHUNK][2];
     unsigned anc[NM];
-    __half xraw[NM][NCH];
+    alignas(16) __half xraw[NM][NCH];
     float4 red[2][VF_CHUNK][RG][LPR];
 };
 
@@ -76,21 +76,44 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
     const float4* sp = (const float4*)(p.state + (((size_t)seq * p.nv + j) * DK + rg * RPT) * DV) + c4;
 #pragma unroll
     for (int i = 0; i < RPT; ++i) S[i] = sp[i * (DV / 4)];
-    pdl_wait();                                  // (states and row descriptors are older than the in-projection)
-
+    // (histories as well; taps and weights of this thread's channels stay in registers until the convolution)
     auto chan = [&](int c) -> int {
         if (c < DK) return kh * DK + c;
         if (c < 2 * DK) return p.nk * DK + kh * DK + (c - DK);
         return 2 * p.nk * DK + j * DV + (c - 2 * DK);
     };
+    constexpr int CPT = (NCH + VF_THREADS - 1) / VF_THREADS;
+    __half hist[CPT][3];
+    __half cw[CPT][4];
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) {
+        const int c = min(tid + q * VF_THREADS, NCH - 1);
+        const int blk = c < 2 * DK ? 0 : (c - 2 * DK) / DN_COLS, hc = c < 2 * DK ? c : 2 * DK + (c - 2 * DK) % DN_COLS;
+        const __half* hp = p.conv_state + ((((size_t)seq * p.nv + j) * CB + blk) * HCH + hc) * 3;
+#pragma unroll
+        for (int e = 0; e < 3; ++e) hist[q][e] = hp[e];
+        const __half* w = p.conv_w + (size_t)chan(c) * 4;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) cw[q][e] = w[e];
+    }
+    pdl_wait();                                  // (states and row descriptors are older than the in-projection)
+
     auto proj_col = [&](int c) -> int {
         if (c < DK) return p.off_q + kh * DK + c;
         if (c < 2 * DK) return p.off_k + kh * DK + (c - DK);
         return p.off_v + j * DV + (c - 2 * DK);
     };
-    for (int i = tid; i < N * NCH; i += VF_THREADS) {
-        const int t = i / NCH, c = i - t * NCH;
-        sm.xraw[t][c] = p.proj[(size_t)(r0 + t) * p.ld + proj_col(c)];
+    if (((p.off_q | p.off_k | p.off_v | p.ld) & 7) == 0 && ((uintptr_t)p.proj & 15) == 0) {
+#pragma unroll 2
+        for (int i = tid; i < N * (NCH / 8); i += VF_THREADS) {
+            const int t = i / (NCH / 8), c = (i - t * (NCH / 8)) * 8;
+            *(uint4*)&sm.xraw[t][c] = *(const uint4*)(p.proj + (size_t)(r0 + t) * p.ld + proj_col(c));
+        }
+    } else {
+        for (int i = tid; i < N * NCH; i += VF_THREADS) {
+            const int t = i / NCH, c = i - t * NCH;
+            sm.xraw[t][c] = p.proj[(size_t)(r0 + t) * p.ld + proj_col(c)];
+        }
     }
     // ancestors of a node inside this sequence's block (bit a <-> node a)
     if (tid < N) sm.anc[tid] = (unsigned)(p.rows[r0 + tid].mask & 0xFFFFull) & ((1u << tid) - 1u);
@@ -140,25 +163,22 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
     }
     __syncthreads();
     // ---- convolution + SiLU along every node's path: a thread keeps its channel's taps and history
-    for (int c = tid; c < NCH; c += VF_THREADS) {
-        const int blk = c < 2 * DK ? 0 : (c - 2 * DK) / DN_COLS, hc = c < 2 * DK ? c : 2 * DK + (c - 2 * DK) % DN_COLS;
-        const __half* hp = p.conv_state + ((((size_t)seq * p.nv + j) * CB + blk) * HCH + hc) * 3;
-        const __half* w = p.conv_w + (size_t)chan(c) * 4;
-        float hist[3], cw[4];
 #pragma unroll
-        for (int q = 0; q < 3; ++q) hist[q] = __half2float(hp[q]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) cw[q] = __half2float(w[q]);
+    for (int q = 0; q < CPT; ++q) {
+        const int c = tid + q * VF_THREADS;
+        if (c >= NCH) break;
+        const float h0 = __half2float(hist[q][0]), h1 = __half2float(hist[q][1]), h2 = __half2float(hist[q][2]);
+        const float w0 = __half2float(cw[q][0]), w1 = __half2float(cw[q][1]), w2 = __half2float(cw[q][2]), w3 = __half2float(cw[q][3]);
         for (int t = 0; t < N; ++t) {
             // taps at distance 1..3 along the path; beyond the root they come from the history
             const unsigned a1 = sm.anc[t];
             const int d = __popc(a1), p1 = top_bit(a1);
             const unsigned a2 = p1 >= 0 ? a1 & ~(1u << p1) : 0u;
             const int p2 = top_bit(a2), p3 = top_bit(p2 >= 0 ? a2 & ~(1u << p2) : 0u);
-            const float x1 = d >= 1 ? __half2float(sm.xraw[p1][c]) : hist[2];
-            const float x2 = d >= 2 ? __half2float(sm.xraw[p2][c]) : (d == 1 ? hist[2] : hist[1]);
-            const float x3 = d >= 3 ? __half2float(sm.xraw[p3][c]) : (d == 2 ? hist[2] : (d == 1 ? hist[1] : hist[0]));
-            const float o = silu_f(x3 * cw[0] + x2 * cw[1] + x1 * cw[2] + __half2float(sm.xraw[t][c]) * cw[3]);
+            const float x1 = d >= 1 ? __half2float(sm.xraw[p1][c]) : h2;
+            const float x2 = d >= 2 ? __half2float(sm.xraw[p2][c]) : (d == 1 ? h2 : h1);
+            const float x3 = d >= 3 ? __half2float(sm.xraw[p3][c]) : (d == 2 ? h2 : (d == 1 ? h1 : h0));
+            const float o = silu_f(x3 * w0 + x2 * w1 + x1 * w2 + __half2float(sm.xraw[t][c]) * w3);
             if (c < DK) sm.cq[t][c] = o; else if (c < 2 * DK) sm.ck[t][c - DK] = o; else sm.cv[t][c - 2 * DK] = o;
         }
     }
