@@ -174,9 +174,9 @@ struct Driver {
     int graph_rows = 0, graph_flags = 0;
     long long launches = 0;               // kernels issued by the last eager step
     int scan_prepass = 2;                 // chunked scan: 1 = q / k convolution and norms in a parallel pre-pass,
-                                          // 2 = also the state-independent products and the triangle inverse of every chunk
+                                          // 2 = the scan in three parts, of which only the middle one is serial
     bool attn_tc = true;                  // prompt attention on tcgen05 (csrc/attention_tc.cu)
-    bool gemm_m256 = true;                // 256-output GEMM tiles where the grid stays large enough
+    bool gemm_m256 = true;                // 256-output GEMM tiles where the work model prefers them
     bool gemm_splitk = true;              // split-K in the many-row GEMMs that add into the residual stream
     const void* pf_span = nullptr; long long pf_span_bytes = 0;   // see run_linear
     bool pf_state = false;                // the in-projection of a DeltaNet layer prefetches that layer's state into L2

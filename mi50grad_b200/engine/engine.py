@@ -36,6 +36,7 @@ from ..utils.quant import DenseLinear, Int4Linear
 from .state import SequenceStates
 
 log = logging.getLogger(__name__)
+
 # Rows of a prompt per pass over the layers.  A pass costs every projection whole waves of tiles over the SMs and a walk
 # over the weights, so few long passes beat many short ones; work buffers grow with it (27B: 0.75 GB for 4096 rows).
 # Measured: 3001 rows at width 4096 24.5 -> 18.3 ms against passes of 512.  Under tensor parallelism the exchange buffers, and
