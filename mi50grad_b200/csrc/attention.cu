@@ -12,9 +12,12 @@
 // once per group.  Each warp takes 16 cache slots at a time and multiplies them on the tensor cores with the
 // heads as the narrow side: S^T = K Q^T is [16 slots x 8 heads] and O^T += V^T P^T [16 dims x 8 heads] a
 // mma.sync m16n8k16, so up to eight heads cost one column tile and no shuffles but those of the running
-// maximum.  The soft-max weights enter the second product as the sum of two fp16 terms (22 bits); everything
-// else in it is fp16 already, sums are fp32.  (max, sum, O) are merged across warps in shared memory and
-// across splits through a scratch buffer by the last CTA to arrive.
+// maximum.  The soft-max weights enter the second product as the sum of two fp16 terms; the largest is 2^15, so that
+// both terms of weights down to 2^-18 of it are normal numbers (23 bits) and what falls off at the bottom is below 2^-40 of it.
+// Everything else in the products is fp16 already.  The tensor core cuts off the bits below its 24 at every addition, so
+// a product's own 16 terms are all that it adds up; the sums over the head dim and over the slots are fp32 additions,
+// which round.  (max, sum, O) are merged across warps in shared memory and across splits through a scratch buffer by
+// the last CTA to arrive.
 //
 // Bound: the cache, and with short contexts the latency of one pass.  With dot products on the FMA pipes a
 // slot cost about 180 warp instructions for six heads (here 10), which was the bound.  Measured per layer,
@@ -26,6 +29,7 @@
 #define ATT_MAX_G 8
 #define ATT_SLOTS 16             // cache slots a warp takes at a time
 #define ATT_MIN_SPLIT_LEN (ATT_WARPS * ATT_SLOTS)      // one pass of one CTA
+#define ATT_WEIGHT 32768.f       // soft-max weight of a score that is the maximum
 #define ATT_LDH(HD) ((HD) + 8)   // halfs per staged row: the 16-byte rows of a matrix meet no bank twice
 
 __device__ __forceinline__ void at_ldsm4(uint32_t (&r)[4], const __half* p) {
@@ -110,14 +114,18 @@ __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnPara
         const bool more = sb + ATT_MIN_SPLIT_LEN < s1;
         cp_async_wait<1>();
         __syncwarp();
-        float s[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};    // two chains: even and odd k steps
+        float s[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int k = 0; k < KS; k += 2) {
-            uint32_t a[4], b[4];
-            at_ldsm4(a, ka + 16 * k);
-            at_ldsm4(b, ka + 16 * k + 16);
-            at_mma(s, a, qf[k][0], qf[k][1]);
-            at_mma(s2, b, qf[k + 1][0], qf[k + 1][1]);
+        for (int k = 0; k < KS; k += 4) {                        // (added in pairs: short chains of roundings)
+            float x[4][4] = {};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                uint32_t a[4];
+                at_ldsm4(a, ka + 16 * (k + i));
+                at_mma(x[i], a, qf[k + i][0], qf[k + i][1]);
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[e] += (x[0][e] + x[1][e]) + (x[2][e] + x[3][e]);
         }
         __syncwarp();
         if (more) stage(Kw, p.kcache, sb + ATT_MIN_SPLIT_LEN);
@@ -127,7 +135,7 @@ __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnPara
         for (int e = 0; e < 4; ++e) {
             const int slot = sb + g + 8 * (e >> 1), d = slot - rm.ctx;
             const bool vis = slot < s1 && (d < 0 || ((rm.mask >> d) & 1ull));
-            s[e] = vis ? (s[e] + s2[e]) * sc : -INFINITY;
+            s[e] = vis ? s[e] * sc : -INFINITY;
         }
         float pw[4];
         float cor[2];
@@ -139,13 +147,9 @@ __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnPara
             const float mn = fmaxf(m[h], mx), ref = mn == -INFINITY ? 0.f : mn;
             cor[h] = exp2f(m[h] - ref);                          // exp2(-inf) = 0 on the first visible slot
             m[h] = mn;
-            pw[h] = exp2f(s[h] - ref);
-            pw[2 + h] = exp2f(s[2 + h] - ref);
+            pw[h] = exp2f(s[h] - ref) * ATT_WEIGHT;
+            pw[2 + h] = exp2f(s[2 + h] - ref) * ATT_WEIGHT;
             l[h] = l[h] * cor[h] + pw[h] + pw[2 + h];
-        }
-        if (__any_sync(0xffffffffu, cor[0] != 1.f || cor[1] != 1.f)) {
-#pragma unroll
-            for (int k = 0; k < KS; ++k) { o[k][0] *= cor[0]; o[k][1] *= cor[1]; o[k][2] *= cor[0]; o[k][3] *= cor[1]; }
         }
         uint32_t ph[2], pl[2];
 #pragma unroll
@@ -161,9 +165,12 @@ __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnPara
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
             uint32_t v[4];
+            float x[4] = {0.f, 0.f, 0.f, 0.f};
             at_ldsm4_t(v, va + 16 * k);
-            at_mma(o[k], v, pl[0], pl[1]);
-            at_mma(o[k], v, ph[0], ph[1]);
+            at_mma(x, v, pl[0], pl[1]);
+            at_mma(x, v, ph[0], ph[1]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) o[k][e] = fmaf(o[k][e], cor[e & 1], x[e]);
         }
         __syncwarp();
         if (more) stage(Vw, p.vcache, sb + ATT_MIN_SPLIT_LEN);
