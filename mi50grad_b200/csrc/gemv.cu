@@ -629,7 +629,9 @@ __global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_int4_kernel(const GemvIn
 // row quad takes 8 adjacent k (16 bytes) of weights and activations and these are its fragments of two products.  The
 // weights of F16_DEPTH blocks of 64 k are in flight, the first of them while the activations are staged.  On the FMA pipes
 // 5 rows cost 8 conversions and 16 FMAs a row and 16 bytes of weights, twice the time of the weights.  Decode of 5 sequences
-// with fp16 attention weights at width 5120: 1.34 -> 1.08 ms a token.
+// with fp16 attention weights at width 5120: 1.34 -> 1.10 ms a token.  Only the 16 terms of a product are summed by the
+// tensor core, which cuts off; longer sums are fp32 additions: error of 5 rows of 5120 1.05e-7 (FMA chains 1.13e-7; sums over
+// all of K on the tensor core 4.8e-7 and 1 % faster).
 // ---------------------------------------------------------------------------
 #define F16_DEPTH 4
 #define F16_PAD(MR) ((MR) > 1 ? 32 : 0)      // halfs: the 16-byte reads of two adjacent rows meet no bank twice
@@ -725,10 +727,14 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Par
                 if (k < klen) {                                      // (kslice is a multiple of 256: no read behind a row)
                     uint4 x0 = *(const uint4*)(xr + k), x1 = *(const uint4*)(xr + k + 32);
                     if (g >= MR) { x0 = make_uint4(0u, 0u, 0u, 0u); x1 = x0; }
-                    mma16816(acc[0], wbuf[d][0].x, wbuf[d][1].x, wbuf[d][0].y, wbuf[d][1].y, x0.x, x0.y);
-                    mma16816(acc[1], wbuf[d][0].z, wbuf[d][1].z, wbuf[d][0].w, wbuf[d][1].w, x0.z, x0.w);
-                    mma16816(acc[0], wbuf[d][2].x, wbuf[d][3].x, wbuf[d][2].y, wbuf[d][3].y, x1.x, x1.y);
-                    mma16816(acc[1], wbuf[d][2].z, wbuf[d][3].z, wbuf[d][2].w, wbuf[d][3].w, x1.z, x1.w);
+                    // (each product from zero: the tensor core cuts its sums off, the additions to acc round)
+                    float y[4][4] = {};
+                    mma16816(y[0], wbuf[d][0].x, wbuf[d][1].x, wbuf[d][0].y, wbuf[d][1].y, x0.x, x0.y);
+                    mma16816(y[1], wbuf[d][0].z, wbuf[d][1].z, wbuf[d][0].w, wbuf[d][1].w, x0.z, x0.w);
+                    mma16816(y[2], wbuf[d][2].x, wbuf[d][3].x, wbuf[d][2].y, wbuf[d][3].y, x1.x, x1.y);
+                    mma16816(y[3], wbuf[d][2].z, wbuf[d][3].z, wbuf[d][2].w, wbuf[d][3].w, x1.z, x1.w);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) { acc[0][e] += y[0][e] + y[1][e]; acc[1][e] += y[2][e] + y[3][e]; }
                     load_w(wbuf[d], k + 64 * F16_DEPTH);
                 }
             }

@@ -56,3 +56,19 @@ def test_decode_attention_sums_round(K, hd, nq, nkv, ctx, splits):
     v = (torch.randn(1, ctx + 1, nkv, hd, generator=g, device="cuda") * 2 + 3).half()
     out = K.decode_attn(q, K.make_rows([(0, ctx, ctx, ctx, 1)] * 6, "cuda"), k, v, nq, nkv, hd, splits=splits)
     assert _misrounded(out, _attention(q, k[0], v[0], nq, nkv)) < 1.5e-3
+
+
+@pytest.mark.parametrize("N,Kd,rows", [(1000, 5120, 5), (1024, 17408, 8), (512, 2048, 2)])
+def test_gemv_f16_of_several_rows_sums_round(K, N, Kd, rows):
+    """A sum of K products in fp32: a rounding of 2^-24 for each of the about 100 additions of an output's longest chain,
+    of random sign, is 1.5e-7 at most; one that is cut off every time loses several times that."""
+    from mi50grad_b200.engine.engine import DeviceLinear
+    from mi50grad_b200.ops import lib as L
+    g = _gen(4)
+    for positive in (False, True):
+        w, x = torch.randn(N, Kd, generator=g, device="cuda") * 0.02, torch.randn(rows, Kd, generator=g, device="cuda")
+        w, x = (w.abs().half(), x.abs().half()) if positive else (w.half(), x.half())
+        out = torch.zeros(rows, N, device="cuda")
+        K.gemv(DeviceLinear(dense=w), x, out=out, mode=L.EPI_STORE_F32)
+        ref = x.double() @ w.double().t()
+        assert float((out.double() - ref).norm() / ref.norm()) < 2e-7
