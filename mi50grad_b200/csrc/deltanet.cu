@@ -1571,8 +1571,11 @@ __global__ void __launch_bounds__(AB_WARPS * 32) ab_proj_kernel(const __half* __
 #pragma unroll
         for (int n = 0; n < AB_OUT / 8; ++n) {
             const uint4 w = v[(2 + n) * 32];
-            ab_mma(acc[n], a0, w.x, w.y);
-            ab_mma(acc[n], a1, w.z, w.w);
+            float y0[4] = {}, y1[4] = {};        // (from zero: the tensor core cuts its sums off, the additions to acc round)
+            ab_mma(y0, a0, w.x, w.y);
+            ab_mma(y1, a1, w.z, w.w);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[n][e] += y0[e] + y1[e];
         }
     }
     __syncthreads();                                 // the partial sums take the ring's place

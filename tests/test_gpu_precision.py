@@ -72,3 +72,10 @@ def test_gemv_f16_of_several_rows_sums_round(K, N, Kd, rows):
         K.gemv(DeviceLinear(dense=w), x, out=out, mode=L.EPI_STORE_F32)
         ref = x.double() @ w.double().t()
         assert float((out.double() - ref).norm() / ref.norm()) < 2e-7
+
+
+def test_gate_projections_sums_round(K):
+    g = _gen(5)
+    x, wa, wb = (torch.randn(n, 5120, generator=g, device="cuda").half() for n in (160, 48, 48))
+    out = K.ab_proj(x, wa, wb)[:, :96]
+    assert _misrounded(out, torch.cat([x.double() @ wa.double().t(), x.double() @ wb.double().t()], 1)) < 1.5e-3
