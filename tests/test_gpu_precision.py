@@ -79,3 +79,19 @@ def test_gate_projections_sums_round(K):
     x, wa, wb = (torch.randn(n, 5120, generator=g, device="cuda").half() for n in (160, 48, 48))
     out = K.ab_proj(x, wa, wb)[:, :96]
     assert _misrounded(out, torch.cat([x.double() @ wa.double().t(), x.double() @ wb.double().t()], 1)) < 1.5e-3
+
+
+@pytest.mark.parametrize("hd,T,past", [(256, 300, 1200), (64, 300, 1200)])
+def test_prompt_attention_with_peaked_scores(K, hd, T, past):
+    """Where one weight outweighs the others, it is exactly 1 in fp16 and the result little more than its rounding to
+    fp16 (2.1e-4 in the 2-norm) away."""
+    g = _gen(6)
+    n = past + T
+    q = (torch.randn(T, 2 * hd, generator=g, device="cuda") * 2.5).half()
+    k = torch.randn(1, n, 1, hd, generator=g, device="cuda").half()
+    v = (torch.randn(1, n, 1, hd, generator=g, device="cuda") * 2).half()
+    out = K.attn_prefill_tc(q, K.make_rows([(0, past + i, past + i, past + i + 1, 0) for i in range(T)], "cuda"), k, v, 2, 1, hd)
+    K.gemm_tc_check_status()
+    mask = torch.arange(n, device="cuda")[None] <= past + torch.arange(T, device="cuda")[:, None]
+    ref = _attention(q, k[0], v[0], 2, 1, mask)
+    assert float((out.double() - ref).norm() / ref.norm()) < 2.4e-4
