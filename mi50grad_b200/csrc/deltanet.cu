@@ -1048,9 +1048,10 @@ template <int DK, int DV> struct ScanBlock {
     static constexpr int U0 = DC_C * DK, W = U0 + DC_C * DV, GATES = W + DC_C * DC_C, FLOATS = GATES + DC_GATES;
 };
 
-// hi + lo = x with hi a TF32 value; the tensor core ignores the low 13 bits of lo, which leaves 2^-21 of x
+// x = hi + lo with hi rounded to a TF32 value (as tf32r does; an addition and a mask take fewer issue slots than the
+// conversion).  At most 13 bits are left for lo, of which the tensor core reads 11: 2^-23 of x is cut off at most.
 __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
-    hi = __uint_as_float(__float_as_uint(x) & 0xffffe000u);
+    hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
     lo = x - hi;
 }
 __device__ __forceinline__ void ldsm4_h(uint32_t (&r)[4], const __half* row_ptr) {
