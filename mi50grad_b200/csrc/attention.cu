@@ -81,11 +81,20 @@ __global__ void __launch_bounds__(ATT_THREADS) decode_attn_kernel(const AttnPara
     // requested as soon as the scores are formed, the V rows as soon as the output is.
     const size_t base = ((size_t)rm.seq * p.max_seq) * p.nkv * HD + (size_t)kvh * HD;
     const size_t stride = (size_t)p.nkv * HD;
+    // 16-byte pieces where both caches start on such a boundary, else as many bytes as a lane's share of a row
+    const bool wide = (((uintptr_t)p.kcache | (uintptr_t)p.vcache) & 15) == 0;
+    auto copy8 = [&](__half* dst, const __half* src) {
+        if (HD == 256 || wide) { cp_async16(dst, src); return; }
+#pragma unroll
+        for (int i = 0; i < 8; i += HD / 32) {
+            if constexpr (HD == 128) cp_async8(dst + i, src + i); else cp_async4(dst + i, src + i);
+        }
+    };
     auto stage = [&](__half* dst, const __half* cache, int sb) {
 #pragma unroll 4
         for (int i = lane; i < ATT_SLOTS * PPR; i += 32) {
             const int row = i / PPR, c = i % PPR * 8;
-            if (sb + row < s1) cp_async16(dst + row * LD + c, cache + base + (size_t)(sb + row) * stride + c);
+            if (sb + row < s1) copy8(dst + row * LD + c, cache + base + (size_t)(sb + row) * stride + c);
             else *(uint4*)(dst + row * LD + c) = make_uint4(0u, 0u, 0u, 0u);
         }
     };

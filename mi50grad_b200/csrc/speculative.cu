@@ -74,8 +74,16 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
 
     float4 S[RPT];
     const float4* sp = (const float4*)(p.state + (((size_t)seq * p.nv + j) * DK + rg * RPT) * DV) + c4;
+    if (((uintptr_t)p.state & 15) == 0) {
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) S[i] = sp[i * (DV / 4)];
+        for (int i = 0; i < RPT; ++i) S[i] = sp[i * (DV / 4)];
+    } else {
+#pragma unroll
+        for (int i = 0; i < RPT; ++i) {
+            const float* f = (const float*)(sp + i * (DV / 4));
+            S[i] = make_float4(f[0], f[1], f[2], f[3]);
+        }
+    }
     // (histories as well; taps and weights of this thread's channels stay in registers until the convolution)
     auto chan = [&](int c) -> int {
         if (c < DK) return kh * DK + c;

@@ -337,6 +337,20 @@ def test_decode_attn_slot_edges(K, hd, nq, nkv, splits):
         assert _rel(out[r].cpu().view(nq, hd), o[0]) < 3e-3, f"row {r}"
 
 
+@pytest.mark.parametrize("hd,off", [(64, 2), (64, 6), (128, 4)])
+def test_decode_attn_caches_off_the_16_byte_boundary(K, hd, off):
+    """Caches that start on a boundary of a lane's share of a row only (4 bytes with heads of 64, 8 with 128): the same
+    copies in smaller pieces."""
+    gen = torch.Generator().manual_seed(24)
+    n, nq, nkv = 150, 6, 2
+    kv = [torch.randn(2 * n * nkv * hd, generator=gen).half().cuda() for _ in range(2)]
+    q, rows = torch.randn(3, nq * hd, generator=gen).half().cuda(), K.make_rows([(0, 99, 99, 99, 1), (1, 0, 0, 0, 1), (1, 149, 149, 149, 1)], _dev())
+    moved = [torch.cat([t.new_zeros(off), t])[off:].view(2, n, nkv, hd) for t in kv]
+    assert all(t.data_ptr() % 16 for t in moved)
+    got = [K.decode_attn(q, rows, k, v, nq, nkv, hd, splits=2) for k, v in ([t.view(2, n, nkv, hd) for t in kv], moved)]
+    assert torch.equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("hd,T,past", [(256, 130, 100), (64, 65, 0), (128, 129, 320), (256, 64, 1)])
 def test_attn_prefill_growing_scores_and_poisoned_slots(K, hd, T, past):
     """Scores that grow along the cache (the reference maximum moves many times, and stays behind by up to 2^8 between), a

@@ -218,3 +218,49 @@ def test_verify_outputs_equal_steps_along_every_path(dk, nk, nv, sizes, kind, ab
                               wb=wb if ab != "proj" else None, ln=lazy(path) if ab == "lazy" else None)[-1]
         err = float((out[r].float() - ref.float()).abs().max() / ref.float().abs().max())
         assert err < 2e-3, (r, err)
+
+
+class _Verify:
+    """One launch of the verify kernel over chains of `n` drafts of `ns` sequences, heads of 64."""
+
+    def __init__(self, nk=2, nv=4, ns=3, n=4, state_offset=0):
+        from mi50grad_b200.ops import kernels as K
+        g = torch.Generator().manual_seed(8)
+        rnd = lambda *s: torch.randn(*s, generator=g)  # noqa: E731
+        d, vd = 64, nv * 64
+        self.cd = cd = 2 * nk * d + vd
+        self.dims, self.offs = (nk, nv, d, d), (0, nk * d, 2 * nk * d, cd, cd + vd, cd + vd + nv)
+        self.proj = rnd(ns * n, cd + vd + 2 * nv).half().cuda()
+        self.w = [(rnd(cd, 4) * 0.3).half().cuda(), (torch.rand(nv, generator=g) * 1.5 - 1.0).cuda(), (rnd(nv) * 0.5).half().cuda(),
+                  (torch.rand(d, generator=g) + 0.5).half().cuda()]
+        self.conv = rnd(ns, nv, d // 32, 2 * d + 32, 3).half().cuda()
+        self.state = torch.cat([torch.zeros(state_offset), (rnd(ns, nv, d, d) * 0.3).flatten()]).cuda()[state_offset:].view(ns, nv, d, d)
+        self.rows = K.make_rows([(s, 0, 0, 0, (2 << i) - 1) for s in range(ns) for i in range(n)], "cuda")
+        self.seq_rows = torch.arange(ns + 1, dtype=torch.int32, device="cuda") * n
+        self.out, self.ns = torch.zeros(ns * n, vd, dtype=torch.float16, device="cuda"), ns
+
+    def __call__(self):
+        import ctypes as C
+        from mi50grad_b200.ops import lib as L
+        nk, nv, dk, dv = self.dims
+        p, st = L.DeltaParams(), L.SpecStage()
+        p.proj, p.ld = self.proj.data_ptr(), self.proj.stride(0)
+        p.off_q, p.off_k, p.off_v, p.off_z, p.off_a, p.off_b = self.offs
+        p.conv_w, p.A_log, p.dt_bias, p.norm_w = (t.data_ptr() for t in self.w)
+        p.conv_state, p.state = self.conv.data_ptr(), self.state.data_ptr()
+        p.seq_rows, p.rows, p.out, p.ldo = self.seq_rows.data_ptr(), self.rows.data_ptr(), self.out.data_ptr(), self.out.stride(0)
+        p.nk, p.nv, p.n_seqs, p.eps = nk, nv, self.ns, 1e-6
+        off = [C.c_int() for _ in range(4)]
+        L.lib().b2_spec_stage_layout.restype = C.c_longlong
+        blk = int(L.lib().b2_spec_stage_layout(nk, nv, dk, dv, *[C.byref(o) for o in off]))
+        self.stage = torch.empty(self.ns * blk, dtype=torch.uint8, device="cuda")
+        st.base, st.seq_stride, st.layer_stride = self.stage.data_ptr(), blk, self.ns * blk
+        st.off_k, st.off_u, st.off_g, st.off_x = (o.value for o in off)
+        L.check(L.lib().b2_deltanet_verify(C.byref(p), C.byref(st), 0, dk, dv, L.stream()), "verify")
+        return self.out
+
+
+def test_verify_of_states_off_the_16_byte_boundary():
+    a, b = _Verify(), _Verify(state_offset=1)
+    assert a.state.data_ptr() % 16 == 0 and b.state.data_ptr() % 16 == 4
+    assert torch.equal(a(), b())
