@@ -34,6 +34,7 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_step_kernel(const DeltaPa
     constexpr int NCH = 2 * DK + DN_COLS;        // conv channels this CTA consumes
     cg::cluster_group cluster = cg::this_cluster();
     pdl_launch_dependents();
+    if (!p.older) pdl_wait();
     const int cb = blockIdx.x, j = blockIdx.y, si = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, kr = tid >> 5, vcol = lane;
     const int kh = j / (p.nv / p.nk);
@@ -255,6 +256,7 @@ __global__ void __launch_bounds__(DV / 32 * 128) deltanet_head_kernel(const Delt
     constexpr int NCH = 2 * DK + DV;             // conv channels of the head: q | k | v
     constexpr int PRE = 5;                       // a/b weight pairs per thread kept in registers
     pdl_launch_dependents();
+    if (!p.older) pdl_wait();
     const int j = blockIdx.x, si = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cb = warp / KR, kr = warp % KR, col = cb * DN_COLS + lane;
@@ -1261,6 +1263,7 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
     extern __shared__ __align__(16) float dsm[];
     ScanSmem<DK>& sm = *(ScanSmem<DK>*)dsm;
     pdl_launch_dependents();
+    if (!p.older) pdl_wait();
     const int cb = blockIdx.x, j = blockIdx.y, kh = j / (p.nv / p.nk);
     const int tid = threadIdx.x, lane = tid & 31, kr = tid >> 5, g = lane >> 2, t = lane & 3;
     const int r0 = p.seq_rows[0], r1 = p.seq_rows[1];
@@ -1309,7 +1312,7 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
             S[n][0] = lo.x; S[n][1] = lo.y; S[n][2] = hi.x; S[n][3] = hi.y;
         }
     }
-    pdl_wait();                                   // (the state is older than the kernels before)
+    pdl_wait();
     stage(0);
     load_u0(0);
     put_s0();

@@ -364,7 +364,7 @@ static void fill_delta(const Driver* d, const LayerDesc& L, DeltaParams& q) {
     q.ldx = m.H; q.H = m.H; q.wa = (const __half*)L.wa; q.wb = (const __half*)L.wb;
     q.conv_w = (const __half*)L.conv_w; q.conv_state = (__half*)L.conv_state; q.state = L.state;
     q.A_log = L.A_log; q.dt_bias = (const __half*)L.dt_bias; q.norm_w = (const __half*)L.la_norm;
-    q.seq_rows = m.seq_rows; q.ldo = m.ld_attn; q.nk = m.la_nk; q.nv = m.la_nv; q.eps = 1e-6f; q.commit = 1;
+    q.seq_rows = m.seq_rows; q.ldo = m.ld_attn; q.nk = m.la_nk; q.nv = m.la_nv; q.eps = 1e-6f; q.commit = 1; q.older = 1;
 }
 
 // After the arg-max of a verify step: accept on the device, then bring DeltaNet states and the
@@ -468,7 +468,7 @@ static int step_impl(Driver* d, int rows, int n_seqs, int flags, cudaStream_t s)
             q.A_log = L.A_log; q.dt_bias = (const __half*)L.dt_bias; q.norm_w = (const __half*)L.la_norm;
             q.seq_rows = m.seq_rows; q.rows = (const RowMeta*)m.rows; q.out = (__half*)m.attn_out; q.ldo = m.ld_attn;
             q.nk = m.la_nk; q.nv = m.la_nv; q.n_seqs = n_seqs; q.eps = 1e-6f;
-            q.commit = (flags & STEP_NO_COMMIT_DELTA) ? 0 : 1;
+            q.commit = (flags & STEP_NO_COMMIT_DELTA) ? 0 : 1; q.older = 1;
             if (flags & STEP_SPEC) CK(b2_deltanet_verify(&q, &m.spec, L.type_index, m.la_dk, m.la_dv, s));
             else CK(b2_deltanet_step(&q, m.la_dk, m.la_dv, s));
             d->launches++;

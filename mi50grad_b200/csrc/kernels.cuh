@@ -34,6 +34,8 @@ struct DeltaParams {
     int ldo, nk, nv, n_seqs;
     float eps;
     int commit;              // 0: leave state and conv history untouched (dry run for tree verification)
+    int older;               // 1: rows, seq_rows, states and histories were complete before the first kernel of this step
+    int pad;                 //    started (the step driver: prepare_rows is a plain launch), so they are read before the wait
     LazyNorm ln;             // if ln.h: the a/b projections read the lazily normalised residual stream
 };
 

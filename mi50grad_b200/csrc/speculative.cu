@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
     extern __shared__ float4 vf_smem[];
     Smem& sm = *(Smem*)vf_smem;
     pdl_launch_dependents();
+    if (!p.older) pdl_wait();
     const int j = blockIdx.x, si = blockIdx.y;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rep = p.nv / p.nk, kh = j / rep;
@@ -104,7 +105,7 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
 #pragma unroll
         for (int e = 0; e < 4; ++e) cw[q][e] = w[e];
     }
-    pdl_wait();                                  // (states and row descriptors are older than the in-projection)
+    pdl_wait();
 
     auto proj_col = [&](int c) -> int {
         if (c < DK) return p.off_q + kh * DK + c;

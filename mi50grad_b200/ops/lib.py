@@ -109,7 +109,7 @@ class DeltaParams(C.Structure):
                 ("off_a", i32), ("off_b", i32), ("xn", vp), ("ldx", i32), ("H", i32), ("wa", vp), ("wb", vp),
                 ("conv_w", vp), ("conv_state", vp), ("state", vp), ("A_log", vp), ("dt_bias", vp),
                 ("norm_w", vp), ("seq_rows", vp), ("rows", vp), ("out", vp), ("ldo", i32), ("nk", i32),
-                ("nv", i32), ("n_seqs", i32), ("eps", f32), ("commit", i32), ("ln", LazyNorm)]
+                ("nv", i32), ("n_seqs", i32), ("eps", f32), ("commit", i32), ("older", i32), ("pad", i32), ("ln", LazyNorm)]
 
 
 class ArgmaxParams(C.Structure):

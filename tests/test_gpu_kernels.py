@@ -318,6 +318,35 @@ def test_deltanet_scan_in_parts_equals_one_kernel(K, dk, nk, nv, rows):
     assert torch.equal(got[1][2], got[0][2])
 
 
+@pytest.mark.parametrize("dk,nk,nv,cuts", [(128, 1, 2, (0, 64, 96, 224, 300)), (64, 1, 2, (0, 32, 64, 96, 128, 160)), (64, 2, 4, (0, 512, 530))])
+def test_deltanet_portions_in_a_row(K, dk, nk, nv, cuts):
+    """Launch after launch on one state: each starts from what the one before left, although it may begin under it.  Portions
+    end where chunks do, so they give the bits of one call; one token after it by the step kernel reads the same state."""
+    gen = torch.Generator().manual_seed(25)
+    rnd = lambda *s: torch.randn(*s, generator=gen)  # noqa: E731
+    n, kd, vd = cuts[-1], nk * dk, nv * dk
+    cd = 2 * kd + vd
+    proj = rnd(n + 1, cd + vd + 2 * nv).half().cuda()
+    w = [(rnd(cd, 4) * 0.3).half().cuda(), (torch.rand(nv, generator=gen) * 1.5 - 1.0).cuda(), (rnd(nv) * 0.5).half().cuda(), (torch.rand(dk, generator=gen) + 0.5).half().cuda()]
+    S0 = (rnd(1, nv, dk, dk) * 0.1).cuda()
+    offs = (0, kd, 2 * kd, cd, cd + vd, cd + vd + nv)
+    meta = K.make_rows([(0, 0, 0, 0, 1)] * (n + 1), _dev())
+    size = lambda m: torch.tensor([0, m], dtype=torch.int32, device=_dev())  # noqa: E731
+    sizes, one = [size(b - a) for a, b in zip(cuts, cuts[1:])], size(1)
+
+    def run(bounds, counts):
+        S, h = S0.clone(), torch.zeros(1, nv, dk // 32, 2 * dk + 32, 3, dtype=torch.float16, device=_dev())
+        out = torch.zeros(n + 1, vd, dtype=torch.float16, device=_dev())
+        for a, b, c in zip(bounds, bounds[1:], counts):
+            K.deltanet_chunk(proj[a:b], offs, proj[a:b, cd + vd:], w[0], h, S, w[1], w[2], w[3], meta, c, nk, nv, dk, dk, out=out[a:b], prepass=2)
+        K.deltanet_step(proj[n:], offs, w[0], h, S, w[1], w[2], w[3], meta, one, nk, nv, dk, dk, out=out[n:])
+        return out, S, h
+    ref = run((0, n), [size(n)])
+    for _ in range(10):
+        for a, b in zip(run(cuts, sizes), ref):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("hd,nq,nkv,splits", [(256, 8, 1, 1), (256, 5, 5, 4), (128, 14, 2, 32), (64, 8, 8, 2)])
 def test_decode_attn_slot_edges(K, hd, nq, nkv, splits):
     """Contexts around the 16 slots of a warp's pass and the 64 of a CTA's, one to eight heads a group, masks with holes,

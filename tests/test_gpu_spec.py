@@ -264,3 +264,22 @@ def test_verify_of_states_off_the_16_byte_boundary():
     a, b = _Verify(), _Verify(state_offset=1)
     assert a.state.data_ptr() % 16 == 0 and b.state.data_ptr() % 16 == 4
     assert torch.equal(a(), b())
+
+
+def test_verify_directly_after_the_step_that_left_its_states():
+    """The verify kernel may begin under the step kernel before it; it reads the states that this leaves all the same."""
+    from mi50grad_b200.ops import kernels as K
+    v = _Verify()
+    nk, nv, dk, dv = v.dims
+    S0, c0, got = v.state.clone(), v.conv.clone(), []
+    one = torch.arange(v.ns + 1, dtype=torch.int32, device="cuda")
+    rows = K.make_rows([(s, 0, 0, 0, 1) for s in range(v.ns)], "cuda")
+    for i in range(8):
+        v.state.copy_(S0)
+        v.conv.copy_(c0)
+        for _ in range(3):
+            K.deltanet_step(v.proj[:v.ns], v.offs, v.w[0], v.conv, v.state, *v.w[1:], rows, one, nk, nv, dk, dv)
+        if i == 0:
+            torch.cuda.synchronize()
+        got.append(v().clone())
+    assert all(torch.equal(g, got[0]) for g in got)
