@@ -801,6 +801,7 @@ static MixRun mixer_run(const Driver* d, bool many, int rows, int n_seqs, int fl
     r.out = many ? m.p_attn : m.attn_out; r.ldo = m.ld_attn; r.commit = (flags & STEP_NO_COMMIT_DELTA) ? 0 : 1;
     r.attn_scratch = x.attn_scratch; r.attn_counters = x.attn_counters; r.ssd_counters = x.ssd_counters;
     r.chunk_state = x.chunk_state; r.chunk_prev = x.chunk_prev; r.chunk_decay = x.chunk_decay;
+    r.older = 1;
     return r;
 }
 

@@ -189,7 +189,7 @@ struct MixRun {
     const RowMeta* rows; const int* seq_rows;             // rows of one sequence are consecutive
     int n_rows, n_seqs;
     void* qbuf;              // [rows][H][dp] normalised, rotated queries
-    void* xbc; int ld_xbc; int pad;                   // [rows][ld_xbc] x | B | C after convolution and SiLU (lightning: the projection rows)
+    void* xbc; int ld_xbc; int older;                 // older 1: as in DeltaParams (the step driver); [rows][ld_xbc] x | B | C after convolution and SiLU (lightning: the projection rows)
     float* dtb; int ld_dt; int splits;                    // [rows][ld_dt] step sizes; cache slices per attention row
     float* ubuf; int ld_u; int fuse_norm;                 // [rows][ld_u] what the recurrence's norm is taken of
     void* out; int ldo; int commit;                       // [rows][ldo]; commit 0: leave recurrent state alone

@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(SS_THREADS) ssd_step_kernel(const MixLayer L, 
     __shared__ float Bs[SS_WARPS * NB], Cs[SS_WARPS * NB], part[SS_WARPS][32], red[32];
     __shared__ int s_last;
     pdl_launch_dependents();
+    if (!R.older) pdl_wait();
     const int h = blockIdx.x, p0 = blockIdx.y * 32, sq = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int grp = h / (L.heads / L.groups), p = p0 + lane;
@@ -339,6 +340,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const MixLayer L, 
 // (2) the pass over the chunks: grid (ceil(N * Pp / 256), heads); leaves the state before every chunk as bf16 planes
 __global__ void __launch_bounds__(256) ssd_chunk_pass_kernel(const MixLayer L, const MixRun R, int chunks) {
     pdl_launch_dependents();
+    if (!R.older) pdl_wait();
     const int Pp = (L.P + 7) & ~7, h = blockIdx.y;
     const int i = blockIdx.x * 256 + threadIdx.x, n = i / Pp, p = i % Pp;
     const bool in = n < L.N, ok = in && p < L.P;

@@ -248,7 +248,7 @@ class MixLayer(C.Structure):
 
 class MixRun(C.Structure):
     _fields_ = [("proj", vp), ("ld_proj", i32), ("dt", i32), ("rows", vp), ("seq_rows", vp), ("n_rows", i32), ("n_seqs", i32),
-                ("qbuf", vp), ("xbc", vp), ("ld_xbc", i32), ("pad", i32), ("dtb", vp), ("ld_dt", i32), ("splits", i32),
+                ("qbuf", vp), ("xbc", vp), ("ld_xbc", i32), ("older", i32), ("dtb", vp), ("ld_dt", i32), ("splits", i32),
                 ("ubuf", vp), ("ld_u", i32), ("fuse_norm", i32), ("out", vp), ("ldo", i32), ("commit", i32),
                 ("attn_scratch", vp), ("attn_counters", vp), ("ssd_counters", vp),
                 ("chunk_state", vp), ("chunk_prev", vp), ("chunk_decay", vp)]

@@ -451,6 +451,24 @@ def test_recurrence_step(dt, shape):
         assert int(x.b["ssd_counters"].abs().sum()) == 0
 
 
+@pytest.mark.parametrize("op,n", [("ssd_step", 1), ("ssd_step", 5), ("ssd_chunk", 70)])
+def test_recurrences_in_a_row(op, n):
+    """Launch after launch on one state: each starts from what the one before left, although it may begin under it."""
+    x = Mix("bf16", **SHAPES[3])
+    x.rows([(0, 0, n)])
+    x.b["proj"][:n] = _rnd(n, x.ld).to(x.T).cuda()
+    S0, got = _rnd(3, x.heads, x.N, x.P, seed=4).cuda(), []
+    x.op("mix_prepare")
+    for i in range(8):
+        x.S.copy_(S0)
+        for _ in range(4):
+            x.op(op)
+            if i == 0:
+                torch.cuda.synchronize()
+        got.append(x.S.clone())
+    assert all(torch.equal(g, got[0]) for g in got)
+
+
 @pytest.mark.parametrize("shape", range(len(SHAPES)))
 @pytest.mark.parametrize("n", [3, 64, 65, 200])
 def test_recurrence_chunked(shape, n):
