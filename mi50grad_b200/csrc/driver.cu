@@ -526,7 +526,7 @@ static int run_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, int 
     if (L.kind != LIN_INT4) return cudaErrorNotSupported;
     GemmTcParams p;
     memset(&p, 0, sizeof(p));
-    p.qfrag = (const uint4*)L.w; p.szfrag = (const uint2*)L.sz;
+    p.qfrag = (const uint4*)L.w; p.szfrag = (const uint2*)L.sz; p.w_older = 1;
     p.K = L.K; p.KB = L.KB; p.NTL = L.NTL; p.G = L.G; p.off32 = L.off32; p.gshift = L.gshift;
     // Token tile, outputs per CTA (128, or 256 as two accumulators that share an activation tile) and K splits (only
     // where the product is added to the residual stream; the parts meet through atomic adds) with the least time by a
@@ -706,7 +706,7 @@ static int rows_impl(Driver* d, int T, int n_seqs, int flags, cudaStream_t s) {
         if (T > m.p_logit_rows || m.lm_head.kind != LIN_F16) return cudaErrorInvalidValue;
         GemmTcParams g;
         memset(&g, 0, sizeof(g));
-        g.K = m.lm_head.K; g.T = T; g.t_tile = T >= 512 ? 512 : ((T + 15) & ~15);
+        g.w_older = 1; g.K = m.lm_head.K; g.T = T; g.t_tile = T >= 512 ? 512 : ((T + 15) & ~15);
         g.n_valid = m.vocab_local; g.ldo = m.ld_logits; g.epi = TC_EPI_STORE_F32; g.out = m.p_logits; g.status = m.tc_status;
         CK(b2_gemm_f16_tc(&g, m.lm_head.w, m.lm_head.ldw, m.p_xn, m.H, s));
         d->launches++;
@@ -748,7 +748,7 @@ static int mixer_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, in
     if (d->mx.dt == DT_F32) {
         GemmF32Params p;
         memset(&p, 0, sizeof(p));
-        p.w = (const float*)L.w; p.x = (const float*)x; p.out = out; p.ldw = L.ldw; p.ldx = ldx; p.K = L.K; p.N = L.N; p.T = T;
+        p.w_older = 1; p.w = (const float*)L.w; p.x = (const float*)x; p.out = out; p.ldw = L.ldw; p.ldx = ldx; p.K = L.K; p.N = L.N; p.T = T;
         p.ldo = ldo; p.mode = mode; p.softcap = softcap;
         if (mode == DG_STORE) p.act_cols = act; else p.act = act;
         if (max_ks > 1) {
@@ -779,7 +779,7 @@ static int mixer_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, in
             }
         }
     }
-    p.K = L.K; p.T = T; p.t_tile = best_t > Tr ? Tr : best_t; p.k_splits = best_ks; p.m_halves = best_w;
+    p.w_older = 1; p.K = L.K; p.T = T; p.t_tile = best_t > Tr ? Tr : best_t; p.k_splits = best_ks; p.m_halves = best_w;
     p.ldo = ldo; p.out = out; p.status = d->m.tc_status; p.bf16 = 1; p.softcap = softcap;
     if (planes) { *planes = b2_gemm_tc_splits(L.K, best_ks); p.plane_stride = (long long)d->m.max_prefill * ldo; }
     p.n_valid = mode == DG_GATE_PAIR ? L.N / 2 : L.N;

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_f32_kernel(const GemmF32Param
     auto stage_x = [&](int kb) { stage_rows(xs + (kb % GF_STAGES) * BT * GF_LD, p.x, p.ldx, BT, t0, p.T, kb); };
 
     pdl_launch_dependents();
-    // weights do not depend on the kernel before
+    if (!p.w_older) pdl_wait();
     for (int s = 0; s < GF_STAGES - 1; ++s)
         if (s < KB) stage_w(s);
     pdl_wait();

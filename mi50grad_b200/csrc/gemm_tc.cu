@@ -143,6 +143,7 @@ gemm_int4_tc_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
     // the activations are; only the TMA warp and the epilogue wait for them.  (Decode
     // of 24 sequences at width 2048, 98 launches a token: 1.12 -> 1.00 ms.)
     pdl_launch_dependents();
+    if (!p.w_older) pdl_wait();
     // split-K: this CTA's k-blocks are [kb_lo, kb_lo + KB) of the p.KB blocks of the matrix
     const int per_kb = (p.KB + (int)gridDim.z - 1) / (int)gridDim.z;
     const int kb_lo = (int)blockIdx.z * per_kb;

@@ -41,7 +41,7 @@ struct GemmTcParams {
     int box_rows;            // set by the launcher: token rows per TMA load
     int act;                 // TC_EPI_SILU_PAIR: 1 = relu(gate) * up instead of silu(gate) * up
     int act_cols;            // TC_EPI_STORE_F16: SiLU on the outputs n < act_cols
-    int pad3;
+    int w_older;             // 1: packed weights were complete before the first kernel of this step started, and are read before the wait
 };
 
 // planes a launch with `want` splits over K columns leaves (no split is empty)

@@ -141,7 +141,8 @@ struct GemmF32Params {
     int ldw, ldx, K, N, T, ldo, mode, act;
     float softcap; int act_cols;
     long long plane_stride;  // DG_STORE_F32: floats between the planes of a product split over K (0: no split)
-    int max_splits, pad;
+    int max_splits;
+    int w_older;             // 1: w was complete before the first kernel of this step started, and is read before the wait
 };
 
 // ---- one mixer: windowed attention and / or a linear recurrence (csrc/attention_window.cu, csrc/ssd.cu).

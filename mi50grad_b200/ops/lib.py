@@ -124,7 +124,7 @@ class GemmTcParams(C.Structure):
                 ("stages", i32), ("out", vp), ("status", vp), ("m_halves", i32), ("dense", i32),
                 ("push", vp * MAX_TP), ("epoch", vp), ("part_stride", i64), ("push_tp", i32), ("push_rank", i32),
                 ("push_per", C.c_uint), ("k_splits", i32), ("cta_pair", i32), ("bf16", i32), ("softcap", f32),
-                ("plane_stride", i64), ("box_rows", i32), ("act", i32), ("act_cols", i32), ("pad3", i32)]
+                ("plane_stride", i64), ("box_rows", i32), ("act", i32), ("act_cols", i32), ("w_older", i32)]
 
 
 TC_EPI_STORE_F16, TC_EPI_SILU_PAIR, TC_EPI_STORE_F32, TC_EPI_RESID_F32 = 0, 1, 2, 3
@@ -231,7 +231,7 @@ class DenseGemvParams(C.Structure):
 
 class GemmF32Params(C.Structure):
     _fields_ = [("w", vp), ("x", vp), ("out", vp), ("ldw", i32), ("ldx", i32), ("K", i32), ("N", i32), ("T", i32), ("ldo", i32),
-                ("mode", i32), ("act", i32), ("softcap", f32), ("act_cols", i32), ("plane_stride", i64), ("max_splits", i32), ("pad", i32)]
+                ("mode", i32), ("act", i32), ("softcap", f32), ("act_cols", i32), ("plane_stride", i64), ("max_splits", i32), ("w_older", i32)]
 
 
 class MixLayer(C.Structure):

@@ -125,6 +125,25 @@ def test_gemm_f32_tiles_and_splits(N, K, T_, pad):
     _close(planes.sum(0), ref, 1e-5)
 
 
+def test_gemm_f32_of_an_operand_that_the_launch_before_writes():
+    """The "weights" are the product of the launch before, under whose end this one may begin."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    a, b, c = (_rnd(200, 512, seed=i).cuda() for i in range(3))
+    got = []
+    for i in range(6):
+        mid, out = torch.zeros(200, 200, device="cuda"), torch.zeros(200, 200, device="cuda")
+        x = c[:, :200].contiguous()
+        for _ in range(3):
+            K_.gemm_f32(a, b, mid, L.DG_STORE_F32)
+        if i == 0:
+            torch.cuda.synchronize()
+        K_.gemm_f32(mid, x, out, L.DG_STORE_F32)
+        got.append(out)
+    _close(got[0], c[:, :200].double().cpu() @ (b.double() @ a.double().T).cpu().T, 1e-5)
+    assert all(torch.equal(g, got[0]) for g in got)
+
+
 @pytest.mark.parametrize("N,K,T_", [(37, 90, 9), (300, 200, 64), (640, 1032, 130), (129, 4096, 511)])
 def test_many_row_gemms(N, K, T_):
     from mi50grad_b200.ops import kernels as K_
