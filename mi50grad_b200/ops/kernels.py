@@ -576,16 +576,18 @@ def gemv_dense(lin, x: Optional[torch.Tensor], out: torch.Tensor, mode: int = L.
 def gemm_f32(w: torch.Tensor, x: torch.Tensor, out: torch.Tensor, mode: int = L.DG_STORE, softcap: float = 0.0,
              act: int = L.ACT_SILU, act_cols: int = 0):
     """out[t][n] = x[t] . w[n] in true fp32.  A three-dimensional out [planes][T][N] has room for a product split over K,
-    which is the sum of the planes; returned are those that were written."""
+    which is the sum of the planes; returned are those that were written: one in every mode but an uncapped
+    DG_STORE_F32, whose planes alone can be added."""
     p = L.GemmF32Params()
     p.w, p.x, p.out, p.ldw, p.ldx, p.ldo = w.data_ptr(), x.data_ptr(), out.data_ptr(), w.stride(0), x.stride(0), out.stride(-2)
-    if out.dim() == 3:
-        p.max_splits, p.plane_stride = out.shape[0], out.stride(0)
+    room = out.shape[0] if out.dim() == 3 and mode == L.DG_STORE_F32 and softcap <= 0.0 else 1
+    if room > 1:
+        p.max_splits, p.plane_stride = room, out.stride(0)
     p.K, p.N, p.T, p.mode, p.softcap = x.shape[1], w.shape[0], x.shape[0], mode, softcap
     p.act, p.act_cols = act, act_cols
     L.check(L.lib().b2_gemm_f32(C.byref(p), L.stream()), "gemm_f32")
     if out.dim() == 3:
-        return out[:L.lib().b2_gemm_f32_splits(p.N, p.K, p.T, out.shape[0])]
+        return out[:L.lib().b2_gemm_f32_splits(p.N, p.K, p.T, room)]
     return out
 
 

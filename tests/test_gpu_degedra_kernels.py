@@ -125,6 +125,20 @@ def test_gemm_f32_tiles_and_splits(N, K, T_, pad):
     _close(planes.sum(0), ref, 1e-5)
 
 
+@pytest.mark.parametrize("mode,softcap", [("DG_STORE", 0.0), ("DG_STORE_F32", 5.0), ("DG_GATE_PAIR", 0.0)])
+def test_gemm_f32_with_room_for_planes_in_modes_without(mode, softcap):
+    """A shape that would be split over K: where the result is not a plain product, all of it is in the one plane returned."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    w, x = _rnd(96, 6144, std=6144 ** -0.5).cuda(), _rnd(49, 6144, seed=1).cuda()
+    assert L.lib().b2_gemm_f32_splits(96, 6144, 49, 4) > 1
+    n = 48 if mode == "DG_GATE_PAIR" else 96
+    flat, planes = torch.zeros(49, n, device="cuda"), torch.full((4, 49, n), float("nan"), device="cuda")
+    K_.gemm_f32(w, x, flat, getattr(L, mode), softcap)
+    got = K_.gemm_f32(w, x, planes, getattr(L, mode), softcap)
+    assert got.shape == (1, 49, n) and torch.equal(got[0], flat) and bool(planes[1:].isnan().all())
+
+
 def test_gemm_f32_of_an_operand_that_the_launch_before_writes():
     """The "weights" are the product of the launch before, under whose end this one may begin."""
     from mi50grad_b200.ops import kernels as K_
