@@ -44,6 +44,28 @@ log = logging.getLogger(__name__)
 PROMPT_ROWS = 4096
 PROMPT_ROWS_FIXED = 512
 
+
+def portion_passes(n: int, want: Sequence[int], few: int, wide: int, logit_rows: int, many: bool = True):
+    """Passes over n tokens of which the places `want` need logits: (first, count, whether logits are formed).  Up to `few`
+    rows go through the few-row step, as the end of a portion or, without a many-row path, all of it; a many-row pass
+    takes `wide` rows, with logits `logit_rows`.  Rows in front of the next wanted place run at full width: only the pass that
+    reaches it is cut."""
+    out, places, i = [], sorted(set(want)), 0
+    while i < n:
+        while places and places[0] < i:
+            places.pop(0)
+        rest, ahead = n - i, (places[0] if places else n) - i
+        if rest <= few or not many:
+            c = min(rest, few)
+        elif ahead >= logit_rows or not places:
+            c = min(wide, ahead)
+        else:
+            c = min(rest, wide, logit_rows)
+        out.append((i, c, ahead < c))
+        i += c
+    return out
+
+
 AR_MODE_ID = {"exact": 0, "deferred_ref": 1, "deferred_consistent": 2}
 
 
@@ -676,24 +698,15 @@ class InferenceEngine:
             self.decode_tokens(1, [seq], collect=False)
             keep(0, 1, self.buf["logits"])
             return out
-        i = 0
-        while i < n:
-            rest = n - i
-            if rest <= self.max_rows or not self.use_tc_prefill:
-                c = min(rest, self.max_rows)
-                hit = any(i <= w < i + c for w in want)
+        for i, c, hit in portion_passes(n, want, self.max_rows, self.max_prefill, self.step_rows, self.use_tc_prefill):
+            if c <= self.max_rows and (i + c == n or not self.use_tc_prefill):
                 self.step_tokens(tokens[i:i + c], seq, logits=hit)
                 keep(i, c, self.buf["logits"])
             else:
-                c = min(rest, self.max_prefill)
-                hit = any(i <= w < i + c for w in want)
-                if hit:
-                    c = min(c, self.step_rows)
-                    hit = any(i <= w < i + c for w in want)
                 self.buf["p_row_tokens"][:c].copy_(torch.tensor(tokens[i:i + c], dtype=torch.int32).to(self.device))
                 self._prefill_rows(c, seq, L.STEP_EMBED_TOKENS | (L.STEP_LM_HEAD if hit else 0))
-                keep(i, c, self.buf["p_logits"])
-            i += c
+                if hit:
+                    keep(i, c, self.buf["p_logits"])
         return out
 
     def score_tokens(self, tokens: Sequence[int], seq: int = 0) -> torch.Tensor:

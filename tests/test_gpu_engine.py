@@ -312,3 +312,26 @@ def test_long_prompt_in_one_pass_equals_passes_of_512():
     assert got[0][0] == got[1][0]
     for a, b in zip(got[0][1:], got[1][1:]):
         assert (a - b).abs().max() <= 2e-2 * b.abs().max()
+
+
+def test_long_portion_with_one_wanted_place_takes_few_passes():
+    """1000 tokens of which the last needs logits, with eight rows of logits to a step: the rows in front of it go through in one
+    pass, and the logits are those of feeding eight at a time."""
+    from mi50grad_b200.config import tiny_config
+    from mi50grad_b200.engine.engine import InferenceEngine
+    from mi50grad_b200.models.weights import random_model
+    cfg = tiny_config()
+    eng = InferenceEngine(cfg, max_seq_len=1100)
+    eng.load_model(random_model(cfg, 4))
+    ids = _prompt(cfg, 1000, seed=6)
+    eng._ensure_driver()
+    assert eng.step_rows == 8
+    before = eng._steps
+    got = eng.forward_tokens(ids, want=[999])
+    assert eng._steps - before <= 3
+    eng.states.reset(0)
+    for i in range(0, 1000, 8):
+        ref = eng.step_tokens(ids[i:i + 8])
+    ref = eng.buf["logits"][7:8, :cfg.vocab_size]
+    assert cosine(got[0].float().cpu(), ref[0].float().cpu()) > 0.999
+
