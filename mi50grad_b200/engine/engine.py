@@ -26,7 +26,7 @@ from typing import Dict, List, Optional, Sequence, Union
 import numpy as np
 import torch
 
-from ..config import EngineConfig, QwenConfig
+from ..config import PROMPT_ROWS, PROMPT_ROWS_FIXED, EngineConfig, QwenConfig, prompt_rows
 from ..models.weights import LayerWeights, ModelWeights
 from ..ops import lib as L
 from ..ops.packing import (PackedInt4, concat_out, concat_out_dense, interleave_gate_up, launch_shape,
@@ -36,13 +36,6 @@ from ..utils.quant import DenseLinear, Int4Linear
 from .state import SequenceStates
 
 log = logging.getLogger(__name__)
-
-# Rows of a prompt per pass over the layers.  A pass costs every projection whole waves of tiles over the SMs and a walk
-# over the weights, so few long passes beat many short ones; work buffers grow with it (27B: 0.75 GB for 4096 rows).
-# Measured: 3001 rows at width 4096 24.5 -> 18.3 ms against passes of 512.  Under tensor parallelism the exchange buffers, and
-# with INT8 activations the quantised rows, are sized for 512.
-PROMPT_ROWS = 4096
-PROMPT_ROWS_FIXED = 512
 
 
 def portion_passes(n: int, want: Sequence[int], few: int, wide: int, logit_rows: int, many: bool = True):
@@ -429,9 +422,9 @@ class InferenceEngine:
         b["out_tokens"] = i32(R)
         b["emb_in"] = f32(R, H)
         # prefill buffers (tensor-core path, up to max_prefill rows per launch)
-        short = self.tp_size > 1 or any(dl.ffn_q8 is not None for dl in self.layers)
-        P = self.max_prefill = min(PROMPT_ROWS_FIXED if short else PROMPT_ROWS, self.max_seq_len)
         self.use_tc_prefill = all(l.packed is not None for l in lins[:-1])
+        fixed = self.tp_size > 1 or not self.use_tc_prefill or any(dl.ffn_q8 is not None for dl in self.layers)
+        P = self.max_prefill = prompt_rows(self.ecfg, PROMPT_ROWS_FIXED if fixed else PROMPT_ROWS, self.max_seq_len)
         b["p_h"], b["p_xn"] = f32(P, H), f16(P, H)
         # sequence-parallel many-row steps: the activations live in symmetric memory, where every rank's
         # reduce-scatter + norm + all-gather kernel stores its rows

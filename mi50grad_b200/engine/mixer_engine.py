@@ -27,13 +27,13 @@ from typing import Dict, List, Optional, Sequence, Union
 import numpy as np
 import torch
 
-from ..config import EngineConfig, WindowAttentionSpec
+from ..config import EngineConfig, WindowAttentionSpec, prompt_rows
 from ..models.mixer_weights import MixerLayerWeights, MixerModelWeights, random_mixer_model
 from ..ops import lib as L
 from .engine import InferenceEngine
 from .state import MixerStates
 
-PROMPT_ROWS = 2048      # rows of a prompt per pass (the planes of split projections and the scan's states grow with it)
+PROMPT_ROWS = 2048      # rows of a prompt per pass unless the engine is given others (the planes of split projections and the scan's states grow with it)
 MAX_STEP_ROWS = 512     # rows of a step that can have logits
 
 DTYPES = {"bfloat16": (torch.bfloat16, L.DT_BF16, L.LIN_BF16), "float32": (torch.float32, L.DT_F32, L.LIN_F32)}
@@ -239,7 +239,7 @@ class MixerEngine(InferenceEngine):
         if any(l is None for l in self.layers) or self.embed is None or self.lm_head is None or self.final_norm is None:
             raise RuntimeError("weights are not fully loaded")
         cfg, R, T = self.config, self.max_rows, self.dtype
-        H, P = cfg.hidden_size, min(PROMPT_ROWS, self.max_seq_len)
+        H, P = cfg.hidden_size, prompt_rows(self.ecfg, PROMPT_ROWS, self.max_seq_len)
         self.max_prefill = P
         runs, n_runs = [self.layers[i] for i in self.runs], len(self.runs)
         alloc = self._work_allocator()

@@ -335,3 +335,21 @@ def test_long_portion_with_one_wanted_place_takes_few_passes():
     ref = eng.buf["logits"][7:8, :cfg.vocab_size]
     assert cosine(got[0].float().cpu(), ref[0].float().cpu()) > 0.999
 
+
+def test_prompt_passes_as_long_as_the_engine_was_told():
+    """Fewer rows per pass: smaller buffers, as the estimate says, and the same answer."""
+    from mi50grad_b200.config import EngineConfig, prompt_work_bytes, tiny_config
+    from mi50grad_b200.engine.engine import InferenceEngine
+    from mi50grad_b200.models.weights import random_model
+    cfg, got = tiny_config(), []
+    w, ids = random_model(cfg, 4), _prompt(cfg, 700, seed=7)
+    for rows in (0, 64):
+        eng = InferenceEngine(cfg, max_seq_len=800, engine_config=EngineConfig(max_prompt_rows=rows))
+        eng.load_model(w)
+        got.append(eng.generate_tokens(ids, 4))
+        assert eng.max_prefill == (rows or 800)
+        held = sum(t.numel() * t.element_size() for k, t in eng.buf.items() if k in (
+            "p_h", "p_xn", "p_proj", "p_attn", "p_act", "p_rows", "p_rows_tmpl", "p_row_tokens", "p_scan"))
+        assert 0.7 * held < prompt_work_bytes(cfg, eng.max_prefill) < 1.5 * held
+    assert got[0] == got[1]
+

@@ -47,3 +47,19 @@ def test_engine_switch_defaults_and_environment(monkeypatch):
     e = EngineConfig.from_env()
     assert e.ar_mode == "deferred_consistent" and not e.use_multimem
     assert e.replace(use_chain=1).use_chain == 1 and e.use_chain == 0
+
+
+def test_prompt_rows_and_their_memory():
+    """A pass takes the rows it was given, never more than the default or the sequence; the budget knows its buffers."""
+    import pytest
+    from mi50grad_b200.config import PROMPT_ROWS, EngineConfig, memory_budget, prompt_rows, prompt_work_bytes, qwen35_27b
+    assert prompt_rows(EngineConfig(), PROMPT_ROWS, 100000) == PROMPT_ROWS and prompt_rows(EngineConfig(), PROMPT_ROWS, 300) == 300
+    assert prompt_rows(EngineConfig(max_prompt_rows=512), PROMPT_ROWS, 100000) == 512
+    assert prompt_rows(EngineConfig(max_prompt_rows=9999), PROMPT_ROWS, 100000) == PROMPT_ROWS
+    with pytest.raises(ValueError):
+        EngineConfig(max_prompt_rows=8)
+    cfg = qwen35_27b()
+    work = prompt_work_bytes(cfg, 4096)
+    assert 0.65e9 < work < 0.75e9 and work == 8 * prompt_work_bytes(cfg, 512)
+    assert memory_budget(cfg, 4096)["scratch_gb"] >= work / 1e9
+
