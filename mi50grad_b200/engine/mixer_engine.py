@@ -259,9 +259,6 @@ class MixerEngine(InferenceEngine):
         b["logits"] = f32(R, b["ld_logits"])
         self.np = -(-H // 8)                                   # one partial sum per CTA of at least 8 outputs
         b["ss"] = f32(R, self.np)
-        M_PLANES = 4                                           # splits over K of a many-row output projection
-        b["p_h"], b["p_m"], b["p_xn"] = f32(P, H), f32(M_PLANES, P, H), elt(P, ld_x)
-        b["p_proj"], b["p_attn"], b["p_act"] = elt(P, b["ld_proj"]), elt(P, b["ld_attn"]), elt(P, ld_act)
         M = max(P, R)
         b["qbuf"] = elt(M, max([m.H * m.dp for m in att] + [8]))
         channels = [s.conv_channels for _, s in cfg.run_mixers() if s is not None]
@@ -274,17 +271,21 @@ class MixerEngine(InferenceEngine):
         b["attn_scratch"] = f32(max([self.lib.b2_window_attn_scratch(m.H, m.G, max(m.dp, m.vp), SR, self.attn_splits) for m in att] + [8]))
         b["attn_counters"] = i32(max([self.lib.b2_window_attn_units(m.H, m.G, SR) for m in att] + [0]) + 8)
         b["ssd_counters"] = i32(max([self.lib.b2_ssd_units(C.byref(m), SR) for m in rec] + [0]) + 8)
+        self.argmax_blocks = max(1, min(64, cfg.vocab_size // 2048))
+        b["argmax_scratch"], b["argmax_counters"] = f32(R * self.argmax_blocks * 2), i32(R + 8)
+        b["rows"], b["rows_tmpl"], b["seq_rows"] = i32(R, 6), i32(R, 6), i32(self.max_batch + 1 + R)
+        b["row_tokens"] = torch.full((R,), -1, dtype=torch.int32, device=self.device)
+        b["out_tokens"], b["tc_status"] = i32(R), i32(4)
+        # buffers of prompt passes only, behind those of the decode step
+        M_PLANES = 4                                           # splits over K of a many-row output projection
+        b["p_h"], b["p_m"], b["p_xn"] = f32(P, H), f32(M_PLANES, P, H), elt(P, ld_x)
+        b["p_proj"], b["p_attn"], b["p_act"] = elt(P, b["ld_proj"]), elt(P, b["ld_attn"]), elt(P, ld_act)
         if self.dt == L.DT_BF16 and rec:
             b["chunk_state"] = f32(max(self.lib.b2_ssd_chunk_state_floats(C.byref(m), P) for m in rec))
             b["chunk_prev"] = alloc((max(self.lib.b2_ssd_chunk_prev_bytes(C.byref(m), P) for m in rec),), torch.uint8)
             b["chunk_decay"] = f32(-(-P // 64) * ld_dt)
-        self.argmax_blocks = max(1, min(64, cfg.vocab_size // 2048))
-        b["argmax_scratch"], b["argmax_counters"] = f32(R * self.argmax_blocks * 2), i32(R + 8)
-        b["rows"], b["rows_tmpl"], b["p_rows"], b["p_rows_tmpl"] = i32(R, 6), i32(R, 6), i32(P, 6), i32(P, 6)
-        b["row_tokens"] = torch.full((R,), -1, dtype=torch.int32, device=self.device)
+        b["p_rows"], b["p_rows_tmpl"], b["p_out_tokens"] = i32(P, 6), i32(P, 6), i32(P)
         b["p_row_tokens"] = torch.full((P,), -1, dtype=torch.int32, device=self.device)
-        b["seq_rows"] = i32(self.max_batch + 1 + R)
-        b["out_tokens"], b["p_out_tokens"], b["tc_status"] = i32(R), i32(P), i32(4)
         # rows of a many-row step that can have logits: what the caller asked for, or 64 MB of them
         want = self.ecfg.max_step_rows or max(8 * self.max_batch, (64 << 20) // (4 * b["ld_logits"]))
         self.step_rows = min(P, MAX_STEP_ROWS, max(8, want))

@@ -68,3 +68,13 @@ def test_long_passes_equal_short_ones(kind, n):
     assert len(S) and len(kv)
     assert _worst(S, S2, 0.1) < BOUND[kind] and _worst(kv, kv2, 0.1) < BOUND[kind]
     assert float((lg - lg2).norm() / lg2.norm()) < BOUND[kind]
+
+
+@pytest.mark.parametrize("kind", ["degedra bfloat16", "vekerax bfloat16"])
+def test_buffers_of_the_decode_step_come_before_those_of_prompts(kind):
+    """The decode step's buffers do not lie between those of prompt passes, however long these are."""
+    eng = _engine(kind, 3000, 0)
+    eng._ensure_driver()
+    names = list(eng.buf)
+    decode = ["h", "xn", "proj", "attn_out", "act", "logits", "ss", "qbuf", "attn_scratch", "argmax_scratch", "rows", "row_tokens", "out_tokens"]
+    assert max(names.index(n) for n in decode) < min(names.index(n) for n in ("p_h", "p_m", "p_xn", "p_proj", "p_attn", "p_act", "p_logits"))
