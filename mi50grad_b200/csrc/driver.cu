@@ -89,7 +89,6 @@ struct ModelDesc {
     int max_prefill; int pad4;
     float* p_h; void* p_xn; void* p_proj; void* p_attn; void* p_act; float* p_partial;
     void* p_rows; void* p_rows_tmpl; int* p_row_tokens; int* tc_status;
-    void* p_ab;                            // [max_prefill][2*la_nv] fp16 a/b projections of the DeltaNet layers
     void* p_scan;                          // DeltaNet scan: b2_deltanet_tw_floats(la_nv, max_prefill) floats
     float* coll_gather[B2_MAX_TP]; float* coll_mc_gather; int* coll_counters;
     // many-row steps (batched decode, speculative verification): logits and arg-max scratch for p_logit_rows rows

@@ -437,7 +437,6 @@ class InferenceEngine:
         b["p_rows"], b["p_rows_tmpl"] = i32(P, 6), i32(P, 6)
         b["p_row_tokens"] = torch.full((P,), -1, dtype=torch.int32, device=dev)
         b["tc_status"] = i32(4)
-        b["p_ab"] = f16(P, max(2, 2 * sp.n_la_v))
         self.lib.b2_deltanet_tw_floats.restype = C.c_longlong
         b["p_scan"] = f32(max(4, int(self.lib.b2_deltanet_tw_floats(sp.n_la_v, P)) if len(self.states.dn.layers) else 0))
         b["coll_counters"] = i32(8)
@@ -493,7 +492,7 @@ class InferenceEngine:
             # (a communicator rebuilt by recover() has a new symmetric block)
             b["p_xn"] = self.comm.xn_view(self.max_prefill, self.config.hidden_size)
         for k in ("p_h", "p_xn", "p_proj", "p_attn", "p_act", "p_partial", "p_rows", "p_rows_tmpl", "p_row_tokens",
-                  "tc_status", "coll_counters", "p_ab", "p_scan"):
+                  "tc_status", "coll_counters", "p_scan"):
             setattr(m, k, b[k].data_ptr())
         for k in ("p_logits", "p_argmax_scratch", "p_argmax_counters", "p_out_tokens", "p_attn_scratch",
                   "p_attn_counters", "spec_acc", "spec_result"):

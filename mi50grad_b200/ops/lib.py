@@ -194,7 +194,7 @@ class ModelDesc(C.Structure):
                 ("out_tokens", vp),
                 ("max_prefill", i32), ("pad4", i32), ("p_h", vp), ("p_xn", vp), ("p_proj", vp), ("p_attn", vp),
                 ("p_act", vp), ("p_partial", vp), ("p_rows", vp), ("p_rows_tmpl", vp), ("p_row_tokens", vp),
-                ("tc_status", vp), ("p_ab", vp), ("p_scan", vp), ("coll_gather", vp * MAX_TP), ("coll_mc_gather", vp), ("coll_counters", vp),
+                ("tc_status", vp), ("p_scan", vp), ("coll_gather", vp * MAX_TP), ("coll_mc_gather", vp), ("coll_counters", vp),
                 ("p_logits", vp), ("p_argmax_scratch", vp), ("p_argmax_counters", vp), ("p_out_tokens", vp),
                 ("p_attn_scratch", vp), ("p_attn_counters", vp),
                 ("p_logit_rows", i32), ("n_lin_layers", i32), ("n_full_layers", i32), ("ab_off", i32),
