@@ -176,7 +176,14 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 // Launch `kern` so that it may become resident while its predecessor in the stream is still running
 // (programmatic dependent launch).  The kernel must call pdl_wait() before it reads anything that a
-// predecessor of the same step writes.
+// predecessor of the same step writes, with one exception: kernels of the step driver read row descriptors,
+// constant weights and what the step before left (states, histories) before they wait.  That is right because a step
+// begins with prepare_rows, a plain launch that does not trigger early: all that was launched before it is complete when
+// it starts, and it is complete when the kernel behind it starts.  So prepare_rows stays a plain launch without
+// pdl_launch_dependents(), and so do the kernels at the end of a verification that write states, caches and lengths
+// (spec_accept, deltanet_commit, kv_compact: plain; they may trigger early only because prepare_rows comes next).
+// DeltaParams.older, MixRun.older and w_older say that a launch belongs to such a step; without them the states and
+// weights are read behind the wait.
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
     cudaLaunchConfig_t cfg = {};
