@@ -527,32 +527,29 @@ static int run_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, int 
     memset(&p, 0, sizeof(p));
     p.qfrag = (const uint4*)L.w; p.szfrag = (const uint2*)L.sz; p.w_older = 1;
     p.K = L.K; p.KB = L.KB; p.NTL = L.NTL; p.G = L.G; p.off32 = L.off32; p.gshift = L.gshift;
-    // Token tile, outputs per CTA (128, or 256 as two accumulators that share an activation tile) and K splits (only
+    // Token tile, outputs per item (128, or 256 as two accumulators that share an activation tile) and K splits (only
     // where the product is added to the residual stream; the parts meet through atomic adds) with the least time by a
-    // model of one CTA per SM: whole waves of CTAs, each a walk over its k-blocks plus a start and an epilogue, and the
-    // traffic of the atomic adds.  us of a 64-k block, measured with one wave: 128 outputs: .39 at 16 tokens, .47 at 128,
-    // .51 at 192, .58 at 256 (to there four pipeline stages fit, beyond it two), .86 at 320, 1.1 at 512; 256 outputs: .64 at
-    // 16, .71 at 128, .84 at 192, .96 at 256.
-    // (256-output tiles of a residual product with few rows would need so many splits that the adds cost more than they
-    // give: at 80 rows the 27B verification step is 2% slower with them.)  Measured against one wave of the widest
-    // tile that fits: prompt of 512 at 27B 37.4 -> 36.1 ms, of 3001 at width 4096 17.5 -> 16.1 ms, of 77 1.78 -> 1.74 ms.
+    // model of one CTA per SM that walks over whole items: k-blocks, an epilogue, and once the launch.  us of a 64-k block, fitted
+    // to 148 CTAs with one to three items of 32 to 128 k-blocks: 128 outputs: .17 at 16 tokens, .205 at 80, .26 at 128, .34 at
+    // 192, .42 at 256; 256 outputs: .40, .415, .49 at 128, .645 at 192; an epilogue 1.5 to 6 us and 2 to 8.5, of the residual
+    // form up to twice that.
     auto block_us = [](int t, bool wide) -> double {
-        if (wide) return t <= 128 ? 0.625 + 0.00065 * t : 0.47 + 0.0019 * t;
-        return t <= 192 ? 0.375 + 0.0007 * t : (t <= 256 ? 0.30 + 0.0011 * t : 0.46 + 0.00125 * t);
+        if (wide) return t <= 80 ? 0.395 + 0.0002 * t : (t <= 128 ? 0.411 + 0.0016 * (t - 80) : 0.488 + 0.00245 * (t - 128));
+        return t <= 80 ? 0.165 + 0.0005 * t : 0.205 + 0.0012 * (t - 80);
     };
-    const bool wide_ok = d->gemm_m256 && (L.NTL * 16) % 256 == 0 && (epi == TC_EPI_STORE_F16 || epi == TC_EPI_SILU_PAIR || epi == TC_EPI_STORE_F32 ||
-                         (epi == TC_EPI_RESID_F32 && T >= 256));
+    const bool wide_ok = d->gemm_m256 && (L.NTL * 16) % 256 == 0;
     const int max_ks = epi == TC_EPI_RESID_F32 && d->gemm_splitk ? 8 : 1;
+    const double epi_f = epi == TC_EPI_RESID_F32 ? 1.8 : 1.0;
     int tt = 16, ks = 1;
     bool wide = false;
     double best = 1e30;
     for (int w = 0; w <= (wide_ok ? 1 : 0); ++w) {
-        const int ctas_n = L.NTL * 16 / (w ? 256 : 128), t_max = w ? 256 : 512, nt0 = (T + t_max - 1) / t_max;
+        const int ctas_n = L.NTL * 16 / (w ? 256 : 128), t_max = w ? 192 : 256, nt0 = (T + t_max - 1) / t_max;
         for (int nt = nt0; nt <= 2 * nt0 + 8; ++nt) {
             const int t = ((T + nt - 1) / nt + 15) & ~15;
             for (int k = 1; k <= max_ks && (k == 1 || L.KB / k >= 8); ++k) {
                 const int waves = (ctas_n * ((T + t - 1) / t) * k + 147) / 148;
-                const double cost = waves * ((L.KB + k - 1) / k * block_us(t, w) + 6.0 + 0.01 * t) + (k > 1 ? 2e-6 * k * T * n_valid : 0.0);
+                const double cost = waves * ((L.KB + k - 1) / k * block_us(t, w) + epi_f * (w ? 2.5 + 0.031 * t : 1.5 + 0.0165 * t)) + (k > 1 ? 1e-6 * k * T * n_valid : 0.0);
                 if (cost < best - 1e-9) { best = cost; tt = t; ks = k; wide = w; }
             }
         }

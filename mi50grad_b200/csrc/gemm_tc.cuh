@@ -1,4 +1,4 @@
-// Parameters of the tcgen05 INT4 GEMM (csrc/gemm_tc.cu).
+// Parameters of the tcgen05 GEMMs (csrc/gemm_int4.cu, csrc/gemm_tc.cu).
 #pragma once
 #include "common.cuh"
 
@@ -19,9 +19,8 @@ struct GemmTcParams {
     int n_valid, ldo, epi, stages;
     void* out;
     int* status;             // [0] set to 1 when a bounded wait expired
-    int m_halves;            // 2: CTAs own 256 outputs (two accumulators sharing each activation tile; t_tile <= 256,
-                             // N a multiple of 256); else 128 outputs
-    int dense;               // set by the launcher: weights are fp16 and come through a tensor map
+    int m_halves;            // 2: CTAs own 256 outputs (two accumulators sharing each activation tile; t_tile <= 256, INT4
+                             // weights 192 and N a multiple of 256); else 128 outputs
     // TC_EPI_PUSH_F32: the flattened output (float4 units) is cut into push_tp slices of push_per; slice o
     // lives on rank o at push[o] + parity offset + (push_rank * push_per + index in slice) * 4 floats
     float* push[B2_MAX_TP];
@@ -33,8 +32,8 @@ struct GemmTcParams {
                                  // partial products are added to out with atomic adds; TC_EPI_STORE_F32 with
                                  // plane_stride: split z stores its own plane, which the consumer sums
                                  // (b2_gemm_tc_splits gives the number of planes)
-    int cta_pair;                // 1: adjacent output tiles run as CTA pairs (cta_group::2 MMAs, M = 256 over two SMs); needs
-                                 // 128-output CTAs, t_tile 256 or 512, and (INT4 weights) an even number of output tiles
+    int cta_pair;                // 1 (dense weights only): adjacent output tiles run as CTA pairs (cta_group::2 MMAs, M = 256 over
+                                 // two SMs); needs 128-output CTAs and t_tile 256 or 512
     int bf16;                // 1 (dense weights only): operands and 16-bit outputs are bf16 instead of fp16
     float softcap;           // TC_EPI_STORE_F32: > 0 stores softcap * tanh(y / softcap)
     long long plane_stride;  // floats between the planes of a split-K TC_EPI_STORE_F32

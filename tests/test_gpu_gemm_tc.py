@@ -162,3 +162,48 @@ def test_gemm_f16_tc_dense_weights(T, N, K):
     ref = x.float() @ w.float().t()
     err = (out[:, :N] - ref).abs().max().item()
     assert err < 2e-3 * max(1.0, ref.abs().max().item()), err
+
+
+@pytest.mark.parametrize("K,N,T,tt,mh,g", [
+    (64, 128, 1, 16, 1, 32),            # a single k-block, half a slot
+    (192, 128, 17, 32, 1, 64),          # an odd number of k-blocks: the second group of warps has one step less
+    (320, 256, 33, 16, 2, 128),         # three token tiles, a ragged one, with two accumulators
+    (704, 200, 65, 80, 1, 128),         # outputs behind the last that is wanted
+    (4096, 256, 192, 192, 2, 128),      # the widest tile with two accumulators: one k-block per slot
+    (448, 512, 193, 512, 2, 256),       # one token too many for it, a group longer than a slot
+    (2048, 128, 257, 512, 1, 128),      # one token more than the widest tile
+    (1024, 20480, 48, 16, 1, 128),      # more items than CTAs: three or four a CTA
+    (192, 37888, 20, 32, 2, 128),       # the same, two accumulators and an odd number of k-blocks
+])
+def test_gemm_int4_tc_items_slots_and_edges(K, N, T, tt, mh, g):
+    """All output forms at the edges of tiles, slots and the walk over items, against the product of the weights as the
+    kernel rounds them.  Bound: a sum of K products in steps of 16 of which each may lose one unit in the last place."""
+    from mi50grad_b200.ops import kernels as Kn
+    from mi50grad_b200.ops import lib as L
+    from mi50grad_b200.ops.packing import pack_int4
+    from mi50grad_b200.utils.quant import random_int4_linear
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator().manual_seed(K + N + T)
+    lin = random_int4_linear(K, N, g, gen)
+    lin.zeros = torch.randint(0, 16, lin.zeros.shape, generator=gen).half()
+    x = torch.randn(T, K, generator=gen).half().to(dev)
+    w = lin.dense().half().to(dev).double()
+    ref, mag = x.double() @ w.t(), x.double().abs() @ w.t().abs()
+    pk = pack_int4(lin, dev)
+    bound = (K / 16 + 4) * 2.0 ** -23 * mag
+    h0 = torch.randn(T, N, device=dev)
+    for pad in (0, 3):                  # rows of outputs off the 16-byte boundary take the scalar stores
+        for epi, ks in ((L.TC_EPI_STORE_F32, 1), (L.TC_EPI_RESID_F32, 1), (L.TC_EPI_RESID_F32, 3), (L.TC_EPI_STORE_F16, 1)):
+            dt = torch.float16 if epi == L.TC_EPI_STORE_F16 else torch.float32
+            buf = torch.full((T, N + pad), 7.0, dtype=dt, device=dev)
+            out = buf[:, :N]
+            resid = epi == L.TC_EPI_RESID_F32
+            if resid:
+                out.copy_(h0)
+            Kn.gemm_int4_tc(pk, x, out, epi=epi, t_tile=tt, m_halves=mh, k_splits=ks)
+            torch.cuda.synchronize()
+            Kn.gemm_tc_check_status()
+            want = ref + h0 if resid else ref
+            lim = bound + (2.0 ** -11 * ref.abs() + 2.0 ** -24 if dt == torch.float16 else (ks + 1) * 2.0 ** -23 * (mag + h0.abs()))
+            assert bool(((out.double() - want).abs() <= lim).all()), (epi, ks, pad)
+            assert bool((buf[:, N:] == 7.0).all())
