@@ -744,7 +744,7 @@ static int mixer_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, in
     if (d->mx.dt == DT_F32) {
         GemmF32Params p;
         memset(&p, 0, sizeof(p));
-        p.w_older = 1; p.w = (const float*)L.w; p.x = (const float*)x; p.out = out; p.ldw = L.ldw; p.ldx = ldx; p.K = L.K; p.N = L.N; p.T = T;
+        p.w_older = 1; p.status = d->m.tc_status; p.w = (const float*)L.w; p.x = (const float*)x; p.out = out; p.ldw = L.ldw; p.ldx = ldx; p.K = L.K; p.N = L.N; p.T = T;
         p.ldo = ldo; p.mode = mode; p.softcap = softcap;
         if (mode == DG_STORE) p.act_cols = act; else p.act = act;
         if (max_ks > 1) {

@@ -1,16 +1,17 @@
 // Many-row projection in true fp32 (no reduced-precision matrix mode): out[t][n] = sum_k x[t][k] w[n][k].
-// It serves models that run entirely in 32 bits.
+// It serves models that run entirely in 32 bits.  Operands whose rows start on 16-byte boundaries, as an engine's do, go to the
+// tensor cores in three bf16 terms each (csrc/gemm_f32_tc.cu); this file has the plan of the splits over K for both, and the
+// kernel for all other operands:
 //
 // Bound: the FMA pipes (74 TFLOP/s).  A CTA of 128 threads owns [8 RT tokens x 128 outputs], a thread RT x 8 of them.
 // Both operands are contiguous in k, so they go from global memory into shared memory as they are (cp.async, four
 // stages of 16 k; rows of 20 floats, so that the 16-byte reads of 8 adjacent rows meet no bank twice) and two
 // adjacent k form one packed FMA (fma.rn.f32x2): half the issue slots, and no operand has to be duplicated.  An
-// output is the sum of its even-k and its odd-k chain.  RT and the splits over K are chosen by b2_gemm_f32 /
-// b2_gemm_f32_splits.
+// output is the sum of its even-k and its odd-k chain.
 // Operands reach the registers at 32 floats a clock and an 8 x 8 thread tile asks for a quarter of a float per FMA, so
 // shared memory and the FMA pipes are about equally busy.  Measured in a prompt of 200 rows (12 layers of width 2048):
-// 30 TFLOP/s, the whole prompt 14.5 ms; 64 x 64 tiles staged by scalar loads gave 5.6 TFLOP/s and 55.9 ms.
-#include "mixers.cuh"
+// 30 TFLOP/s, the whole prompt 14.5 ms; on the tensor cores 6.4 ms.
+#include "gemm_f32.cuh"
 
 #define GF_BN 128
 #define GF_K 16
@@ -18,22 +19,17 @@
 #define GF_STAGES 4
 #define GF_THREADS 128
 
-// B bytes (16 or 4), of which the last B - valid are zeros
-template <int B>
+// four bytes, or (valid 0) a zero
 __device__ __forceinline__ void cp_async_zfill(float* dst, const float* src, int valid) {
-    if constexpr (B == 16)
-        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(valid) : "memory");
 }
 __device__ __forceinline__ void fma_x2(unsigned long long& c, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
 }
 
-// VEC: floats per copy (4: rows of both operands start on 16-byte boundaries; 1: any)
-template <int RT, int VEC>
+template <int RT>
 __global__ void __launch_bounds__(GF_THREADS) gemm_f32_kernel(const GemmF32Params p) {
-    constexpr int BT = 8 * RT, PER_ROW = GF_K / VEC;
+    constexpr int BT = 8 * RT;
     extern __shared__ float4 gf_smem[];
     float* ws = (float*)gf_smem;                          // [GF_STAGES][GF_BN][GF_LD]
     float* xs = ws + GF_STAGES * GF_BN * GF_LD;           // [GF_STAGES][BT][GF_LD]
@@ -43,10 +39,10 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_f32_kernel(const GemmF32Param
     const int kb0 = (int)blockIdx.z * per, KB = max(0, min(blocks, kb0 + per) - kb0);
     // rows beyond the matrix and columns beyond K are zeros
     auto stage_rows = [&](float* dst, const float* src, int ld, int rows, int row0, int row_end, int kb) {
-        for (int i = tid; i < rows * PER_ROW; i += GF_THREADS) {
-            const int r = i / PER_ROW, c = (i % PER_ROW) * VEC, k = (kb0 + kb) * GF_K + c;
-            const int valid = row0 + r < row_end ? max(0, min(VEC, p.K - k)) * 4 : 0;
-            cp_async_zfill<VEC * 4>(dst + r * GF_LD + c, valid ? src + (size_t)(row0 + r) * ld + k : src, valid);
+        for (int i = tid; i < rows * GF_K; i += GF_THREADS) {
+            const int r = i / GF_K, c = i % GF_K, k = (kb0 + kb) * GF_K + c;
+            const int valid = row0 + r < row_end && k < p.K ? 4 : 0;
+            cp_async_zfill(dst + r * GF_LD + c, valid ? src + (size_t)(row0 + r) * ld + k : src, valid);
         }
     };
     auto stage_w = [&](int kb) { stage_rows(ws + (kb % GF_STAGES) * GF_BN * GF_LD, p.w, p.ldw, GF_BN, n0, p.N, kb); };
@@ -117,37 +113,28 @@ __global__ void __launch_bounds__(GF_THREADS) gemm_f32_kernel(const GemmF32Param
     }
 }
 
-template <int RT, int VEC>
+template <int RT>
 static int launch_f32(const GemmF32Params* p, int splits, cudaStream_t s) {
     constexpr size_t smem = (size_t)GF_STAGES * (GF_BN + 8 * RT) * GF_LD * 4;
     static SmemOptIn optin;
-    if (cudaError_t e = optin.ensure(gemm_f32_kernel<RT, VEC>, smem)) return e;
+    if (cudaError_t e = optin.ensure(gemm_f32_kernel<RT>, smem)) return e;
     const dim3 grid((p->N + GF_BN - 1) / GF_BN, (p->T + 8 * RT - 1) / (8 * RT), splits);
-    return launch_pdl(gemm_f32_kernel<RT, VEC>, grid, dim3(GF_THREADS), smem, s, *p);
+    return launch_pdl(gemm_f32_kernel<RT>, grid, dim3(GF_THREADS), smem, s, *p);
 }
 
-// Tokens of a CTA (8 rt) and splits over K with the least time on the busiest SM.  Measured, us a 16-k block with n CTAs
-// on an SM: about 0.5 + s n, s = .38, .54, .62, .73, .85, 1.02 for rt = 2, 4, 5, 6, 7, 8 (one CTA alone does not cover its own
-// latencies, so splits pay beyond one CTA an SM: 200 rows, 4096 -> 2048 in two splits 192 us, in four 129 us); a start
-// and an end cost 10, a further plane 1 in its consumer.
-static void plan_f32(int N, int K, int T, int max_splits, int* rt, int* splits) {
-    static const double slope[9] = {0, 0, 0.38, 0, 0.54, 0.62, 0.73, 0.85, 1.02};
-    const int nt = (N + GF_BN - 1) / GF_BN, blocks = (K + GF_K - 1) / GF_K;
-    double best = 1e30;
-    for (int r = 8; r >= 2; --r) {
-        if (r == 3) continue;
-        for (int want = 1; want <= max_splits; ++want) {
-            const int per = (blocks + want - 1) / want, ks = (blocks + per - 1) / per;      // no split is empty
-            const int n = (nt * ((T + 8 * r - 1) / (8 * r)) * ks + 147) / 148;
-            const double cost = per * (0.5 + slope[r] * n) + 10.0 + (ks - 1);
-            if (cost < best - 1e-9) { best = cost; *rt = r; *splits = ks; }
-        }
-    }
-}
+// Splits over K with the least time on the busiest SM: a 64-k block of t <= 128 tokens takes a tensor-core CTA about 0.95 +
+// 0.003 t us (9 tokens 1.0, 128 tokens 1.3), a start and an end 5, a further plane 1 in its consumer; whole waves of CTAs.
+static int tc_tile_f32(int T) { const int n = (T + 127) / 128; return ((T + n - 1) / n + 15) & ~15; }
 B2_API int b2_gemm_f32_splits(int N, int K, int T, int max_splits) {
-    int rt = 8, ks = 1;
-    plan_f32(N, K, T, max_splits < 1 ? 1 : max_splits, &rt, &ks);
-    return ks;
+    const int t = tc_tile_f32(T), ctas = (N + 127) / 128 * ((T + t - 1) / t), blocks = (K + 63) / 64;
+    int best = 1;
+    double least = 1e30;
+    for (int want = 1; want <= (max_splits < 1 ? 1 : max_splits); ++want) {
+        const int per = (blocks + want - 1) / want, ks = (blocks + per - 1) / per, waves = (ctas * ks + 147) / 148;      // no split is empty
+        const double cost = waves * (per * (0.95 + 0.003 * t) + 5.0) + (ks - 1);
+        if (cost < least - 1e-9) { least = cost; best = ks; }
+    }
+    return best;
 }
 
 // p->max_splits > 1 (DG_STORE_F32 without a cap): the product may be split over K; split z stores its own plane,
@@ -156,16 +143,26 @@ B2_API int b2_gemm_f32(const GemmF32Params* p, cudaStream_t s) {
     if (p->T < 1 || p->N < 1 || p->K < 1 || p->ldx < p->K || p->ldw < p->K) return cudaErrorInvalidValue;
     if (p->mode == DG_GATE_PAIR && (p->N & 15)) return cudaErrorInvalidValue;
     const bool planes = p->mode == DG_STORE_F32 && p->softcap <= 0.f && p->plane_stride > 0;
-    int rt = 8, ks = 1;
-    plan_f32(p->N, p->K, p->T, planes && p->max_splits > 1 ? p->max_splits : 1, &rt, &ks);
-    const bool vec = !((p->ldx | p->ldw) & 3) && !(((uintptr_t)p->x | (uintptr_t)p->w) & 15);
+    const int ks = b2_gemm_f32_splits(p->N, p->K, p->T, planes && p->max_splits > 1 ? p->max_splits : 1);
+    if (!((p->ldx | p->ldw) & 3) && !(((uintptr_t)p->x | (uintptr_t)p->w) & 15)) return gemm_f32_tc_launch(p, tc_tile_f32(p->T), ks, s);
+    // Tokens of an FMA CTA (8 rt): us a 16-k block with n CTAs on an SM, about 0.5 + s n, s = .38, .54, .62, .73, .85, 1.02 for
+    // rt = 2, 4, 5, 6, 7, 8 (one CTA alone does not cover its own latencies)
+    static const double slope[9] = {0, 0, 0.38, 0, 0.54, 0.62, 0.73, 0.85, 1.02};
+    int rt = 8;
+    double least = 1e30;
+    for (int r = 8; r >= 2; --r) {
+        if (r == 3) continue;
+        const int n = ((p->N + GF_BN - 1) / GF_BN * ((p->T + 8 * r - 1) / (8 * r)) * ks + 147) / 148;
+        const double cost = 0.5 + slope[r] * n;
+        if (cost < least - 1e-9) { least = cost; rt = r; }
+    }
     switch (rt) {
-        case 2: return vec ? launch_f32<2, 4>(p, ks, s) : launch_f32<2, 1>(p, ks, s);
-        case 4: return vec ? launch_f32<4, 4>(p, ks, s) : launch_f32<4, 1>(p, ks, s);
-        case 5: return vec ? launch_f32<5, 4>(p, ks, s) : launch_f32<5, 1>(p, ks, s);
-        case 6: return vec ? launch_f32<6, 4>(p, ks, s) : launch_f32<6, 1>(p, ks, s);
-        case 7: return vec ? launch_f32<7, 4>(p, ks, s) : launch_f32<7, 1>(p, ks, s);
-        default: return vec ? launch_f32<8, 4>(p, ks, s) : launch_f32<8, 1>(p, ks, s);
+        case 2: return launch_f32<2>(p, ks, s);
+        case 4: return launch_f32<4>(p, ks, s);
+        case 5: return launch_f32<5>(p, ks, s);
+        case 6: return launch_f32<6>(p, ks, s);
+        case 7: return launch_f32<7>(p, ks, s);
+        default: return launch_f32<8>(p, ks, s);
     }
 }
 B2_API int b2_sizeof_gemm_f32_params() { return (int)sizeof(GemmF32Params); }

@@ -143,6 +143,7 @@ struct GemmF32Params {
     long long plane_stride;  // DG_STORE_F32: floats between the planes of a product split over K (0: no split)
     int max_splits;
     int w_older;             // 1: w was complete before the first kernel of this step started, and is read before the wait
+    int* status;             // optional: [0] set to 1 when a bounded wait expired (the result is right all the same)
 };
 
 // ---- one mixer: windowed attention and / or a linear recurrence (csrc/attention_window.cu, csrc/ssd.cu).

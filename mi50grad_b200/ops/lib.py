@@ -231,7 +231,7 @@ class DenseGemvParams(C.Structure):
 
 class GemmF32Params(C.Structure):
     _fields_ = [("w", vp), ("x", vp), ("out", vp), ("ldw", i32), ("ldx", i32), ("K", i32), ("N", i32), ("T", i32), ("ldo", i32),
-                ("mode", i32), ("act", i32), ("softcap", f32), ("act_cols", i32), ("plane_stride", i64), ("max_splits", i32), ("w_older", i32)]
+                ("mode", i32), ("act", i32), ("softcap", f32), ("act_cols", i32), ("plane_stride", i64), ("max_splits", i32), ("w_older", i32), ("status", vp)]
 
 
 class MixLayer(C.Structure):

@@ -546,3 +546,49 @@ def test_recurrence_keeps_a_distant_token():
     other = proj.clone()
     other[3] = 0
     assert float((x.ref_ssd(other)[0] - out)[-50:].abs().mean()) > 0.1
+
+
+@pytest.mark.parametrize("N,K,T_", [(1, 4, 1), (128, 64, 16), (129, 68, 17), (200, 132, 128), (300, 1000, 129), (2048, 520, 257)])
+def test_gemm_f32_three_terms(N, K, T_):
+    """Edges of the tensor-core tiles (128 outputs, 128 tokens, 64 k), with weights that are bf16 numbers in some 64-k blocks
+    and rows and need all 24 bits in others.  Bound: half a unit in the last place for each of K / 64 additions and for the
+    products left out (2 ** -24 of their size each), and one unit for each of the four steps of a block that the tensor core cuts off."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    w, x = _rnd(N, K).cuda(), _rnd(T_, K, seed=1).cuda()
+    w[:, 64:192] = w[:, 64:192].bfloat16().float()
+    w[N // 2:] = w[N // 2:].bfloat16().float()
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    bound = 2.0 ** -24 * (K / 64 + 2 + 8) * mag
+    out = torch.full((T_, N), float("nan"), device="cuda")
+    K_.gemm_f32(w, x, out, L.DG_STORE_F32)
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    planes = torch.full((4, T_, N), float("nan"), device="cuda")
+    got = K_.gemm_f32(w, x, planes, L.DG_STORE_F32).sum(0)
+    assert bool(((got.double() - ref).abs() <= bound + 2.0 ** -22 * mag).all())
+
+
+def test_gemm_f32_infinities_and_the_largest_numbers():
+    """What does not fit three bf16 terms comes out as in fp32 arithmetic: infinities, NaNs, numbers above the largest bf16."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    w, x = _rnd(130, 96).cuda(), _rnd(20, 96, seed=1).cuda()
+    top = 3.4e38                                   # rounds to infinity as bf16
+    x[3, 5], w[7, 5] = float("inf"), 0.25
+    x[4, 9] = float("nan")
+    x[5] = 0.0
+    x[5, 0], w[:, 0] = top, 0.5
+    x[6], x[6, 1] = 0.0, 2.0
+    w[9] = 0.0
+    w[9, 1] = -top / 4
+    w[11] = 0.0                                    # an infinity times zero
+    x[8] = 1e-30
+    w[12] = 1e-30                                  # below the smallest normal number
+    out = torch.zeros(20, 130, device="cuda")
+    K_.gemm_f32(w, x, out, L.DG_STORE_F32)
+    ref = x.double() @ w.double().T
+    finite = ref.isfinite() & (ref.abs() < 3.4028e38)
+    finite[4] = False
+    assert bool(out[4].isnan().all()) and bool(torch.equal(out[3].isnan(), ref[3].isnan())) and float(out[3, 7]) == float("inf")
+    assert bool(((out.double() - ref).abs()[finite] <= 1e-5 * (x.double().abs() @ w.double().abs().T)[finite] + 1e-37).all())
+    assert bool(out[5].isfinite().all()) and float(out[6, 9]) == 2.0 * float(torch.tensor(-top / 4, dtype=torch.float32))
