@@ -592,3 +592,28 @@ def test_gemm_f32_infinities_and_the_largest_numbers():
     assert bool(out[4].isnan().all()) and bool(torch.equal(out[3].isnan(), ref[3].isnan())) and float(out[3, 7]) == float("inf")
     assert bool(((out.double() - ref).abs()[finite] <= 1e-5 * (x.double().abs() @ w.double().abs().T)[finite] + 1e-37).all())
     assert bool(out[5].isfinite().all()) and float(out[6, 9]) == 2.0 * float(torch.tensor(-top / 4, dtype=torch.float32))
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f32"])
+@pytest.mark.parametrize("shape", range(len(SHAPES)))
+@pytest.mark.parametrize("n", [2, 4, 8, 9, 17])
+def test_recurrence_turns(dt, shape, n):
+    """Several tokens a turn (eight, or four of a state of 256) give the bits of one token a launch."""
+    x = Mix(dt, **SHAPES[shape])
+    x.rows([(0, 0, n)])
+    x.r.fuse_norm = 0
+    x.b["proj"][:n] = _rnd(n, x.ld).to(x.T).cuda()
+    S0 = _rnd(3, x.heads, x.N, x.P, seed=4).cuda()
+    x.S.copy_(S0)
+    x.op("mix_prepare")
+    x.op("ssd_step")
+    S, u = x.S.clone(), x.b["ubuf"][:n].clone()
+    rows = {k: x.b[k][:n].clone() for k in ("proj", "xbc", "dtb")}
+    x.S.copy_(S0)
+    x.rows([(0, 0, 1)])
+    for i in range(n):
+        for k, t in rows.items():
+            x.b[k][0] = t[i]
+        x.op("ssd_step")
+        assert torch.equal(x.b["ubuf"][0], u[i])
+    assert torch.equal(x.S, S)
