@@ -236,6 +236,7 @@ static int run_linear(Driver* d, const LinearDesc& L, const void* x, int ldx, co
     memset(&p, 0, sizeof(p));
     p.w = (const __half*)L.w; p.x = (const __half*)x; p.ldw = L.ldw; p.ldx = ldx; p.rows = rows;
     p.K = L.K; p.N = L.N; p.k_splits = L.k_splits; p.kslice = L.kslice;
+    b2_gemv_f16_shape(L.K, rows, &p.k_splits, &p.kslice);
     p.scratch = d->m.gemv_scratch; p.counters = d->m.gemv_counters; p.ln = ln; p.epi = epi; p.comm = d->m.comm;
     return b2_gemv_f16(&p, s);
 }

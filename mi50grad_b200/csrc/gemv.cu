@@ -39,6 +39,7 @@ namespace cg = cooperative_groups;
 #define GEMV_NT 4            // 16-wide n-tiles per warp
 #define GEMV_STAGE_UN 3         // activation items per thread whose loads are in flight together
 #define GEMV_TILE_N (GEMV_WN * GEMV_NT * 16)   // 128
+#define GEMV_RED_FLOATS (GEMV_WK * GEMV_WN * GEMV_NT * 128 + B2_MAX_ROWS * GEMV_TILE_N)
 #define GEMV_STAGES 4        // cp.async ring depth per warp (k64-blocks in flight)
 
 __device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
@@ -375,13 +376,15 @@ __device__ __forceinline__ void prefetch_next_weights(const GemvInt4Params& p, i
 // ---------------------------------------------------------------------------
 // INT4 kernel
 // ---------------------------------------------------------------------------
-template <bool FAST>
+// ONE: a single row, as in decode of one sequence
+template <bool FAST, bool ONE>
 __global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_int4_kernel(const GemvInt4Params p) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wn = warp % GEMV_WN, wk = warp / GEMV_WN;
     const int g = lane >> 2, t = lane & 3;
-    const int M = p.rows;
+    constexpr int UN = ONE ? GEMV_STAGE_UN : GEMV_STAGE_UN + 1;
+    const int M = ONE ? 1 : p.rows;
     const int maxCh = 2 * GEMV_WK * p.L;
     const int cta_b0 = blockIdx.y * (GEMV_WK * p.L);
     const int cta_b1 = min(p.KB, cta_b0 + GEMV_WK * p.L);
@@ -390,10 +393,13 @@ __global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_int4_kernel(const GemvIn
 
     uint4* xf = (uint4*)smem;                                        // [maxCh][M][4] (+1 zero entry)
     float2* cs = (float2*)(smem + ((size_t)maxCh * M * 4 + 4) * 16); // [maxCh][8]
-    float* redbuf = (float*)((unsigned char*)cs + (size_t)maxCh * 8 * 8);   // [WK*WN*NT*128]
-    float* ybuf = redbuf + GEMV_WK * GEMV_WN * GEMV_NT * 128;        // [8][128]
-    float* red32 = ybuf + B2_MAX_ROWS * GEMV_TILE_N;                 // [32]
+    // (several rows: the buffers of the reduction take the place of the weight ring, which is read by then; so two CTAs fit an
+    // SM up to seven rows of slices of 2560: 5 rows of 17408 -> 5120 24.9 -> 17.2 us; of 5120 -> 16384 23.8 -> 17.8)
+    unsigned char* mid = (unsigned char*)cs + (size_t)maxCh * 8 * 8;
+    float* red32 = (float*)mid + (ONE ? GEMV_RED_FLOATS : 0);      // [32]
     int* s_flag = (int*)(red32 + 32);          // 4 ints, then the weight ring (16-byte aligned)
+    float* redbuf = ONE ? (float*)mid : (float*)(s_flag + 4);      // [WK*WN*NT*128]
+    float* ybuf = redbuf + GEMV_WK * GEMV_WN * GEMV_NT * 128;        // [8][128]
 
     // ---- this warp owns GEMV_NT n-tiles (contiguous in memory per k-block) over blocks [wb0, wb1).
     // Weights stream through a per-warp cp.async ring: GEMV_STAGES-1 blocks of 2 KB are in
@@ -443,20 +449,31 @@ __global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_int4_kernel(const GemvIn
     if (tid < 4) xf[(size_t)maxCh * M * 4 + tid] = make_uint4(0u, 0u, 0u, 0u);
     const int items = nCh * 4;
     float* s_inv = red32;                       // [rows] 1/rms per row when the input is lazy-normed
-    // Loads first, arithmetic after: the inputs of up to GEMV_STAGE_UN items per thread (and, under them, the
+    // Loads first, arithmetic after: the inputs of up to UN items per thread (and, under them, the
     // partial sums of squares of the lazy RMSNorm) are requested before anything waits on one of them, so
     // staging costs one trip to L2 instead of one per item.
-    bool inv_ready = !p.ln.h;
-    for (int m = 0; m < M; ++m) {
-        const __half* xr = p.x + (size_t)m * p.ldx;
-        const float* hr = p.ln.h ? p.ln.h + (size_t)m * p.ln.H : nullptr;
-        for (int base0 = 0; base0 < items; base0 += GEMV_STAGE_UN * GEMV_THREADS) {
-            float2 hv[GEMV_STAGE_UN][4];
-            __half2 wv[GEMV_STAGE_UN][4];
+    const bool lazy = p.ln.h != nullptr;
+    bool inv_ready = !lazy;
+    {
+        // (the items of all rows form one list: row by row, every row cost a trip to L2 of its own; groups of four lanes have
+        // items of one row)
+        const int all = items * M;
+        struct Item { int m, i; };               // row and item of the row; a step is GEMV_THREADS further in the list
+        Item at = {ONE ? 0 : tid / max(items, 1), 0}, done;
+        at.i = tid - at.m * items;
+        done = at;
+        auto advance = [&](Item& a) {
+            a.i += GEMV_THREADS;
+            if (!ONE) while (a.i >= items) { a.i -= items; ++a.m; }
+        };
+        for (int base0 = 0; base0 < all; base0 += UN * GEMV_THREADS) {
+            float2 hv[UN][4];
+            __half2 wv[UN][4];
 #pragma unroll
-            for (int u = 0; u < GEMV_STAGE_UN; ++u) {
-                const int item = base0 + u * GEMV_THREADS + tid;
-                const bool valid = item < items;
+            for (int u = 0; u < UN; ++u) {
+                const int m = at.m, item = at.i;
+                const bool valid = base0 + u * GEMV_THREADS + tid < all;
+                advance(at);
                 const int k0 = (cta_b0 * 2 + (item >> 2)) * 32 + 2 * (item & 3);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
@@ -464,8 +481,8 @@ __global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_int4_kernel(const GemvIn
                     hv[u][q] = make_float2(0.f, 0.f);
                     wv[u][q] = __float2half2_rn(0.f);
                     if (valid && k < p.K) {
-                        if (hr) { hv[u][q] = *(const float2*)(hr + k); wv[u][q] = *(const __half2*)(p.ln.w + k); }
-                        else wv[u][q] = *(const __half2*)(xr + k);
+                        if (lazy) { hv[u][q] = *(const float2*)(p.ln.h + (size_t)m * p.ln.H + k); wv[u][q] = *(const __half2*)(p.ln.w + k); }
+                        else wv[u][q] = *(const __half2*)(p.x + (size_t)m * p.ldx + k);
                     }
                 }
             }
@@ -474,15 +491,16 @@ __global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_int4_kernel(const GemvIn
                 __syncthreads();
                 inv_ready = true;
             }
-            const float inv = hr ? s_inv[m] : 0.f;
 #pragma unroll
-            for (int u = 0; u < GEMV_STAGE_UN; ++u) {
-                const int item = base0 + u * GEMV_THREADS + tid;
-                if (base0 + u * GEMV_THREADS >= items) break;          // uniform: no thread has an item here
-                const bool valid = item < items;
+            for (int u = 0; u < UN; ++u) {
+                if (base0 + u * GEMV_THREADS >= all) break;            // uniform: no thread has an item here
+                const bool valid = base0 + u * GEMV_THREADS + tid < all;
+                const int m = valid ? done.m : 0, item = done.i;
+                advance(done);
                 const int tt = item & 3, cl = item >> 2;
+                const float inv = lazy ? s_inv[m] : 0.f;
                 __half2 a0, a1, b0, b1;
-                if (hr) {
+                if (lazy) {
                     auto nrm = [&](int q) -> __half2 {
                         const float2 w = __half22float2(wv[u][q]);
                         return __floats2half2_rn(hv[u][q].x * inv * w.x, hv[u][q].y * inv * w.y);
@@ -597,6 +615,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_int4_kernel(const GemvIn
     else if (cur >= 0) flush(cur);
 
     // ---- in-CTA reduction over the k-warps into ybuf[row][n_local]
+    if (!ONE) __syncthreads();                 // (every warp has read its ring)
 #pragma unroll
     for (int i = 0; i < GEMV_NT; ++i)
         *(float4*)&redbuf[(((wk * GEMV_WN + wn) * GEMV_NT + i) * 32 + lane) * 4] =
@@ -636,7 +655,7 @@ __global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_int4_kernel(const GemvIn
 #define F16_DEPTH 4
 #define F16_PAD(MR) ((MR) > 1 ? 32 : 0)      // halfs: the 16-byte reads of two adjacent rows meet no bank twice
 template <int MR>
-__global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Params p) {
+__global__ void __launch_bounds__(GEMV_THREADS, 2) gemv_f16_kernel(const GemvF16Params p) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int M = p.rows;
@@ -668,7 +687,7 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Par
     // to GEMV_STAGE_UN pieces per thread, and under them the partial sums of the norm, are requested before
     // anything waits on one of them
     bool inv_ready = !p.ln.h;
-    for (int i0 = tid * 8; i0 < MR * p.kslice; i0 += GEMV_STAGE_UN * GEMV_THREADS * 8) {
+    for (int i0 = tid * 8; i0 < M * p.kslice; i0 += GEMV_STAGE_UN * GEMV_THREADS * 8) {
         uint4 raw[GEMV_STAGE_UN];
         float2 hv[GEMV_STAGE_UN][4];
 #pragma unroll
@@ -678,7 +697,7 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Par
             raw[u] = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (int q = 0; q < 4; ++q) hv[u][q] = make_float2(0.f, 0.f);
-            if (i < MR * p.kslice && m < M && kk < klen) {
+            if (i < M * p.kslice && kk < klen) {
                 if (p.ln.h) {
                     const float* hr = p.ln.h + (size_t)m * p.ln.H + k0 + kk;
                     raw[u] = *(const uint4*)(p.ln.w + k0 + kk);
@@ -697,11 +716,11 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Par
 #pragma unroll
         for (int u = 0; u < GEMV_STAGE_UN; ++u) {
             const int i = i0 + u * GEMV_THREADS * 8;
-            if (i >= MR * p.kslice) break;
+            if (i >= M * p.kslice) break;
             const int m = i / p.kslice;
             uint4 v = raw[u];
             if (p.ln.h) {
-                const float inv = m < M ? red32[m] : 0.f;
+                const float inv = red32[m];
                 const __half2* wv = (const __half2*)&raw[u];
                 __half2* o = (__half2*)&v;
 #pragma unroll
@@ -719,14 +738,14 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Par
 
     if constexpr (MR > 1) {
         float acc[2][4] = {};
-        const __half* xr = xs + (g < MR ? g : 0) * ldx_s + t * 8;
+        const __half* xr = xs + (g < M ? g : 0) * ldx_s + t * 8;
         for (int kb = 0; kb < klen; kb += 64 * F16_DEPTH) {
 #pragma unroll
             for (int d = 0; d < F16_DEPTH; ++d) {
                 const int k = kb + 64 * d;
                 if (k < klen) {                                      // (kslice is a multiple of 256: no read behind a row)
                     uint4 x0 = *(const uint4*)(xr + k), x1 = *(const uint4*)(xr + k + 32);
-                    if (g >= MR) { x0 = make_uint4(0u, 0u, 0u, 0u); x1 = x0; }
+                    if (g >= M) { x0 = make_uint4(0u, 0u, 0u, 0u); x1 = x0; }
                     // (each product from zero: the tensor core cuts its sums off, the additions to acc round)
                     float y[4][4] = {};
                     mma16816(y[0], wbuf[d][0].x, wbuf[d][1].x, wbuf[d][0].y, wbuf[d][1].y, x0.x, x0.y);
@@ -800,7 +819,7 @@ __global__ void __launch_bounds__(GEMV_THREADS) gemv_f16_kernel(const GemvF16Par
 // ---------------------------------------------------------------------------
 B2_API size_t b2_gemv_int4_smem(int rows, int L) {
     size_t maxCh = 2 * GEMV_WK * (size_t)L;
-    return (maxCh * rows + 1) * 64 + maxCh * 64 + (GEMV_WK * GEMV_WN * GEMV_NT * 128 + B2_MAX_ROWS * GEMV_TILE_N + 32 + 4) * 4
+    return (maxCh * rows + 1) * 64 + maxCh * 64 + ((rows > 1 ? 0 : GEMV_RED_FLOATS) + 32 + 4) * 4
            + (size_t)(GEMV_THREADS / 32) * GEMV_STAGES * (GEMV_NT * 512 + 256);
 }
 
@@ -810,11 +829,12 @@ B2_API int b2_gemv_int4(const GemvInt4Params* p, cudaStream_t stream) {
     size_t smem = b2_gemv_int4_smem(p->rows, p->L);
     // groups of 128 aligned to even k-blocks let the kernel drop all per-chunk group bookkeeping
     const bool fast = p->gshift == 2 && p->off32 == 0 && (p->L % 2 == 0);
-    static SmemOptIn optin[2];
-    {
-        cudaError_t e = fast ? optin[1].ensure(gemv_int4_kernel<true>, smem) : optin[0].ensure(gemv_int4_kernel<false>, smem);
-        if (e != cudaSuccess) return e;
-    }
+    const bool one = p->rows == 1;
+    void (*const kern)(GemvInt4Params) = fast ? (one ? gemv_int4_kernel<true, true> : gemv_int4_kernel<true, false>)
+                                              : (one ? gemv_int4_kernel<false, true> : gemv_int4_kernel<false, false>);
+    const int which = 2 * fast + one;
+    static SmemOptIn optin[4];
+    if (cudaError_t e = optin[which].ensure(kern, smem)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p->NTL * 16 / GEMV_TILE_N, p->k_splits);
     cfg.blockDim = dim3(GEMV_THREADS);
@@ -832,19 +852,18 @@ B2_API int b2_gemv_int4(const GemvInt4Params* p, cudaStream_t stream) {
         static std::mutex occ_mu;
         static int sms = 0, n_cached = 0;
         static size_t cached_smem[64];
-        static int cached_fast[64], cached_per_sm[64];
+        static int cached_which[64], cached_per_sm[64];
         int per_sm = 0;
         {
             std::lock_guard<std::mutex> lock(occ_mu);
             if (!sms) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev); }
             for (int i = 0; i < n_cached; ++i)
-                if (cached_smem[i] == smem && cached_fast[i] == (int)fast) per_sm = cached_per_sm[i];
+                if (cached_smem[i] == smem && cached_which[i] == which) per_sm = cached_per_sm[i];
             if (!per_sm) {
                 int n = 0;
-                cudaError_t e = fast ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gemv_int4_kernel<true>, GEMV_THREADS, smem)
-                                     : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, gemv_int4_kernel<false>, GEMV_THREADS, smem);
+                const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, GEMV_THREADS, smem);
                 per_sm = (e == cudaSuccess && n > 0) ? n : -1;
-                if (n_cached < 64) { cached_smem[n_cached] = smem; cached_fast[n_cached] = (int)fast; cached_per_sm[n_cached++] = per_sm; }
+                if (n_cached < 64) { cached_smem[n_cached] = smem; cached_which[n_cached] = which; cached_per_sm[n_cached++] = per_sm; }
             }
         }
         if (per_sm < 0 || (long long)cfg.gridDim.x * cfg.gridDim.y > (long long)sms * per_sm) q.tag_word = nullptr;
@@ -858,19 +877,26 @@ B2_API int b2_gemv_int4(const GemvInt4Params* p, cudaStream_t stream) {
         attr[1].id = cudaLaunchAttributeClusterDimension;
         attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = p->k_splits; attr[1].val.clusterDim.z = 1;
         cfg.numAttrs = 2;
-        static int ok_cache[2][9] = {{0}};                      // 0 unknown, 1 fits, -1 does not
-        int& ok = ok_cache[fast][p->k_splits];
+        static int ok_cache[4][9] = {{0}};                      // 0 unknown, 1 fits, -1 does not
+        int& ok = ok_cache[which][p->k_splits];
         if (ok == 0) {
             int n = 0;
-            cudaError_t e = fast ? cudaOccupancyMaxActiveClusters(&n, gemv_int4_kernel<true>, &cfg)
-                                 : cudaOccupancyMaxActiveClusters(&n, gemv_int4_kernel<false>, &cfg);
+            const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kern, &cfg);
             ok = (e == cudaSuccess && n >= 1) ? 1 : -1;
             if (e != cudaSuccess) cudaGetLastError();
         }
         if (ok == 1) q.cluster_splitk = 1; else cfg.numAttrs = 1;
     }
-    if (fast) return cudaLaunchKernelEx(&cfg, gemv_int4_kernel<true>, q);
-    return cudaLaunchKernelEx(&cfg, gemv_int4_kernel<false>, q);
+    return cudaLaunchKernelEx(&cfg, kern, q);
+}
+
+// Launch shape for `rows` rows of an fp16 matrix cut for (k_splits, kslice): with five rows and more, slices of 2560 at most.  The
+// activations of longer ones take so much shared memory that the L1 holds too few loads in flight (5 rows of 5120 -> 65536:
+// 161 us whole, 131 in two slices).
+B2_API void b2_gemv_f16_shape(int K, int rows, int* k_splits, int* kslice) {
+    if (rows <= 4 || *kslice <= 2560) return;
+    *kslice = 2560;
+    *k_splits = (K + 2559) / 2560;
 }
 
 template <int MR>

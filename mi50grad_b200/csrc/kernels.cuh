@@ -138,6 +138,7 @@ B2_API int b2_kv_compact(const KvCompactParams* p, cudaStream_t s);
 B2_API int b2_allreduce(const CollParams* p, int max_ctas, cudaStream_t s);
 B2_API int b2_rs_norm_ag(const SeqParParams* p, cudaStream_t s);
 B2_API int b2_gemv_int4(const GemvInt4Params* p, cudaStream_t stream);
+B2_API void b2_gemv_f16_shape(int K, int rows, int* k_splits, int* kslice);
 B2_API int b2_gemv_f16(const GemvF16Params* p, cudaStream_t stream);
 B2_API int b2_decode_attn(const AttnParams* p, int hd, cudaStream_t s);
 B2_API int b2_attn_rows(const AttnParams* p, const int* seq_rows, int n_seqs, int hd, cudaStream_t s);

@@ -29,6 +29,7 @@ import torch
 from ..config import PROMPT_ROWS, PROMPT_ROWS_FIXED, EngineConfig, QwenConfig, prompt_rows
 from ..models.weights import LayerWeights, ModelWeights
 from ..ops import lib as L
+from ..ops.kernels import gemv_f16_shape
 from ..ops.packing import (PackedInt4, concat_out, concat_out_dense, interleave_gate_up, launch_shape,
                            pack_int4, random_packed_int4)
 from ..parallel.sharding import ShardSpec, make_shard_spec
@@ -81,8 +82,9 @@ class DeviceLinear:
         return self.packed.n_pad if self.packed is not None else -(-self.N // 128) * 128
 
     def scratch_floats(self, rows: int) -> int:
-        ks = self.packed.k_splits if self.packed is not None else self.k_splits
-        return ks * rows * self.n_pad if ks > 1 else 0
+        if self.packed is not None:
+            return self.packed.k_splits * rows * self.n_pad if self.packed.k_splits > 1 else 0
+        return max([ks * r * self.n_pad for r in range(1, rows + 1) for ks in [gemv_f16_shape(self, r)[0]] if ks > 1] or [0])
 
     def desc(self) -> L.LinearDesc:
         d = L.LinearDesc()

@@ -47,6 +47,13 @@ def lazy_norm(h: torch.Tensor, ss: torch.Tensor, w: torch.Tensor, eps: float = 1
     return ln
 
 
+def gemv_f16_shape(lin, rows: int):
+    """(k_splits, kslice) of a launch with this many rows."""
+    ks, sl = C.c_int(lin.k_splits), C.c_int(lin.kslice)
+    L.lib().b2_gemv_f16_shape(lin.K, rows, C.byref(ks), C.byref(sl))
+    return ks.value, sl.value
+
+
 def gemv(lin, x: Optional[torch.Tensor], out: Optional[torch.Tensor] = None, mode: int = L.EPI_STORE_F16,
          scratch: Optional[torch.Tensor] = None, counters: Optional[torch.Tensor] = None,
          comm: Optional[L.CommCtx] = None, fin_flags: int = 0, h=None, norm_w=None, xn=None,
@@ -63,8 +70,12 @@ def gemv(lin, x: Optional[torch.Tensor], out: Optional[torch.Tensor] = None, mod
     pk, dense = getattr(lin, "packed", None), getattr(lin, "dense", None)
     if pk is None and dense is None:
         pk = lin
-    ks = k_splits or (pk.k_splits if pk is not None else lin.k_splits)
+    ks, kslice = k_splits or (pk.k_splits if pk is not None else lin.k_splits), getattr(lin, "kslice", None)
     n_pad = pk.n_pad if pk is not None else -(-dense.shape[0] // 128) * 128
+    if pk is None and not k_splits:
+        more, cut = gemv_f16_shape(lin, rows)
+        if scratch is None or scratch.numel() >= more * rows * n_pad:      # (a caller's scratch may be for the shape of few rows)
+            ks, kslice = more, cut
     if scratch is None:
         scratch = torch.empty(max(1, ks * rows * n_pad), dtype=torch.float32, device=dev)
     if counters is None:
@@ -99,7 +110,7 @@ def gemv(lin, x: Optional[torch.Tensor], out: Optional[torch.Tensor] = None, mod
         p.w, p.x, p.ldw, p.ldx, p.rows = dense.data_ptr(), xptr, dense.stride(0), ldx, rows
         if ln is not None:
             p.ln = ln
-        p.K, p.N, p.k_splits, p.kslice = dense.shape[1], dense.shape[0], ks, lin.kslice
+        p.K, p.N, p.k_splits, p.kslice = dense.shape[1], dense.shape[0], ks, kslice
         p.scratch, p.counters, p.epi, p.comm = scratch.data_ptr(), counters.data_ptr(), epi, cm
         L.check(lib.b2_gemv_f16(C.byref(p), L.stream()), "gemv_f16")
     return ss_part if mode == L.EPI_FINISH else out

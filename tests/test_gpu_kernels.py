@@ -698,3 +698,52 @@ def test_device_sampler_distribution_matches_host(K, temp, top_k, top_p, pen):
         counts[t] = counts.get(t, 0) + 1
     top = int(np.argmax(ref))
     assert abs(counts.get(top, 0) / 400.0 - ref[top]) < 0.1
+
+
+@pytest.mark.parametrize("rows,K,N", [(2, 2560, 256), (5, 5120, 128), (7, 2560, 4224), (8, 5120, 640), (8, 704, 128)])
+@pytest.mark.parametrize("lazy", [False, True])
+def test_gemv_int4_rows_share_one_list(rows, K, N, lazy):
+    """Rows whose activations are staged together: slices that are longer and shorter than a pass of the threads, an odd
+    number of rows, and grids of one and of two CTAs an SM; every row as a launch of its own gives it."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    from mi50grad_b200.ops.packing import pack_int4
+    from mi50grad_b200.utils.quant import random_int4_linear
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator().manual_seed(rows + K)
+    pk = pack_int4(random_int4_linear(K, N, 128, gen), dev)
+    x = torch.randn(rows, K, generator=gen).to(dev)
+    w = torch.randn(K, generator=gen).half().to(dev)
+    ss = x.pow(2).sum(1, keepdim=True)
+
+    def run(a, b):
+        ln = L.LazyNorm()
+        part = ss[a:b].contiguous()
+        ln.h, ln.ss, ln.w, ln.np, ln.H, ln.eps = x[a:b].data_ptr(), part.data_ptr(), w.data_ptr(), 1, K, 1e-6
+        out = torch.zeros(b - a, N, dtype=torch.float16, device=dev)
+        if lazy:
+            K_.gemv(pk, None, out=out, ln=ln, rows=b - a)
+        else:
+            K_.gemv(pk, x[a:b].half(), out=out)
+        torch.cuda.synchronize()
+        return out
+    got = run(0, rows)
+    assert all(torch.equal(got[r], run(r, r + 1)[0]) for r in range(rows))
+
+
+@pytest.mark.parametrize("rows", [4, 5, 8])
+@pytest.mark.parametrize("K,N", [(2816, 300), (5120, 19000)])
+def test_gemv_f16_slices_of_many_rows(rows, K, N):
+    """From five rows on a slice of K has 2560 at most; bound: fp32 sums of fp16 products, and the fp16 result."""
+    from mi50grad_b200.engine.engine import DeviceLinear
+    from mi50grad_b200.ops import kernels as K_
+    dev = torch.device("cuda", 0)
+    gen = torch.Generator().manual_seed(rows + N)
+    w, x = (torch.randn(N, K, generator=gen) * K ** -0.5).half().to(dev), torch.randn(rows, K, generator=gen).half().to(dev)
+    out = torch.zeros(rows, N, dtype=torch.float16, device=dev)
+    lin = DeviceLinear(dense=w)
+    assert lin.scratch_floats(rows) > 0 or rows == 4
+    K_.gemv(lin, x, out=out)
+    torch.cuda.synchronize()
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    assert bool(((out.double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -24 * (K / 16) * mag).all())
