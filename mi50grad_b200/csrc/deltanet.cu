@@ -983,53 +983,68 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_chunk_kernel(const Del
 // Pre-pass of the chunked scan: causal conv + SiLU + L2 norm of the q and k channels of every row, once
 // per key head and fully parallel over the rows (the scan kernel would otherwise redo it in each of the
 // dv/32 column CTAs of each of the nv/nk value heads that share a key head, on its sequential path).
-// Output fp16 [rows][2 * nk * DK]: q (scaled by 1/sqrt(DK)) | k.  grid = (row blocks of QP_ROWS, key heads),
-// 2 * DK threads: thread c owns one channel for QP_ROWS rows.
+// Output fp16 [rows][2 * nk * DK]: q (scaled by 1/sqrt(DK)) | k.  A warp owns a head's q or k over QP_ROWS rows: a lane has
+// DK / 32 adjacent channels, so rows are read and written in pieces of 256 bytes a warp and the norm stays inside the warp.
+// Bound: the rows' bytes.  (A thread with one channel of 16 rows: 12 us for 512 rows of 16 heads, 75 us for 3001; now 10 and 41.)
+// grid = (row blocks of QP_ROWS, 2 nk / 8), eight warps.
 // ---------------------------------------------------------------------------
-#define QP_ROWS 16
+#define QP_ROWS 8
 template <int DK>
-__global__ void __launch_bounds__(2 * DK) deltanet_qk_prep_kernel(const DeltaParams p, __half* __restrict__ qk_pre, int ld_qk,
-                                                                  int cb_copies, int nch) {
+__global__ void __launch_bounds__(256) deltanet_qk_prep_kernel(const DeltaParams p, __half* __restrict__ qk_pre, int ld_qk,
+                                                               int cb_copies, int nch) {
+    constexpr int CH = DK / 32;                    // channels of a lane: 4 or 2
+    struct alignas(2 * CH) Chans { __half v[CH]; };
     pdl_launch_dependents();
     pdl_wait();
-    const int kh = blockIdx.y, c = threadIdx.x, lane = c & 31, warp = c >> 5;
+    const int lane = threadIdx.x & 31, unit = blockIdx.y * 8 + (threadIdx.x >> 5);       // q heads, then k heads
     const int r0 = p.seq_rows[0], r1 = p.seq_rows[1];
     const int rb = r0 + blockIdx.x * QP_ROWS;
-    if (rb >= r1) return;
+    if (rb >= r1 || unit >= 2 * p.nk) return;
     const int seq = p.rows[r0].seq;
-    const bool is_q = c < DK;
-    const int gch = is_q ? kh * DK + c : p.nk * DK + kh * DK + (c - DK);
-    const int col = is_q ? p.off_q + kh * DK + c : p.off_k + kh * DK + (c - DK);
-    const __half* w = p.conv_w + (size_t)gch * 4;
-    const float w0 = __half2float(w[0]), w1 = __half2float(w[1]), w2 = __half2float(w[2]), w3 = __half2float(w[3]);
+    const bool is_q = unit < p.nk;
+    const int kh = is_q ? unit : unit - p.nk, c = lane * CH;
+    const int col = (is_q ? p.off_q : p.off_k) + kh * DK + c;
+    float w[CH][4];
+#pragma unroll
+    for (int e = 0; e < CH; ++e)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[e][q] = __half2float(p.conv_w[(size_t)(unit * DK + c + e) * 4 + q]);
     // rows before the sequence start come from the saved history of the first value head of this key head
-    const __half* hist = p.conv_state + ((((size_t)seq * p.nv + kh * (p.nv / p.nk)) * cb_copies) * nch + c) * 3;
-    auto input = [&](int ri) -> float {
-        if (ri >= r1) return 0.f;
-        return ri >= r0 ? __half2float(p.proj[(size_t)ri * p.ld + col]) : __half2float(hist[ri - r0 + 3]);
-    };
-    float x[QP_ROWS + 3];
+    const __half* hist = p.conv_state + ((((size_t)seq * p.nv + kh * (p.nv / p.nk)) * cb_copies) * nch + (is_q ? 0 : DK) + c) * 3;
+    const bool whole = ((p.ld | col) & (CH - 1)) == 0 && ((uintptr_t)p.proj & (2 * CH - 1)) == 0;
+    float x[QP_ROWS + 3][CH];
 #pragma unroll
-    for (int i = 0; i < QP_ROWS + 3; ++i) x[i] = input(rb - 3 + i);
-    __shared__ float part[2 * DK / 32][QP_ROWS];
-    float y[QP_ROWS];
+    for (int i = 0; i < QP_ROWS + 3; ++i) {
+        const int ri = rb - 3 + i;
+        Chans v = {};
+        if (ri >= r0 && ri < r1) {
+            const __half* src = p.proj + (size_t)ri * p.ld + col;
+            if (whole) v = *(const Chans*)src;
+            else
 #pragma unroll
-    for (int i = 0; i < QP_ROWS; ++i) {
-        y[i] = silu_fast(x[i] * w0 + x[i + 1] * w1 + x[i + 2] * w2 + x[i + 3] * w3);
-        const float ss = warp_sum(y[i] * y[i]);
-        if (lane == 0) part[warp][i] = ss;
+                for (int e = 0; e < CH; ++e) v.v[e] = src[e];
+        } else if (ri < r0) {
+#pragma unroll
+            for (int e = 0; e < CH; ++e) v.v[e] = hist[e * 3 + ri - r0 + 3];
+        }
+#pragma unroll
+        for (int e = 0; e < CH; ++e) x[i][e] = __half2float(v.v[e]);
     }
-    __syncthreads();
-    const int w_lo = is_q ? 0 : DK / 32;
     const float qscale = is_q ? rsqrtf((float)DK) : 1.f;
 #pragma unroll
     for (int i = 0; i < QP_ROWS; ++i) {
-        if (rb + i >= r1) break;
-        float ss = 0.f;
+        float y[CH], ss = 0.f;
 #pragma unroll
-        for (int k = 0; k < DK / 32; ++k) ss += part[w_lo + k][i];
-        qk_pre[(size_t)(rb - r0 + i) * ld_qk + (is_q ? kh * DK + c : p.nk * DK + kh * DK + (c - DK))] =
-            __float2half_rn(y[i] * rsqrtf(ss + 1e-6f) * qscale);
+        for (int e = 0; e < CH; ++e) {
+            y[e] = silu_fast(x[i][e] * w[e][0] + x[i + 1][e] * w[e][1] + x[i + 2][e] * w[e][2] + x[i + 3][e] * w[e][3]);
+            ss += y[e] * y[e];
+        }
+        const float inv = rsqrtf(warp_sum(ss) + 1e-6f) * qscale;
+        if (rb + i >= r1) break;
+        Chans o;
+#pragma unroll
+        for (int e = 0; e < CH; ++e) o.v[e] = __float2half_rn(y[e] * inv);
+        *(Chans*)(qk_pre + (size_t)(rb - r0 + i) * ld_qk + unit * DK + c) = o;
     }
 }
 
@@ -1232,15 +1247,19 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const Delt
     }
 }
 
-// The walk over the chunks.  A CTA owns 32 columns of a value head's state: as accumulator fragments in registers (warp w:
+// The walk over the chunks.  A CTA owns COLS columns of a value head's state: as accumulator fragments in registers (warp w:
 // rows 16 w ..) and, TF32-rounded and transposed, as the B operand in shared memory.  Two barriers a chunk:
-//   A  warp (m, n) forms its 16 x 8 tiles of Wt S0 (Wt as hi + lo) and Q S0, and writes U, twice (plain, and times
+//   A  warp (m, n) forms its 16 x 8 tiles (one, or of 64 columns two) of Wt S0 (Wt as hi + lo) and Q S0, and writes U, twice (plain, and times
 //      exp(G_C - G) for the state), as a transposed B operand;
 //   B  the same warp finishes its tile of Y = exp(G) Q S0 + W U, and every warp updates its rows of the state.
 // The operands of the next chunk travel meanwhile (cp.async, two stages).  The order of k inside a product is free: a
 // 16-k block is taken as (2t, 2t + 1) and (8 + 2t, 9 + 2t), which is what ldmatrix gives of fp16 rows and one 8-byte
 // load of fp32 rows.  Bound: the latency of this chain.  Measured (48 value heads of 128, 512 rows):
-// 60 us, and 37 + 8 us for the parts before and behind it; one kernel with nine barriers a chunk took 144 + 16 us.
+// 53 us, and 37 + 8 us for the parts before and behind it; one kernel with nine barriers a chunk took 144 + 16 us.
+// COLS: two CTAs on an SM hinder one another (1.7 us a chunk alone, 3.8 both), so the grid has at most one for each SM where
+// that can be: 32 columns up to 37 value heads, 64 up to 74 (their second tile takes the loaded Wt and Q again), else
+// 32 and two CTAs an SM.  48 heads, 512 rows: 32 columns 60 us, 64 53; 32 heads, 3001 rows: two CTAs on some SMs, because the
+// first SMs that the kernel before left took two, 360 us, one on each 218.
 #define SC_LDH(D) ((D) + 8)      // halfs: 16-byte rows of 8 adjacent lanes meet no bank twice
 #define SC_LDF(D) ((D) + 8)      // floats: the 8-byte reads of a half warp neither
 template <int DK>
@@ -1248,20 +1267,21 @@ struct ScanStage {
     __half q[DC_C][SC_LDH(DK)], k[DC_C][SC_LDH(DK)];
     float wt[DC_C][SC_LDF(DK)], w[DC_C][SC_LDF(DC_C)], gates[DC_GATES];
 };
-template <int DK>
+template <int DK, int COLS>
 struct ScanSmem {
     ScanStage<DK> st[2];
-    float s0[DN_COLS][SC_LDF(DK)], u[DN_COLS][SC_LDF(DC_C)], ut[DN_COLS][SC_LDF(DC_C)];
+    float s0[COLS][SC_LDF(DK)], u[COLS][SC_LDF(DC_C)], ut[COLS][SC_LDF(DC_C)];
 };
 
-template <int DK, int DV>
-__global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const DeltaParams p, const __half* __restrict__ qk_pre, int ld_qk,
+template <int DK, int DV, int COLS>
+__global__ void __launch_bounds__(DN_THREADS, COLS == 32 ? 2 : 1) deltanet_scan_kernel(const DeltaParams p, const __half* __restrict__ qk_pre, int ld_qk,
                                                                      float* __restrict__ tw, int n_chunks) {
     typedef ScanBlock<DK, DV> B;
     constexpr int MT = DK / 16;                   // warps that own 16 rows of the state
-    static_assert(DC_C == 32 && DN_COLS == 32 && MT <= 8, "eight warps: two row tiles by four column tiles");
+    constexpr int NT = COLS / 32, NS = COLS / 8;  // column tiles of a warp in A (32 columns apart), of the state
+    static_assert(DC_C == 32 && COLS % 32 == 0 && MT <= 8, "eight warps: two row tiles by four column tiles");
     extern __shared__ __align__(16) float dsm[];
-    ScanSmem<DK>& sm = *(ScanSmem<DK>*)dsm;
+    ScanSmem<DK, COLS>& sm = *(ScanSmem<DK, COLS>*)dsm;
     pdl_launch_dependents();
     if (!p.older) pdl_wait();
     const int cb = blockIdx.x, j = blockIdx.y, kh = j / (p.nv / p.nk);
@@ -1285,28 +1305,31 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
         if (tid < DC_GATES / 4) cp_async16(&s.gates[4 * tid], src + B::GATES + 4 * tid);
         cp_async_commit();
     };
-    // this lane's elements of its 16 x 8 tile of U0 (and later Y)
+    // this lane's elements of its 16 x 8 tiles of U0 (and later Y)
     const int mi = kr & 1, ni = kr >> 1;
-    const size_t u0_off = (size_t)B::U0 + (size_t)(16 * mi + g) * DV + cb * DN_COLS + 8 * ni + 2 * t;
-    float2 u0[2], u0n[2] = {};
+    const size_t u0_off = (size_t)B::U0 + (size_t)(16 * mi + g) * DV + cb * COLS + 8 * ni + 2 * t;
+    float2 u0[NT][2], u0n[NT][2] = {};
     auto load_u0 = [&](int ci) {
         const float* src = blocks + (size_t)ci * B::FLOATS + u0_off;
-        u0n[0] = *(const float2*)src;
-        u0n[1] = *(const float2*)(src + 8 * DV);
+#pragma unroll
+        for (int c = 0; c < NT; ++c) {
+            u0n[c][0] = *(const float2*)(src + 32 * c);
+            u0n[c][1] = *(const float2*)(src + 32 * c + 8 * DV);
+        }
     };
-    float S[4][4];
-    float* sp = p.state + (((size_t)seq * p.nv + j) * DK) * DV + cb * DN_COLS;
+    float S[NS][4];
+    float* sp = p.state + (((size_t)seq * p.nv + j) * DK) * DV + cb * COLS;
     auto put_s0 = [&]() {
         if (kr < MT) {
 #pragma unroll
-            for (int n = 0; n < 4; ++n)
+            for (int n = 0; n < NS; ++n)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) sm.s0[8 * n + 2 * t + (e & 1)][16 * kr + g + 8 * (e >> 1)] = tf32r(S[n][e]);
         }
     };
     if (kr < MT) {
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
+        for (int n = 0; n < NS; ++n) {
             const float2 lo = *(const float2*)(sp + (size_t)(16 * kr + g) * DV + 8 * n + 2 * t);
             const float2 hi = *(const float2*)(sp + (size_t)(16 * kr + g + 8) * DV + 8 * n + 2 * t);
             S[n][0] = lo.x; S[n][1] = lo.y; S[n][2] = hi.x; S[n][3] = hi.y;
@@ -1322,11 +1345,12 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
         cp_async_wait<0>();
         __syncthreads();                          // the chunk's operands and S0 are in place; everyone left the chunk before
         if (ci + 1 < chunks) stage(ci + 1);
-        u0[0] = u0n[0]; u0[1] = u0n[1];
+#pragma unroll
+        for (int c = 0; c < NT; ++c) { u0[c][0] = u0n[c][0]; u0[c][1] = u0n[c][1]; }
         if (ci + 1 < chunks) load_u0(ci + 1);
         const ScanStage<DK>& s = sm.st[ci & 1];
         // ---- A
-        float wh[4] = {0.f, 0.f, 0.f, 0.f}, wl[4] = {0.f, 0.f, 0.f, 0.f}, y[4] = {0.f, 0.f, 0.f, 0.f};
+        float wh[NT][4] = {}, wl[NT][4] = {}, y[NT][4] = {};
         {
             const float* wr = &s.wt[16 * mi + g][2 * t];
             const float* br = &sm.s0[8 * ni + g][2 * t];
@@ -1337,26 +1361,31 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
                 ldsm4_h(q, qr + k0);
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const float2 b = *(const float2*)(br + k0 + 8 * h);
                     const float2 x = *(const float2*)(wr + k0 + 8 * h), z = *(const float2*)(wr + 8 * SC_LDF(DK) + k0 + 8 * h);
                     const float2 qa = h2f(q[2 * h]), qb = h2f(q[2 * h + 1]);
                     float hi[4], lo[4];
                     split_tf32(x.x, hi[0], lo[0]); split_tf32(z.x, hi[1], lo[1]);
                     split_tf32(x.y, hi[2], lo[2]); split_tf32(z.y, hi[3], lo[3]);
-                    mma_tf32(wh, hi[0], hi[1], hi[2], hi[3], b.x, b.y);
-                    mma_tf32(wl, lo[0], lo[1], lo[2], lo[3], b.x, b.y);
-                    mma_tf32(y, qa.x, qb.x, qa.y, qb.y, b.x, b.y);
+#pragma unroll
+                    for (int c = 0; c < NT; ++c) {
+                        const float2 b = *(const float2*)(br + 32 * c * SC_LDF(DK) + k0 + 8 * h);
+                        mma_tf32(wh[c], hi[0], hi[1], hi[2], hi[3], b.x, b.y);
+                        mma_tf32(wl[c], lo[0], lo[1], lo[2], lo[3], b.x, b.y);
+                        mma_tf32(y[c], qa.x, qb.x, qa.y, qb.y, b.x, b.y);
+                    }
                 }
             }
         }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int i = 16 * mi + g + 8 * (e >> 1), c = 8 * ni + 2 * t + (e & 1);
-            const float u = ((e & 2) ? ((e & 1) ? u0[1].y : u0[1].x) : ((e & 1) ? u0[0].y : u0[0].x)) - (wh[e] + wl[e]);
-            sm.u[c][i] = tf32r(u);
-            sm.ut[c][i] = tf32r(u * s.gates[DC_C + i]);
-            y[e] *= s.gates[i];
-        }
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = 16 * mi + g + 8 * (e >> 1), c = 32 * n + 8 * ni + 2 * t + (e & 1);
+                const float u = ((e & 2) ? ((e & 1) ? u0[n][1].y : u0[n][1].x) : ((e & 1) ? u0[n][0].y : u0[n][0].x)) - (wh[n][e] + wl[n][e]);
+                sm.u[c][i] = tf32r(u);
+                sm.ut[c][i] = tf32r(u * s.gates[DC_C + i]);
+                y[n][e] *= s.gates[i];
+            }
         __syncthreads();
         // ---- B: Y
         {
@@ -1366,18 +1395,24 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
             for (int k0 = 0; k0 < DC_C; k0 += 8) {
                 if (k0 >= 16 * (mi + 1)) break;   // (W is zero above the diagonal)
                 const float2 x = *(const float2*)(wr + k0), z = *(const float2*)(wr + 8 * SC_LDF(DC_C) + k0);
-                const float2 b = *(const float2*)(br + k0);
-                mma_tf32(y, x.x, z.x, x.y, z.y, b.x, b.y);
+#pragma unroll
+                for (int c = 0; c < NT; ++c) {
+                    const float2 b = *(const float2*)(br + 32 * c * SC_LDF(DC_C) + k0);
+                    mma_tf32(y[c], x.x, z.x, x.y, z.y, b.x, b.y);
+                }
             }
             float* dst = blocks + (size_t)ci * B::FLOATS + u0_off;
-            *(float2*)dst = make_float2(y[0], y[1]);
-            *(float2*)(dst + 8 * DV) = make_float2(y[2], y[3]);
+#pragma unroll
+            for (int c = 0; c < NT; ++c) {
+                *(float2*)(dst + 32 * c) = make_float2(y[c][0], y[c][1]);
+                *(float2*)(dst + 32 * c + 8 * DV) = make_float2(y[c][2], y[c][3]);
+            }
         }
         // ---- B: S' = exp(G_C) S0 + K^T (exp(G_C - G) U)
         if (kr < MT) {
             const float egC = s.gates[2 * DC_C];
 #pragma unroll
-            for (int n = 0; n < 4; ++n)
+            for (int n = 0; n < NS; ++n)
 #pragma unroll
                 for (int e = 0; e < 4; ++e) S[n][e] *= egC;
 #pragma unroll
@@ -1388,7 +1423,7 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
                 for (int h = 0; h < 2; ++h) {
                     const float2 lo = h2f(kt[h]), hi = h2f(kt[2 + h]);
 #pragma unroll
-                    for (int n = 0; n < 4; ++n) {
+                    for (int n = 0; n < NS; ++n) {
                         const float2 b = *(const float2*)&sm.ut[8 * n + g][k0 + 8 * h + 2 * t];
                         mma_tf32(S[n], lo.x, hi.x, lo.y, hi.y, b.x, b.y);
                     }
@@ -1400,7 +1435,7 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_scan_kernel(const Delt
     if (!p.commit) return;
     if (kr < MT) {
 #pragma unroll
-        for (int n = 0; n < 4; ++n) {
+        for (int n = 0; n < NS; ++n) {
             *(float2*)(sp + (size_t)(16 * kr + g) * DV + 8 * n + 2 * t) = make_float2(S[n][0], S[n][1]);
             *(float2*)(sp + (size_t)(16 * kr + g + 8) * DV + 8 * n + 2 * t) = make_float2(S[n][2], S[n][3]);
         }
@@ -1452,17 +1487,21 @@ template <int DK, int DV>
 static int launch_delta_chunk(const DeltaParams* p, const void* ab, int ld_ab, __half* qk_pre, int ld_qk, int n_rows,
                               float* tw, cudaStream_t s) {
     if (qk_pre) {
-        dim3 grid((n_rows + QP_ROWS - 1) / QP_ROWS, p->nk);
-        if (cudaError_t e = launch_pdl(deltanet_qk_prep_kernel<DK>, grid, dim3(2 * DK), 0, s, *p, qk_pre, ld_qk, DV / DN_COLS, 2 * DK + DN_COLS)) return e;
+        dim3 grid((n_rows + QP_ROWS - 1) / QP_ROWS, (2 * p->nk + 7) / 8);
+        if (cudaError_t e = launch_pdl(deltanet_qk_prep_kernel<DK>, grid, dim3(256), 0, s, *p, qk_pre, ld_qk, DV / DN_COLS, 2 * DK + DN_COLS)) return e;
     }
     if (qk_pre && tw) {
         const int n_chunks = (n_rows + DC_C - 1) / DC_C;
         constexpr size_t psm = (size_t)(2 * DC_C * DC_LDK(DK) + DC_C * (DV + 8) + 3 * DC_C * DC_LDA + 3 * DC_C) * sizeof(float);
-        static SmemOptIn opt_tw, opt_scan;
+        static SmemOptIn opt_tw, opt_scan[2];
         if (cudaError_t e = opt_tw.ensure(deltanet_tw_prep_kernel<DK, DV>, psm)) return e;
         if (cudaError_t e = launch_pdl(deltanet_tw_prep_kernel<DK, DV>, dim3(n_chunks, p->nv), dim3(DN_THREADS), psm, s, *p, (const __half*)ab, ld_ab, qk_pre, ld_qk, tw, n_chunks)) return e;
-        if (cudaError_t e = opt_scan.ensure(deltanet_scan_kernel<DK, DV>, sizeof(ScanSmem<DK>))) return e;
-        if (cudaError_t e = launch_pdl(deltanet_scan_kernel<DK, DV>, dim3(DV / DN_COLS, p->nv), dim3(DN_THREADS), sizeof(ScanSmem<DK>), s, *p, qk_pre, ld_qk, tw, n_chunks)) return e;
+        // (more than half of an SM's shared memory keeps a second CTA off)
+        const bool one = p->nv * (DV / 32) <= 148, wide = !one && p->nv * (DV / 64) <= 148;
+        const size_t half = 120 * 1024, need = wide ? sizeof(ScanSmem<DK, 64>) : sizeof(ScanSmem<DK, 32>), ssm = (one || wide) && need < half ? half : need;
+        const auto scan = wide ? deltanet_scan_kernel<DK, DV, 64> : deltanet_scan_kernel<DK, DV, 32>;
+        if (cudaError_t e = opt_scan[wide].ensure(scan, ssm)) return e;
+        if (cudaError_t e = launch_pdl(scan, dim3(DV / (wide ? 64 : 32), p->nv), dim3(DN_THREADS), ssm, s, *p, (const __half*)qk_pre, ld_qk, tw, n_chunks)) return e;
         const int row_ctas = (int)(((long long)n_rows * p->nv + DN_THREADS / 32 - 1) / (DN_THREADS / 32));
         return launch_pdl(deltanet_scan_out_kernel<DK, DV>, dim3(row_ctas + p->nv * (DV / DN_COLS)), dim3(DN_THREADS), 0, s, *p, tw, n_chunks, row_ctas);
     }

@@ -50,7 +50,7 @@ def lazy_norm(h: torch.Tensor, ss: torch.Tensor, w: torch.Tensor, eps: float = 1
 def gemv_f16_shape(lin, rows: int):
     """(k_splits, kslice) of a launch with this many rows."""
     ks, sl = C.c_int(lin.k_splits), C.c_int(lin.kslice)
-    L.lib().b2_gemv_f16_shape(lin.K, rows, C.byref(ks), C.byref(sl))
+    L.lib().b2_gemv_f16_shape(lin.dense.shape[1], rows, C.byref(ks), C.byref(sl))
     return ks.value, sl.value
 
 

@@ -747,3 +747,36 @@ def test_gemv_f16_slices_of_many_rows(rows, K, N):
     torch.cuda.synchronize()
     ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
     assert bool(((out.double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -24 * (K / 16) * mag).all())
+
+
+@pytest.mark.parametrize("dk,heads", [(128, 38), (128, 74), (128, 76), (64, 75), (64, 150)])
+@pytest.mark.parametrize("n,shift", [(33, 0), (70, 1)])
+def test_deltanet_scan_columns_of_a_cta(K, dk, heads, n, shift):
+    """Grids of 32 or 64 columns a CTA, one or two CTAs an SM, give every head the bits that it gets in a launch of its own few
+    heads; with projection rows on and off the boundary of the vector loads."""
+    gen = torch.Generator().manual_seed(31)
+    rnd = lambda *s: torch.randn(*s, generator=gen)  # noqa: E731
+    cd = 3 * heads * dk
+    wide = torch.zeros(n, 4 * heads * dk + 2 * heads + shift, dtype=torch.float16)
+    wide[:, shift:] = rnd(n, wide.shape[1] - shift).half()
+    proj = wide.cuda()[:, shift:]
+    cw, al, dtb, nw = (rnd(cd, 4) * 0.3).half().cuda(), (torch.rand(heads, generator=gen) * 1.5 - 1.0).cuda(), (rnd(heads) * 0.5).half().cuda(), (torch.rand(dk, generator=gen) + 0.5).half().cuda()
+    S0 = (rnd(1, heads, dk, dk) * 0.1).cuda()
+    h0 = rnd(1, heads, dk // 32, 2 * dk + 32, 3).half().cuda()
+    h0[:, :, :, :2 * dk] = h0[:, :, :1, :2 * dk]
+    meta, rows = K.make_rows([(0, 0, 0, 0, 1)] * n, _dev()), torch.tensor([0, n], dtype=torch.int32, device=_dev())
+    ab = proj[:, 4 * heads * dk:]
+
+    def run(a, b):
+        m = b - a
+        offs = tuple(i * heads * dk + a * dk for i in range(4)) + (-1, -1)
+        S, h = S0[:, a:b].clone(), h0[:, a:b].clone()
+        c = torch.cat([cw[i * heads * dk + a * dk:i * heads * dk + b * dk] for i in range(3)])
+        gates = torch.cat([ab[:, a:b], ab[:, heads + a:heads + b]], 1).contiguous()
+        out = K.deltanet_chunk(proj, offs, gates, c, h, S, al[a:b].clone(), dtb[a:b].clone(), nw, meta, rows, m, m, dk, dk, prepass=2)
+        return out.reshape(n, m, dk), S[0], h[0]
+    got = run(0, heads)
+    for a in range(0, heads, 30):
+        b = min(heads, a + 30)
+        few = run(a, b)
+        assert torch.equal(got[0][:, a:b], few[0]) and torch.equal(got[1][a:b], few[1]) and torch.equal(got[2][a:b], few[2])
