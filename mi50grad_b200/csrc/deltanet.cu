@@ -985,7 +985,7 @@ __global__ void __launch_bounds__(DN_THREADS, 2) deltanet_chunk_kernel(const Del
 // dv/32 column CTAs of each of the nv/nk value heads that share a key head, on its sequential path).
 // Output fp16 [rows][2 * nk * DK]: q (scaled by 1/sqrt(DK)) | k.  A warp owns a head's q or k over QP_ROWS rows: a lane has
 // DK / 32 adjacent channels, so rows are read and written in pieces of 256 bytes a warp and the norm stays inside the warp.
-// Bound: the rows' bytes.  (A thread with one channel of 16 rows: 12 us for 512 rows of 16 heads, 75 us for 3001; now 10 and 41.)
+// Bound: the rows' bytes.  (A thread with one channel of 16 rows: 12 us for 512 rows of 16 heads, 75 us for 3001; now 8 and 25.)
 // grid = (row blocks of QP_ROWS, 2 nk / 8), eight warps.
 // ---------------------------------------------------------------------------
 #define QP_ROWS 8
@@ -1012,24 +1012,28 @@ __global__ void __launch_bounds__(256) deltanet_qk_prep_kernel(const DeltaParams
     // rows before the sequence start come from the saved history of the first value head of this key head
     const __half* hist = p.conv_state + ((((size_t)seq * p.nv + kh * (p.nv / p.nk)) * cb_copies) * nch + (is_q ? 0 : DK) + c) * 3;
     const bool whole = ((p.ld | col) & (CH - 1)) == 0 && ((uintptr_t)p.proj & (2 * CH - 1)) == 0;
+    // all rows are requested before the first is looked at (rows outside the launch read one inside and are replaced)
+    Chans v[QP_ROWS + 3];
+    if (whole) {
+#pragma unroll
+        for (int i = 0; i < QP_ROWS + 3; ++i) v[i] = *(const Chans*)(p.proj + (size_t)min(max(rb - 3 + i, r0), r1 - 1) * p.ld + col);
+    } else {
+#pragma unroll
+        for (int i = 0; i < QP_ROWS + 3; ++i)
+#pragma unroll
+            for (int e = 0; e < CH; ++e) v[i].v[e] = p.proj[(size_t)min(max(rb - 3 + i, r0), r1 - 1) * p.ld + col + e];
+    }
+    if (rb == r0) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int e = 0; e < CH; ++e) v[i].v[e] = hist[e * 3 + i];
+    }
     float x[QP_ROWS + 3][CH];
 #pragma unroll
-    for (int i = 0; i < QP_ROWS + 3; ++i) {
-        const int ri = rb - 3 + i;
-        Chans v = {};
-        if (ri >= r0 && ri < r1) {
-            const __half* src = p.proj + (size_t)ri * p.ld + col;
-            if (whole) v = *(const Chans*)src;
-            else
+    for (int i = 0; i < QP_ROWS + 3; ++i)
 #pragma unroll
-                for (int e = 0; e < CH; ++e) v.v[e] = src[e];
-        } else if (ri < r0) {
-#pragma unroll
-            for (int e = 0; e < CH; ++e) v.v[e] = hist[e * 3 + ri - r0 + 3];
-        }
-#pragma unroll
-        for (int e = 0; e < CH; ++e) x[i][e] = __half2float(v.v[e]);
-    }
+        for (int e = 0; e < CH; ++e) x[i][e] = __half2float(v[i].v[e]);
     const float qscale = is_q ? rsqrtf((float)DK) : 1.f;
 #pragma unroll
     for (int i = 0; i < QP_ROWS; ++i) {
@@ -1103,60 +1107,84 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const Delt
     float* Ts = Ws + DC_C * DC_LDA;
     float* Gs = Ts + DC_C * DC_LDA;           // [C]
     float* bs = Gs + DC_C;
-    float* gs = bs + DC_C;
     const int ci = blockIdx.x, j = blockIdx.y, kh = j / (p.nv / p.nk);
     const int tid = threadIdx.x, lane = tid & 31, kr = tid >> 5, g = lane >> 2, t = lane & 3;
     const int r0 = p.seq_rows[0], r1 = p.seq_rows[1];
     const int rb = r0 + ci * DC_C;
     if (rb >= r1) return;
     const int Ce = min(DC_C, r1 - rb), seq = p.rows[r0].seq;
-    for (int idx = tid; idx < DC_C * (DK / 8) * 2; idx += DN_THREADS) {
-        const int which = idx / (DC_C * (DK / 8)), rem = idx % (DC_C * (DK / 8));
-        const int row = rem / (DK / 8), c = (rem % (DK / 8)) * 8;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (row < Ce) v = *(const uint4*)(qk_pre + (size_t)(rb - r0 + row) * ld_qk + (which ? p.nk * DK : 0) + kh * DK + c);
-        const __half2* h2 = (const __half2*)&v;
-        float* dst = (which ? Ks : Qs) + row * LDK + c;
+    // everything is requested before the first value is looked at: loads behind conditions, each with its conversion, were
+    // taken one after the other, which was half of this kernel's time (14 600 of 30 000 clocks)
+    constexpr int NQK = DC_C * (DK / 8) * 2 / DN_THREADS, NV = DV * (DC_C / 8) / DN_THREADS;
+    static_assert(NQK * DN_THREADS == DC_C * (DK / 8) * 2 && NV * DN_THREADS == DV * (DC_C / 8), "whole turns of the threads");
+    uint4 qk[NQK];
+    __half vx[NV][11], vw[NV][4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) { const float2 f = __half22float2(h2[q]); dst[2 * q] = f.x; dst[2 * q + 1] = f.y; }
+    for (int q = 0; q < NQK; ++q) {
+        const int idx = tid + q * DN_THREADS, which = idx / (DC_C * (DK / 8)), rem = idx % (DC_C * (DK / 8));
+        const int row = rem / (DK / 8), c = (rem % (DK / 8)) * 8;
+        qk[q] = *(const uint4*)(qk_pre + (size_t)(rb - r0 + min(row, Ce - 1)) * ld_qk + (which ? p.nk * DK : 0) + kh * DK + c);
     }
     // values: causal convolution + SiLU of a channel over a run of rows; rows before the sequence come from the history
-    for (int idx = tid; idx < DV * (DC_C / 8); idx += DN_THREADS) {
-        const int c = idx % DV, i0 = idx / DV * 8;
-        const __half* hist = p.conv_state + ((((size_t)seq * p.nv + j) * (DV / DN_COLS) + c / DN_COLS) * (2 * DK + DN_COLS) + 2 * DK + c % DN_COLS) * 3;
-        const __half* w = p.conv_w + (size_t)(2 * p.nk * DK + j * DV + c) * 4;
-        const float w0 = __half2float(w[0]), w1 = __half2float(w[1]), w2 = __half2float(w[2]), w3 = __half2float(w[3]);
-        const __half* col = p.proj + p.off_v + j * DV + c;
-        float x[11];
 #pragma unroll
-        for (int i = 0; i < 11; ++i) {
-            const int ri = rb + i0 - 3 + i;
-            x[i] = ri >= r1 ? 0.f : (ri >= r0 ? __half2float(col[(size_t)ri * p.ld]) : __half2float(hist[ri - r0 + 3]));
+    for (int q = 0; q < NV; ++q) {
+        const int idx = tid + q * DN_THREADS, c = idx % DV, i0 = idx / DV * 8;
+        const __half* col = p.proj + p.off_v + j * DV + c;
+        const __half* w = p.conv_w + (size_t)(2 * p.nk * DK + j * DV + c) * 4;
+#pragma unroll
+        for (int i = 0; i < 11; ++i) vx[q][i] = col[(size_t)min(max(rb + i0 - 3 + i, r0), r1 - 1) * p.ld];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) vw[q][i] = w[i];
+        if (ci == 0 && i0 == 0) {
+            const __half* hist = p.conv_state + ((((size_t)seq * p.nv + j) * (DV / DN_COLS) + c / DN_COLS) * (2 * DK + DN_COLS) + 2 * DK + c % DN_COLS) * 3;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) vx[q][i] = hist[i];
         }
+    }
+    __half ga = __float2half(0.f), gb = ga, g_bias = ga;
+    float g_log = 0.f;
+    if (tid < DC_C) {
+        const __half* abr = ab + (size_t)(rb + min(tid, Ce - 1)) * ld_ab;
+        ga = abr[j]; gb = abr[p.nv + j]; g_bias = p.dt_bias[j]; g_log = p.A_log[j];
+    }
+#pragma unroll
+    for (int q = 0; q < NQK; ++q) {
+        const int idx = tid + q * DN_THREADS, which = idx / (DC_C * (DK / 8)), rem = idx % (DC_C * (DK / 8));
+        const int row = rem / (DK / 8), c = (rem % (DK / 8)) * 8;
+        const __half2* h2 = (const __half2*)&qk[q];
+        float f[8];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { const float2 v = __half22float2(h2[e]); f[2 * e] = row < Ce ? v.x : 0.f; f[2 * e + 1] = row < Ce ? v.y : 0.f; }
+        float* dst = (which ? Ks : Qs) + row * LDK + c;
+        *(float4*)dst = make_float4(f[0], f[1], f[2], f[3]);
+        *(float4*)(dst + 4) = make_float4(f[4], f[5], f[6], f[7]);
+    }
+#pragma unroll
+    for (int q = 0; q < NV; ++q) {
+        const int idx = tid + q * DN_THREADS, c = idx % DV, i0 = idx / DV * 8;
+        float x[11], w[4];
+#pragma unroll
+        for (int i = 0; i < 11; ++i) x[i] = __half2float(vx[q][i]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = __half2float(vw[q][i]);
 #pragma unroll
         for (int i = 0; i < 8; ++i)
-            Vs[(i0 + i) * LDV + c] = i0 + i < Ce ? silu_fast(x[i] * w0 + x[i + 1] * w1 + x[i + 2] * w2 + x[i + 3] * w3) : 0.f;
+            Vs[(i0 + i) * LDV + c] = i0 + i < Ce ? silu_fast(x[i] * w[0] + x[i + 1] * w[1] + x[i + 2] * w[2] + x[i + 3] * w[3]) : 0.f;
     }
     if (tid < DC_C) {
         float gl = 0.f, beta = 0.f;
         if (tid < Ce) {
-            const __half* abr = ab + (size_t)(rb + tid) * ld_ab;
-            const float sp_ = __half2float(abr[j]) + __half2float(p.dt_bias[j]);
-            gl = fmaxf(-__expf(p.A_log[j]) * (sp_ > 20.f ? sp_ : log1pf(__expf(sp_))), -20.f);
-            beta = sigmoid_f(__half2float(abr[p.nv + j]));
+            const float sp_ = __half2float(ga) + __half2float(g_bias);
+            gl = fmaxf(-__expf(g_log) * (sp_ > 20.f ? sp_ : log1pf(__expf(sp_))), -20.f);
+            beta = sigmoid_f(__half2float(gb));
         }
-        gs[tid] = gl;
         bs[tid] = beta;
-    }
-    __syncthreads();
-    if (kr == 0) {
-        float a = gs[lane];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float ua = __shfl_up_sync(0xffffffffu, a, o);
-            if (lane >= o) a += ua;
+        for (int o = 1; o < 32; o <<= 1) {           // (the first warp has the chunk's rows)
+            const float ua = __shfl_up_sync(0xffffffffu, gl, o);
+            if (lane >= o) gl += ua;
         }
-        Gs[lane] = a;
+        Gs[tid] = gl;
     }
     __syncthreads();
     {
@@ -1190,19 +1218,40 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const Delt
         }
     }
     __syncthreads();
-    if (kr == 0) {
-        // column `lane` of T: t_i = [i == lane] - sum_{j < i} A_ij t_j
-        float tc[DC_C];
+    // T = [T1 0; -T2 A21 T1  T2] with T1, T2 the inverses of the diagonal 16 x 16 triangles of I + A: a warp forms one by
+    // forward substitution, a column per lane (t_i = [i == c] - sum_{j < i} A_ij t_j); then all threads two 16 x 16 products.
+    // (One warp over all 32 rows took 3500-4200 clocks, while the others waited.)
+    constexpr int HC = DC_C / 2;
+    if (kr < 2) {
+        const float* Ad = As + kr * (HC * DC_LDA + HC);
+        float* Td = Ts + kr * (HC * DC_LDA + HC);
+        const int c = lane & (HC - 1);
+        float tc[HC];
 #pragma unroll
-        for (int i = 0; i < DC_C; ++i) {
-            float v = (i == lane) ? 1.f : 0.f;
+        for (int i = 0; i < HC; ++i) {
+            float v = (i == c) ? 1.f : 0.f;
 #pragma unroll
-            for (int jj = 0; jj < DC_C; ++jj)
-                if (jj < i) v = fmaf(-As[i * DC_LDA + jj], tc[jj], v);
+            for (int jj = 0; jj < HC; ++jj)
+                if (jj < i) v = fmaf(-Ad[i * DC_LDA + jj], tc[jj], v);
             tc[i] = v;
-            Ts[i * DC_LDA + lane] = v;
+            if (lane < HC) Td[i * DC_LDA + c] = v;
         }
     }
+    __syncthreads();
+    const int hr = tid / HC, hc = tid % HC;                    // 256 threads: an element each
+    {
+        float v = 0.f;                                         // A21 T1, kept where T is zero
+#pragma unroll
+        for (int k = 0; k < HC; ++k) v = fmaf(As[(HC + hr) * DC_LDA + k], Ts[k * DC_LDA + hc], v);
+        Ts[hr * DC_LDA + HC + hc] = v;
+    }
+    __syncthreads();
+    float t21 = 0.f;
+#pragma unroll
+    for (int k = 0; k < HC; ++k) t21 = fmaf(-Ts[(HC + hr) * DC_LDA + HC + k], Ts[k * DC_LDA + HC + hc], t21);
+    __syncthreads();
+    Ts[(HC + hr) * DC_LDA + hc] = t21;
+    Ts[hr * DC_LDA + HC + hc] = 0.f;
     __syncthreads();
     typedef ScanBlock<DK, DV> B;
     float* dst = tw + ((size_t)j * n_chunks + ci) * B::FLOATS;
@@ -1255,7 +1304,7 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const Delt
 // The operands of the next chunk travel meanwhile (cp.async, two stages).  The order of k inside a product is free: a
 // 16-k block is taken as (2t, 2t + 1) and (8 + 2t, 9 + 2t), which is what ldmatrix gives of fp16 rows and one 8-byte
 // load of fp32 rows.  Bound: the latency of this chain.  Measured (48 value heads of 128, 512 rows):
-// 53 us, and 37 + 8 us for the parts before and behind it; one kernel with nine barriers a chunk took 144 + 16 us.
+// 53 us, and 26 + 8 us for the parts before and behind it; one kernel with nine barriers a chunk took 144 + 16 us.
 // COLS: two CTAs on an SM hinder one another (1.7 us a chunk alone, 3.8 both), so the grid has at most one for each SM where
 // that can be: 32 columns up to 37 value heads, 64 up to 74 (their second tile takes the loaded Wt and Q again), else
 // 32 and two CTAs an SM.  48 heads, 512 rows: 32 columns 60 us, 64 53; 32 heads, 3001 rows: two CTAs on some SMs, because the
@@ -1492,7 +1541,7 @@ static int launch_delta_chunk(const DeltaParams* p, const void* ab, int ld_ab, _
     }
     if (qk_pre && tw) {
         const int n_chunks = (n_rows + DC_C - 1) / DC_C;
-        constexpr size_t psm = (size_t)(2 * DC_C * DC_LDK(DK) + DC_C * (DV + 8) + 3 * DC_C * DC_LDA + 3 * DC_C) * sizeof(float);
+        constexpr size_t psm = (size_t)(2 * DC_C * DC_LDK(DK) + DC_C * (DV + 8) + 3 * DC_C * DC_LDA + 2 * DC_C) * sizeof(float);
         static SmemOptIn opt_tw, opt_scan[2];
         if (cudaError_t e = opt_tw.ensure(deltanet_tw_prep_kernel<DK, DV>, psm)) return e;
         if (cudaError_t e = launch_pdl(deltanet_tw_prep_kernel<DK, DV>, dim3(n_chunks, p->nv), dim3(DN_THREADS), psm, s, *p, (const __half*)ab, ld_ab, qk_pre, ld_qk, tw, n_chunks)) return e;
