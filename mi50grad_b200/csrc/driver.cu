@@ -528,19 +528,18 @@ static int run_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, int 
     memset(&p, 0, sizeof(p));
     p.qfrag = (const uint4*)L.w; p.szfrag = (const uint2*)L.sz; p.w_older = 1;
     p.K = L.K; p.KB = L.KB; p.NTL = L.NTL; p.G = L.G; p.off32 = L.off32; p.gshift = L.gshift;
-    // Token tile, outputs per item (128, or 256 as two accumulators that share an activation tile) and K splits (only
+    // Token tile, outputs per CTA (128, or 256 as two accumulators that share an activation tile) and K splits (only
     // where the product is added to the residual stream; the parts meet through atomic adds) with the least time by a
-    // model of one CTA per SM that walks over whole items: k-blocks, an epilogue, and once the launch.  us of a 64-k block, fitted
-    // to 148 CTAs with one to three items of 32 to 128 k-blocks: 128 outputs: .17 at 16 tokens, .205 at 80, .26 at 128, .34 at
-    // 192, .42 at 256; 256 outputs: .40, .415, .49 at 128, .645 at 192; an epilogue 1.5 to 6 us and 2 to 8.5, of the residual
-    // form up to twice that.
+    // model of one CTA per SM: whole waves of CTAs, each a walk over its k-blocks plus a start and an epilogue, and the traffic of the
+    // atomic adds.  us of a 64-k block, measured with one to three waves of 64 and 128 blocks: 128 outputs: .17 at 16 tokens, .21 at 80, .26
+    // at 128, .34 at 192, .41 at 256; 256 outputs: .37 up to 80, .45 at 128, .58 at 192.  80 rows, 17408 -> 5120: 256 outputs in seven splits
+    // 21.3 us, 128 in three 25.8; 512 rows: 256 x 176 in two 73, 128 x 256 in three 75.
     auto block_us = [](int t, bool wide) -> double {
-        if (wide) return t <= 80 ? 0.395 + 0.0002 * t : (t <= 128 ? 0.411 + 0.0016 * (t - 80) : 0.488 + 0.00245 * (t - 128));
-        return t <= 80 ? 0.165 + 0.0005 * t : 0.205 + 0.0012 * (t - 80);
+        if (wide) return t <= 80 ? 0.365 + 0.0001 * t : (t <= 128 ? 0.373 + 0.0016 * (t - 80) : 0.45 + 0.0021 * (t - 128));
+        return t <= 80 ? 0.17 + 0.00045 * t : (t <= 128 ? 0.206 + 0.001 * (t - 80) : 0.254 + 0.00125 * (t - 128));
     };
-    const bool wide_ok = d->gemm_m256 && (L.NTL * 16) % 256 == 0;
-    const int max_ks = epi == TC_EPI_RESID_F32 && d->gemm_splitk ? 8 : 1;
-    const double epi_f = epi == TC_EPI_RESID_F32 ? 1.8 : 1.0;
+    const bool wide_ok = d->gemm_m256 && (L.NTL * 16) % 256 == 0, resid = epi == TC_EPI_RESID_F32;
+    const int max_ks = resid && d->gemm_splitk ? 12 : 1;
     int tt = 16, ks = 1;
     bool wide = false;
     double best = 1e30;
@@ -550,7 +549,7 @@ static int run_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, int 
             const int t = ((T + nt - 1) / nt + 15) & ~15;
             for (int k = 1; k <= max_ks && (k == 1 || L.KB / k >= 8); ++k) {
                 const int waves = (ctas_n * ((T + t - 1) / t) * k + 147) / 148;
-                const double cost = waves * ((L.KB + k - 1) / k * block_us(t, w) + epi_f * (w ? 2.5 + 0.031 * t : 1.5 + 0.0165 * t)) + (k > 1 ? 1e-6 * k * T * n_valid : 0.0);
+                const double cost = waves * ((L.KB + k - 1) / k * block_us(t, w) + (w ? 3.0 + 0.02 * t : 3.5) + (resid ? 1.5 : 0.0)) + (k > 1 ? 0.8e-6 * k * T * n_valid : 0.0);
                 if (cost < best - 1e-9) { best = cost; tt = t; ks = k; wide = w; }
             }
         }

@@ -5,8 +5,7 @@
 // gemm_int4_prefill_v2.hip:41, src/asm/gemm_*.s), which runs 64x64x16 tiles on vector ALUs.
 //
 // The WEIGHT tile is the MMA's A operand (M = 128 outputs) and comes from TENSOR MEMORY; the activations are the B operand
-// (N = tokens, any multiple of 16) in shared memory.  A work item is [128 MH outputs x t_tile tokens x a range of K]; a CTA
-// per SM walks over its items.
+// (N = tokens, any multiple of 16) in shared memory.  A CTA, one on an SM, has [128 MH outputs x t_tile tokens x a range of K].
 //   * warps 0-15 dequantise.  A lane's packed weights of a 16 x 64 tile are one 16-byte load (fragment order of the decode
 //     GEMV), held two steps ahead in registers; expanded to fp16 ((q - zero) * scale, the 0x6400 trick) they are in the
 //     order of tcgen05.st.16x128b, so they go from registers into tensor memory as they are.
@@ -14,13 +13,16 @@
 //     some k-blocks ahead in L2;
 //   * warp 17 (and 18: one for each accumulator) issues tcgen05.mma (A in tensor memory) and releases slots and stages
 //     with tcgen05.commit.
-//   * warps 0-15 then read the accumulators back and store them, while the activations of the next item arrive.
+//   * warps 0-15 then read the accumulators back and store them.
 // Tensor memory (512 columns): MH accumulators of t_tile columns and four slots of weights, two for each group of eight
 // dequantising warps; a slot has [128 outputs x 64 KS k].
 //
 // Why tensor memory: with the dequantised tile in shared memory its stores waited for the operand reads of the MMAs, which go
 // first: four stmatrix and a proxy fence of 16 warps took 600-1270 cycles beside them, tcgen05.st of the same tile takes
 // 65-105.  It also takes the A operand off the shared-memory port (n = 16: 75 instead of 157 cycles a k-block).
+// (CTAs that walk over several tiles, with the first weights of a tile before the epilogue of the one before, or over equal
+// shares of all tiles' k-blocks, were no faster than as many CTAs and splits over K: what they have to keep in mind costs
+// the dequantising warps 2 us in 20 with few tokens.)
 // What bounds it: few tokens, the dequantisation (see block_us in csrc/driver.cu for the measured k-block times); many
 // tokens, the tensor pipe.
 // Every mbarrier wait is bounded; on expiry the kernel records a status, skips the rest of its work, releases its tensor
@@ -37,7 +39,9 @@
 #define TS_SLOTS 4
 #define TS_MAX_STAGES 16
 #define TS_STAGE_SMEM (192 * 1024)
-#define TS_AHEAD 24               // k-blocks that the weights are requested ahead into L2
+// k-blocks that the weights are requested ahead into L2, in front of the two steps that are held in registers.  256 outputs, 16 tokens,
+// 37888 x 5120: 28.6 us; 8 ahead 29.8, 24 ahead 31.2; nothing 27.5, but then 128 outputs take 4 % longer
+#define TS_AHEAD 4
 
 __device__ __forceinline__ uint32_t ts_nib_lo(uint32_t w) {
     uint32_t r;
@@ -97,13 +101,12 @@ __device__ __forceinline__ void ts_dequant(uint32_t w0, uint32_t w1, uint2 sz, u
     r[6] = hi(w1, ch_lo, s_lo); r[7] = hi(w1 >> 8, ch_hi, s_hi);
 }
 
-// MH: accumulators of 128 outputs per item.  KS: k-blocks per slot and stage: two, since a slot's waits, commits and
+// MH: accumulators of 128 outputs.  KS: k-blocks per slot and stage: two, since a slot's waits, commits and
 // instructions around them cost an MMA warp as much as the products of few tokens, or one where the accumulators leave
 // room for no more.  UNI: a pair of k-blocks is a group of 128, with one scale per output; else every 32 k look theirs up.
 template <int MH, int KS, bool UNI>
 __global__ void __launch_bounds__((TS_PRODUCERS + 1 + MH) * 32, 1)
-gemm_int4_ts_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xmap, const int n_mt, const int n_tt, const int n_items,
-                    const int per_kb) {
+gemm_int4_ts_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xmap, const int n_mt, const int n_tt, const int per_kb) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* sB = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);      // [S][KS][t_tile rows of 128 bytes]
     // (the broadcast and the votes below tell the compiler that roles and loop exits are warp-uniform)
@@ -115,8 +118,7 @@ gemm_int4_ts_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
     uint64_t* a_full = b_empty + S;                 // [4] one arrival per warp of the group
     uint64_t* a_empty = a_full + TS_SLOTS;          // [4] a commit
     uint64_t* acc_full = a_empty + TS_SLOTS;        // a commit of every MMA warp
-    uint64_t* acc_empty = acc_full + 1;             // one arrival per epilogue warp
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 1);
+    uint32_t* tmem_slot = (uint32_t*)(acc_full + 1);
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     const int acc_cols = (p.t_tile + 31) & ~31;     // columns of an accumulator
 
@@ -124,7 +126,6 @@ gemm_int4_ts_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
         for (int s = 0; s < S; ++s) { mbar_init(&b_full[s], 1); mbar_init(&b_empty[s], MH); }
         for (int s = 0; s < TS_SLOTS; ++s) { mbar_init(&a_full[s], TS_PRODUCERS / 2); mbar_init(&a_empty[s], 1); }
         mbar_init(acc_full, MH);
-        mbar_init(acc_empty, TS_PRODUCERS);
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -142,16 +143,10 @@ gemm_int4_ts_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
     pdl_launch_dependents();
     if (!p.w_older) pdl_wait();
 
-    // an item: output tile mt, token tile tt, K range z; the token tiles of an output tile run side by side and share its
-    // weights in L2
-    struct Item { int mt, tt, kb0, kbs; };
-    auto item = [&](int i) {
-        Item it;
-        const int z = i / (n_mt * n_tt), r = i - z * (n_mt * n_tt);
-        it.mt = r / n_tt; it.tt = r - it.mt * n_tt;
-        it.kb0 = z * per_kb; it.kbs = min(p.KB - it.kb0, per_kb);
-        return it;
-    };
+    // output tile mt, token tile tt, K range z; the token tiles of an output tile run side by side and share its weights in L2
+    const int z = (int)blockIdx.x / (n_mt * n_tt), tile = (int)blockIdx.x - z * (n_mt * n_tt);
+    const int mt = tile / n_tt, tt = tile - mt * n_tt;
+    const int kb0 = z * per_kb, kbs = min(p.KB - kb0, per_kb);
 
     if (warp < TS_PRODUCERS) {
         // ================= dequantising warps, then epilogue =================
@@ -162,53 +157,39 @@ gemm_int4_ts_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
         constexpr int NSZ = UNI ? 1 : 4;
         uint4 wq[2][2] = {};
         uint2 sz[2][NSZ] = {};
-        const int first = MH == 2 ? 0 : grp, stride = MH == 2 ? 1 : 2;     // steps of this group
-        // load cursor: item, step, pointers of the item's tile
-        int l_item = blockIdx.x, l_step = first, l_steps = 0, l_kb = 0, l_kbs = 0;
-        const uint4* l_q = nullptr;
-        const uint2* l_s = nullptr;
-        auto l_begin = [&]() {
-            // the next item in which this group has a step
-            while (l_item < n_items) {
-                const Item it = item(l_item);
-                l_kbs = it.kbs; l_steps = (it.kbs + 1) >> 1; l_step = first; l_kb = it.kb0;
-                const int wt = (it.mt * MH + (MH == 2 ? grp : 0)) * 2 + (rt >> 2);
-                l_q = p.qfrag + (((size_t)wt * p.KB + it.kb0 + 2 * first) * 4 + (rt & 3)) * 32 + lane;
-                l_s = p.szfrag + ((size_t)wt * p.G * 4 + (rt & 3)) * 8 + g;
-                if (UNI) l_s += (size_t)(((p.off32 + 2 * it.kb0) >> 2) + first) * 32;
-                if (first < l_steps) return;
-                l_item += gridDim.x;
-            }
-        };
-        // (buffers 0 and 1 take the steps of an item in turn, beginning with 0; an odd last one leaves buffer 1 idle)
+        const int first = MH == 2 ? 0 : grp, stride = MH == 2 ? 1 : 2, steps = (kbs + 1) >> 1;     // steps of this group
+        const int wt = (mt * MH + (MH == 2 ? grp : 0)) * 2 + (rt >> 2);
+        const uint4* l_q = p.qfrag + (((size_t)wt * p.KB + kb0 + 2 * first) * 4 + (rt & 3)) * 32 + lane;
+        const uint2* l_s = p.szfrag + ((size_t)wt * p.G * 4 + (rt & 3)) * 8 + g;
+        if (UNI) l_s += (size_t)(((p.off32 + 2 * kb0) >> 2) + first) * 32;
+        int l_step = first;
+        if (first >= steps) { l_q = p.qfrag + (((size_t)wt * p.KB + kb0) * 4 + (rt & 3)) * 32 + lane; if (UNI) l_s -= first * 32; }
+        // (buffers 0 and 1 take the steps in turn)
+        // A step behind the last reads the last again, a half one its first block twice: no branch stands between the loads.
         auto load = [&](int b) __attribute__((always_inline)) {
-            if (l_item >= n_items) return;
-            if (l_step < l_steps) {
-                const int kb = 2 * l_step;
-                wq[b][0] = ts_load_w(l_q);
-                if (kb + 1 < l_kbs) wq[b][1] = ts_load_w(l_q + 128);
-                if (UNI) sz[b][0] = __ldg(l_s);
-                else {
-                    const int c = p.off32 + 2 * (l_kb + kb);
+            wq[b][0] = ts_load_w(l_q);
+            wq[b][1] = ts_load_w(l_q + (2 * l_step + 1 < kbs ? 128 : 0));
+            if (UNI) sz[b][0] = __ldg(l_s);
+            else {
+                const int c = p.off32 + 2 * (kb0 + 2 * l_step);
 #pragma unroll
-                    for (int j = 0; j < NSZ; ++j)
-                        if (j < 2 || kb + 1 < l_kbs) sz[b][j] = __ldg(l_s + (size_t)((c + j) >> p.gshift) * 32);
-                }
+                for (int j = 0; j < NSZ; ++j) sz[b][j] = __ldg(l_s + (size_t)min((c + j) >> p.gshift, p.G - 1) * 32);
+            }
+            l_step += stride;
+            if (l_step < steps) {
                 l_q += stride * 256;
                 if (UNI) l_s += stride * 32;
             }
-            l_step += stride;
-            if (b == 1 && l_step >= l_steps) { l_item += gridDim.x; l_begin(); }
         };
-        l_begin();
         load(0);
         load(1);
         const uint32_t a_lane = tmem_a + ((uint32_t)(rt * 16) << 16) + (uint32_t)(grp * 2 * 32 * KS);
         bool ok = true;
         uint32_t q = 0;                            // slots that this group has filled: it has two, in turn
-        uint32_t item_ph = 0;
-        auto wait_slot = [&]() __attribute__((always_inline)) {
-            uint64_t* bar = &a_empty[grp * 2 + (q & 1)];
+        // (with a whole step a slot the buffers alternate just as the slots do)
+        auto slot = [&](int b) __attribute__((always_inline)) { return KS == 2 ? b : (int)(q & 1); };
+        auto wait_slot = [&](int b) __attribute__((always_inline)) {
+            uint64_t* bar = &a_empty[grp * 2 + slot(b)];
             const uint32_t parity = ((q >> 1) & 1) ^ 1;
             if (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
                 int o = 1;
@@ -217,149 +198,127 @@ gemm_int4_ts_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
             }
             tc_fence_after();
         };
-        auto filled = [&]() __attribute__((always_inline)) {
+        auto filled = [&](int b) __attribute__((always_inline)) {
             ts_wait_store();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&a_full[grp * 2 + (q & 1)]);
+            if (lane == 0) mbar_arrive(&a_full[grp * 2 + slot(b)]);
             ++q;
         };
-        auto step = [&](int b, int i, int kbs) __attribute__((always_inline)) {
+        auto step = [&](int b, int i) __attribute__((always_inline)) {
             const bool two = 2 * i + 1 < kbs;
             uint32_t r[16];
             ts_dequant(wq[b][0].x, wq[b][0].y, sz[b][0], r);
             ts_dequant(wq[b][0].z, wq[b][0].w, sz[b][UNI ? 0 : 1], r + 8);
-            wait_slot();
+            wait_slot(b);
             if (!ok) return;
-            ts_store(a_lane + (q & 1) * 32 * KS, r);
-            if (KS == 1) filled();
+            ts_store(a_lane + slot(b) * 32 * KS, r);
+            if (KS == 1) filled(b);
             if (two) {
                 ts_dequant(wq[b][1].x, wq[b][1].y, sz[b][UNI ? 0 : 2], r);
                 ts_dequant(wq[b][1].z, wq[b][1].w, sz[b][UNI ? 0 : 3], r + 8);
-                if (KS == 1) { wait_slot(); if (!ok) return; }
-                ts_store(a_lane + (q & 1) * 32 * KS + (KS - 1) * 32, r);
+                if (KS == 1) { wait_slot(b); if (!ok) return; }
+                ts_store(a_lane + slot(b) * 32 * KS + (KS - 1) * 32, r);
             }
             load(b);
-            if (KS == 2 || two) filled();
+            if (KS == 2 || two) filled(b);
         };
-        for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
-            const Item it = item(i);
-            const int steps = (it.kbs + 1) >> 1;
-#pragma unroll 1
-            for (int s = first; ok && s < steps; s += 2 * stride) {
-                step(0, s, it.kbs);
-                if (!ok) break;
-                if (s + stride < steps) step(1, s + stride, it.kbs);
-                else load(1);
-            }
-            // ---- epilogue (one lane polls, the other warps sleep at a hardware barrier)
-            if (warp == 0) {
-                if (lane == 0 && ok) mbar_wait(acc_full, item_ph, abort_flag);
-                __syncwarp();
-            }
-            asm volatile("bar.sync 1, %0;" :: "n"(TS_PRODUCERS * 32) : "memory");
-            item_ph ^= 1;
-            pdl_wait();
-            ok = ok && !*abort_flag;
-            tc_fence_after();
-            if (ok) {
-                const int lg = warp & 3, t0 = it.tt * p.t_tile, Tn = min(p.t_tile, p.T - t0);
-                const size_t plane = (size_t)(it.kb0 / per_kb) * (size_t)p.plane_stride;     // (split-K of TC_EPI_STORE_F32)
-                const int chunks = (Tn + TC_EPI_COLS - 1) / TC_EPI_COLS;
-                for (int c = warp >> 2; c < MH * chunks; c += TS_PRODUCERS / 4) {
-                    const int hc = MH == 2 && c >= chunks ? 1 : 0, c0 = (c - hc * chunks) * TC_EPI_COLS;
-                    uint32_t r[TC_EPI_COLS];
-                    tc_ld16(tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(hc * acc_cols + c0), r);
-                    tc_wait_ld();
-                    tc_epilogue(p, r, lane, (it.mt * MH + hc) * TS_BM + lg * 32, t0 + c0, Tn - c0, plane, per_kb < p.KB, sE + warp * TC_EPI_STAGE);
-                }
-            }
-            tc_fence_before();
+        for (int s = first; s < steps; s += 2 * stride) {
+            step(0, s);
+            if (!ok) break;
+            if (s + stride < steps) step(1, s + stride);
+            if (!ok) break;
+        }
+        // ---- epilogue (one lane polls, the other warps sleep at a hardware barrier)
+        if (warp == 0) {
+            if (lane == 0 && ok) mbar_wait(acc_full, 0, abort_flag);
             __syncwarp();
-            if (lane == 0) mbar_arrive(acc_empty);
+        }
+        asm volatile("bar.sync 1, %0;" :: "n"(TS_PRODUCERS * 32) : "memory");
+        pdl_wait();
+        ok = ok && !*abort_flag;
+        tc_fence_after();
+        if (ok) {
+            const int lg = warp & 3, t0 = tt * p.t_tile, Tn = min(p.t_tile, p.T - t0);
+            const size_t plane = (size_t)z * (size_t)p.plane_stride;     // (split-K of TC_EPI_STORE_F32)
+            const int chunks = (Tn + TC_EPI_COLS - 1) / TC_EPI_COLS;
+            for (int c = warp >> 2; c < MH * chunks; c += TS_PRODUCERS / 4) {
+                const int hc = MH == 2 && c >= chunks ? 1 : 0, c0 = (c - hc * chunks) * TC_EPI_COLS;
+                uint32_t r[TC_EPI_COLS];
+                tc_ld16(tmem_base + ((uint32_t)(lg * 32) << 16) + (uint32_t)(hc * acc_cols + c0), r);
+                tc_wait_ld();
+                tc_epilogue(p, r, lane, (mt * MH + hc) * TS_BM + lg * 32, t0 + c0, Tn - c0, plane, per_kb < p.KB, sE + warp * TC_EPI_STAGE);
+            }
         }
     } else if (warp == TS_PRODUCERS) {
         // ================= activation producer (TMA) =================
         int st = 0;
         uint32_t ph = 0;
-        bool ok = true, waited = false;
         unsigned char* b = sB;
-        for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
-            const Item it = item(i);
-            const unsigned char* w0 = (const unsigned char*)(p.qfrag + ((size_t)it.mt * (2 * MH) * p.KB + it.kb0) * 128);
-            // (2 KB of weights a k-block and 64 outputs, k-blocks side by side)
-            auto ahead = [&](int kb, int n) {
-                n = min(n, it.kbs - kb);
-                if (n > 0) for (int j = 0; j < 2 * MH; ++j) ts_prefetch_l2(w0 + ((size_t)j * p.KB + kb) * 2048, (uint32_t)n * 2048u);
-            };
-            if (elect_one()) ahead(0, TS_AHEAD);
-            __syncwarp();
-            if (!waited) { pdl_wait(); waited = true; }
-            for (int kb = 0, kx = it.kb0 * TS_BK; kb < it.kbs; kb += KS, kx += KS * TS_BK) {
-                ok = __all_sync(0xffffffffu, mbar_wait(&b_empty[st], ph ^ 1, abort_flag));
-                if (!ok) break;
-                if (elect_one()) {
-                    const bool two = KS == 2 && kb + 1 < it.kbs;
-                    mbar_arrive_expect_tx(&b_full[st], (uint32_t)(two ? 2 * box_bytes : box_bytes));
-                    tma_load_2d(b, &xmap, kx, it.tt * p.t_tile, &b_full[st]);
-                    if (two) tma_load_2d(b + box_bytes, &xmap, kx + TS_BK, it.tt * p.t_tile, &b_full[st]);
-                    if ((kb & 7) == 0) ahead(kb + TS_AHEAD, 8);
-                }
-                __syncwarp();
-                b += stage_bytes;
-                if (++st == S) { st = 0; ph ^= 1; b = sB; }
+        const unsigned char* w0 = (const unsigned char*)(p.qfrag + ((size_t)mt * (2 * MH) * p.KB + kb0) * 128);
+        // (2 KB of weights a k-block and 64 outputs, k-blocks side by side)
+        auto ahead = [&](int kb, int n) {
+            n = min(n, kbs - kb);
+            if (n > 0) for (int j = 0; j < 2 * MH; ++j) ts_prefetch_l2(w0 + ((size_t)j * p.KB + kb) * 2048, (uint32_t)n * 2048u);
+        };
+        if (elect_one()) ahead(0, TS_AHEAD);
+        __syncwarp();
+        pdl_wait();
+        for (int kb = 0, kx = kb0 * TS_BK; kb < kbs; kb += KS, kx += KS * TS_BK) {
+            if (!__all_sync(0xffffffffu, mbar_wait(&b_empty[st], ph ^ 1, abort_flag))) break;
+            if (elect_one()) {
+                const bool two = KS == 2 && kb + 1 < kbs;
+                mbar_arrive_expect_tx(&b_full[st], (uint32_t)(two ? 2 * box_bytes : box_bytes));
+                tma_load_2d(b, &xmap, kx, tt * p.t_tile, &b_full[st]);
+                if (two) tma_load_2d(b + box_bytes, &xmap, kx + TS_BK, tt * p.t_tile, &b_full[st]);
+                if ((kb & 3) == 0) ahead(kb + TS_AHEAD, 4);
             }
+            __syncwarp();
+            b += stage_bytes;
+            if (++st == S) { st = 0; ph ^= 1; b = sB; }
         }
     } else {
         // ================= MMA issuers: warp 17 + h for accumulator h =================
         // descriptors differ between stages and k16 steps only in the start-address field (16-byte units)
         const int h = MH == 2 ? warp - TS_PRODUCERS - 1 : 0;
         const uint64_t bd0 = make_desc_sw128(smem_u32(sB)), b_step = (uint64_t)(stage_bytes >> 4), b_box = (uint64_t)(box_bytes >> 4);
-        const uint32_t acc = tmem_base + h * acc_cols;
+        const uint32_t acc = tmem_base + h * acc_cols, idesc = make_idesc_f16((min(p.t_tile, p.T - tt * p.t_tile) + 15) & ~15);
         uint64_t bd = bd0;
         int st = 0;
-        uint32_t ph = 0, item_ph = 0;
+        uint32_t ph = 0;
         uint32_t q[2] = {0, 0};                    // slots of the group taken; MH = 2: only that of group h counts
+        uint32_t odd = 0;                          // MH = 1: pairs of k-blocks come from the groups in turn
         bool ok = true;
-        for (int i = blockIdx.x; i < n_items && ok; i += gridDim.x) {
-            const Item it = item(i);
-            const int Tp = (min(p.t_tile, p.T - it.tt * p.t_tile) + 15) & ~15;
-            const uint32_t idesc = make_idesc_f16(Tp);
-            // (the first wait passes at once: no item has used the accumulators)
-            ok = __all_sync(0xffffffffu, mbar_wait(acc_empty, item_ph ^ 1, abort_flag));
-            item_ph ^= 1;
-            uint32_t odd = 0;                      // MH = 1: pairs of k-blocks come from the groups in turn
-            for (int kb = 0; ok && kb < it.kbs; kb += KS) {
-                const uint32_t grp = MH == 2 ? (uint32_t)h : odd;
-                const uint32_t n = MH == 2 || !odd ? q[0] : q[1];
-                const uint32_t sl = grp * 2 + (n & 1);
-                // (both barriers are asked before either answer is needed)
-                const bool r0 = mbar_try_wait(&b_full[st], ph), r1 = mbar_try_wait(&a_full[sl], (n >> 1) & 1);
-                if (!__all_sync(0xffffffffu, r0 && r1)) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(&b_full[st], ph, abort_flag) && mbar_wait(&a_full[sl], (n >> 1) & 1, abort_flag));
-                    if (!ok) break;
-                }
-                tc_fence_after();
-                const uint32_t a = tmem_a + sl * (32 * KS);
-                if (elect_one()) {
-#pragma unroll
-                    for (int k16 = 0; k16 < TS_BK / 16; ++k16) ts_mma(acc, a + 8 * k16, bd + 2 * k16, idesc, (kb | k16) ? 1u : 0u);
-                    if (KS == 2 && kb + 1 < it.kbs) {
-#pragma unroll
-                        for (int k16 = 0; k16 < TS_BK / 16; ++k16) ts_mma(acc, a + 32 + 8 * k16, bd + b_box + 2 * k16, idesc, 1u);
-                    }
-                    tc_commit(&a_empty[sl]);
-                    tc_commit(&b_empty[st]);
-                }
-                __syncwarp();
-                if (MH == 2 || !odd) ++q[0]; else ++q[1];
-                if (MH == 1) odd ^= 1;
-                bd += b_step;
-                if (++st == S) { st = 0; ph ^= 1; bd = bd0; }
+        for (int kb = 0; kb < kbs; kb += KS) {
+            const uint32_t grp = MH == 2 ? (uint32_t)h : odd;
+            const uint32_t n = MH == 2 || !odd ? q[0] : q[1];
+            const uint32_t sl = grp * 2 + (n & 1);
+            // (both barriers are asked before either answer is needed)
+            const bool r0 = mbar_try_wait(&b_full[st], ph), r1 = mbar_try_wait(&a_full[sl], (n >> 1) & 1);
+            if (!__all_sync(0xffffffffu, r0 && r1)) {
+                ok = __all_sync(0xffffffffu, mbar_wait(&b_full[st], ph, abort_flag) && mbar_wait(&a_full[sl], (n >> 1) & 1, abort_flag));
+                if (!ok) break;
             }
-            if (ok && elect_one()) tc_commit(acc_full);
+            tc_fence_after();
+            const uint32_t a = tmem_a + sl * (32 * KS);
+            if (elect_one()) {
+#pragma unroll
+                for (int k16 = 0; k16 < TS_BK / 16; ++k16) ts_mma(acc, a + 8 * k16, bd + 2 * k16, idesc, (kb | k16) ? 1u : 0u);
+                if (KS == 2 && kb + 1 < kbs) {
+#pragma unroll
+                    for (int k16 = 0; k16 < TS_BK / 16; ++k16) ts_mma(acc, a + 32 + 8 * k16, bd + b_box + 2 * k16, idesc, 1u);
+                }
+                tc_commit(&a_empty[sl]);
+                tc_commit(&b_empty[st]);
+            }
             __syncwarp();
+            if (MH == 2 || !odd) ++q[0]; else ++q[1];
+            if (MH == 1) odd ^= 1;
+            bd += b_step;
+            if (++st == S) { st = 0; ph ^= 1; bd = bd0; }
         }
+        if (ok && elect_one()) tc_commit(acc_full);
+        __syncwarp();
     }
     if (*abort_flag && tid == 0 && p.status) atomicExch(p.status, 1);
     tc_fence_before();
@@ -370,7 +329,7 @@ gemm_int4_ts_kernel(const GemmTcParams p, const __grid_constant__ CUtensorMap xm
 }
 
 // x: [T][ldx] fp16 activations (ldx multiple of 8, base 16-byte aligned).  t_tile, m_halves and k_splits are the wanted
-// shape; an item takes at most 256 tokens with 128 outputs and 192 with 256 (their accumulators leave room for the weights).
+// shape; a CTA takes at most 256 tokens with 128 outputs and 192 with 256 (their accumulators leave room for the weights).
 B2_API int b2_gemm_int4_tc(const GemmTcParams* p, const void* x, int ldx, cudaStream_t stream) {
     if (p->bf16) return cudaErrorInvalidValue;             // INT4 weights are dequantised to fp16
     if (p->T < 1 || p->t_tile < 16 || p->t_tile > 512 || (p->t_tile & 15) || (ldx & 7) || ((uintptr_t)x & 15))
@@ -397,18 +356,17 @@ B2_API int b2_gemm_int4_tc(const GemmTcParams* p, const void* x, int ldx, cudaSt
     if (ks > 1 && !planes) per = (per + 1) & ~1;
     ks = (q.KB + per - 1) / per;
     const bool uni = q.gshift == 2 && (q.off32 & 3) == 0 && (ks == 1 || (per & 1) == 0);
-    const int n_mt = (q.NTL * 16) / (TS_BM * q.m_halves), n_tt = (q.T + q.t_tile - 1) / q.t_tile, items = n_mt * n_tt * ks;
+    const int n_mt = (q.NTL * 16) / (TS_BM * q.m_halves), n_tt = (q.T + q.t_tile - 1) / q.t_tile;
     const int acc = ((q.t_tile + 31) & ~31) * q.m_halves, KS = acc <= 256 ? 2 : 1;
     // as many stages as 192 KB hold: their depth covers the latency of the loads.  (A CTA has the SM's tensor memory to
     // itself; its registers keep a second one off.)
     const int stage = q.t_tile * 128 * KS;
     int stages = TS_STAGE_SMEM / stage;
     q.stages = stages > TS_MAX_STAGES ? TS_MAX_STAGES : stages;
-    const size_t smem = 1024 + (size_t)q.stages * stage + TS_PRODUCERS * TC_EPI_STAGE + (2 * q.stages + 2 * TS_SLOTS + 2) * 8 + 16;
-    const dim3 grid(items < 148 ? items : 148);
+    const size_t smem = 1024 + (size_t)q.stages * stage + TS_PRODUCERS * TC_EPI_STAGE + (2 * q.stages + 2 * TS_SLOTS + 1) * 8 + 16;
     auto go = [&](auto kern, SmemOptIn& optin) -> int {
         if (cudaError_t e = optin.ensure(kern, smem)) return e;
-        return launch_pdl(kern, grid, dim3((TS_PRODUCERS + 1 + q.m_halves) * 32), smem, stream, q, map, n_mt, n_tt, items, per);
+        return launch_pdl(kern, dim3(n_mt * n_tt * ks), dim3((TS_PRODUCERS + 1 + q.m_halves) * 32), smem, stream, q, map, n_mt, n_tt, per);
     };
     static SmemOptIn o[6];
     if (q.m_halves == 1) return uni ? go(gemm_int4_ts_kernel<1, 2, true>, o[0]) : go(gemm_int4_ts_kernel<1, 2, false>, o[1]);

@@ -172,11 +172,11 @@ def test_gemm_f16_tc_dense_weights(T, N, K):
     (4096, 256, 192, 192, 2, 128),      # the widest tile with two accumulators: one k-block per slot
     (448, 512, 193, 512, 2, 256),       # one token too many for it, a group longer than a slot
     (2048, 128, 257, 512, 1, 128),      # one token more than the widest tile
-    (1024, 20480, 48, 16, 1, 128),      # more items than CTAs: three or four a CTA
-    (192, 37888, 20, 32, 2, 128),       # the same, two accumulators and an odd number of k-blocks
+    (1024, 20480, 48, 16, 1, 128),      # more CTAs than SMs
+    (192, 37888, 20, 32, 2, 128),       # two accumulators and an odd number of k-blocks
 ])
-def test_gemm_int4_tc_items_slots_and_edges(K, N, T, tt, mh, g):
-    """All output forms at the edges of tiles, slots and the walk over items, against the product of the weights as the
+def test_gemm_int4_tc_slots_and_edges(K, N, T, tt, mh, g):
+    """All output forms at the edges of tiles and slots, against the product of the weights as the
     kernel rounds them.  Bound: a sum of K products in steps of 16 of which each may lose one unit in the last place."""
     from mi50grad_b200.ops import kernels as Kn
     from mi50grad_b200.ops import lib as L
