@@ -48,10 +48,12 @@ struct VerifySmem {
     float mm[NM][DV], sq[NM][DV];                         // S0^T k, S0^T q; later the update vectors and the outputs
     float dk[NM][NM], dq[NM][NM];                         // k_t . k_a, q_t . k_a (t == a: k.k, q.k), then their coefficients
     float qq[NM], invq[NM], invk[NM], gl[NM], G[NM], beta[NM], ab[NM][2];
-    float ss[NM][DV / 32];
+    float eG[NM], eGp[NM], egl[NM];                       // exp of G, of the parent's G, of the node's own log decay
+    float ss[NM];
+    uchar4 tap[NM];                                       // rows of xraw that hold the inputs at distance 1, 2, 3 on the path
     float abp[VF_THREADS / 32][VF_CHUNK][2];
     unsigned anc[NM];
-    alignas(16) __half xraw[NM][NCH];
+    alignas(16) __half xraw[NM + 3][NCH];                 // the nodes' inputs; then the history, oldest first
     float4 red[2][VF_CHUNK][RG][LPR];
 };
 
@@ -105,7 +107,21 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
 #pragma unroll
         for (int e = 0; e < 4; ++e) cw[q][e] = w[e];
     }
+    // (and the constants of the last phases, each of which would wait for its own trip there)
+    const float a_log = p.A_log[j], dt_bias = __half2float(p.dt_bias[j]), norm_w = __half2float(p.norm_w[tid % DV]);
+    static_assert(VF_THREADS % DV == 0, "a thread keeps to one column of the outputs");
+#pragma unroll
+    for (int q = 0; q < CPT; ++q) {
+        const int c = tid + q * VF_THREADS;
+        if (c < NCH)
+#pragma unroll
+            for (int e = 0; e < 3; ++e) sm.xraw[NM + e][c] = hist[q][e];
+    }
     pdl_wait();
+    constexpr int TZ = VF_THREADS / DV, NZ = 4;                        // gate inputs of the thread's first NZ outputs (nodes TZ apart)
+    __half zv[NZ];
+#pragma unroll
+    for (int q = 0; q < NZ; ++q) zv[q] = p.proj[(size_t)(r0 + min(tid / DV + q * TZ, N - 1)) * p.ld + p.off_z + j * DV + tid % DV];
 
     auto proj_col = [&](int c) -> int {
         if (c < DK) return p.off_q + kh * DK + c;
@@ -125,7 +141,19 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
         }
     }
     // ancestors of a node inside this sequence's block (bit a <-> node a)
-    if (tid < N) sm.anc[tid] = (unsigned)(p.rows[r0 + tid].mask & 0xFFFFull) & ((1u << tid) - 1u);
+    if (tid < N) {
+        const unsigned m = (unsigned)(p.rows[r0 + tid].mask & 0xFFFFull) & ((1u << tid) - 1u);
+        sm.anc[tid] = m;
+        // beyond the root the path goes on in the history
+        int row[3];
+        unsigned rest = m;
+        for (int e = 0, h = NM + 2; e < 3; ++e) {
+            const int a = top_bit(rest);
+            row[e] = a >= 0 ? a : h--;
+            if (a >= 0) rest &= ~(1u << a);
+        }
+        sm.tap[tid] = make_uchar4((unsigned char)row[0], (unsigned char)row[1], (unsigned char)row[2], 0);
+    }
     // ---- a / b inputs of the gates
     const bool inkernel_ab = p.off_a < 0;
     if (inkernel_ab) {
@@ -176,17 +204,11 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
     for (int q = 0; q < CPT; ++q) {
         const int c = tid + q * VF_THREADS;
         if (c >= NCH) break;
-        const float h0 = __half2float(hist[q][0]), h1 = __half2float(hist[q][1]), h2 = __half2float(hist[q][2]);
         const float w0 = __half2float(cw[q][0]), w1 = __half2float(cw[q][1]), w2 = __half2float(cw[q][2]), w3 = __half2float(cw[q][3]);
+#pragma unroll 2
         for (int t = 0; t < N; ++t) {
-            // taps at distance 1..3 along the path; beyond the root they come from the history
-            const unsigned a1 = sm.anc[t];
-            const int d = __popc(a1), p1 = top_bit(a1);
-            const unsigned a2 = p1 >= 0 ? a1 & ~(1u << p1) : 0u;
-            const int p2 = top_bit(a2), p3 = top_bit(p2 >= 0 ? a2 & ~(1u << p2) : 0u);
-            const float x1 = d >= 1 ? __half2float(sm.xraw[p1][c]) : h2;
-            const float x2 = d >= 2 ? __half2float(sm.xraw[p2][c]) : (d == 1 ? h2 : h1);
-            const float x3 = d >= 3 ? __half2float(sm.xraw[p3][c]) : (d == 2 ? h2 : (d == 1 ? h1 : h0));
+            const uchar4 r = sm.tap[t];
+            const float x1 = __half2float(sm.xraw[r.x][c]), x2 = __half2float(sm.xraw[r.y][c]), x3 = __half2float(sm.xraw[r.z][c]);
             const float o = silu_f(x3 * w0 + x2 * w1 + x1 * w2 + __half2float(sm.xraw[t][c]) * w3);
             if (c < DK) sm.cq[t][c] = o; else if (c < 2 * DK) sm.ck[t][c - DK] = o; else sm.cv[t][c - 2 * DK] = o;
         }
@@ -194,37 +216,45 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
     __syncthreads();
     // ---- dot products of every node with itself and with its ancestors, a warp each
     {
-        int n = 0;
-        for (int t = 0; t < N; ++t)
-            for (unsigned m = sm.anc[t] | (1u << t); m; m &= m - 1, ++n) {
-                if (n % WARPS != warp) continue;
-                const int a = __ffs(m) - 1;
-                float kk = 0.f, qk = 0.f, qq = 0.f;
-                for (int i = lane; i < DK; i += 32) {
-                    const float ka = sm.ck[a][i], q = sm.cq[t][i];
-                    kk = fmaf(sm.ck[t][i], ka, kk);
-                    qk = fmaf(q, ka, qk);
-                    qq = fmaf(q, q, qq);
-                }
-                kk = warp_sum(kk);
-                qk = warp_sum(qk);
-                if (a == t) qq = warp_sum(qq);
-                if (lane == 0) { sm.dk[t][a] = kk; sm.dq[t][a] = qk; if (a == t) sm.qq[t] = qq; }
+        constexpr int E = DK / 32;                        // elements of a lane
+        struct alignas(4 * E) Elems { float v[E]; };
+        for (int n = warp; n < N * (N + 1) / 2; n += WARPS) {
+            int t = (int)((sqrtf(8.f * n + 1.f) - 1.f) * 0.5f);          // pair (t, a), a <= t
+            if ((t + 1) * (t + 2) / 2 <= n) ++t;
+            if (t * (t + 1) / 2 > n) --t;
+            const int a = n - t * (t + 1) / 2;
+            if (a != t && !(sm.anc[t] >> a & 1)) continue;
+            const Elems ka = *(const Elems*)&sm.ck[a][lane * E], kt = *(const Elems*)&sm.ck[t][lane * E], qt = *(const Elems*)&sm.cq[t][lane * E];
+            float kk = 0.f, qk = 0.f, qq = 0.f;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                kk = fmaf(kt.v[e], ka.v[e], kk);
+                qk = fmaf(qt.v[e], ka.v[e], qk);
+                qq = fmaf(qt.v[e], qt.v[e], qq);
             }
+            kk = warp_sum(kk);
+            qk = warp_sum(qk);
+            if (a == t) qq = warp_sum(qq);
+            if (lane == 0) { sm.dk[t][a] = kk; sm.dq[t][a] = qk; if (a == t) sm.qq[t] = qq; }
+        }
     }
     __syncthreads();
     if (tid < N) {
         sm.invq[tid] = rsqrtf(sm.qq[tid] + 1e-6f) * rsqrtf((float)DK);
         sm.invk[tid] = rsqrtf(sm.dk[tid][tid] + 1e-6f);
-        const float x = sm.ab[tid][0] + __half2float(p.dt_bias[j]);
-        sm.gl[tid] = fmaxf(-__expf(p.A_log[j]) * (x > 20.f ? x : log1pf(__expf(x))), -20.f);
+        const float x = sm.ab[tid][0] + dt_bias;
+        sm.gl[tid] = fmaxf(-__expf(a_log) * (x > 20.f ? x : log1pf(__expf(x))), -20.f);
         sm.beta[tid] = sigmoid_f(sm.ab[tid][1]);
     }
     __syncthreads();
     if (tid < N) {
         float g = 0.f;                                    // summed log-decay along the path
-        for (unsigned m = sm.anc[tid] | (1u << tid); m; m &= m - 1) g += sm.gl[__ffs(m) - 1];
-        sm.G[tid] = g;
+        for (unsigned m = sm.anc[tid]; m; m &= m - 1) g += sm.gl[__ffs(m) - 1];
+        const float own = sm.gl[tid];
+        sm.eGp[tid] = __expf(g);                          // (the parent's path is the node's without itself)
+        sm.G[tid] = g + own;
+        sm.eG[tid] = __expf(g + own);
+        sm.egl[tid] = __expf(own);
     }
     // ---- S0^T k and S0^T q of all nodes
     for (int t0 = 0; t0 < N; t0 += VF_CHUNK) {
@@ -274,35 +304,42 @@ __global__ void __launch_bounds__(VF_THREADS, 2) deltanet_verify_kernel(const De
     if (tid < DV) {
         for (int t = 0; t < N; ++t) {
             const unsigned m0 = sm.anc[t];
-            const float Gp = m0 ? sm.G[top_bit(m0)] : 0.f;
-            float Sk = __expf(Gp) * sm.mm[t][tid], ys = __expf(sm.G[t]) * sm.sq[t][tid];
+            float Sk = sm.eGp[t] * sm.mm[t][tid], ys = sm.eG[t] * sm.sq[t][tid];
             for (unsigned m = m0; m; m &= m - 1) {
                 const int a = __ffs(m) - 1;
                 const float u = sm.mm[a][tid];
                 Sk = fmaf(sm.dk[t][a], u, Sk);
                 ys = fmaf(sm.dq[t][a], u, ys);
             }
-            const float delta = (sm.cv[t][tid] - __expf(sm.gl[t]) * Sk) * sm.beta[t];
-            const float y = fmaf(delta, sm.dq[t][t], ys);
+            const float delta = (sm.cv[t][tid] - sm.egl[t] * Sk) * sm.beta[t];
             sm.mm[t][tid] = delta;
-            sm.sq[t][tid] = y;
-            const float s = warp_sum(y * y);
-            if (lane == 0) sm.ss[t][warp] = s;
+            sm.sq[t][tid] = fmaf(delta, sm.dq[t][t], ys);
         }
+    }
+    __syncthreads();
+    for (int t = warp; t < N; t += WARPS) {
+        float y2 = 0.f;
+#pragma unroll
+        for (int q = 0; q < DV / 32; ++q) { const float y = sm.sq[t][lane + 32 * q]; y2 = fmaf(y, y, y2); }
+        y2 = warp_sum(y2);
+        if (lane == 0) sm.ss[t] = rsqrtf(y2 / (float)DV + p.eps);
     }
     __syncthreads();
     // ---- gated RMSNorm over the head's dv outputs; staging for the commit
     unsigned char* blk = st.base + (size_t)layer * st.layer_stride + (size_t)si * st.seq_stride;
     float* su = (float*)(blk + st.off_u);
-    for (int i = tid; i < N * DV; i += VF_THREADS) {
-        const int t = i / DV, c = i - t * DV;
-        float tot = 0.f;
+    {
+        const int c = tid % DV;
+        int q = 0;
+        for (int t = tid / DV; t < N; t += TZ, ++q) {
+            __half zh = zv[0];
 #pragma unroll
-        for (int q = 0; q < DV / 32; ++q) tot += sm.ss[t][q];
-        const float z = __half2float(p.proj[(size_t)(r0 + t) * p.ld + p.off_z + j * DV + c]);
-        const float o = sm.sq[t][c] * rsqrtf(tot / (float)DV + p.eps) * __half2float(p.norm_w[c]) * silu_f(z);
-        p.out[(size_t)(r0 + t) * p.ldo + j * DV + c] = __float2half(o);
-        su[((size_t)t * p.nv + j) * DV + c] = sm.mm[t][c];
+            for (int e = 1; e < NZ; ++e) if (q == e) zh = zv[e];
+            if (q >= NZ) zh = p.proj[(size_t)(r0 + t) * p.ld + p.off_z + j * DV + c];
+            const float o = sm.sq[t][c] * sm.ss[t] * norm_w * silu_f(__half2float(zh));
+            p.out[(size_t)(r0 + t) * p.ldo + j * DV + c] = __float2half(o);
+            su[((size_t)t * p.nv + j) * DV + c] = sm.mm[t][c];
+        }
     }
     const int conv_dim = 2 * p.nk * DK + p.nv * DV;
     __half* sx = (__half*)(blk + st.off_x);
