@@ -808,6 +808,11 @@ static int mixer_block(Driver* d, const MixerLayerDesc& L, const MixRun& run, bo
     if (L.kind == MIX_RECURRENCE) { r.xbc = (void*)r.proj; r.ld_xbc = r.ld_proj; }     // the projection's epilogue has applied the SiLU
     else {
         CK(L.kind == MIX_ATTENTION ? b2_head_prepare(&L.mix, &r, s) : b2_mix_prepare(&L.mix, &r, s));
+        if (L.kind != MIX_ATTENTION && !one && b2_mix_decode_takes(&L.mix, &r)) {
+            CK(b2_mix_decode(&L.mix, &r, s));
+            d->launches += 2;
+            return 0;
+        }
         if (one && r.n_rows >= 16) CK(b2_window_attn_rows(&L.mix, &r, s)); else CK(b2_window_attn_decode(&L.mix, &r, s));
         d->launches += 2;
     }

@@ -228,5 +228,8 @@ B2_API int b2_head_prepare(const MixLayer* l, const MixRun* r, cudaStream_t s);
 B2_API int b2_window_attn_decode(const MixLayer* l, const MixRun* r, cudaStream_t s);
 B2_API int b2_window_attn_rows(const MixLayer* l, const MixRun* r, cudaStream_t s);
 B2_API int b2_ssd_step(const MixLayer* l, const MixRun* r, cudaStream_t s);
+// b2_window_attn_decode and b2_ssd_step in one launch, where it is taken (csrc/mix_decode.cu)
+B2_API int b2_mix_decode_takes(const MixLayer* l, const MixRun* r);
+B2_API int b2_mix_decode(const MixLayer* l, const MixRun* r, cudaStream_t s);
 B2_API int b2_ssd_chunk(const MixLayer* l, const MixRun* r, cudaStream_t s);
 #define SSD_CHUNK 64

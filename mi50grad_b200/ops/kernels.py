@@ -657,5 +657,5 @@ def stream_rows(x: torch.Tensor, coef: torch.Tensor, w: torch.Tensor, xb: torch.
 
 
 def mix_op(name: str, layer: L.MixLayer, run: L.MixRun):
-    """Launch one mixer kernel: 'mix_prepare', 'head_prepare', 'window_attn_decode', 'window_attn_rows', 'ssd_step', 'ssd_chunk'."""
+    """Launch one mixer kernel: 'mix_prepare', 'head_prepare', 'window_attn_decode', 'window_attn_rows', 'ssd_step', 'mix_decode', 'ssd_chunk'."""
     L.check(getattr(L.lib(), "b2_" + name)(C.byref(layer), C.byref(run), L.stream()), name)

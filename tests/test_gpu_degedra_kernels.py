@@ -484,6 +484,48 @@ def test_recurrence_step(dt, shape):
         assert int(x.b["ssd_counters"].abs().sum()) == 0
 
 
+MERGED = SHAPES + [dict(H=1, G=1, d=8, rot=8, heads=1, P=1, N=1, groups=1, ngroups=1, taps=2), dict(H=16, G=4, d=128, rot=64, heads=16, P=64, N=128, groups=2, ngroups=8, taps=4),
+                   dict(H=6, G=2, d=64, rot=32, heads=3, P=40, N=65, groups=3, ngroups=1, taps=3), dict(H=2, G=2, d=72, rot=32, heads=4, P=32, N=64, groups=1, ngroups=4, taps=1)]
+
+
+@pytest.mark.parametrize("dt", ["bf16", "f32"])
+@pytest.mark.parametrize("shape", range(len(MERGED)))
+@pytest.mark.parametrize("window,commit", [(1, 1), (130, 0), (0, 1)])
+def test_both_halves_of_a_mixer_in_one_launch(dt, shape, window, commit):
+    """The launch that holds attention and recurrence gives the bits of the two launches it replaces: outputs, states,
+    histories and counters; what it does not take (wide heads, many of them to a key head, large states, several rows of a
+    sequence) it refuses."""
+    from mi50grad_b200.ops import lib as L
+    x = Mix(dt, window=window, **MERGED[shape])
+    S0, h0 = _rnd(3, x.heads, x.N, x.P, seed=4), _rnd(3, x.taps - 1, x.C, seed=9).to(x.T)
+    for s in range(3):
+        _fill_cache(x, s, 300, seed=10 * s)
+    takes = lambda: bool(L.lib().b2_mix_decode_takes(C.byref(x.m), C.byref(x.r)))
+    for parts in ([(1, 250, 1)], [(2, 0, 1), (0, 299, 1), (1, 63, 1)]):
+        n = x.rows(parts)
+        x.b["proj"][:n] = _rnd(n, x.ld).to(x.T).cuda()
+        x.r.commit = commit
+        want = x.H // x.G <= 4 and x.d <= 128 and x.N <= 128
+        assert takes() == want
+        got = []
+        for ops in (("window_attn_decode", "ssd_step"), ("mix_decode",)):
+            if ops == ("mix_decode",) and not want:
+                with pytest.raises(Exception):
+                    x.op("mix_decode")
+                continue
+            x.S.copy_(S0); x.hist.copy_(h0)
+            x.b["out"].fill_(9.0); x.b["ubuf"].fill_(9.0)
+            x.op("mix_prepare")
+            for op in ops:
+                x.op(op)
+            got.append([t.clone() for t in (x.b["out"], x.b["ubuf"], x.S, x.hist)])
+            assert int(x.b["attn_counters"].abs().sum()) == 0 and int(x.b["ssd_counters"].abs().sum()) == 0
+        for a, b in zip(*(got if want else got * 2)):
+            assert torch.equal(a, b)
+    x.rows([(1, 5, 3), (0, 0, 1)])
+    assert not takes()
+
+
 @pytest.mark.parametrize("op,n", [("ssd_step", 1), ("ssd_step", 5), ("ssd_chunk", 70)])
 def test_recurrences_in_a_row(op, n):
     """Launch after launch on one state: each starts from what the one before left, although it may begin under it."""
