@@ -99,15 +99,15 @@ __device__ __forceinline__ void sc_cumsum(const MixLayer& L, const MixRun& R, in
 __device__ __forceinline__ void sc_stage(const MixRun& R, int t0, int n, int c0, int w, int wp, bf16* dst, int ld, int tid, int nthr) {
     const bf16* src = (const bf16*)R.xbc + c0;
     const bool vec = ((R.ld_xbc | c0) & 7) == 0;
-    const int ppr = wp >> 3;
-    for (int i = tid; i < SC_T * ppr; i += nthr) {
-        const int r = i / ppr, c = (i % ppr) * 8;
-        bf16* d = dst + r * ld + c;
-        if (vec && r < n && c + 8 <= w) cp_async16(d, src + (size_t)(t0 + r) * R.ld_xbc + c);
-        else
+    const int ppr = wp >> 3, sh = ppr > 1 ? 32 - __clz(ppr - 1) : 0, c = (tid & ((1 << sh) - 1)) * 8;      // (no division for each piece)
+    if (c < wp)
+        for (int r = tid >> sh; r < SC_T; r += nthr >> sh) {
+            bf16* d = dst + r * ld + c;
+            if (vec && r < n && c + 8 <= w) cp_async16(d, src + (size_t)(t0 + r) * R.ld_xbc + c);
+            else
 #pragma unroll
-            for (int e = 0; e < 8; ++e) d[e] = (r < n && c + e < w) ? src[(size_t)(t0 + r) * R.ld_xbc + c + e] : __float2bfloat16(0.f);
-    }
+                for (int e = 0; e < 8; ++e) d[e] = (r < n && c + e < w) ? src[(size_t)(t0 + r) * R.ld_xbc + c + e] : __float2bfloat16(0.f);
+        }
     cp_async_commit();
 }
 
@@ -126,17 +126,43 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const MixLayer L, 
     const float A = rec_rate(L, h);
     pdl_wait();
     sc_stage(R, t0, n, L.rB + grp * L.N, L.N, Np, Bs, LDN, tid, 128);
+    // x in pieces of eight columns, all of a thread's requested at once: element by element between the stores of W they were
+    // a trip to L2 each (1000 rows, 80 heads of 128 x 64: 63 -> 29 us, bound by its shared-memory traffic now)
+    constexpr int PIECES = SC_T * (SC_P / 8) / 128;
+    uint4 xr[PIECES];
+    const int x0 = L.rx + h * L.P + p0;
+    const bool vec = ((R.ld_xbc | x0) & 7) == 0;
+#pragma unroll
+    for (int j = 0; j < PIECES; ++j) {
+        const int i = tid + 128 * j, s = i / (SC_P / 8), p = i % (SC_P / 8) * 8;
+        const bf16* src = (const bf16*)R.xbc + (size_t)(t0 + s) * R.ld_xbc + x0 + p;
+        if (s < n && vec && p + 8 <= pw) xr[j] = *(const uint4*)src;
+        else {
+            bf16 e8[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) e8[e] = s < n && p + e < pw ? src[e] : __float2bfloat16(0.f);
+            xr[j] = make_uint4(sc_pack(e8[0], e8[1]), sc_pack(e8[2], e8[3]), sc_pack(e8[4], e8[5]), sc_pack(e8[6], e8[7]));
+        }
+    }
     if (warp == 0) sc_cumsum(L, R, t0, n, h, A, la, dts, lane);
     __syncthreads();
     const float end = la[SC_T - 1];
-    for (int i = tid; i < SC_T * SC_P; i += 128) {
-        const int s = i / SC_P, p = i % SC_P;
-        float v = 0.f;
-        if (s < n && p < pw) v = ld_f((const bf16*)R.xbc + (size_t)(t0 + s) * R.ld_xbc + L.rx + h * L.P + p0 + p) * (dts[s] * expf(end - la[s]));
-        bf16 q[SC_TERMS];
-        sc_split(v, q);
 #pragma unroll
-        for (int k = 0; k < SC_TERMS; ++k) W[(k * SC_T + s) * SC_LDP + p] = q[k];
+    for (int j = 0; j < PIECES; ++j) {
+        const int i = tid + 128 * j, s = i / (SC_P / 8), p = i % (SC_P / 8) * 8;
+        const float f = s < n ? dts[s] * expf(end - la[s]) : 0.f;
+        const uint32_t w[4] = {xr[j].x, xr[j].y, xr[j].z, xr[j].w};
+        uint32_t o[SC_TERMS][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            bf16 q0[SC_TERMS], q1[SC_TERMS];
+            sc_split(__uint_as_float(w[e] << 16) * f, q0);
+            sc_split(__uint_as_float(w[e] & 0xffff0000u) * f, q1);
+#pragma unroll
+            for (int k = 0; k < SC_TERMS; ++k) o[k][e] = sc_pack(q0[k], q1[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < SC_TERMS; ++k) *(uint4*)(W + (k * SC_T + s) * SC_LDP + p) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
     }
     cp_async_wait<0>();
     __syncthreads();
@@ -165,15 +191,20 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const MixLayer L, 
 #pragma unroll
         for (int j = 0; j < SC_P / 8; ++j)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const int nn = mt * 16 + g + 8 * (e >> 1), p = 8 * j + 2 * t + (e & 1);
-                if (nn < L.N && p < pw) out[(size_t)nn * L.P + p] = acc[j][e];
+            for (int e = 0; e < 4; e += 2) {
+                const int nn = mt * 16 + g + 4 * e, p = 8 * j + 2 * t;
+                if (nn >= L.N || p >= pw) continue;
+                float* o = out + (size_t)nn * L.P + p;
+                if ((L.P & 1) == 0) *(float2*)o = make_float2(acc[j][e], acc[j][e + 1]);
+                else { o[0] = acc[j][e]; if (p + 1 < pw) o[1] = acc[j][e + 1]; }
             }
     }
     if (tid == 0 && blockIdx.z == 0) R.chunk_decay[c * L.heads + h] = end;
     // nothing of this launch reads the convolution history: carry it over here
     if (c == 0 && R.commit) conv_history_of<bf16>(L, R, R.rows[0].seq, 0, R.n_rows, h, p0, SC_P, tid, 128);
 }
+
+#define SC_AHEAD 4               // chunks whose states are requested at once
 
 // (2) the pass over the chunks: grid (ceil(N * Pp / 256), heads); leaves the state before every chunk as bf16 planes
 __global__ void __launch_bounds__(256) ssd_chunk_pass_kernel(const MixLayer L, const MixRun R, int chunks) {
@@ -190,15 +221,15 @@ __global__ void __launch_bounds__(256) ssd_chunk_pass_kernel(const MixLayer L, c
     const size_t cst = (size_t)L.heads * L.N * L.P;
     bf16* prev = (bf16*)R.chunk_prev + ((size_t)h * SC_TERMS * L.N + n) * Pp + p;
     const size_t pst = (size_t)L.heads * SC_TERMS * L.N * Pp;
-    for (int c0 = 0; c0 < chunks; c0 += 4) {
-        float v[4], d[4];
+    for (int c0 = 0; c0 < chunks; c0 += SC_AHEAD) {
+        float v[SC_AHEAD], d[SC_AHEAD];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < SC_AHEAD; ++u) {
             v[u] = (ok && c0 + u < chunks) ? cs[(c0 + u) * cst] : 0.f;
             d[u] = c0 + u < chunks ? R.chunk_decay[(c0 + u) * L.heads + h] : 0.f;
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < SC_AHEAD; ++u) {
             if (c0 + u >= chunks) break;
             bf16 q[SC_TERMS];
             sc_split(s, q);
@@ -232,15 +263,33 @@ __global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const MixLayer L, co
     sc_stage(R, t0, n, L.rx + h * L.P + p0, pw, SC_P, Xs, SC_LDP, tid, 128);
     {
         const bf16* src = (const bf16*)R.chunk_prev + ((size_t)c * L.heads + h) * SC_TERMS * L.N * Pp + p0;
-        const int ppr = SC_P / 8;
-        for (int i = tid; i < SC_TERMS * Np * ppr; i += 128) {
-            const int col = (i % ppr) * 8, nn = (i / ppr) % Np, q = i / (ppr * Np);
-            bf16* d = Sp + (q * Np + nn) * SC_LDP + col;
-            if (nn < L.N && col < pwp) cp_async16(d, src + ((size_t)q * L.N + nn) * Pp + col);
-            else *(uint4*)d = make_uint4(0u, 0u, 0u, 0u);
-        }
+        const int col = tid % (SC_P / 8) * 8;
+        for (int nn = tid / (SC_P / 8); nn < Np; nn += 128 / (SC_P / 8))
+#pragma unroll
+            for (int q = 0; q < SC_TERMS; ++q) {
+                bf16* d = Sp + (q * Np + nn) * SC_LDP + col;
+                if (nn < L.N && col < pwp) cp_async16(d, src + ((size_t)q * L.N + nn) * Pp + col);
+                else *(uint4*)d = make_uint4(0u, 0u, 0u, 0u);
+            }
         cp_async_commit();
     }
+    // The gates of this lane's outputs are requested here: read between the stores of the outputs, they were a trip to L2
+    // for each of 32 elements (1000 rows, 80 heads of 128 x 64: 124 -> 84 us, with staging free of divisions; bound by the instructions of eight
+    // warps an SM, a third of them the splits into three terms)
+    const int zc = L.off_z + h * L.P + p0;
+    const bool z2 = ((zc | R.ld_proj) & 1) == 0;
+    uint32_t zz[SC_P / 8][2];
+#pragma unroll
+    for (int j = 0; j < SC_P / 8; ++j)
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            const int r = warp * 16 + g + 8 * hf, p = 8 * j + 2 * t;
+            const bf16* z = (const bf16*)R.proj + (size_t)(t0 + r) * R.ld_proj + zc + p;
+            zz[j][hf] = 0u;
+            if (!gated || r >= n || p >= pw) continue;
+            if (z2 && p + 1 < pw) zz[j][hf] = *(const uint32_t*)z;
+            else zz[j][hf] = sc_pack(z[0], p + 1 < pw ? z[1] : __float2bfloat16(0.f));
+        }
     if (warp == 0) sc_cumsum(L, R, t0, n, h, A, la, dts, lane);
     cp_async_wait<0>();
     __syncthreads();
@@ -308,16 +357,19 @@ __global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const MixLayer L, co
             }
         }
     }
+    const bool u2 = ((R.ld_u | (h * L.P + p0)) & 1) == 0;
 #pragma unroll
     for (int j = 0; j < SC_P / 8; ++j)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int r = e >= 2 ? r_hi : r_lo, p = 8 * j + 2 * t + (e & 1);
-            if (r < n && p < pw) {
-                float u = o[j][e] + Dh * ld_f(Xs + r * SC_LDP + p);
-                if (gated) u *= silu_p(ld_f((const bf16*)R.proj + (size_t)(t0 + r) * R.ld_proj + L.off_z + h * L.P + p0 + p));
-                R.ubuf[(size_t)(t0 + r) * R.ld_u + h * L.P + p0 + p] = u;
-            }
+        for (int hf = 0; hf < 2; ++hf) {
+            const int r = hf ? r_hi : r_lo, p = 8 * j + 2 * t;
+            if (r >= n || p >= pw) continue;
+            const uint32_t xw = *(const uint32_t*)(Xs + r * SC_LDP + p);
+            float u0 = o[j][2 * hf] + Dh * __uint_as_float(xw << 16), u1 = o[j][2 * hf + 1] + Dh * __uint_as_float(xw & 0xffff0000u);
+            if (gated) { u0 *= silu_p(__uint_as_float(zz[j][hf] << 16)); u1 *= silu_p(__uint_as_float(zz[j][hf] & 0xffff0000u)); }
+            float* u = R.ubuf + (size_t)(t0 + r) * R.ld_u + h * L.P + p0 + p;
+            if (u2 && p + 1 < pw) *(float2*)u = make_float2(u0, u1);
+            else { u[0] = u0; if (p + 1 < pw) u[1] = u1; }
         }
 }
 

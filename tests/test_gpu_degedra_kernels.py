@@ -353,15 +353,27 @@ SHAPES = [dict(), dict(H=12, G=1, d=32, rot=32, heads=5, P=33, N=17, groups=1, n
 @pytest.mark.parametrize("dt", ["bf16", "f32"])
 @pytest.mark.parametrize("shape", range(len(SHAPES)))
 def test_prepare(dt, shape):
+    _check_prepare(dt, shape, [(1, 5, 4), (0, 0, 1), (2, 100, 7)])
+
+
+# tiles of eight rows: of one sequence from its history on, in the middle of it, with a remainder; two sequences in one
+@pytest.mark.parametrize("dt", ["bf16", "f32"])
+@pytest.mark.parametrize("shape", range(len(SHAPES)))
+@pytest.mark.parametrize("parts", [[(1, 5, 21)], [(2, 9, 8), (0, 0, 16)], [(0, 30, 9), (1, 2, 2), (2, 77, 14)]])
+def test_prepare_many_rows(dt, shape, parts):
+    _check_prepare(dt, shape, parts)
+
+
+def _check_prepare(dt, shape, parts):
     x = Mix(dt, **SHAPES[shape])
-    n = x.rows([(1, 5, 4), (0, 0, 1), (2, 100, 7)])
+    n = x.rows(parts)
     proj = _rnd(n, x.ld).to(x.T)
     hist = _rnd(3, x.taps - 1, x.C, seed=9).to(x.T)
     x.b["proj"][:n] = proj.cuda()
     x.hist.copy_(hist)
     x.op("mix_prepare")
     row = 0
-    for slot, p0, cnt in ((1, 5, 4), (0, 0, 1), (2, 100, 7)):
+    for slot, p0, cnt in parts:
         pr = proj[row:row + cnt]
         q, k, v = x.ref_qkv(pr, p0)
         got = x.b["qbuf"][row:row + cnt].reshape(cnt, x.H, x.dp)
