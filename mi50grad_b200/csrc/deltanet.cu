@@ -1607,19 +1607,23 @@ __device__ __forceinline__ void ab_mma(float (&d)[4], const uint32_t (&a)[4], ui
 // warps divide K in steps of 32; they meet in shared memory.  The order of k inside a product is free, so lane t of a row
 // quad takes 8 adjacent k of its rows (16 bytes) and these are its fragments of two mma.sync.  Measured: 8.4 us for 512 rows of
 // 5120 and 96 outputs (27 before), 4.8 us for 24 rows of 2048.
+// Few rows: there are fewer CTAs than SMs, and the 20 steps of a width of 5120, three on their way at a time, were most of
+// the time of a launch that nothing runs beside.  AB_SPLIT CTAs, a cluster, share K then, have all their steps (five) on
+// their way at once and add up through distributed shared memory: verification of 80 rows of 5120 (48 such launches) 11.51 -> 11.16 ms, decode
+// of 24 rows of 2048 2.88 -> 2.85 ms (12 launches).  What bounds it: one trip to memory, the exchange, and the launch.
 #define AB_TOK 16
 #define AB_OUT 32
 #define AB_WARPS 8
-#define AB_RING 4
+#define AB_SPLIT 4
 #define AB_ITEMS (2 + AB_OUT / 8)   // 16-byte pieces of a lane and step: two token rows, four output rows
+template <int RING, bool SPLIT>
 __global__ void __launch_bounds__(AB_WARPS * 32) ab_proj_kernel(const __half* __restrict__ x, int ldx, const __half* __restrict__ wa,
                                                                 const __half* __restrict__ wb, int nv, int H,
                                                                 __half* __restrict__ ab, int ld_ab, int rows) {
-    extern __shared__ uint4 ab_smem[];               // [AB_WARPS][AB_RING][AB_ITEMS][32 lanes]
+    extern __shared__ uint4 ab_smem[];               // [AB_WARPS][RING][AB_ITEMS][32 lanes]
     pdl_launch_dependents();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-    uint4* ring = ab_smem + warp * (AB_RING * AB_ITEMS * 32) + lane;
-    pdl_wait();
+    uint4* ring = ab_smem + warp * (RING * AB_ITEMS * 32) + lane;
     const int r0 = blockIdx.x * AB_TOK, o0 = blockIdx.y * AB_OUT;
     const __half* xr[2];
     const __half* wr[AB_OUT / 8];
@@ -1630,10 +1634,22 @@ __global__ void __launch_bounds__(AB_WARPS * 32) ab_proj_kernel(const __half* __
         const int o = min(o0 + 8 * n + g, 2 * nv - 1);
         wr[n] = (o < nv ? wa + (size_t)o * H : wb + (size_t)(o - nv) * H) + 8 * t;
     }
+    const int all = (H + AB_WARPS * 32 - 1) / (AB_WARPS * 32), per = SPLIT ? (all + AB_SPLIT - 1) / AB_SPLIT : all;
+    const int i0 = SPLIT ? (int)blockIdx.z * per : 0, steps = min(all, i0 + per);
+    if (SPLIT) {
+        // (into L2 only, where whatever wrote them is seen)
+        for (int i = i0; i < steps; ++i) {
+            const int k0 = (i * AB_WARPS + warp) * 32;
+            if (k0 + 8 * t < H)
+#pragma unroll
+                for (int n = 0; n < AB_OUT / 8; ++n) asm volatile("prefetch.global.L2 [%0];" :: "l"(wr[n] + k0));
+        }
+    }
+    pdl_wait();
     float acc[AB_OUT / 8][4];
 #pragma unroll
     for (int n = 0; n < AB_OUT / 8; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
-    // a lane copies what it reads back itself (cp.async), AB_RING - 1 steps ahead: no barrier
+    // a lane copies what it reads back itself (cp.async), RING - 1 steps ahead: no barrier
     auto issue = [&](int i, int slot) {
         const int k0 = (i * AB_WARPS + warp) * 32;
         uint4* d = ring + slot * AB_ITEMS * 32;
@@ -1647,17 +1663,16 @@ __global__ void __launch_bounds__(AB_WARPS * 32) ab_proj_kernel(const __half* __
             for (int q = 0; q < AB_ITEMS; ++q) d[q * 32] = make_uint4(0u, 0u, 0u, 0u);
         }
     };
-    const int steps = (H + AB_WARPS * 32 - 1) / (AB_WARPS * 32);
 #pragma unroll
-    for (int i = 0; i < AB_RING - 1; ++i) {
-        if (i < steps) issue(i, i);
+    for (int j = 0; j < RING - 1; ++j) {
+        if (i0 + j < steps) issue(i0 + j, j);
         cp_async_commit();
     }
-    for (int i = 0; i < steps; ++i) {
-        if (i + AB_RING - 1 < steps) issue(i + AB_RING - 1, (i + AB_RING - 1) % AB_RING);
+    for (int i = i0; i < steps; ++i) {
+        if (i + RING - 1 < steps) issue(i + RING - 1, (i - i0 + RING - 1) % RING);
         cp_async_commit();
-        cp_async_wait<AB_RING - 1>();
-        const uint4* v = ring + (i % AB_RING) * AB_ITEMS * 32;
+        cp_async_wait<RING - 1>();
+        const uint4* v = ring + ((i - i0) % RING) * AB_ITEMS * 32;
         const uint4 lo = v[0], hi = v[32];
         const uint32_t a0[4] = {lo.x, hi.x, lo.y, hi.y}, a1[4] = {lo.z, hi.z, lo.w, hi.w};
 #pragma unroll
@@ -1678,20 +1693,52 @@ __global__ void __launch_bounds__(AB_WARPS * 32) ab_proj_kernel(const __half* __
         *(float2*)&red[warp][g + 8][8 * n + 2 * t] = make_float2(acc[n][2], acc[n][3]);
     }
     __syncthreads();
+    float* part = (float*)(red + AB_WARPS);          // this CTA's share of the sums (SPLIT)
     for (int i = tid; i < AB_TOK * AB_OUT; i += AB_WARPS * 32) {
         const int r = i / AB_OUT, o = i % AB_OUT;
         float s = 0.f;
 #pragma unroll
         for (int w = 0; w < AB_WARPS; ++w) s += red[w][r][o];
+        if (SPLIT) { part[i] = s; continue; }
         if (r0 + r < rows && o0 + o < 2 * nv) ab[(size_t)(r0 + r) * ld_ab + o0 + o] = __float2half(s);
+    }
+    if (SPLIT) {
+        cg::cluster_group cl = cg::this_cluster();
+        cl.sync();
+        constexpr int EACH = AB_TOK * AB_OUT / AB_SPLIT;     // every CTA ends a share of the tile
+        if (tid < EACH) {
+            const int i = (int)blockIdx.z * EACH + tid, r = i / AB_OUT, o = i % AB_OUT;
+            float v[AB_SPLIT], s = 0.f;
+#pragma unroll
+            for (int z = 0; z < AB_SPLIT; ++z) v[z] = cl.map_shared_rank(part, z)[i];
+#pragma unroll
+            for (int z = 0; z < AB_SPLIT; ++z) s += v[z];
+            if (r0 + r < rows && o0 + o < 2 * nv) ab[(size_t)(r0 + r) * ld_ab + o0 + o] = __float2half(s);
+        }
+        cl.sync();                                   // (no CTA leaves while its sums are read)
     }
 }
 B2_API int b2_ab_proj(const void* x, int ldx, const void* wa, const void* wb, int nv, int H, void* ab, int ld_ab,
                       int rows, cudaStream_t s) {
     if (H % 8 || (ldx % 8)) return cudaErrorInvalidValue;
-    constexpr size_t smem = (size_t)AB_WARPS * AB_RING * AB_ITEMS * 32 * 16;
-    static SmemOptIn optin;
-    if (cudaError_t e = optin.ensure(ab_proj_kernel, smem)) return e;
-    return launch_pdl(ab_proj_kernel, dim3((rows + AB_TOK - 1) / AB_TOK, (2 * nv + AB_OUT - 1) / AB_OUT), dim3(AB_WARPS * 32), smem, s,
-                      (const __half*)x, ldx, (const __half*)wa, (const __half*)wb, nv, H, (__half*)ab, ld_ab, rows);
+    const dim3 tiles((rows + AB_TOK - 1) / AB_TOK, (2 * nv + AB_OUT - 1) / AB_OUT);
+    auto smem = [](int ring) { return (size_t)AB_WARPS * ring * AB_ITEMS * 32 * 16; };
+    static SmemOptIn optin[2];
+    // with at most 148 CTAs in all, and a step at least for each of them
+    if (tiles.x * tiles.y * AB_SPLIT <= 148 && (H + AB_WARPS * 32 - 1) / (AB_WARPS * 32) >= AB_SPLIT) {
+        auto kern = ab_proj_kernel<6, true>;
+        if (cudaError_t e = optin[0].ensure(kern, smem(6))) return e;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(tiles.x, tiles.y, AB_SPLIT); cfg.blockDim = dim3(AB_WARPS * 32); cfg.dynamicSmemBytes = smem(6); cfg.stream = s;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = 1; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = AB_SPLIT;
+        cfg.attrs = attr; cfg.numAttrs = 2;
+        return cudaLaunchKernelEx(&cfg, kern, (const __half*)x, ldx, (const __half*)wa, (const __half*)wb, nv, H, (__half*)ab, ld_ab, rows);
+    }
+    auto kern = ab_proj_kernel<4, false>;
+    if (cudaError_t e = optin[1].ensure(kern, smem(4))) return e;
+    return launch_pdl(kern, tiles, dim3(AB_WARPS * 32), smem(4), s, (const __half*)x, ldx, (const __half*)wa, (const __half*)wb, nv, H, (__half*)ab, ld_ab, rows);
 }

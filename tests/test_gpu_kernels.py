@@ -284,9 +284,11 @@ def test_decode_attn(K, hd, nq, nkv, splits):
         assert _rel(out[r].cpu().view(nq, hd), o[0]) < 3e-3, f"row {r}"
 
 
-@pytest.mark.parametrize("rows,nv,H", [(1, 1, 8), (16, 16, 256), (17, 17, 264), (80, 48, 5120), (33, 3, 2056)])
+@pytest.mark.parametrize("rows,nv,H", [(1, 1, 8), (16, 16, 256), (17, 17, 264), (80, 48, 5120), (33, 3, 2056), (1, 1, 776), (9, 16, 1024), (150, 32, 1288),
+                                       (192, 48, 4096), (193, 48, 4096), (24, 24, 8200), (592, 16, 2048), (593, 16, 2048)])
 def test_ab_proj_edges(K, rows, nv, H):
-    """Row and output tiles of 16 and 32, widths that end inside a step: fp32 sums rounded to fp16 once."""
+    """Row and output tiles of 16 and 32, widths that end inside a step, K shared by a cluster and not, with shares that
+    differ or are empty: fp32 sums rounded to fp16 once."""
     gen = torch.Generator().manual_seed(22)
     x, wa, wb = (torch.randn(n, H, generator=gen).half() for n in (rows, nv, nv))
     ab = K.ab_proj(x.to(_dev()), wa.to(_dev()), wb.to(_dev())).cpu()[:, :2 * nv]
