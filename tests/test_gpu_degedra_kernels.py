@@ -59,7 +59,8 @@ def test_gemv_dense(dt, N, K, rows, rpc, mma):
 
 @pytest.mark.parametrize("dt", ["bf16", "f32"])
 @pytest.mark.parametrize("mma", [False, True])
-@pytest.mark.parametrize("H,rows", [(90, 3), (256, 8), (5000, 1), (168, 2)])
+# one row: widths of one float4, with a ragged end, one float4 beyond what the threads hold at once, beyond what is staged at once
+@pytest.mark.parametrize("H,rows", [(90, 3), (256, 8), (5000, 1), (168, 2), (4, 1), (36, 1), (90, 1), (5124, 1), (33000, 1)])
 def test_gemv_dense_forms_the_residual_update(dt, H, rows, mma):
     from mi50grad_b200.ops import kernels as K_
     from mi50grad_b200.ops import lib as L
