@@ -44,12 +44,14 @@ def _up8(n: int) -> int:
 
 
 def gemv_outputs_per_cta(n: int, tensor_core: bool, pair: bool = False) -> int:
-    """Outputs per CTA of a decode projection with n outputs: as many as leave every SM about one and a half
-    CTAs (the tensor-core kernel takes at least 16, the other at least 8, a gate / up pair at least 16)."""
-    for r in (32, 16):
-        if n >= r * 222:
+    """Outputs per CTA of a decode projection with n outputs (the tensor-core kernel and a gate / up pair take at least 16, the
+    other at least 8): the fewest whose CTAs all find a place at once, two an SM, so that none starts behind another;
+    else 32.  One row, with 8 / 16 / 32 outputs: 4096 -> 2368 6.5 / 7.6 / 9.6 us, 4096 -> 4736 10.9 / 10.1 / 11.4, 17408 -> 5120 37.9 / 41.7 /
+    35.7 (320 CTAs with 16); eight rows of 17408 -> 5120 68.9 with 16, 62.7 with 32, of 12288 -> 4096 28.6 and 43.7."""
+    for r in (8, 16, 32):
+        if -(-n // r) <= 296 and not (r == 8 and (tensor_core or pair)):
             return r
-    return 16 if tensor_core or pair else 8
+    return 32
 
 
 class MixerLinear:

@@ -111,6 +111,9 @@ def test_gate_up_interleave():
     for n in (1, 7, 500, 5000, 50000, 200000):
         assert gemv_outputs_per_cta(n, True) in (16, 32, 64, 128)
         assert gemv_outputs_per_cta(n, False) in (8, 16, 32) and gemv_outputs_per_cta(n, False, True) in (16, 32)
+    # the fewest whose CTAs are resident at once, two on each of 148 SMs
+    for n, few in ((1, 8), (2368, 8), (2369, 16), (4736, 16), (4737, 32), (65536, 32)):
+        assert gemv_outputs_per_cta(n, False) == few and gemv_outputs_per_cta(n, True) == gemv_outputs_per_cta(n, False, True) == max(few, 16)
 
 
 @pytest.mark.parametrize("name", ["mixed", "odd_width"])
