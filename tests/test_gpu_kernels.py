@@ -455,6 +455,20 @@ def test_attn_rows_few_rows_per_sequence(K, hd, nq, nkv, sizes, splits):
         assert _rel(out[r].cpu().view(nq, hd), o[0]) < 4e-3, f"row {r}"
 
 
+@pytest.mark.parametrize("hd,splits", [(256, 2), (256, 4), (256, 5), (256, 9), (64, 5), (64, 8)])
+@pytest.mark.parametrize("gated", [True, False])
+def test_merge_of_cache_slices(K, hd, splits, gated):
+    """As many slices as are requested at once, one more, two rounds and one more, with gates and without, against one slice:
+    both round the output to fp16 once."""
+    gen = torch.Generator().manual_seed(17)
+    d, nq, nkv, ctx, n = _dev(), 4, 2, 600, 3
+    kc, vc = (torch.randn(n, 700, nkv, hd, generator=gen).half().to(d) for _ in range(2))
+    q = torch.randn(n, 2 * nq * hd, generator=gen).half().to(d)
+    rows, seq_rows = K.make_rows([(s, ctx, ctx, ctx - 250 * s, 1) for s in range(n)], d), torch.arange(n + 1, dtype=torch.int32, device=d)
+    one, many = (K.attn_rows(q, rows, seq_rows, kc, vc, nq, nkv, hd, gate_off=nq * hd if gated else -1, splits=s) for s in (1, splits))
+    assert _rel(many.cpu(), one.float().cpu()) < 1e-3
+
+
 @pytest.mark.parametrize("hd,nq,nkv,T,past", [(64, 4, 2, 40, 5), (64, 2, 1, 200, 0), (256, 6, 1, 130, 7),
                                               (256, 12, 2, 512, 0), (128, 4, 4, 300, 64)])
 def test_attn_prefill_tcgen05(K, hd, nq, nkv, T, past):
