@@ -41,10 +41,13 @@ static int launch_md_t(const MixLayer* l, const MixRun* r, cudaStream_t s) {
     return l->dp <= 64 ? launch_md_heads<T, 2>(l, r, s) : launch_md_heads<T, 4>(l, r, s);
 }
 
-// One row a sequence, plain windows, at most four query heads a key head of at most 128, states of at most 128.
+// One row a sequence, plain windows, at most four query heads a key head of at most 128, states of at most 128; and all CTAs
+// resident at once: beyond that the recurrence, which alone has three CTAs on an SM, is slowed more than a launch costs (seven
+// sequences of 64 heads, 960 CTAs: decode of 7 tokens 11.37 ms merged, 11.27 apart).
 B2_API int b2_mix_decode_takes(const MixLayer* l, const MixRun* r) {
     return attn_valid(l) && ssd_valid(l) && r->n_seqs >= 1 && r->n_rows == r->n_seqs && r->fuse_norm && r->splits >= 1 && r->splits <= WD_MAX_SPLITS &&
-           l->keep_first <= 0 && l->softcap <= 0.f && !l->sink && l->dv == l->d && l->vp == l->dp && l->H / l->G <= 4 && l->dp <= 128 && l->N <= 128;
+           l->keep_first <= 0 && l->softcap <= 0.f && !l->sink && l->dv == l->d && l->vp == l->dp && l->H / l->G <= 4 && l->dp <= 128 && l->N <= 128 &&
+           l->G * r->n_rows * window_decode_splits(l, r, 2 * 148) + l->heads * ((l->P + 31) / 32) * r->n_seqs <= 2 * 148;
 }
 B2_API int b2_mix_decode(const MixLayer* l, const MixRun* r, cudaStream_t s) {
     if (!b2_mix_decode_takes(l, r)) return cudaErrorInvalidValue;

@@ -537,6 +537,9 @@ def test_both_halves_of_a_mixer_in_one_launch(dt, shape, window, commit):
             assert torch.equal(a, b)
     x.rows([(1, 5, 3), (0, 0, 1)])
     assert not takes()
+    x.r.n_rows = x.r.n_seqs = 148                       # more CTAs than are resident at once
+    x.r.fuse_norm = 1
+    assert not takes()
 
 
 @pytest.mark.parametrize("op,n", [("ssd_step", 1), ("ssd_step", 5), ("ssd_chunk", 70)])
