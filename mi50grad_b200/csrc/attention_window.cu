@@ -203,8 +203,9 @@ __device__ __forceinline__ void mp_conv(const MixLayer& L, const MixRun& R, int 
         for (int i = 0; i < MP_MAX_ROWS; ++i) {
             if (i >= rows) break;
             float a0 = b0, a1 = b1;
+            // (with fewer taps the first places hold inputs that this row does not see: an infinity there times a weight of zero is NaN)
 #pragma unroll
-            for (int j = 0; j < MP_TAPS; ++j) { a0 = fmaf(w0[j], v[i + j].x, a0); a1 = fmaf(w1[j], v[i + j].y, a1); }
+            for (int j = 0; j < MP_TAPS; ++j) if (j >= lead) { a0 = fmaf(w0[j], v[i + j].x, a0); a1 = fmaf(w1[j], v[i + j].y, a1); }
             put(r0 + i, a0, a1);
         }
         return;

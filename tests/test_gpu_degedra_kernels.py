@@ -365,6 +365,22 @@ def test_prepare_many_rows(dt, shape, parts):
     _check_prepare(dt, shape, parts)
 
 
+@pytest.mark.parametrize("dt", ["bf16", "f32"])
+@pytest.mark.parametrize("taps", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_convolution_inputs_beyond_the_taps(dt, taps, bad):
+    """An infinity or NaN reaches the rows whose taps cover it and no other, also inside a tile of eight rows."""
+    x = Mix(dt, heads=2, P=20, N=24, groups=1, ngroups=1, taps=taps)
+    n, at = 43, 18
+    x.rows([(1, 5, n)])
+    proj = _rnd(n, x.ld).to(x.T)
+    proj[at, x.m.off_x:x.m.off_x + x.C] = bad
+    x.b["proj"][:n] = proj.cuda()
+    x.op("mix_prepare")
+    lost = [i for i in range(n) if not bool(x.b["xbc"][i, :x.C].isfinite().all())]
+    assert lost == list(range(at, at + taps))
+
+
 def _check_prepare(dt, shape, parts):
     x = Mix(dt, **SHAPES[shape])
     n = x.rows(parts)
