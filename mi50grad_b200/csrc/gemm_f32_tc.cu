@@ -15,7 +15,7 @@
 // is multiplied while the other is split.
 // Bound: the splitting (about 250 instructions a warp and block); the tensor pipe is busy less than half of the time.  200 rows,
 // 2048 -> 8736: 52 us (60 with weights that need all 24 bits), FMAs 245; 128 rows, 8192 -> 18944: 175 (226), FMAs 1132 us.
-// A result that is not finite is formed again by fp32 FMAs: infinities and numbers that no bf16 reaches come out as they do there.
+// A result that is not finite is formed again by fp32 FMAs (ft_again): infinities and numbers that no bf16 reaches come out as they do there.
 // Every mbarrier wait is bounded; on expiry a CTA records a status and forms its outputs by fp32 FMAs.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -51,6 +51,89 @@ __device__ __forceinline__ uint32_t ft_term(float& x, float& y) {
     x -= __uint_as_float(u << 16);
     y -= __uint_as_float(u & 0xffff0000u);
     return u;
+}
+// (of all worker warps; also a barrier among them)
+__device__ __forceinline__ bool ft_any_worker(bool mine) {
+    uint32_t any;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, 1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+                 : "=r"(any) : "r"((uint32_t)mine), "n"(FT_WARPS * 32) : "memory");
+    return any != 0;
+}
+__device__ __forceinline__ void ft_copy16(unsigned char* dst, const float* src, int bytes) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+// The results marked in `again` (bit c: acc[c], token t0 + c0 + c of output n) once more, as chains of fp32 FMAs over
+// k_lo .. k_hi - 1.  All worker warps take part: both operands pass through the shared memory that held their raw blocks, two blocks of
+// 64 k in turn, a row's 16-byte pieces permuted by its number (lanes read one piece of 32 rows without conflicts).  Bound: a few
+// results the staging, many the reads of x, which all lanes make alike.  128 rows, 6144 -> 2048: one row of NaN 306 us, all rows
+// 2.2 ms (a lane's chain straight from global memory: 1.0 and 93 ms; the product by FMAs, which needs no second pass, 309 us).
+__device__ __forceinline__ void ft_again(const GemmF32Params& p, unsigned char* buf, float* keep, volatile int* abort_flag, float (&acc)[32], uint32_t again, int n, int row,
+                                         int n0, int t0, int t_tile, int c0, int k_lo, int k_hi, int tid) {
+    if (*abort_flag) {                       // copies may still be on their way to shared memory
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+            if (!(again >> c & 1)) continue;
+            const float *xt = p.x + (size_t)(t0 + c0 + c) * p.ldx, *wn = p.w + (size_t)n * p.ldw;
+            float v = 0.f;
+#pragma unroll 1
+            for (int k = k_lo; k < k_hi; ++k) v = fmaf(xt[k], wn[k], v);
+            acc[c] = v;
+        }
+        return;
+    }
+    const uint32_t of_warp = __reduce_or_sync(0xffffffffu, again);
+    auto stage = [&](int b) {
+        for (int i = tid; i < (FT_BM + t_tile) * 16; i += FT_WARPS * 32) {
+            const int r = i >> 4, ch = i & 15, k = k_lo + b * FT_BK + 4 * ch, g = r < FT_BM ? n0 + r : t0 + r - FT_BM;
+            const int bytes = g < (r < FT_BM ? p.N : p.T) ? 4 * max(0, min(4, k_hi - k)) : 0;
+            const float* src = r < FT_BM ? p.w + (size_t)g * p.ldw + k : p.x + (size_t)g * p.ldx + k;
+            ft_copy16(buf + (b & 1) * FT_RAW + r * 256 + ((ch ^ (r & 7)) << 4), bytes ? src : p.w, bytes);
+        }
+        cp_async_commit();
+    };
+    auto fma4 = [](const float4& x, const float4& w, float v) { return fmaf(x.w, w.w, fmaf(x.z, w.z, fmaf(x.y, w.y, fmaf(x.x, w.x, v)))); };
+    const int blocks = (k_hi - k_lo + FT_BK - 1) / FT_BK;
+    constexpr int LD = FT_WARPS * 32;        // results and sums wait in shared memory, a column a thread
+#pragma unroll
+    for (int c = 0; c < 32; ++c) keep[c * LD] = (again >> c & 1) ? 0.f : acc[c];
+    stage(0);
+#pragma unroll 1
+    for (int b = 0; b < blocks; ++b) {
+        if (b + 1 < blocks) stage(b + 1); else cp_async_commit();
+        cp_async_wait<1>();
+        ft_any_worker(false);
+        const unsigned char* wr = buf + (b & 1) * FT_RAW + row * 256;
+        const unsigned char* xr = buf + (b & 1) * FT_RAW + (FT_BM + c0) * 256;      // (c0 is a multiple of 32)
+#pragma unroll 1
+        for (int h = 0; h < 32; h += 8) {
+            uint32_t m = of_warp >> h & 0xffu;
+            if (__popc(m) > 2) {             // most of the eight: all of them
+                float v[8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) v[c] = keep[(h + c) * LD];
+#pragma unroll 2
+                for (int ch = 0; ch < FT_BK / 4; ++ch) {
+                    const float4 w = *(const float4*)(wr + ((ch ^ (row & 7)) << 4));
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) v[c] = fma4(*(const float4*)(xr + (h + c) * 256 + ((ch ^ c) << 4)), w, v[c]);
+                }
+#pragma unroll
+                for (int c = 0; c < 8; ++c) if (again >> (h + c) & 1) keep[(h + c) * LD] = v[c];
+            } else
+                for (; m; m &= m - 1) {
+                    const int c = __ffs(m) - 1;
+                    float v = keep[(h + c) * LD];
+#pragma unroll 4
+                    for (int ch = 0; ch < FT_BK / 4; ++ch)
+                        v = fma4(*(const float4*)(xr + (h + c) * 256 + ((ch ^ c) << 4)), *(const float4*)(wr + ((ch ^ (row & 7)) << 4)), v);
+                    if (again >> (h + c) & 1) keep[(h + c) * LD] = v;
+                }
+        }
+        ft_any_worker(false);                // (the block is read before it is overwritten)
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int c = 0; c < 32; ++c) acc[c] = keep[c * LD];
 }
 __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc_kernel(const GemmF32Params p, const __grid_constant__ CUtensorMap wmap,
                                                                      const __grid_constant__ CUtensorMap xmap, const int t_tile, const int per_kb) {
@@ -197,33 +280,34 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
             }
         }
         // ---- epilogue: a lane has one output of 32 tokens
-        const int n = n0 + (warp & 3) * 32 + lane;
-        const size_t plane = (size_t)blockIdx.z * (size_t)p.plane_stride;
-        float* out = (float*)p.out;
-        const float* wn = p.w + (size_t)min(n, p.N - 1) * p.ldw;
+        const int n = n0 + (warp & 3) * 32 + lane, nt = min(32, min(t_tile, p.T - t0) - c0);      // (tokens of this warp; none if negative)
         pdl_wait();
-        const int k_lo = kb0 * FT_BK, k_hi = min(p.K, (kb0 + KB) * FT_BK);
+        uint32_t again = 0;                  // tokens whose result is not finite (or, if a wait expired, all)
+        if (n < p.N) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-            const int tt = t0 + c0 + c;
-            if (c0 + c >= t_tile || tt >= p.T) break;                // (uniform)
-            float v = acc[c];
-            if (!ok || (n < p.N && !isfinite(v))) {
-                const float* xt = p.x + (size_t)tt * p.ldx;
-                v = 0.f;
-#pragma unroll 1
-                for (int k = k_lo; k < k_hi; ++k) v = fmaf(xt[k], wn[k], v);
+            for (int c = 0; c < 32; ++c) if (c < nt && (!ok || !isfinite(acc[c]))) again |= 1u << c;
+        }
+        if (ft_any_worker(again != 0)) ft_again(p, sR, (float*)sB + tid, abort_flag, acc, again, n, (warp & 3) * 32 + lane, n0, t0, t_tile, c0, kb0 * FT_BK, min(p.K, (kb0 + KB) * FT_BK), tid);
+        const size_t plane = (size_t)blockIdx.z * (size_t)p.plane_stride;
+        if (p.mode == DG_GATE_PAIR) {
+            float* out = (float*)p.out + (size_t)(t0 + c0) * p.ldo + (n >> 4) * 8 + (n & 7);
+            const bool mine = !(lane & 8) && n + 8 < p.N;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) {
+                const float up = __shfl_down_sync(0xffffffffu, acc[c], 8);
+                if (mine && c < nt) out[(size_t)c * p.ldo] = (p.act == ACT_RELU ? fmaxf(acc[c], 0.f) : silu_p(acc[c])) * up;
             }
-            __syncwarp();
-            if (p.mode == DG_GATE_PAIR) {
-                const float up = __shfl_down_sync(0xffffffffu, v, 8);
-                if (!(lane & 8) && n + 8 < p.N)
-                    out[(size_t)tt * p.ldo + (n >> 4) * 8 + (n & 7)] = (p.act == ACT_RELU ? fmaxf(v, 0.f) : silu_p(v)) * up;
-            } else if (n < p.N) {
-                if (p.mode == DG_STORE_F32 && p.softcap > 0.f) v = p.softcap * tanhf(v / p.softcap);
-                else if (p.mode == DG_STORE && n < p.act_cols) v = silu_p(v);
-                out[(size_t)tt * p.ldo + n + plane] = v;
+        } else if (n < p.N) {
+            if (p.mode == DG_STORE_F32 && p.softcap > 0.f) {
+#pragma unroll
+                for (int c = 0; c < 32; ++c) acc[c] = p.softcap * tanhf(acc[c] / p.softcap);
+            } else if (p.mode == DG_STORE && n < p.act_cols) {
+#pragma unroll
+                for (int c = 0; c < 32; ++c) acc[c] = silu_p(acc[c]);
             }
+            float* out = (float*)p.out + (size_t)(t0 + c0) * p.ldo + n + plane;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) if (c < nt) out[(size_t)c * p.ldo] = acc[c];
         }
     } else if (warp == FT_WARPS + 1) {
         // ---- fp32 operands; the weights of the first two blocks need not wait for the kernel before this one

@@ -668,6 +668,49 @@ def test_gemm_f32_infinities_and_the_largest_numbers():
     assert bool(out[5].isfinite().all()) and float(out[6, 9]) == 2.0 * float(torch.tensor(-top / 4, dtype=torch.float32))
 
 
+@pytest.mark.parametrize("N,K,T_,planes", [(1, 4, 1, 0), (130, 100, 17, 0), (257, 64, 128, 0), (300, 1000, 129, 0), (96, 2050, 49, 4), (160, 132, 300, 0)])
+def test_gemm_f32_results_formed_again(N, K, T_, planes):
+    """Rows and columns with infinities, NaNs and numbers that no bf16 reaches among ordinary ones, at the edges of the tiles:
+    where the result is finite it is a chain of at most K fp32 FMAs, else the infinity or NaN of the exact sum."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    w, x = _rnd(N, K + -K % 4, std=1e-3).cuda()[:, :K], _rnd(T_, K + -K % 4, seed=1).cuda()[:, :K]
+    x[T_ // 2, K - 1], x[T_ - 1, 0] = 3.4e38, -3.4e38                  # finite results by way of a term that is infinite
+    x[T_ // 3, K // 2] = float("inf")
+    w[N // 2, K // 3] = float("nan")
+    w[N - 1, K - 1] = float("-inf")
+    ref = x.double() @ w.double().T
+    mag = x.double().abs() @ w.double().abs().T
+    out = torch.full((planes, T_, N) if planes else (T_, N), 7.0, device="cuda")
+    got = K_.gemm_f32(w, x, out, L.DG_STORE_F32)
+    got = got.sum(0) if planes else got
+    fin = ref.isfinite()
+    assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got[ref.isinf()].double(), ref[ref.isinf()])
+    assert bool(((got.double() - ref).abs()[fin] <= 2.0 ** -24 * (K + 4) * mag[fin]).all())
+
+
+def test_gemm_f32_of_nans_takes_a_products_time():
+    """Results that are not finite cost about one product by FMAs (a few times the tensor cores'), not a walk of every lane
+    over global memory (230 times)."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    w, x, out = _rnd(2048, 2048).cuda(), _rnd(128, 2048, seed=1).cuda(), torch.zeros(128, 2048, device="cuda")
+
+    def ms(x):
+        best = 1e9
+        for _ in range(6):
+            a, b = torch.cuda.Event(True), torch.cuda.Event(True)
+            a.record()
+            for _ in range(4):
+                K_.gemm_f32(w, x, out, L.DG_STORE_F32)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+    plain, nans = ms(x), ms(torch.full_like(x, float("nan")))
+    assert bool(out.isnan().all()) and nans < 15 * plain, (plain, nans)
+
+
 @pytest.mark.parametrize("dt", ["bf16", "f32"])
 @pytest.mark.parametrize("shape", range(len(SHAPES)))
 @pytest.mark.parametrize("n", [2, 4, 8, 9, 17])
