@@ -2,7 +2,9 @@
 //
 // An fp32 number is the sum of three bf16 numbers (8 + 8 + 8 bits): w = w0 + w1 + w2, x = x0 + x1 + x2.  Of the nine products
 // the six that are not below the last bit are formed by tcgen05.mma kind::f16, which multiplies bf16 exactly:
-// w0 x0 + (w0 x1 + w1 x0) + (w0 x2 + w1 x1 + w2 x0), the smallest first.  Where the 128 x 64 weights of a block are bf16 numbers
+// w0 x0 + (w0 x1 + w1 x0) + (w0 x2 + w1 x1 + w2 x0), the smallest first.  (bf16 has the exponents of fp32, so the third term of a
+// number below 2^-110 would lie among its subnormals or below them: both operands are split times 2^24, which loses nothing
+// and costs 1 % of the time (weights that need all 24 bits 3 %).  Numbers above 2^103 and sums above 2^79 become infinite by that and are formed again, see below.)  Where the 128 x 64 weights of a block are bf16 numbers
 // (a bf16 checkpoint run in 32 bits), w1 and w2 are zero, and their three products are left out.
 // The tensor core cuts its sums off where fp32 additions round, so it never sums more than one block of 64 k: every block starts
 // from zero in tensor memory, and the warps add the blocks' sums in registers.  Error against 64 bits (2-norms, 200 rows,
@@ -14,7 +16,7 @@
 // activations a lane into shared memory (B operand, 128-byte swizzle), then take in the block before.  Two stages here too: one
 // is multiplied while the other is split.
 // Bound: the splitting (about 250 instructions a warp and block); the tensor pipe is busy less than half of the time.  200 rows,
-// 2048 -> 8736: 52 us (60 with weights that need all 24 bits), FMAs 245; 128 rows, 8192 -> 18944: 175 (226), FMAs 1132 us.
+// 2048 -> 8736: 46 us (53 with weights that need all 24 bits), FMAs 245; 128 rows, 8192 -> 18944: 172 (232), FMAs 1132 us.
 // A result that is not finite is formed again by fp32 FMAs (ft_again): infinities and numbers that no bf16 reaches come out as they do there.
 // Every mbarrier wait is bounded; on expiry a CTA records a status and forms its outputs by fp32 FMAs.
 #include <cuda.h>
@@ -32,6 +34,7 @@
 #define FT_STAGE (3 * FT_PLANE)
 #define FT_RAW (2 * (FT_BM + FT_BT) * 128)    // fp32 operands of a block: two boxes of 32 k each
 #define FT_SMEM (1024 + 2 * FT_STAGE + 2 * FT_RAW)
+#define FT_SCALE 16777216.f                  // both operands are split times 2^24, the sums of a block taken in times 2^-48 (exact)
 
 __device__ __forceinline__ void ft_mma(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -43,6 +46,10 @@ __device__ __forceinline__ void ft_mma(uint32_t d, uint32_t a, uint64_t b, uint3
 __device__ __forceinline__ void ft_store(uint32_t a, const uint32_t (&r)[8]) {
     asm volatile("tcgen05.st.sync.aligned.16x128b.x4.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
                  :: "r"(a), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]) : "memory");
+}
+__device__ __forceinline__ uint32_t ft_scale2(uint32_t two) {
+    const __nv_bfloat162 b = __hmul2(*(const __nv_bfloat162*)&two, __float2bfloat162_rn(FT_SCALE));
+    return *(const uint32_t*)&b;
 }
 // the next bf16 term of two numbers, which are left with what it does not hold
 __device__ __forceinline__ uint32_t ft_term(float& x, float& y) {
@@ -220,8 +227,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const int e = 4 * (j >> 1) + (j & 1);
-                        r[e] = __byte_perm(__float_as_uint(a[j].x), __float_as_uint(a[j].y), 0x7632);
-                        r[e + 2] = __byte_perm(__float_as_uint(a[j].z), __float_as_uint(a[j].w), 0x7632);
+                        r[e] = ft_scale2(__byte_perm(__float_as_uint(a[j].x), __float_as_uint(a[j].y), 0x7632));
+                        r[e + 2] = ft_scale2(__byte_perm(__float_as_uint(a[j].z), __float_as_uint(a[j].w), 0x7632));
                     }
                     ft_store(t_st + (uint32_t)(s * 96), r);
                     if (!(s ? zeros[1] : zeros[0])) {
@@ -231,6 +238,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
                         ft_store(t_st + (uint32_t)(s * 96 + 64), r);
                     }
                 } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { a[j].x *= FT_SCALE; a[j].y *= FT_SCALE; a[j].z *= FT_SCALE; a[j].w *= FT_SCALE; }
 #pragma unroll
                     for (int i = 0; i < 3; ++i) {
 #pragma unroll
@@ -245,6 +254,8 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
                 if (s) zeros[1] = !rest; else zeros[0] = !rest;
                 if (rest && lane == 0) s_terms[s] = (uint32_t)(kb + 1);
                 if (has_x) {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) { x[q].x *= FT_SCALE; x[q].y *= FT_SCALE; x[q].z *= FT_SCALE; x[q].w *= FT_SCALE; }
 #pragma unroll
                     for (int i = 0; i < 3; ++i) {
                         uint4 lo, hi;
@@ -273,7 +284,7 @@ __global__ void __launch_bounds__(FT_THREADS, 1) gemm_f32_tc_kernel(const GemmF3
                         tc_ld16(t_ld + (uint32_t)((s ^ 1) * 128 + h * 16), r);
                         tc_wait_ld();
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) acc[h * 16 + c] += __uint_as_float(r[c]);
+                        for (int c = 0; c < 16; ++c) acc[h * 16 + c] = fmaf(__uint_as_float(r[c]), 1.f / (FT_SCALE * FT_SCALE), acc[h * 16 + c]);
                     }
                 }
                 tc_fence_before();

@@ -668,6 +668,27 @@ def test_gemm_f32_infinities_and_the_largest_numbers():
     assert bool(out[5].isfinite().all()) and float(out[6, 9]) == 2.0 * float(torch.tensor(-top / 4, dtype=torch.float32))
 
 
+@pytest.mark.parametrize("N,K,T_", [(130, 196, 17), (64, 1000, 129)])
+@pytest.mark.parametrize("ex,ew", [(-120, 90), (-149, 100), (90, -118), (100, -149), (-70, -62), (-90, 60), (-30, 90), (80, 20)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_gemm_f32_over_the_range_of_exponents(N, K, T_, ex, ew, bf16):
+    """Operands down to the smallest subnormal keep all their bits, and so do results: times a power of two the same bound
+    as test_gemm_f32_three_terms, or a chain of K FMAs where sums come near the largest numbers, and half a unit of the smallest
+    subnormal for each of K / 64 additions."""
+    from mi50grad_b200.ops import kernels as K_
+    from mi50grad_b200.ops import lib as L
+    grow = torch.randint(0, 8, (K,), generator=torch.Generator().manual_seed(7))
+    w, x = torch.ldexp(_rnd(N, K).double(), ew + grow).float().cuda(), torch.ldexp(_rnd(T_, K, seed=1).double(), ex + grow).float().cuda()
+    if bf16:
+        w = w.bfloat16().float()
+    ref, mag = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+    out = torch.full((T_, N), float("nan"), device="cuda")
+    K_.gemm_f32(w, x, out, L.DG_STORE_F32)
+    units = K / 64 + 2 + 8 if ex + ew < 60 else K
+    err = (out.double() - ref).abs()
+    assert bool((err <= 2.0 ** -24 * units * mag + 2.0 ** -150 * (K / 64 + 1)).all()), float((err / mag).max() * 2 ** 24)
+
+
 @pytest.mark.parametrize("N,K,T_,planes", [(1, 4, 1, 0), (130, 100, 17, 0), (257, 64, 128, 0), (300, 1000, 129, 0), (96, 2050, 49, 4), (160, 132, 300, 0)])
 def test_gemm_f32_results_formed_again(N, K, T_, planes):
     """Rows and columns with infinities, NaNs and numbers that no bf16 reaches among ordinary ones, at the edges of the tiles:
