@@ -357,10 +357,11 @@ def test_prepare(dt, shape):
     _check_prepare(dt, shape, [(1, 5, 4), (0, 0, 1), (2, 100, 7)])
 
 
-# tiles of eight rows: of one sequence from its history on, in the middle of it, with a remainder; two sequences in one
+# tiles of eight rows: of one sequence from its history on, in the middle of it, with a remainder; two sequences in one, also
+# between rows of the same third
 @pytest.mark.parametrize("dt", ["bf16", "f32"])
 @pytest.mark.parametrize("shape", range(len(SHAPES)))
-@pytest.mark.parametrize("parts", [[(1, 5, 21)], [(2, 9, 8), (0, 0, 16)], [(0, 30, 9), (1, 2, 2), (2, 77, 14)]])
+@pytest.mark.parametrize("parts", [[(1, 5, 21)], [(2, 9, 8), (0, 0, 16)], [(0, 30, 9), (1, 2, 2), (2, 77, 14)], [(0, 5, 3), (1, 9, 2), (0, 60, 4), (2, 3, 9)]])
 def test_prepare_many_rows(dt, shape, parts):
     _check_prepare(dt, shape, parts)
 
