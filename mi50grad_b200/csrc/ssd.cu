@@ -98,7 +98,7 @@ __device__ __forceinline__ void sc_cumsum(const MixLayer& L, const MixRun& R, in
 // rows [t0, t0 + n) x columns [c0, c0 + w) of xbc into smem [64][ld], zero-padded to wp columns (wp % 8 == 0)
 __device__ __forceinline__ void sc_stage(const MixRun& R, int t0, int n, int c0, int w, int wp, bf16* dst, int ld, int tid, int nthr) {
     const bf16* src = (const bf16*)R.xbc + c0;
-    const bool vec = ((R.ld_xbc | c0) & 7) == 0;
+    const bool vec = ((R.ld_xbc | c0) & 7) == 0 && ((uintptr_t)R.xbc & 15) == 0;
     const int ppr = wp >> 3, sh = ppr > 1 ? 32 - __clz(ppr - 1) : 0, c = (tid & ((1 << sh) - 1)) * 8;      // (no division for each piece)
     if (c < wp)
         for (int r = tid >> sh; r < SC_T; r += nthr >> sh) {
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const MixLayer L, 
     constexpr int PIECES = SC_T * (SC_P / 8) / 128;
     uint4 xr[PIECES];
     const int x0 = L.rx + h * L.P + p0;
-    const bool vec = ((R.ld_xbc | x0) & 7) == 0;
+    const bool vec = ((R.ld_xbc | x0) & 7) == 0 && ((uintptr_t)R.xbc & 15) == 0;
 #pragma unroll
     for (int j = 0; j < PIECES; ++j) {
         const int i = tid + 128 * j, s = i / (SC_P / 8), p = i % (SC_P / 8) * 8;
@@ -169,6 +169,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const MixLayer L, 
     const int g = lane >> 2, t = lane & 3;
     const int v_row = (lane & 7) + ((lane >> 3) & 1) * 8, v_col = (lane >> 4) * 8;
     float* out = R.chunk_state + ((size_t)c * L.heads + h) * L.N * L.P + p0;
+    const bool pairs = (L.P & 1) == 0 && ((uintptr_t)R.chunk_state & 7) == 0;
     for (int mt = warp; mt < Np / 16; mt += 4) {
         float acc[SC_P / 8][4];
 #pragma unroll
@@ -195,7 +196,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_state_kernel(const MixLayer L, 
                 const int nn = mt * 16 + g + 4 * e, p = 8 * j + 2 * t;
                 if (nn >= L.N || p >= pw) continue;
                 float* o = out + (size_t)nn * L.P + p;
-                if ((L.P & 1) == 0) *(float2*)o = make_float2(acc[j][e], acc[j][e + 1]);
+                if (pairs) *(float2*)o = make_float2(acc[j][e], acc[j][e + 1]);
                 else { o[0] = acc[j][e]; if (p + 1 < pw) o[1] = acc[j][e + 1]; }
             }
     }
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const MixLayer L, co
     // for each of 32 elements (1000 rows, 80 heads of 128 x 64: 124 -> 84 us, with staging free of divisions; bound by the instructions of eight
     // warps an SM, a third of them the splits into three terms)
     const int zc = L.off_z + h * L.P + p0;
-    const bool z2 = ((zc | R.ld_proj) & 1) == 0;
+    const bool z2 = ((zc | R.ld_proj) & 1) == 0 && ((uintptr_t)R.proj & 3) == 0;
     uint32_t zz[SC_P / 8][2];
 #pragma unroll
     for (int j = 0; j < SC_P / 8; ++j)
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(128) ssd_chunk_out_kernel(const MixLayer L, co
             }
         }
     }
-    const bool u2 = ((R.ld_u | (h * L.P + p0)) & 1) == 0;
+    const bool u2 = ((R.ld_u | (h * L.P + p0)) & 1) == 0 && ((uintptr_t)R.ubuf & 7) == 0;
 #pragma unroll
     for (int j = 0; j < SC_P / 8; ++j)
 #pragma unroll

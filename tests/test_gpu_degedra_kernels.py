@@ -604,6 +604,33 @@ def test_recurrence_chunked(shape, n):
     assert torch.equal(x.S[0].cpu(), S0[0]) and torch.equal(x.hist[1].cpu(), h0[1])
 
 
+@pytest.mark.parametrize("P,moved", [(21, ("proj",)), (21, ("ubuf",)), (21, ("xbc",)), (24, ("xbc",)), (22, ("ubuf", "chunk_state"))])
+def test_recurrence_chunked_off_the_wide_boundaries(P, moved):
+    """Buffers that begin one element behind a wide boundary, with sizes that do not ask for one: the same bits."""
+    x = Mix("bf16", H=3, G=1, d=10, rot=4, heads=3, P=P, N=24, groups=1, ngroups=1, taps=2)
+    n = 130
+    x.r.ld_u = 3 * P + P % 2
+    x.b["ubuf"] = torch.zeros(n, x.r.ld_u, device="cuda")
+    x.r.ubuf = x.b["ubuf"].data_ptr()
+    x.rows([(0, 0, n)])
+    x.r.fuse_norm = 0
+    x.b["proj"][:n] = _rnd(n, x.ld).to(x.T).cuda()
+    x.op("mix_prepare")
+    got, names = [], ("ubuf", "out")
+    for move in (False, True):
+        if move:
+            for name in moved:
+                t = x.b[name]
+                flat = torch.zeros(t.numel() + 1, dtype=t.dtype, device="cuda")
+                flat[1:].copy_(t.flatten())
+                x.b[name] = flat[1:].view(t.shape)
+                setattr(x.r, name, x.b[name].data_ptr())
+        x.S.zero_()
+        x.op("ssd_chunk")
+        got.append([x.b[k][:n].clone() for k in names] + [x.S.clone()])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
 def test_recurrence_keeps_a_distant_token():
     """Decay close to one: a single large input must still be in the output hundreds of tokens and several
     chunks later."""
