@@ -256,6 +256,12 @@ template <> struct DgVec<float> {
     }
 };
 
+// (by way of the L1: the other CTAs of an SM read the same activations.  One row of 17408 -> 5120 36.1 -> 35.2 us, two rows of
+// 4096 -> 6144 15.5 -> 15.2)
+__device__ __forceinline__ void dg_copy16(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" :: "r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
 template <typename T, int MR, bool EXT>
 __global__ void __launch_bounds__(DG_THREADS, 2) gemv_fma_kernel(const DenseGemvParams p, int KC) {
     constexpr int V = DgVec<T>::V;
@@ -296,12 +302,29 @@ __global__ void __launch_bounds__(DG_THREADS, 2) gemv_fma_kernel(const DenseGemv
         // ---- stage the input of this K chunk.  All its loads are on their way at once, those of the residual stream also while
         // the inverses are formed: a loop of load and store took a trip to L2 for each of up to six pieces, in every CTA
         // (one row: 12288 -> 4096 19.8 -> 18.7 us, 17408 -> 5120 43.7 -> 40.9; a step of decode at width 4096 1.126 -> 1.099 ms)
-        if (p.x && (p.ldx & 7) == 0) {
+        if (MR == 1 && p.x && (p.ldx & 7) == 0 && cl <= 2 * DG_THREADS * V) {
+            // (two pieces a thread at most: through registers, which is the shorter way: one row of 2048 -> 2048 4.42 us by cp.async,
+            // 4.07 so; 2048 -> 12288 13.7 and 13.1, 4096 -> 12288 22.7 and 21.8)
+            uint4 v[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int kk = (tid + u * DG_THREADS) * V, kg = c0 + kk;
+                if (kk < cl && kg + V <= p.K) v[u] = *(const uint4*)((const T*)p.x + kg);
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int kk = (tid + u * DG_THREADS) * V, kg = c0 + kk;
+                if (kk >= cl) break;
+                if (kg + V <= p.K) *(uint4*)(xs + kk) = v[u];
+                else
+                    for (int e = 0; e < V; ++e) xs[kk + e] = kg + e < p.K ? ((const T*)p.x)[kg + e] : to_t<T>(0.f);
+            }
+        } else if (p.x && (p.ldx & 7) == 0) {
             for (int i = tid * V; i < p.rows * KC; i += DG_THREADS * V) {
                 const int m = MR == 1 ? 0 : i / KC, kk = i - m * KC, kg = c0 + kk;
                 if (kk >= cl) continue;
                 const T* src = (const T*)p.x + (size_t)m * p.ldx + kg;
-                if (kg + V <= p.K) cp_async16(xs + i, src);
+                if (kg + V <= p.K) dg_copy16(xs + i, src);
                 else
                     for (int e = 0; e < V; ++e) xs[i + e] = kg + e < p.K ? src[e] : to_t<T>(0.f);
             }

@@ -34,7 +34,9 @@ def _lin(w, dtype, rpc):
 @pytest.mark.parametrize("dt", ["bf16", "f32"])
 @pytest.mark.parametrize("mma", [False, True])
 @pytest.mark.parametrize("N,K,rows,rpc", [(37, 90, 1, 8), (333, 5000, 2, 128), (64, 200, 3, 16), (301, 2056, 8, 32), (1000, 5000, 2, 8),
-                                          (40, 17000, 8, 16), (129, 4096, 5, 32), (700, 1500, 7, 64)])
+                                          (40, 17000, 8, 16), (129, 4096, 5, 32), (700, 1500, 7, 64),
+                                          # one row: one and two pieces a thread (fp32: of half as many numbers), and one number more
+                                          (33, 1024, 1, 8), (33, 2048, 1, 8), (33, 2049, 1, 16), (33, 4096, 1, 8), (33, 4097, 1, 16)])
 def test_gemv_dense(dt, N, K, rows, rpc, mma):
     from mi50grad_b200.ops import kernels as K_
     from mi50grad_b200.ops import lib as L
