@@ -124,62 +124,94 @@ __device__ __forceinline__ void ssd_step_cta(const MixLayer& L, const MixRun& R,
     const float A = rec_rate(L, h), Dh = L.D ? L.D[h] : 0.f, a_const = L.decay ? L.decay[h] : 0.f;
     const bool gated = L.gate == REC_GATE_SILU_NORM;
     pdl_wait();
-    float nb[LD], nc[LD], nx[U], ndt[U], nz = 0.f;            // the next turn's
-    auto load = [&](int r) {
-#pragma unroll
-        for (int i = 0; i < LD; ++i) {
-            const int e = tid + i * SS_THREADS, u = e / NN, n = e % NN;
-            const T* xbc = (const T*)R.xbc + (size_t)(r + u) * R.ld_xbc + grp * L.N + n;
-            const bool in = e < U * NN && r + u < r1 && n < L.N;
-            nb[i] = in ? ld_f(xbc + L.rB) : 0.f;
-            nc[i] = in ? ld_f(xbc + L.rC) : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const bool in = r + u < r1;
-            nx[u] = in && pv ? ld_f((const T*)R.xbc + (size_t)(r + u) * R.ld_xbc + L.rx + h * L.P + p) : 0.f;
-            ndt[u] = in ? rec_dt(L, R, r + u, h) : 0.f;
-        }
-        // (the token that this warp sums)
-        nz = (gated && warp < U && r + warp < r1 && pv) ? ld_f((const T*)R.proj + (size_t)(r + warp) * R.ld_proj + L.off_z + h * L.P + p) : 0.f;
-    };
-    auto put = [&]() {
-#pragma unroll
-        for (int i = 0; i < LD; ++i) {
-            const int e = tid + i * SS_THREADS;
-            if (e < U * NN) { Bs[e] = nb[i]; Cs[e] = nc[i]; }
-        }
-    };
-    load(r0);
-    for (int r = r0; r < r1; r += U) {
-        put();
-        float x[U], dt[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) { x[u] = nx[u]; dt[u] = ndt[u]; }
-        const float z = nz;
-        __syncthreads();
-        if (r + U < r1) load(r + U);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            if (r + u >= r1) break;
-            const float a = L.decay ? a_const : expf(A * dt[u]), dx = dt[u] * x[u];
+    if constexpr (U == 1) {
+        // one token at a time, as in decode: nothing to overlap, and a turn's detour through registers costs 1 to 5 % (one sequence of
+        // 64 heads 8.26 us, by a turn of one 8.48; six 13.9 and 14.5)
+        for (int r = r0; r < r1; ++r) {
+            const T* xbc = (const T*)R.xbc + (size_t)r * R.ld_xbc;
+            for (int n = tid; n < NN; n += SS_THREADS) {
+                Bs[n] = n < L.N ? ld_f(xbc + L.rB + grp * L.N + n) : 0.f;
+                Cs[n] = n < L.N ? ld_f(xbc + L.rC + grp * L.N + n) : 0.f;
+            }
+            const float x = pv ? ld_f(xbc + L.rx + h * L.P + p) : 0.f;
+            const float dt = rec_dt(L, R, r, h);
+            const float z = (gated && warp == 0 && pv) ? ld_f((const T*)R.proj + (size_t)r * R.ld_proj + L.off_z + h * L.P + p) : 0.f;
+            const float a = L.decay ? a_const : expf(A * dt), dx = dt * x;
+            __syncthreads();
             float y = 0.f;
 #pragma unroll
             for (int i = 0; i < NB; ++i) {
-                const int n = u * NN + warp + SS_WARPS * i;
+                const int n = warp + SS_WARPS * i;
                 st[i] = fmaf(a, st[i], Bs[n] * dx);
                 y = fmaf(st[i], Cs[n], y);
             }
-            part[u][warp][lane] = y;
+            part[0][warp][lane] = y;
+            __syncthreads();
+            if (warp == 0 && pv) {
+                float s = 0.f;
+#pragma unroll
+                for (int w = 0; w < SS_WARPS; ++w) s += part[0][w][lane];
+                R.ubuf[(size_t)r * R.ld_u + h * L.P + p] = (s + Dh * x) * (gated ? silu_p(z) : 1.f);
+            }
         }
-        __syncthreads();
-        if (warp < U && r + warp < r1 && pv) {
-            float s = 0.f, xs = x[0];
+    } else {
+        float nb[LD], nc[LD], nx[U], ndt[U], nz = 0.f;            // the next turn's
+        auto load = [&](int r) {
 #pragma unroll
-            for (int u = 1; u < U; ++u) if (warp == u) xs = x[u];
+            for (int i = 0; i < LD; ++i) {
+                const int e = tid + i * SS_THREADS, u = e / NN, n = e % NN;
+                const T* xbc = (const T*)R.xbc + (size_t)(r + u) * R.ld_xbc + grp * L.N + n;
+                const bool in = e < U * NN && r + u < r1 && n < L.N;
+                nb[i] = in ? ld_f(xbc + L.rB) : 0.f;
+                nc[i] = in ? ld_f(xbc + L.rC) : 0.f;
+            }
 #pragma unroll
-            for (int w = 0; w < SS_WARPS; ++w) s += part[warp][w][lane];
-            R.ubuf[(size_t)(r + warp) * R.ld_u + h * L.P + p] = (s + Dh * xs) * (gated ? silu_p(z) : 1.f);
+            for (int u = 0; u < U; ++u) {
+                const bool in = r + u < r1;
+                nx[u] = in && pv ? ld_f((const T*)R.xbc + (size_t)(r + u) * R.ld_xbc + L.rx + h * L.P + p) : 0.f;
+                ndt[u] = in ? rec_dt(L, R, r + u, h) : 0.f;
+            }
+            // (the token that this warp sums)
+            nz = (gated && warp < U && r + warp < r1 && pv) ? ld_f((const T*)R.proj + (size_t)(r + warp) * R.ld_proj + L.off_z + h * L.P + p) : 0.f;
+        };
+        auto put = [&]() {
+#pragma unroll
+            for (int i = 0; i < LD; ++i) {
+                const int e = tid + i * SS_THREADS;
+                if (e < U * NN) { Bs[e] = nb[i]; Cs[e] = nc[i]; }
+            }
+        };
+        load(r0);
+        for (int r = r0; r < r1; r += U) {
+            put();
+            float x[U], dt[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) { x[u] = nx[u]; dt[u] = ndt[u]; }
+            const float z = nz;
+            __syncthreads();
+            if (r + U < r1) load(r + U);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (r + u >= r1) break;
+                const float a = L.decay ? a_const : expf(A * dt[u]), dx = dt[u] * x[u];
+                float y = 0.f;
+#pragma unroll
+                for (int i = 0; i < NB; ++i) {
+                    const int n = u * NN + warp + SS_WARPS * i;
+                    st[i] = fmaf(a, st[i], Bs[n] * dx);
+                    y = fmaf(st[i], Cs[n], y);
+                }
+                part[u][warp][lane] = y;
+            }
+            __syncthreads();
+            if (warp < U && r + warp < r1 && pv) {
+                float s = 0.f, xs = x[0];
+#pragma unroll
+                for (int u = 1; u < U; ++u) if (warp == u) xs = x[u];
+#pragma unroll
+                for (int w = 0; w < SS_WARPS; ++w) s += part[warp][w][lane];
+                R.ubuf[(size_t)(r + warp) * R.ld_u + h * L.P + p] = (s + Dh * xs) * (gated ? silu_p(z) : 1.f);
+            }
         }
     }
     if (R.commit) {
