@@ -890,11 +890,13 @@ B2_API int b2_gemv_int4(const GemvInt4Params* p, cudaStream_t stream) {
     return cudaLaunchKernelEx(&cfg, kern, q);
 }
 
-// Launch shape for `rows` rows of an fp16 matrix cut for (k_splits, kslice): with five rows and more, slices of 2560 at most.  The
-// activations of longer ones take so much shared memory that the L1 holds too few loads in flight (5 rows of 5120 -> 65536:
-// 161 us whole, 131 in two slices).
+// Launch shape for `rows` rows of an fp16 matrix cut for (k_splits, kslice): with five rows and more, slices of 4096 and longer become
+// slices of 2560.  The activations of long ones take so much shared memory that the L1 holds too few loads in flight (5 rows of
+// 5120 -> 65536: 161 us whole, 131 in two slices).  Shorter ones lose more by the merge of the slices (8 rows of 2816 -> 65536: 66 us whole,
+// 77 cut, of 3840 87 and 96).  A short last slice is no loss: its CTAs fill the last wave (8 rows of 4096 -> 20480: 2560 + 1536 48 us,
+// 2048 + 2048 54; of 4096 -> 65536 114 and 112).
 B2_API void b2_gemv_f16_shape(int K, int rows, int* k_splits, int* kslice) {
-    if (rows <= 4 || *kslice <= 2560) return;
+    if (rows <= 4 || *kslice < 4096) return;
     *kslice = 2560;
     *k_splits = (K + 2559) / 2560;
 }
@@ -908,9 +910,10 @@ static int launch_f16(const GemvF16Params* p, cudaStream_t stream) {
         if (e != cudaSuccess) return e;
     }
     dim3 grid((p->N + GEMV_TILE_N - 1) / GEMV_TILE_N, p->k_splits);
-    // A plain launch: with the programmatic-serialisation attribute this kernel (nothing to do before its
+    // A plain launch: with the programmatic-serialisation attribute the kernel of one row (nothing to do before its
     // dependency wait, 40-170 MB to stream after it) measured 10 % slower in the decode step (fp16 attention
-    // weights: 149.1 against 167.1 tok/s).
+    // weights: 149.1 against 167.1 tok/s).  With more rows, where the first weights are requested in front of the activations, it was
+    // not measured.
     gemv_f16_kernel<MR><<<grid, GEMV_THREADS, smem, stream>>>(*p);
     return cudaGetLastError();
 }

@@ -750,7 +750,7 @@ def test_gemv_int4_rows_share_one_list(rows, K, N, lazy):
 @pytest.mark.parametrize("rows", [4, 5, 8])
 @pytest.mark.parametrize("K,N", [(2816, 300), (5120, 19000)])
 def test_gemv_f16_slices_of_many_rows(rows, K, N):
-    """From five rows on a slice of K has 2560 at most; bound: fp32 sums of fp16 products, and the fp16 result."""
+    """From five rows on a whole K of 5120 is cut into two slices; bound: fp32 sums of fp16 products, and the fp16 result."""
     from mi50grad_b200.engine.engine import DeviceLinear
     from mi50grad_b200.ops import kernels as K_
     dev = torch.device("cuda", 0)

@@ -63,3 +63,28 @@ def test_prompt_rows_and_their_memory():
     assert 0.65e9 < work < 0.75e9 and work == 8 * prompt_work_bytes(cfg, 512)
     assert memory_budget(cfg, 4096)["scratch_gb"] >= work / 1e9
 
+
+
+def test_fp16_gemv_slices_of_many_rows():
+    """Five rows and more: slices of 4096 and longer become slices of 2560, none empty; up to four rows, and where slices are
+    shorter, as the matrix was cut."""
+    import ctypes as C
+    from mi50grad_b200.ops import lib as L
+    lib = L.lib()
+
+    def shape(K, rows, ks, kslice):
+        a, b = C.c_int(ks), C.c_int(kslice)
+        lib.b2_gemv_f16_shape(K, rows, C.byref(a), C.byref(b))
+        return a.value, b.value
+
+    for K in list(range(256, 20000, 37)) + [2816, 3840, 4096, 5120, 8192, 17408, 65536]:
+        cut = min(8192, -(-K // 256) * 256)
+        given = (-(-K // cut), cut)
+        assert shape(K, 4, *given) == given and shape(K, 8, -(-K // 3840), 3840) == (-(-K // 3840), 3840)
+        for rows in (5, 8):
+            ks, kslice = shape(K, rows, *given)
+            assert (ks - 1) * kslice < K <= ks * kslice
+            if cut < 4096:
+                assert (ks, kslice) == given
+            else:
+                assert kslice == 2560
