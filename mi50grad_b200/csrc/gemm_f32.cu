@@ -1,7 +1,6 @@
-// Many-row projection in true fp32 (no reduced-precision matrix mode): out[t][n] = sum_k x[t][k] w[n][k].
-// It serves models that run entirely in 32 bits.  Operands whose rows start on 16-byte boundaries, as an engine's do, go to the
-// tensor cores in three bf16 terms each (csrc/gemm_f32_tc.cu); this file has the plan of the splits over K for both, and the
-// kernel for all other operands:
+// Many-row projection in fp32: out[t][n] = sum_k x[t][k] w[n][k].  It serves models that run entirely in 32 bits.  Operands
+// whose rows start on 16-byte boundaries, as an engine's do, go to the tensor cores in three bf16 terms each (csrc/gemm_f32_tc.cu);
+// this file has the plan of the splits over K for both, and the kernel of fp32 FMAs for all other operands and for a short K:
 //
 // Bound: the FMA pipes (74 TFLOP/s).  A CTA of 128 threads owns [8 RT tokens x 128 outputs], a thread RT x 8 of them.
 // Both operands are contiguous in k, so they go from global memory into shared memory as they are (cp.async, four
@@ -10,7 +9,7 @@
 // output is the sum of its even-k and its odd-k chain.
 // Operands reach the registers at 32 floats a clock and an 8 x 8 thread tile asks for a quarter of a float per FMA, so
 // shared memory and the FMA pipes are about equally busy.  Measured in a prompt of 200 rows (12 layers of width 2048):
-// 30 TFLOP/s, the whole prompt 14.5 ms; on the tensor cores 6.4 ms.
+// 30 TFLOP/s, the whole prompt 14.5 ms; on the tensor cores 4.8 ms.
 #include "gemm_f32.cuh"
 
 #define GF_BN 128
@@ -144,7 +143,11 @@ B2_API int b2_gemm_f32(const GemmF32Params* p, cudaStream_t s) {
     if (p->mode == DG_GATE_PAIR && (p->N & 15)) return cudaErrorInvalidValue;
     const bool planes = p->mode == DG_STORE_F32 && p->softcap <= 0.f && p->plane_stride > 0;
     const int ks = b2_gemm_f32_splits(p->N, p->K, p->T, planes && p->max_splits > 1 ? p->max_splits : 1);
-    if (!((p->ldx | p->ldw) & 3) && !(((uintptr_t)p->x | (uintptr_t)p->w) & 15)) return gemm_f32_tc_launch(p, tc_tile_f32(p->T), ks, s);
+    // A short K is over before the tensor-core CTA is set up: with one FMA CTA an SM at most, K = 32 3.9 to 5.5 us against 4.8 to 7.7 (9 to 500
+    // rows), K = 64 and 128 rows of 512 outputs 6.2 against 7.5; but K = 64, 33 rows 6.2 and 6.1, 128 rows of 2048 outputs 8.4 and 7.7
+    const long long fma_ctas = (long long)((p->N + GF_BN - 1) / GF_BN) * ((p->T + 15) / 16);
+    const bool brief = (p->K <= 32 && fma_ctas <= 148) || (p->K <= 64 && p->T > 64 && fma_ctas <= 64);
+    if (!brief && !((p->ldx | p->ldw) & 3) && !(((uintptr_t)p->x | (uintptr_t)p->w) & 15)) return gemm_f32_tc_launch(p, tc_tile_f32(p->T), ks, s);
     // Tokens of an FMA CTA (8 rt): us a 16-k block with n CTAs on an SM, about 0.5 + s n, s = .38, .54, .62, .73, .85, 1.02 for
     // rt = 2, 4, 5, 6, 7, 8 (one CTA alone does not cover its own latencies)
     static const double slope[9] = {0, 0, 0.38, 0, 0.54, 0.62, 0.73, 0.85, 1.02};

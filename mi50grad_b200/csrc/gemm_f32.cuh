@@ -2,5 +2,5 @@
 #pragma once
 #include "mixers.cuh"
 
-// rows of both operands on 16-byte boundaries; t_tile a multiple of 16 up to 128; splits as plan_f32 counts them
+// rows of both operands on 16-byte boundaries; t_tile a multiple of 16 up to 128; splits as b2_gemm_f32_splits counts them
 int gemm_f32_tc_launch(const GemmF32Params* p, int t_tile, int splits, cudaStream_t s);

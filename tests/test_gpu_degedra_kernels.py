@@ -112,10 +112,15 @@ def test_gate_up_pair(dt, F, K, rows):
 
 
 @pytest.mark.parametrize("N,K,T_,pad", [(1, 1, 1, 0), (130, 15, 17, 3), (128, 16, 33, 4), (257, 50, 41, 4), (2048, 1000, 200, 0), (96, 6144, 49, 8),
-                                        (4500, 66, 57, 2), (12288, 36, 65, 4), (16, 2049, 300, 1)])
+                                        (4500, 66, 57, 2), (12288, 36, 65, 4), (16, 2049, 300, 1),
+                                        # by FMAs, 16 to 64 tokens a CTA: the heights whose CTAs just fit the SMs
+                                        (256, 201, 1184, 0), (256, 201, 2368, 0), (256, 201, 2960, 0), (256, 201, 3552, 0), (256, 201, 4144, 0), (256, 201, 4736, 0),
+                                        (300, 1031, 1500, 0),
+                                        # on 16-byte boundaries: by FMAs (a short K) and on the tensor cores
+                                        (100, 32, 500, 4), (300, 64, 90, 0), (300, 64, 900, 0), (300, 68, 90, 0), (130, 33, 40, 3)])
 def test_gemm_f32_tiles_and_splits(N, K, T_, pad):
-    """Every tile height, ragged edges, rows that allow 16-byte copies and rows that do not, splits over K.  Two fp32
-    chains of at most K terms: the error stays below sqrt(K) roundings of terms of size K ** -0.5."""
+    """Rows off the 16-byte boundary and a short K (every tile height of the FMA kernel) and the tensor-core kernel, ragged
+    edges, splits over K.  Two fp32 chains of at most K terms: the error stays below sqrt(K) roundings of terms of size K ** -0.5."""
     from mi50grad_b200.ops import kernels as K_
     from mi50grad_b200.ops import lib as L
     w, x = _rnd(N, K + pad, std=K ** -0.5).cuda()[:, :K], _rnd(T_, K + pad, seed=1).cuda()[:, :K]
