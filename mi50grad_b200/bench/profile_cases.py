@@ -70,20 +70,19 @@ def case_gemv(which: str, timed: bool):
 def case_gemm(which: str, timed: bool):
     dev = torch.device("cuda")
     if which == "gemm_int4":
-        # (K, N, T, tokens per CTA, 128-output halves per CTA, CTA pairs)
-        shapes = [(17408, 5120, 512, 176, 1, 0), (5120, 34816, 512, 512, 1, 0), (5120, 34816, 80, 80, 1, 0),
-                  (5120, 34816, 512, 512, 1, 1)]
+        # (K, N, T, tokens per CTA, 128-output halves per CTA, splits over K): a CTA takes at most 256 tokens, of 256 outputs 192
+        shapes = [(17408, 5120, 512, 176, 2, 2), (5120, 34816, 512, 256, 1, 1), (5120, 34816, 80, 80, 2, 1)]
         if timed:
-            shapes += [(5120, 34816, 512, 256, 1, 1), (5120, 34816, 512, 256, 2, 0),
-                       (5120, 16384, 512, 512, 1, 0), (5120, 16384, 512, 512, 1, 1), (5120, 16384, 512, 256, 1, 1),
-                       (5120, 16384, 512, 256, 2, 0), (17408, 5120, 512, 512, 1, 1), (5120, 34816, 80, 80, 2, 0)]
-        for Kd, N, T, tt, mh, pair in shapes:
+            shapes += [(5120, 34816, 512, 176, 2, 1), (5120, 34816, 80, 80, 1, 1), (5120, 16384, 512, 256, 1, 1), (5120, 16384, 512, 176, 2, 1),
+                       (17408, 5120, 512, 256, 1, 3), (17408, 5120, 80, 80, 2, 7), (17408, 5120, 80, 80, 1, 3)]
+        for Kd, N, T, tt, mh, ks in shapes:
             pk = random_packed_int4(Kd, N, 128, dev)
             x = torch.randn(T, Kd, device=dev).half()
             out = torch.zeros(T, pk.n_pad, dtype=torch.float32, device=dev)
-            run = lambda i=0: K.gemm_int4_tc(pk, x, out, epi=L.TC_EPI_STORE_F32, t_tile=tt, m_halves=mh, cta_pair=bool(pair))
+            epi = L.TC_EPI_RESID_F32 if ks > 1 else L.TC_EPI_STORE_F32
+            run = lambda i=0: K.gemm_int4_tc(pk, x, out, epi=epi, t_tile=tt, m_halves=mh, k_splits=ks)
             if timed:
-                _report(f"gemm_int4 K={Kd} N={N} T={T} t_tile={tt} outputs/CTA={128 * mh}{' CTA pairs' if pair else ''}",
+                _report(f"gemm_int4 K={Kd} N={N} T={T} t_tile={tt} outputs/CTA={128 * mh} splits={ks}",
                         time_launches(run, 1, 6), bytes_=pk.nbytes(), flops=2.0 * T * Kd * N)
             else:
                 _profiled(run, 1)

@@ -91,8 +91,8 @@ def test_gemm_int4_tc_256_output_tiles(K, N, T, g, ks):
 
 @pytest.mark.parametrize("K,N,T,tt", [(1024, 512, 512, 256), (2176, 768, 256, 256), (5120, 1024, 768, 256),
                                       (1024, 512, 512, 512), (5120, 1280, 1024, 512)])
-def test_gemm_int4_tc_cta_pairs(K, N, T, tt):
-    """Adjacent output tiles as CTA pairs: cta_group::2 MMAs, each CTA loading its half of the token operand."""
+def test_gemm_int4_tc_wide_token_tiles(K, N, T, tt):
+    """The widest tiles of tokens, also where more are asked for than a CTA takes.  (CTA pairs are the dense kernel's alone.)"""
     from mi50grad_b200.ops import kernels as Kn
     from mi50grad_b200.ops import lib as L
     from mi50grad_b200.ops.packing import pack_int4
@@ -105,10 +105,12 @@ def test_gemm_int4_tc_cta_pairs(K, N, T, tt):
     ref = x.float() @ lin.dense().t()
     pk = pack_int4(lin, dev)
     out32 = torch.zeros(T, N, dtype=torch.float32, device=dev)
-    Kn.gemm_int4_tc(pk, x.to(dev), out32, epi=L.TC_EPI_STORE_F32, t_tile=tt, cta_pair=True)
+    Kn.gemm_int4_tc(pk, x.to(dev), out32, epi=L.TC_EPI_STORE_F32, t_tile=tt)
     torch.cuda.synchronize()
     Kn.gemm_tc_check_status()
     assert _rel(out32.cpu(), ref) < 2e-3
+    with pytest.raises(TypeError):
+        Kn.gemm_int4_tc(pk, x.to(dev), out32, epi=L.TC_EPI_STORE_F32, t_tile=tt, cta_pair=True)
 
 
 def test_gemm_int4_tc_silu_pair_256_output_tiles():
