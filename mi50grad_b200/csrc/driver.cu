@@ -758,8 +758,9 @@ static int mixer_gemm(Driver* d, const LinearDesc& L, const void* x, int ldx, in
     // Token tile, outputs per CTA and K splits from a fit to measured times (us): a 64-k block of a [128 x t] tile costs
     // about 0.22 + t / 1000, of a [256 x t] tile (both halves share the activation tile, so a product of the same size
     // moves two thirds of the bytes out of L2, which is what bounds the narrow form) 0.20 + 2.6 t / 1000; a tile about
-    // 6 + t / 33, or 8, outside its k loop, a further plane 0.7 in its consumer.  1000 rows: 5120 -> 18512 204 -> 157 us
-    // (1206 TFLOP/s), 17408 -> 5120 245 -> 144 us.
+    // 6 + t / 33, or 8, outside its k loop, a further plane 0.7 in its consumer.  (Fitted to an epilogue that stored two bytes a lane; the
+    // present one is shorter, so what lies outside the k loop is counted too high.)  1000 rows, by that fit against the one before:
+    // 5120 -> 18512 204 -> 157 us (1206 TFLOP/s), 17408 -> 5120 245 -> 144 us.
     const int KB = (L.K + 63) / 64, Tr = (T + 15) & ~15;
     int best_t = 64, best_ks = 1, best_w = 1;
     double best = 1e30;

@@ -2,10 +2,11 @@
 //
 // An fp32 number is the sum of three bf16 numbers (8 + 8 + 8 bits): w = w0 + w1 + w2, x = x0 + x1 + x2.  Of the nine products
 // the six that are not below the last bit are formed by tcgen05.mma kind::f16, which multiplies bf16 exactly:
-// w0 x0 + (w0 x1 + w1 x0) + (w0 x2 + w1 x1 + w2 x0), the smallest first.  (bf16 has the exponents of fp32, so the third term of a
-// number below 2^-110 would lie among its subnormals or below them: both operands are split times 2^24, which loses nothing
-// and costs 1 % of the time (weights that need all 24 bits 3 %).  Numbers above 2^103 and sums above 2^79 become infinite by that and are formed again, see below.)  Where the 128 x 64 weights of a block are bf16 numbers
+// w0 x0 + (w0 x1 + w1 x0) + (w0 x2 + w1 x1 + w2 x0), the smallest first.  Where the 128 x 64 weights of a block are bf16 numbers
 // (a bf16 checkpoint run in 32 bits), w1 and w2 are zero, and their three products are left out.
+// bf16 has the exponents of fp32, so the third term of a number below 2^-110 would lie among its subnormals or below them: both
+// operands are split times 2^24, which loses nothing and costs 1 % of the time (weights that need all 24 bits 3 %).  Numbers above
+// 2^103 and sums above 2^79 become infinite by that and are formed again, see below.
 // The tensor core cuts its sums off where fp32 additions round, so it never sums more than one block of 64 k: every block starts
 // from zero in tensor memory, and the warps add the blocks' sums in registers.  Error against 64 bits (2-norms, 200 rows,
 // K = 2048 / 6144): 1.3e-7 / 1.95e-7; two chains of fp32 FMAs, as before: 5.7e-7 / 9.9e-7.
@@ -15,7 +16,8 @@
 // (tcgen05.st 16x128b; a lane takes 16 bytes of a row, so the k of a 16-group are permuted, in both operands alike), split 16
 // activations a lane into shared memory (B operand, 128-byte swizzle), then take in the block before.  Two stages here too: one
 // is multiplied while the other is split.
-// Bound: the splitting (about 250 instructions a warp and block); the tensor pipe is busy less than half of the time.  200 rows,
+// Bound: the splitting (about 280 instructions a warp and block: 63 % of the issue slots at 200 rows, 2048 -> 8736, beside loads from
+// shared memory; the tensor pipe is busy 42 % of the time).  200 rows,
 // 2048 -> 8736: 46 us (53 with weights that need all 24 bits), FMAs 245; 128 rows, 8192 -> 18944: 172 (232), FMAs 1132 us.
 // A result that is not finite is formed again by fp32 FMAs (ft_again): infinities and numbers that no bf16 reaches come out as they do there.
 // Every mbarrier wait is bounded; on expiry a CTA records a status and forms its outputs by fp32 FMAs.

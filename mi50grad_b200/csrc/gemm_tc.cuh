@@ -15,7 +15,7 @@ struct GemmTcParams {
     const uint2* szfrag;     // [NTL/4][G][4][8]
     int K, KB, NTL, G, off32, gshift;
     int T;                   // token rows in this launch's activation matrix
-    int t_tile;              // tokens per CTA (multiple of 16, <= 512)
+    int t_tile;              // tokens per CTA (multiple of 16, <= 512; INT4 weights take 256 of more, of 256 outputs 192)
     int n_valid, ldo, epi, stages;
     void* out;
     int* status;             // [0] set to 1 when a bounded wait expired

