@@ -16,9 +16,9 @@
 // (tcgen05.st 16x128b; a lane takes 16 bytes of a row, so the k of a 16-group are permuted, in both operands alike), split 16
 // activations a lane into shared memory (B operand, 128-byte swizzle), then take in the block before.  Two stages here too: one
 // is multiplied while the other is split.
-// Bound: the splitting (about 280 instructions a warp and block: 63 % of the issue slots at 200 rows, 2048 -> 8736, beside loads from
-// shared memory; the tensor pipe is busy 42 % of the time).  200 rows,
-// 2048 -> 8736: 46 us (53 with weights that need all 24 bits), FMAs 245; 128 rows, 8192 -> 18944: 172 (232), FMAs 1132 us.
+// Bound: the splitting and what surrounds it, 490 instructions a warp and block with weights of 24 bits (63 % of the issue slots
+// at 200 rows, 2048 -> 8736; tensor pipe 42 % of the time).  That shape takes 46 us (53 with weights that need all 24 bits), FMAs 245;
+// 128 rows, 8192 -> 18944: 172 (232), FMAs 1132 us.
 // A result that is not finite is formed again by fp32 FMAs (ft_again): infinities and numbers that no bf16 reaches come out as they do there.
 // Every mbarrier wait is bounded; on expiry a CTA records a status and forms its outputs by fp32 FMAs.
 #include <cuda.h>
