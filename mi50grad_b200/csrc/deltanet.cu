@@ -1086,14 +1086,14 @@ __device__ __forceinline__ void ldsm4_ht(uint32_t (&r)[4], const __half* row_ptr
 __device__ __forceinline__ float2 h2f(uint32_t x) { return __half22float2(*(const __half2*)&x); }
 
 // Everything of a chunk that does not depend on the state: the gates, A = beta decay (K K^T) below the diagonal,
-// W = decay (Q K^T) on and below it, T = (I + A)^-1 (forward substitution on the 32 x 32 unit triangle, one column per
-// lane), the convolved values V, and with them U0 and Wt.  T enters its products as hi + lo TF32 parts (and V too; K is
+// W = decay (Q K^T) on and below it, T = (I + A)^-1 (forward substitution on the two 16 x 16 diagonal triangles, one column per
+// lane, and two products for the block below them), the convolved values V, and with them U0 and Wt.  T enters its products as hi + lo TF32 parts (and V too; K is
 // fp16), so they keep fp32 accuracy.  grid = (chunks, value heads), 256 threads.
 template <int DK, int DV>
 __global__ void __launch_bounds__(DN_THREADS) deltanet_tw_prep_kernel(const DeltaParams p, const __half* __restrict__ ab, int ld_ab,
                                                                       const __half* __restrict__ qk_pre, int ld_qk,
                                                                       float* __restrict__ tw, int n_chunks) {
-    static_assert(DC_C == 32, "one lane per column of the triangle");
+    static_assert(DC_C == 32, "a warp has the chunk's rows, half of one a column of a triangle each");
     constexpr int LDK = DC_LDK(DK), LDV = DV + 8;
     constexpr int MB = DC_C / 16;
     extern __shared__ __align__(16) float psm[];
