@@ -302,9 +302,10 @@ __global__ void __launch_bounds__(DG_THREADS, 2) gemv_fma_kernel(const DenseGemv
         // ---- stage the input of this K chunk.  All its loads are on their way at once, those of the residual stream also while
         // the inverses are formed: a loop of load and store took a trip to L2 for each of up to six pieces, in every CTA
         // (one row: 12288 -> 4096 19.8 -> 18.7 us, 17408 -> 5120 43.7 -> 40.9; a step of decode at width 4096 1.126 -> 1.099 ms)
-        if (MR == 1 && p.x && (p.ldx & 7) == 0 && cl <= 2 * DG_THREADS * V) {
-            // (two pieces a thread at most: through registers, which is the shorter way: one row of 2048 -> 2048 4.42 us by cp.async,
-            // 4.07 so; 2048 -> 12288 13.7 and 13.1, 4096 -> 12288 22.7 and 21.8)
+        if (sizeof(T) == 2 && MR == 1 && p.x && (p.ldx & 7) == 0 && cl <= 2 * DG_THREADS * V) {
+            // (two pieces a thread at most: through registers, which is the shorter way: one bf16 row of 2048 -> 2048 4.42 us by cp.async,
+            // 4.07 so; 2048 -> 12288 13.7 and 13.1, 4096 -> 12288 22.7 and 21.8.  In fp32, where the kernel has no registers to spare, 2048 ->
+            // 8736 14.3 and 14.7)
             uint4 v[2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
